@@ -16,7 +16,13 @@ extern "C" {
 #define BF_MAX_PEERS 8
 #define BF_FLAG_CHANNELS 64      // barrier channels per flag page (uint32[BF_FLAG_CHANNELS][BF_MAX_PEERS])
 
-#define BF_HUB_DEGREE 1024   // rows longer than this use the chunked hub kernels
+// Edge attention: query rows with more than BF_LONG_ROW edges are cut into work items of BF_LONG_CHUNK edges.  A row below
+// the line is one lane group's serial walk, two gathers at a time: 64 rounds of roughly 0.7 us at 128 edges, about what an
+// item, its scratch and the two reduction launches cost.
+#define BF_LONG_ROW 128
+#define BF_LONG_CHUNK 64
+// allocation-free forward entry point (bf_noalloc.h): its callers list the rows with more than BF_HUB_DEGREE edges
+#define BF_HUB_DEGREE 1024
 #define BF_HUB_CHUNK 8192    // edges per hub chunk (one thread block)
 
 // ---- edge attention (edge_attn.cu) ----------------------------------------------------------
@@ -56,6 +62,17 @@ typedef struct {
   long long slab_row0;              // this (source) rank's slab: source index * rows_per
 } bf_attn_route;
 
+// Query rows with more than min_degree edges, as work items: item i is slot i of the scratch and the items of a row are
+// adjacent.  n_task == 0: none (rows of any length are walked by the regular kernels).
+typedef struct {
+  const int* task;                  // [n_task, 4] int32, 16-byte aligned: row, first edge, end edge, slot
+  int n_task;
+  const int* split;                 // [n_split, 3] int32: row, first slot, slot count
+  int n_split;
+  float* partial;                   // [n_task, pitch] fp32 scratch, 16-byte aligned
+  int min_degree;
+} bf_long_rows;
+
 typedef struct {
   const void* dout;                 // [n, hl, hn] contiguous
   void *dq, *dk, *dv;               // [n, hl, hn], common row stride ldg (elements; 0 = hl*hn)
@@ -63,16 +80,13 @@ typedef struct {
   float* zd;                        // [n, hl, 2] fp32 workspace (written by the dQ pass)
   const int *t_rowptr, *t_row, *t_eid;  // transposed CSR over keys
   float* detab;                     // zero-filled [2, hl, hn] fp32 or NULL
-  const int* t_hub_rows;
-  int n_t_hub, max_t_hub_degree;
-  float* hub_scratch_q;             // zero-filled [n_hub, hl*hn]
-  float* hub_scratch_kv;            // zero-filled [n_t_hub, 2*hl*hn]
-  // Optional balanced dK/dV work list (replaces the t_hub_* path when kv_task != NULL)
+  bf_long_rows long_rows;           // scratch row: hl*hn floats
+  // balanced dK/dV work list; the n_kv_slots items of split keys come first, in slot order
   const int* kv_task;               // [n_kv_task, 4] int32, 16-byte aligned: key row, first edge, end edge, slot (-1 direct)
   int n_kv_task;
   const int* kv_split;              // [n_kv_split, 3] int32: key row, first slot, slot count
-  int n_kv_split;
-  float* kv_partial;                // [total slots, 2*hl*hn] fp32 scratch
+  int n_kv_split, n_kv_slots;
+  float* kv_partial;                // [n_kv_slots, 2*hl*hn] fp32 scratch
   // Optional workspace for narrow rows (hl*hn elements of 64 bytes or less), used with kv_task: the dQ pass leaves one
   // contiguous record [q | dout / (Z + eps)] per (row, head) in qg and D / (Z + eps) in cz, and the dK/dV pass gathers
   // those instead of q, dout and zd separately.
@@ -85,8 +99,10 @@ typedef struct {
 } bf_attn_bwd_params;
 
 int bf_edge_attn_fwd(const bf_attn_params* p, cudaStream_t st);
-// as above; additionally every output row is stored into its owner's buffer (route may be NULL)
-int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_route* route, cudaStream_t st);
+// as above; additionally every output row is stored into its owner's buffer (route may be NULL), and long rows come as
+// work items (long_rows may be NULL; its scratch has bf_attn_fwd_long_pitch floats per item)
+int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_route* route, const bf_long_rows* long_rows, cudaStream_t st);
+size_t bf_attn_fwd_long_pitch(int hl, int hn);
 int bf_edge_attn_bwd(const bf_attn_params* p, const bf_attn_bwd_params* q, cudaStream_t st);
 
 // ---- attention-graph construction (edge_build.cu) -------------------------------------------
@@ -250,10 +266,13 @@ size_t bf_graph_transpose_scratch(int n, long long n_edges);
 int bf_graph_transpose(const int* rowptr, const int* col, int n, long long n_edges, int* t_rowptr /* [n+1] */,
                        int* t_row /* [E] */, int* t_eid /* [E] */, void* scratch, size_t scratch_bytes, cudaStream_t st);
 size_t bf_kv_task_scratch(int n);
-int bf_kv_task_counts(const int* t_rowptr, int n, int chunk, int* item_first /* [n+1] */, int* slot_first /* [n+1] */,
-                      int* split_first /* [n+1] */, void* scratch, size_t scratch_bytes, cudaStream_t st);
+// rows with more than min_split (>= chunk) edges become several items of `chunk` edges
+int bf_kv_task_counts(const int* t_rowptr, int n, int chunk, int min_split, int* item_first /* [n+1] */,
+                      int* slot_first /* [n+1] */, int* split_first /* [n+1] */, void* scratch, size_t scratch_bytes,
+                      cudaStream_t st);
+// singles == 0: only the items of split rows are written ([slots, 4])
 int bf_kv_task_fill(const int* t_rowptr, const int* item_first, const int* slot_first, const int* split_first, int n,
-                    int chunk, int* tasks /* [T, 4] */, int* splits /* [S, 3] */, cudaStream_t st);
+                    int chunk, int singles, int* tasks /* [T, 4] */, int* splits /* [S, 3] */, cudaStream_t st);
 
 // ---- row kernels (norm_fused.cu) -----------------------------------------------------------------
 int bf_layernorm_fwd(const void* x, long long ldx, const float* gamma, const float* beta, void* y, long long ldy,

@@ -38,24 +38,67 @@ void check_qkv(const Tensor& t, const char* name) {
 
 const int* iptr(const Tensor& t) { return t.data_ptr<int>(); }
 
-struct HubInfo {
-  Tensor rows;
-  int n = 0;
-  int max_deg = 0;
+// Work items of the CSR rows with more than min_split edges: items of `chunk` edges, split rows, and with `singles` one item
+// for every other row behind them.  The totals size the outputs: one host read.
+struct RowTasks {
+  Tensor tasks, splits, sizes;       // [T, 4], [S, 3], int64 [3] on the host = items, slots, split rows
 };
-
-// Rows of a CSR longer than BF_HUB_DEGREE.  `known_max` >= 0 skips the device query.
-HubInfo find_hubs(const Tensor& rowptr, int64_t known_max) {
-  HubInfo h;
-  if (known_max >= 0 && known_max <= BF_HUB_DEGREE) return h;
-  auto deg = rowptr.slice(0, 1) - rowptr.slice(0, 0, rowptr.size(0) - 1);
-  auto rows = torch::nonzero(deg > BF_HUB_DEGREE).flatten().to(torch::kInt);
-  h.n = (int)rows.size(0);
-  if (h.n > 0) {
-    h.rows = rows;
-    h.max_deg = deg.max().item<int>();
+RowTasks row_tasks(const Tensor& rowptr, int64_t n, int64_t chunk, int64_t min_split, bool singles, cudaStream_t st) {
+  auto iopt = rowptr.options();
+  Tensor firsts = torch::empty({3, n + 1}, iopt);
+  {
+    const size_t bytes = bf_kv_task_scratch((int)n);
+    Tensor scratch = torch::empty({(int64_t)bytes}, iopt.dtype(torch::kUInt8));
+    check_cuda(bf_kv_task_counts(rowptr.data_ptr<int>(), (int)n, (int)chunk, (int)min_split, firsts[0].data_ptr<int>(),
+                                 firsts[1].data_ptr<int>(), firsts[2].data_ptr<int>(), scratch.data_ptr(), bytes, st),
+               "kv_task_counts");
   }
-  return h;
+  RowTasks r;
+  r.sizes = firsts.select(1, n).to(torch::kCPU).to(torch::kLong);
+  const int64_t n_items = r.sizes[singles ? 0 : 1].item<int64_t>(), n_splits = r.sizes[2].item<int64_t>();
+  r.tasks = torch::empty({n_items, 4}, iopt);
+  r.splits = torch::empty({n_splits, 3}, iopt);
+  if (n_items > 0)
+    check_cuda(bf_kv_task_fill(rowptr.data_ptr<int>(), firsts[0].data_ptr<int>(), firsts[1].data_ptr<int>(),
+                               firsts[2].data_ptr<int>(), (int)n, (int)chunk, singles ? 1 : 0, r.tasks.data_ptr<int>(),
+                               r.splits.data_ptr<int>(), st), "kv_task_fill");
+  return r;
+}
+
+// (tasks, splits) of the query rows with more than BF_LONG_ROW edges (empty tensors: none)
+std::vector<Tensor> long_row_tasks(Tensor rowptr) {
+  TORCH_CHECK(rowptr.is_cuda() && rowptr.scalar_type() == torch::kInt && rowptr.is_contiguous() && rowptr.numel() >= 1);
+  c10::cuda::CUDAGuard guard(rowptr.device());
+  if (rowptr.numel() == 1) return {torch::empty({0, 4}, rowptr.options()), torch::empty({0, 3}, rowptr.options())};
+  RowTasks r = row_tasks(rowptr, rowptr.numel() - 1, BF_LONG_CHUNK, BF_LONG_ROW, false, at::cuda::getCurrentCUDAStream());
+  return {r.tasks, r.splits};
+}
+
+// The long rows of a call: the caller's list, or a list made here.  A known bound on the row length of at most BF_LONG_ROW
+// means that there are none.
+struct LongRows {
+  Tensor tasks, splits, partial;
+  bf_long_rows c{};
+};
+LongRows take_long_rows(const Tensor& rowptr, int64_t known_max, const OptTensor& tasks, const OptTensor& splits, size_t pitch) {
+  LongRows r;
+  if (known_max >= 0 && known_max <= BF_LONG_ROW) return r;
+  if (tasks.has_value() && splits.has_value()) {
+    r.tasks = *tasks; r.splits = *splits;
+    TORCH_CHECK(r.tasks.is_cuda() && r.tasks.scalar_type() == torch::kInt && r.tasks.is_contiguous() && r.tasks.dim() == 2 &&
+                r.tasks.size(1) == 4 && ((uintptr_t)r.tasks.data_ptr()) % 16 == 0, "long rows: tasks int32 [T, 4]");
+    TORCH_CHECK(r.splits.is_cuda() && r.splits.scalar_type() == torch::kInt && r.splits.is_contiguous() && r.splits.dim() == 2 &&
+                r.splits.size(1) == 3, "long rows: splits int32 [S, 3]");
+  } else {
+    auto v = long_row_tasks(rowptr);
+    r.tasks = v[0]; r.splits = v[1];
+  }
+  if (r.tasks.size(0) == 0) return r;
+  r.partial = torch::empty({r.tasks.size(0), (int64_t)pitch}, rowptr.options().dtype(torch::kFloat));
+  r.c.task = r.tasks.data_ptr<int>(); r.c.n_task = (int)r.tasks.size(0);
+  r.c.split = r.splits.data_ptr<int>(); r.c.n_split = (int)r.splits.size(0);
+  r.c.partial = r.partial.data_ptr<float>(); r.c.min_degree = BF_LONG_ROW;
+  return r;
 }
 
 // out_drop = {p, seed, rows per owning rank, column offset} or empty: dropout fused into the attention output
@@ -97,26 +140,20 @@ bf_attn_route parse_route(const std::vector<int64_t>& route, size_t header) {
 
 void edge_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor rowptr, Tensor col, OptTensor etype,
                    OptTensor etab, int64_t variant, double dropout_p, int64_t seed, int64_t known_max_degree,
-                   std::vector<double> out_drop, std::vector<int64_t> route) {
+                   std::vector<double> out_drop, std::vector<int64_t> route, OptTensor long_task, OptTensor long_split) {
   c10::cuda::CUDAGuard guard(q.device());
   bf_attn_params p{};
   fill_common(p, q, k, v, out, z, rowptr, col, etype, etab, variant, dropout_p, seed, out_drop);
-  HubInfo hub = find_hubs(rowptr, known_max_degree);
-  Tensor scratch;
-  if (hub.n > 0) {
-    scratch = torch::zeros({hub.n, (int64_t)p.hl * p.hn + p.hl}, q.options().dtype(torch::kFloat));
-    p.hub_rows = iptr(hub.rows); p.n_hub = hub.n; p.max_hub_degree = hub.max_deg;
-    p.hub_scratch = scratch.data_ptr<float>();
-  }
+  LongRows lr = take_long_rows(rowptr, known_max_degree, long_task, long_split, bf_attn_fwd_long_pitch(p.hl, p.hn));
   const bf_attn_route r = parse_route(route, 3);
-  check_cuda(bf_edge_attn_fwd_routed(&p, &r, at::cuda::getCurrentCUDAStream()), "edge_attn_fwd");
+  check_cuda(bf_edge_attn_fwd_routed(&p, &r, &lr.c, at::cuda::getCurrentCUDAStream()), "edge_attn_fwd");
 }
 
 void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor dout, Tensor dq, Tensor dk, Tensor dv,
                    Tensor zd, Tensor rowptr, Tensor col, OptTensor etype, Tensor t_rowptr, Tensor t_row, Tensor t_eid,
                    OptTensor etab, OptTensor detab, int64_t variant, double dropout_p, int64_t seed,
                    int64_t known_max_degree, OptTensor kv_task, OptTensor kv_split, int64_t kv_slots,
-                   std::vector<double> out_drop, std::vector<int64_t> route) {
+                   std::vector<double> out_drop, std::vector<int64_t> route, OptTensor long_task, OptTensor long_split) {
   c10::cuda::CUDAGuard guard(q.device());
   bf_attn_params p{};
   fill_common(p, q, k, v, out, z, rowptr, col, etype, etab, variant, dropout_p, seed, out_drop);
@@ -130,36 +167,23 @@ void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor do
   b.zd = zd.data_ptr<float>();
   b.t_rowptr = iptr(t_rowptr); b.t_row = iptr(t_row); b.t_eid = iptr(t_eid);
   b.detab = detab.has_value() ? detab->data_ptr<float>() : nullptr;
-  HubInfo hub = find_hubs(rowptr, known_max_degree);
-  const bool use_tasks = kv_task.has_value() && kv_task->numel() > 0;
-  HubInfo thub = use_tasks ? HubInfo() : find_hubs(t_rowptr, -1);
-  Tensor sq, skv, partial, qg, cz;
-  if (use_tasks && (int64_t)p.hl * p.hn * q.element_size() <= 64) {
+  const int64_t w = (int64_t)p.hl * p.hn;
+  LongRows lr = take_long_rows(rowptr, known_max_degree, long_task, long_split, (size_t)w);
+  b.long_rows = lr.c;
+  Tensor partial, qg, cz;
+  if (w * q.element_size() <= 64) {
     // narrow rows: one packed record per (query, head) for the dK/dV pass (see bf_attn_bwd_params)
     qg = torch::empty({q.size(0), (int64_t)p.hl, 2, (int64_t)p.hn}, q.options());
     cz = torch::empty({q.size(0), (int64_t)p.hl}, q.options().dtype(torch::kFloat));
     b.qg = qg.data_ptr(); b.cz = cz.data_ptr<float>();
   }
-  if (use_tasks) {
-    TORCH_CHECK(kv_task->scalar_type() == torch::kInt && kv_task->is_contiguous() && kv_task->size(1) == 4 &&
-                ((uintptr_t)kv_task->data_ptr()) % 16 == 0, "kv_task must be contiguous int32 [T, 4]");
-    b.kv_task = kv_task->data_ptr<int>(); b.n_kv_task = (int)kv_task->size(0);
-    if (kv_split.has_value() && kv_split->numel() > 0 && kv_slots > 0) {
-      b.kv_split = kv_split->data_ptr<int>(); b.n_kv_split = (int)kv_split->size(0);
-      partial = torch::empty({kv_slots, 2 * (int64_t)p.hl * p.hn}, q.options().dtype(torch::kFloat));
-      b.kv_partial = partial.data_ptr<float>();
-    }
-  }
-  const int64_t w = (int64_t)p.hl * p.hn;
-  if (hub.n > 0) {
-    sq = torch::zeros({hub.n, w}, q.options().dtype(torch::kFloat));
-    p.hub_rows = iptr(hub.rows); p.n_hub = hub.n; p.max_hub_degree = hub.max_deg;
-    b.hub_scratch_q = sq.data_ptr<float>();
-  }
-  if (thub.n > 0) {
-    skv = torch::zeros({thub.n, 2 * w}, q.options().dtype(torch::kFloat));
-    b.t_hub_rows = iptr(thub.rows); b.n_t_hub = thub.n; b.max_t_hub_degree = thub.max_deg;
-    b.hub_scratch_kv = skv.data_ptr<float>();
+  TORCH_CHECK(kv_task.has_value() && kv_task->scalar_type() == torch::kInt && kv_task->is_contiguous() && kv_task->size(1) == 4 &&
+              ((uintptr_t)kv_task->data_ptr()) % 16 == 0, "kv_task must be contiguous int32 [T, 4]");
+  b.kv_task = kv_task->data_ptr<int>(); b.n_kv_task = (int)kv_task->size(0);
+  if (kv_split.has_value() && kv_split->numel() > 0 && kv_slots > 0) {
+    b.kv_split = kv_split->data_ptr<int>(); b.n_kv_split = (int)kv_split->size(0); b.n_kv_slots = (int)kv_slots;
+    partial = torch::empty({kv_slots, 2 * w}, q.options().dtype(torch::kFloat));
+    b.kv_partial = partial.data_ptr<float>();
   }
   if (!route.empty()) {
     // {rows per destination, slab row, row stride, column of dq, of dk, of dv, destination pointers...}
@@ -382,23 +406,8 @@ std::vector<Tensor> graph_transpose(Tensor rowptr, Tensor col, int64_t n, int64_
                                   t_row.data_ptr<int>(), t_eid.data_ptr<int>(), scratch.data_ptr(), bytes, st),
                "graph_transpose");
   }
-  Tensor firsts = torch::empty({3, n + 1}, iopt);
-  {
-    const size_t bytes = bf_kv_task_scratch((int)n);
-    Tensor scratch = torch::empty({(int64_t)bytes}, iopt.dtype(torch::kUInt8));
-    check_cuda(bf_kv_task_counts(t_rowptr.data_ptr<int>(), (int)n, (int)chunk, firsts[0].data_ptr<int>(),
-                                 firsts[1].data_ptr<int>(), firsts[2].data_ptr<int>(), scratch.data_ptr(), bytes, st),
-               "kv_task_counts");
-  }
-  // the three totals size the outputs: the one host read of this build
-  Tensor sizes = firsts.select(1, n).to(torch::kCPU).to(torch::kLong);
-  const int64_t n_tasks = sizes[0].item<int64_t>(), n_splits = sizes[2].item<int64_t>();
-  Tensor tasks = torch::empty({n_tasks, 4}, iopt), splits = torch::empty({n_splits, 3}, iopt);
-  check_cuda(bf_kv_task_fill(t_rowptr.data_ptr<int>(), firsts[0].data_ptr<int>(), firsts[1].data_ptr<int>(),
-                             firsts[2].data_ptr<int>(), (int)n, (int)chunk, tasks.data_ptr<int>(),
-                             splits.data_ptr<int>(), st),
-             "kv_task_fill");
-  return {t_rowptr, t_row, t_eid, tasks, splits, sizes};
+  RowTasks r = row_tasks(t_rowptr, n, chunk, chunk, true, st);
+  return {t_rowptr, t_row, t_eid, r.tasks, r.splits, r.sizes};
 }
 
 // C = A * W^T with fused epilogue.  `dst_ptrs` holds one device pointer per destination (1 = plain output).
@@ -768,8 +777,19 @@ bool gemm_supported(int64_t M, int64_t N, int64_t K) { return bf_gemm_supported(
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
-  m.def("edge_attn_fwd", &edge_attn_fwd);
-  m.def("edge_attn_bwd", &edge_attn_bwd);
+  namespace py = pybind11;
+  m.def("edge_attn_fwd", &edge_attn_fwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("out"), py::arg("z"), py::arg("rowptr"),
+        py::arg("col"), py::arg("etype"), py::arg("etab"), py::arg("variant"), py::arg("dropout_p"), py::arg("seed"),
+        py::arg("known_max_degree"), py::arg("out_drop"), py::arg("route"), py::arg("long_task") = py::none(),
+        py::arg("long_split") = py::none());
+  m.def("edge_attn_bwd", &edge_attn_bwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("out"), py::arg("z"), py::arg("dout"),
+        py::arg("dq"), py::arg("dk"), py::arg("dv"), py::arg("zd"), py::arg("rowptr"), py::arg("col"), py::arg("etype"),
+        py::arg("t_rowptr"), py::arg("t_row"), py::arg("t_eid"), py::arg("etab"), py::arg("detab"), py::arg("variant"),
+        py::arg("dropout_p"), py::arg("seed"), py::arg("known_max_degree"), py::arg("kv_task"), py::arg("kv_split"),
+        py::arg("kv_slots"), py::arg("out_drop"), py::arg("route"), py::arg("long_task") = py::none(),
+        py::arg("long_split") = py::none());
+  m.def("long_row_tasks", &long_row_tasks);
+  m.attr("LONG_ROW") = (int64_t)BF_LONG_ROW;
   m.attr("BUILD_HUB_DEGREE") = (int64_t)BF_BUILD_HUB_DEGREE;
   m.def("build_attn_graph", &build_attn_graph);
   m.def("budget_select_rows", &budget_select_rows);

@@ -1,9 +1,10 @@
 // Budgeted sparse edge attention for sm_100a: forward, dQ pass (over queries) and dK/dV pass
 // (over the transposed graph).  Gather-only on regular rows: every query owns <= B sampled
 // in-edges, so one lane group streams them with 16-byte loads and keeps the running
-// numerator / normaliser in registers.  Rows longer than BF_HUB_DEGREE (the Graphormer virtual
-// node, popular keys in the transposed graph) are split into chunks whose partial sums meet in
-// an fp32 scratch buffer through atomics and are finalised by a second small kernel.
+// numerator / normaliser in registers.  Rows longer than BF_LONG_ROW (the Graphormer virtual node,
+// hubs of a graph without a budget, popular keys in the transposed graph) are cut into work items of
+// BF_LONG_CHUNK edges, one warp each, whose fp32 partial sums are added in a fixed order by two small
+// kernels: no atomics, bit-reproducible.
 //
 // Math (reference: models/graphormer_dist_node_level.py:231-263, models/gt_dist_node_level.py:
 // 224-262, models/graphgps_dist_node_level.py:151-177, models/exphormer_dist_node_level.py:92-121):
@@ -168,10 +169,17 @@ struct AttnArgs {
   int variant;                 // 0 plain, 1 gps, 2 exphormer
   float inv_keep;              // 1/(1-p)
   uint32_t thresh, seed;
-  // hub path
+  int long_row;                // rows with more edges are left to the long-row kernels (0: every row is walked here)
+  // long rows as work items (see bf_long_rows)
+  const int4* long_task;       // [n_long_task]: row, first edge, end edge, slot
+  int n_long_task;
+  const int* long_split;       // [n_long_split, 3]: row, first slot, slot count
+  int n_long_split;
+  float* long_partial;         // [n_long_task, forward: fwd_pitch(Hl*HN, Hl); backward: Hl*HN]
+  // long rows of the allocation-free entry point: fixed scratch, atomics
   const int* hub_rows;         // [n_hub]
   int n_hub, hub_chunk;
-  float* hub_scratch;          // forward: [n_hub, Hl*HN + Hl]
+  float* hub_scratch;          // [n_hub, Hl*HN + Hl]
   // fused dropout on the stored output (out_thresh == 0: off)
   uint32_t out_thresh, out_seed;
   float out_inv_keep, out_keep;
@@ -260,8 +268,8 @@ __global__ void __launch_bounds__(256) edge_attn_fwd_kernel(AttnArgs a) {
   const int off = hsafe * HN + (lt % LPH) * VN;
   int beg = 0, end = 0;
   if (head_ok) { beg = a.rowptr[row]; end = a.rowptr[row + 1]; }
-  // long rows go to the hub kernels when the caller listed them; without a list they are walked here (slow, complete)
-  const bool hub = a.n_hub > 0 && (end - beg) > BF_HUB_DEGREE;
+  // long rows have kernels of their own when the caller listed them; without a list they are walked here (slow, complete)
+  const bool hub = a.long_row > 0 && (end - beg) > a.long_row;
   if (hub) end = beg;
   float qs0[VN], qs1[VN], acc[VN];
   float zsum = 0.f;
@@ -286,7 +294,57 @@ __global__ void __launch_bounds__(256) edge_attn_fwd_kernel(AttnArgs a) {
   }
 }
 
-// Hub rows: grid = (n_hub * chunks_per_hub) blocks; each warp strides over its block's chunk.
+// Long rows.  One warp per (work item, head chunk): the 32 / TL lane groups take consecutive quarters (halves, ...) of the
+// item's edges and meet in shuffles; the item's numerator and normaliser go to its slot of the scratch.  An item is
+// BF_LONG_CHUNK = 64 edges, so a virtual node over 169 k nodes is 2,646 warps side by side (18 per SM, each 16 dependent
+// gathers deep) instead of the 21 blocks of 8,192 edges it used to be: 25 us against 340 us (8 heads x 16, bf16), the dQ
+// pass 24 against 421 us, and a 720 k-edge power-law graph without a budget (4 heads x 64, fp32) 31 against 781 us.
+__host__ __device__ inline int fwd_pitch(int w, int hl) { return w + ((hl + 3) & ~3); }
+
+// lanes of the first lane group receive the sum over the warp's lane groups (tl a power of two)
+__device__ __forceinline__ float group_total(float x, int tl) {
+  for (int o = tl; o < 32; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+template <typename T, int HN>
+__global__ void __launch_bounds__(256) edge_attn_fwd_long_kernel(AttnArgs a) {
+  constexpr int VN = Vec<T>::N;
+  constexpr int LPH = HN / VN;
+  const Geo g = make_geo<T, HN>(a.hl);
+  const int lane = threadIdx.x & 31;
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (warp >= (long long)a.n_long_task * g.n_hc) return;
+  const int tpw = 32 / g.tl, sub = lane / g.tl, lt = lane % g.tl;
+  const int item = (int)(warp / g.n_hc), hc = (int)(warp % g.n_hc);
+  const int head = hc * g.hpt + lt / LPH;
+  const bool head_ok = head < a.hl;
+  const int hsafe = head_ok ? head : 0;
+  const int off = hsafe * HN + (lt % LPH) * VN;
+  const int4 it = __ldg(a.long_task + item);
+  const int per = (it.z - it.y + tpw - 1) / tpw;
+  const int beg = it.y + sub * per, end = min(it.z, beg + per);
+  float qs0[VN], qs1[VN], acc[VN];
+  float zsum = 0.f;
+#pragma unroll
+  for (int i = 0; i < VN; ++i) acc[i] = 0.f;
+  load_q_scaled<T, HN>(a, it.x, hsafe, off, qs0, qs1);
+  const unsigned hm = head_mask<LPH>();
+  for (int e = beg; e < end; e += 2) fwd_pair<T, HN>(a, hsafe, off, e, e + 1, e + 1 < end, hm, qs0, qs1, acc, zsum);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < VN; ++i) acc[i] = group_total(acc[i], g.tl);
+  zsum = group_total(zsum, g.tl);
+  if (sub == 0 && head_ok) {
+    const int w = a.hl * HN;
+    float* pp = a.long_partial + (long long)it.w * fwd_pitch(w, a.hl);
+#pragma unroll
+    for (int i = 0; i < VN; i += 4) *reinterpret_cast<float4*>(pp + off + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+    if ((lt % LPH) == 0) pp[w + head] = zsum;
+  }
+}
+
+// Hub rows of the allocation-free entry point: grid = (n_hub * chunks_per_hub) blocks; each warp strides over its block's chunk.
 template <typename T, int HN>
 __global__ void __launch_bounds__(256) edge_attn_fwd_hub_kernel(AttnArgs a, int chunks_per_hub) {
   constexpr int VN = Vec<T>::N;
@@ -360,16 +418,12 @@ struct BwdArgs {
   float2* zd;                  // [n, Hl]: (1/(Z+eps), D = <dout,out>)
   const int *t_rowptr, *t_row, *t_eid;
   float* detab;                // [T, Hl, HN] fp32 or null
-  const int* t_hub_rows;
-  int n_t_hub;
-  float* hub_scratch_q;        // [n_hub, Hl*HN]
-  float* hub_scratch_kv;       // [n_t_hub, 2*Hl*HN]
   // balanced dK/dV work list
   const int4* kv_task;         // [n_kv_task]: key row, first edge, end edge, partial slot (-1 = direct store)
   int n_kv_task;
   const int* kv_split;         // [n_kv_split, 3]: key row, first slot, number of slots
-  int n_kv_split;
-  float* kv_partial;           // [slots, 2*Hl*HN] fp32
+  int n_kv_split, n_kv_slots;
+  float* kv_partial;           // [n_kv_slots, 2*Hl*HN] fp32
   // Packed query records for narrow rows (optional): the dQ pass writes, per (row, head), [q | dout / (Z + eps)] next to
   // each other plus one float D / (Z + eps); the dK/dV pass then gathers one contiguous record per edge instead of
   // three separate short rows (q, dout, (1/Z, D)), which matters when a row of q is only 32 or 64 bytes.
@@ -386,46 +440,6 @@ template <typename T>
 __device__ __forceinline__ T* grad_row(const BwdArgs& b, void* local, int col0, long long row) {
   if (b.route.n_dest == 0) return static_cast<T*>(local) + row * b.ldg;
   return routed<T>(b.route, row, col0);
-}
-
-// One edge of the dQ pass for one task lane.
-template <typename T, int HN>
-__device__ __forceinline__ void dq_edge(const BwdArgs& b, int e, int head, int off, const float* qs0, const float* qs1,
-                                        const float* qraw, const float* dof, float invz, float dterm, float* dq,
-                                        float* de0, float* de1, unsigned hm) {
-  constexpr int VN = Vec<T>::N;
-  constexpr int LPH = HN / VN;
-  const AttnArgs& a = b.f;
-  const float scale = inv_sqrt_hn<HN>();
-  const int j = __ldg(a.col + e);
-  float kf[VN], vf[VN];
-  load_vec<T>(static_cast<const T*>(a.k) + (long long)j * a.ldk + off, kf);
-  load_vec<T>(static_cast<const T*>(a.v) + (long long)j * a.ldv + off, vf);
-  const int t = (a.variant == 2) ? a.etype[e] : 0;
-  float d = 0.f, dv = 0.f;
-#pragma unroll
-  for (int i = 0; i < VN; ++i) { d += (t ? qs1[i] : qs0[i]) * kf[i]; dv += dof[i] * vf[i]; }
-  d = head_sum<LPH>(d, hm);
-  dv = head_sum<LPH>(dv, hm);
-  const bool inr = (d > -kClamp) && (d < kClamp);
-  const float w = __expf(fminf(fmaxf(d, -kClamp), kClamp));
-  float mf = 1.f;
-  if (a.variant == 1 && a.thresh) mf = keep_edge(a.seed, (uint32_t)e, (uint32_t)head, a.thresh) ? a.inv_keep : 0.f;
-  else if (a.variant == 1) mf = a.inv_keep;
-  const float ds = inr ? (dv * mf - dterm) * invz * w : 0.f;
-  if (a.variant == 2) {
-    const float* et = a.etab + (t ? a.hl * HN : 0) + off;
-#pragma unroll
-    for (int i = 0; i < VN; ++i) {
-      dq[i] += ds * scale * kf[i] * et[i];
-      const float g = ds * scale * qraw[i] * kf[i];
-      de0[i] += t ? 0.f : g;
-      de1[i] += t ? g : 0.f;
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < VN; ++i) dq[i] += ds * scale * kf[i];
-  }
 }
 
 // Four edges of one query at a time (see dkv_edge4).
@@ -528,7 +542,7 @@ __global__ void __launch_bounds__(256, EXPH ? 3 : 4) edge_attn_bwd_q_kernel(BwdA
   const int off = hsafe * HN + (lt % LPH) * VN;
   int beg = 0, end = 0;
   if (head_ok) { beg = a.rowptr[row]; end = a.rowptr[row + 1]; }
-  const bool hub = a.n_hub > 0 && (end - beg) > BF_HUB_DEGREE;
+  const bool hub = a.long_row > 0 && (end - beg) > a.long_row;
   float qs0[VN], qs1[VN], qraw[VN], dof[VN], of[VN], dq[VN], de0[VN], de1[VN];
   load_q_scaled<T, HN>(a, row, hsafe, off, qs0, qs1);
   load_vec<T>(static_cast<const T*>(a.q) + (long long)row * a.ldq + off, qraw);
@@ -570,100 +584,59 @@ __global__ void __launch_bounds__(256, EXPH ? 3 : 4) edge_attn_bwd_q_kernel(BwdA
   }
 }
 
-template <typename T, int HN>
-__global__ void __launch_bounds__(256) edge_attn_bwd_q_hub_kernel(BwdArgs b, int chunks_per_hub) {
+// Long rows of the dQ pass: work items as in edge_attn_fwd_long_kernel, partial dQ rows to the scratch.
+template <typename T, int HN, bool EXPH>
+__global__ void __launch_bounds__(256, EXPH ? 2 : 3) edge_attn_bwd_q_long_kernel(BwdArgs b) {
   constexpr int VN = Vec<T>::N;
   constexpr int LPH = HN / VN;
   const AttnArgs& a = b.f;
   const Geo g = make_geo<T, HN>(a.hl);
   const int w_row = a.hl * HN;
-  const int hub_i = blockIdx.x / chunks_per_hub;
-  const int row = a.hub_rows[hub_i];
-  const int rbeg = a.rowptr[row], rend = a.rowptr[row + 1];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  const int tpw = 32 / g.tl;
-  const int lt = lane % g.tl;
-  const int streams = nwarp * tpw;
-  const int stream = warp * tpw + lane / g.tl;
-  float* scratch = b.hub_scratch_q + (long long)hub_i * w_row;
-  for (int chunk = blockIdx.x % chunks_per_hub; (long long)chunk * a.hub_chunk < rend - rbeg; chunk += chunks_per_hub) {
-  const int cbeg = rbeg + chunk * a.hub_chunk;
-  const int cend = min(rend, cbeg + a.hub_chunk);
-  for (int hc = 0; hc < g.n_hc; ++hc) {
-    const int head = hc * g.hpt + lt / LPH;
-    const bool head_ok = head < a.hl;
-    const int hsafe = head_ok ? head : 0;
-    const int off = hsafe * HN + (lt % LPH) * VN;
-    float qs0[VN], qs1[VN], qraw[VN], dof[VN], of[VN], dq[VN], de0[VN], de1[VN];
-    load_q_scaled<T, HN>(a, row, hsafe, off, qs0, qs1);
-    load_vec<T>(static_cast<const T*>(a.q) + (long long)row * a.ldq + off, qraw);
-    load_vec<T>(static_cast<const T*>(b.dout) + (long long)row * w_row + off, dof);
-    load_vec<T>(static_cast<const T*>(a.out) + (long long)row * w_row + off, of);
-    float dterm = 0.f;
+  const int lane = threadIdx.x & 31;
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (warp >= (long long)a.n_long_task * g.n_hc) return;
+  const int tpw = 32 / g.tl, sub = lane / g.tl, lt = lane % g.tl;
+  const int item = (int)(warp / g.n_hc), hc = (int)(warp % g.n_hc);
+  const int head = hc * g.hpt + lt / LPH;
+  const bool head_ok = head < a.hl;
+  const int hsafe = head_ok ? head : 0;
+  const int off = hsafe * HN + (lt % LPH) * VN;
+  const int4 it = __ldg(a.long_task + item);
+  const int row = it.x;
+  const int per = (it.z - it.y + tpw - 1) / tpw;
+  const int beg = it.y + sub * per, end = min(it.z, beg + per);
+  float qs0[VN], qs1[VN], qraw[VN], dof[VN], of[VN], dq[VN], de0[VN], de1[VN];
+  load_q_scaled<T, HN>(a, row, hsafe, off, qs0, qs1);
+  load_vec<T>(static_cast<const T*>(a.q) + (long long)row * a.ldq + off, qraw);
+  load_vec<T>(static_cast<const T*>(b.dout) + (long long)row * w_row + off, dof);
+  load_vec<T>(static_cast<const T*>(a.out) + (long long)row * w_row + off, of);
+  float dterm = 0.f;
 #pragma unroll
-    for (int i = 0; i < VN; ++i) { dterm += dof[i] * of[i]; dq[i] = 0.f; de0[i] = 0.f; de1[i] = 0.f; }
-    const unsigned hm = head_mask<LPH>();
-    dterm = head_sum<LPH>(dterm, hm);
-    if (a.out_thresh) dterm *= a.out_keep;
-    const float invz = 1.f / (a.z[(long long)row * a.hl + hsafe] + kEps);
-    if (head_ok)
-      for (int e = cbeg + stream; e < cend; e += streams)
-        dq_edge<T, HN>(b, e, hsafe, off, qs0, qs1, qraw, dof, invz, dterm, dq, de0, de1, hm);
-    if (head_ok) {
+  for (int i = 0; i < VN; ++i) { dterm += dof[i] * of[i]; dq[i] = 0.f; de0[i] = 0.f; de1[i] = 0.f; }
+  const unsigned hm = head_mask<LPH>();
+  dterm = head_sum<LPH>(dterm, hm);
+  if (a.out_thresh) dterm *= a.out_keep;
+  const float invz = 1.f / (a.z[(long long)row * a.hl + hsafe] + kEps);
+  for (int e = beg; e < end; e += 2)
+    dq_edge4<T, HN, EXPH, 2>(b, e, end, hsafe, off, qs0, qs1, qraw, dof, invz, dterm, dq, de0, de1, hm);
+  __syncwarp();
 #pragma unroll
-      for (int i = 0; i < VN; ++i) atomicAdd(scratch + off + i, dq[i]);
-      if (a.variant == 2) {
+  for (int i = 0; i < VN; ++i) dq[i] = group_total(dq[i], g.tl);
+  if (EXPH) {
 #pragma unroll
-        for (int i = 0; i < VN; ++i) {
-          atomicAdd(b.detab + off + i, de0[i]);
-          atomicAdd(b.detab + w_row + off + i, de1[i]);
-        }
+    for (int i = 0; i < VN; ++i) { de0[i] = group_total(de0[i], g.tl); de1[i] = group_total(de1[i], g.tl); }
+  }
+  if (sub == 0 && head_ok) {
+    float* pp = a.long_partial + (long long)it.w * w_row;
+#pragma unroll
+    for (int i = 0; i < VN; i += 4) *reinterpret_cast<float4*>(pp + off + i) = make_float4(dq[i], dq[i + 1], dq[i + 2], dq[i + 3]);
+    if (EXPH) {
+#pragma unroll
+      for (int i = 0; i < VN; ++i) {
+        atomicAdd(b.detab + off + i, de0[i]);
+        atomicAdd(b.detab + w_row + off + i, de1[i]);
       }
     }
-  }
-  }
-}
-
-// One transposed edge (key j fixed, query i varies) for one task lane.
-template <typename T, int HN>
-__device__ __forceinline__ void dkv_edge(const BwdArgs& b, int te, int head, int off, const float* kf, const float* vf,
-                                         float* dk, float* dv, unsigned hm) {
-  constexpr int VN = Vec<T>::N;
-  constexpr int LPH = HN / VN;
-  const AttnArgs& a = b.f;
-  const float scale = inv_sqrt_hn<HN>();
-  const int w_row = a.hl * HN;
-  const int i_row = __ldg(b.t_row + te);
-  const int eid = __ldg(b.t_eid + te);
-  float qf[VN], dof[VN];
-  load_vec<T>(static_cast<const T*>(a.q) + (long long)i_row * a.ldq + off, qf);
-  load_vec<T>(static_cast<const T*>(b.dout) + (long long)i_row * w_row + off, dof);
-  const float2 zd = __ldg(b.zd + (long long)i_row * a.hl + head);
-  const int t = (a.variant == 2) ? a.etype[eid] : 0;
-  float et[VN];
-  if (a.variant == 2) {
-#pragma unroll
-    for (int i = 0; i < VN; ++i) et[i] = a.etab[(t ? w_row : 0) + off + i];
-  } else {
-#pragma unroll
-    for (int i = 0; i < VN; ++i) et[i] = 1.f;
-  }
-  float d = 0.f, dotv = 0.f;
-#pragma unroll
-  for (int i = 0; i < VN; ++i) { d += qf[i] * kf[i] * et[i]; dotv += dof[i] * vf[i]; }
-  d = head_sum<LPH>(d, hm) * scale;
-  dotv = head_sum<LPH>(dotv, hm);
-  const bool inr = (d > -kClamp) && (d < kClamp);
-  const float w = __expf(fminf(fmaxf(d, -kClamp), kClamp));
-  float mf = 1.f;
-  if (a.variant == 1 && a.thresh) mf = keep_edge(a.seed, (uint32_t)eid, (uint32_t)head, a.thresh) ? a.inv_keep : 0.f;
-  else if (a.variant == 1) mf = a.inv_keep;
-  const float ds = inr ? (dotv * mf - zd.y) * zd.x * w : 0.f;
-  const float wn = w * mf * zd.x;
-#pragma unroll
-  for (int i = 0; i < VN; ++i) {
-    dk[i] += ds * scale * qf[i] * et[i];
-    dv[i] += wn * dof[i];
   }
 }
 
@@ -772,143 +745,119 @@ __global__ void __launch_bounds__(256, MINB) edge_attn_bwd_kv_task_kernel(BwdArg
   }
 }
 
-// Adds the partials of every split key row (fixed association => bit-reproducible).  A hub key owns thousands of
-// slots, so a block spreads them over G thread groups (slot j goes to group j % G), every thread keeps 16 independent
-// sums in flight, and the groups' results meet in shared memory in group order.
-constexpr int KV_REDUCE_THREADS = 1024;
-template <typename T>
-__global__ void __launch_bounds__(KV_REDUCE_THREADS) edge_attn_bwd_kv_reduce_kernel(BwdArgs b, int w_row) {
-  extern __shared__ float s_part[];           // [G, 2 * w_row]
-  const int s = blockIdx.x;
-  const int row = b.kv_split[3 * s], first = b.kv_split[3 * s + 1], n = b.kv_split[3 * s + 2];
-  const int ncol = 2 * w_row;
-  const int G = ncol <= KV_REDUCE_THREADS ? KV_REDUCE_THREADS / ncol : 1;
-  const int grp = ncol <= KV_REDUCE_THREADS ? (int)threadIdx.x / ncol : 0;
-  for (int c0 = 0; c0 < ncol; c0 += KV_REDUCE_THREADS) {
-    const int c = c0 + (ncol <= KV_REDUCE_THREADS ? (int)threadIdx.x % ncol : (int)threadIdx.x);
-    const bool act = c < ncol && grp < G;
-    float acc = 0.f;
-    if (act) {
-      float a16[16];
-#pragma unroll
-      for (int u = 0; u < 16; ++u) a16[u] = 0.f;
-      const float* pp = b.kv_partial + (long long)first * ncol + c;
-      int j = grp;
-      for (; j + 15 * G < n; j += 16 * G) {
-#pragma unroll
-        for (int u = 0; u < 16; ++u) a16[u] += pp[(long long)(j + u * G) * ncol];
-      }
-      for (; j < n; j += G) a16[0] += pp[(long long)j * ncol];
-#pragma unroll
-      for (int w = 8; w > 0; w >>= 1) {
-#pragma unroll
-        for (int u = 0; u < w; ++u) a16[u] += a16[u + w];
-      }
-      acc = a16[0];
+// ---------------------------------------------------------------------------------------------
+// Rows cut into work items: their partial sums lie side by side in slot order.  Pass 1 gives every window of SPLIT_WINDOW
+// slots to a block, which adds the slots of each row inside its window (threads run along the columns, so every slot is one
+// coalesced read) and finishes the rows that lie in the window whole; of a row that goes on, the window's sum replaces its
+// first slot there.  Pass 2 adds those window sums for the rows that cross a window's end.  The association depends on the
+// slot numbers alone: bit-reproducible.  A row of 10^6 edges (16 k slots) is thus 244 blocks and one short tail instead of
+// one block's walk, and 10^4 rows of two or three slots are a few hundred blocks instead of 10^4 (each of 1,024 threads):
+// both passes over the dK/dV slots take 84 us on a 612 k-node power-law graph at h = 256 (632 us with a block per row),
+// 42 us at 700 k nodes / h = 128 (78 us).
+// ---------------------------------------------------------------------------------------------
+constexpr int SPLIT_WINDOW = 64;
+constexpr int SPLIT_THREADS = 256;
+constexpr int SPLIT_FWD = 0, SPLIT_DQ = 1, SPLIT_KV = 2;
+
+// s[0 .. ncol) holds the finished sums of row `row`
+template <typename T, int MODE>
+__device__ __forceinline__ void split_finish(const BwdArgs& b, int row, int w, int hn, const float* s) {
+  const AttnArgs& a = b.f;
+  if (MODE == SPLIT_FWD) {
+    for (int c = threadIdx.x; c < w; c += blockDim.x) {
+      const int head = c / hn;
+      const float zs = s[w + head];
+      float inv = 1.f / (zs + kEps);
+      if (a.variant == 1) inv *= a.inv_keep;
+      float ov = s[c] * inv;
+      if (a.out_thresh) ov = keep_out(a, row, c) ? ov * a.out_inv_keep : 0.f;
+      static_cast<T*>(a.out)[(long long)row * w + c] = from_float<T>(ov);
+      if (a.route_out.n_dest) *routed<T>(a.route_out, row, c) = from_float<T>(ov);
+      if (c % hn == 0) a.z[(long long)row * a.hl + head] = zs;
     }
-    if (G > 1) {
-      if (act) s_part[grp * ncol + c] = acc;
+  } else if (MODE == SPLIT_DQ) {
+    T* dst = grad_row<T>(b, b.dq, b.cq, row);
+    for (int c = threadIdx.x; c < w; c += blockDim.x) dst[c] = from_float<T>(s[c]);
+  } else {
+    T* dk = grad_row<T>(b, b.dk, b.ck, row);
+    T* dv = grad_row<T>(b, b.dv, b.cv, row);
+    for (int c = threadIdx.x; c < 2 * w; c += blockDim.x) (c < w ? dk + c : dv + (c - w))[0] = from_float<T>(s[c]);
+  }
+}
+
+template <typename T, int MODE>
+__global__ void __launch_bounds__(SPLIT_THREADS) split_window_kernel(BwdArgs b, const int4* __restrict__ task, int n_slots,
+                                                                     float* partial, int pitch, int ncol, int w, int hn) {
+  extern __shared__ float s_sum[];            // [ncol]
+  __shared__ int s_key[SPLIT_WINDOW];
+  const int s0 = blockIdx.x * SPLIT_WINDOW, s1 = min(s0 + SPLIT_WINDOW, n_slots);
+  for (int i = threadIdx.x; i < s1 - s0; i += blockDim.x) s_key[i] = task[s0 + i].x;
+  const int before = s0 > 0 ? task[s0 - 1].x : -1, after = s1 < n_slots ? task[s1].x : -1;
+  __syncthreads();
+  for (int i = s0; i < s1;) {
+    const int key = s_key[i - s0];
+    int j = i + 1;
+    while (j < s1 && s_key[j - s0] == key) ++j;
+    const bool whole = !(i == s0 && before == key) && !(j == s1 && after == key);
+    for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
+      const float* pp = partial + (long long)i * pitch + c;
+      float acc[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc[u] = 0.f;
+      int n = j - i;
+      for (; n >= 8; n -= 8, pp += 8 * (long long)pitch) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc[u] += pp[u * (long long)pitch];
+      }
+#pragma unroll
+      for (int u = 0; u < 7; ++u)
+        if (u < n) acc[u] += pp[u * (long long)pitch];
+      const float sum = ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
+      if (whole) s_sum[c] = sum;
+      else partial[(long long)i * pitch + c] = sum;
+    }
+    if (whole) {
       __syncthreads();
-      if (act && grp == 0) {
-        for (int q = 1; q < G; ++q) acc += s_part[q * ncol + c];
+      split_finish<T, MODE>(b, key, w, hn, s_sum);
+      __syncthreads();
+    }
+    i = j;
+  }
+}
+
+template <typename T, int MODE>
+__global__ void __launch_bounds__(SPLIT_THREADS) split_cross_kernel(BwdArgs b, const int* __restrict__ split, int n_split,
+                                                                    const float* partial, int pitch, int ncol, int w, int hn) {
+  extern __shared__ float s_sum[];            // [ncol]
+  for (int s = blockIdx.x; s < n_split; s += gridDim.x) {
+    const int first = split[3 * s + 1];
+    const int w0 = first / SPLIT_WINDOW, w1 = (first + split[3 * s + 2] - 1) / SPLIT_WINDOW;
+    if (w0 == w1) continue;                   // finished by its window
+    for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
+      float acc[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc[u] = 0.f;
+      const float* pp = partial + c;
+      int k = w0 + 1;
+      for (; k + 7 <= w1; k += 8) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc[u] += pp[(long long)(k + u) * SPLIT_WINDOW * pitch];
       }
+      for (; k <= w1; ++k) acc[0] += pp[(long long)k * SPLIT_WINDOW * pitch];
+      s_sum[c] = pp[(long long)first * pitch] + ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
     }
-    if (act && grp == 0) {
-      T* dst = c < w_row ? grad_row<T>(b, b.dk, b.ck, row) : grad_row<T>(b, b.dv, b.cv, row);
-      dst[c < w_row ? c : c - w_row] = from_float<T>(acc);
-    }
-    if (G > 1) __syncthreads();
+    __syncthreads();
+    split_finish<T, MODE>(b, split[3 * s], w, hn, s_sum);
+    __syncthreads();
   }
 }
 
-template <typename T, int HN>
-__global__ void __launch_bounds__(256) edge_attn_bwd_kv_kernel(BwdArgs b) {
-  constexpr int VN = Vec<T>::N;
-  constexpr int LPH = HN / VN;
-  const AttnArgs& a = b.f;
-  const Geo g = make_geo<T, HN>(a.hl);
-  const int w_row = a.hl * HN;
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int tpw = 32 / g.tl;
-  const long long task = (long long)warp * tpw + lane / g.tl;
-  const int lt = lane % g.tl;
-  const long long n_task = (long long)a.n * g.n_hc;
-  const bool live = task < n_task;
-  const int row = live ? (int)(task / g.n_hc) : 0;
-  const int hc = live ? (int)(task % g.n_hc) : 0;
-  const int head = hc * g.hpt + lt / LPH;
-  const bool head_ok = live && head < a.hl;
-  const int hsafe = head_ok ? head : 0;
-  const int off = hsafe * HN + (lt % LPH) * VN;
-  int beg = 0, end = 0;
-  if (head_ok) { beg = b.t_rowptr[row]; end = b.t_rowptr[row + 1]; }
-  const bool hub = b.n_t_hub > 0 && (end - beg) > BF_HUB_DEGREE;
-  if (hub) end = beg;
-  float kf[VN], vf[VN], dk[VN], dv[VN];
-  load_vec<T>(static_cast<const T*>(a.k) + (long long)row * a.ldk + off, kf);
-  load_vec<T>(static_cast<const T*>(a.v) + (long long)row * a.ldv + off, vf);
-#pragma unroll
-  for (int i = 0; i < VN; ++i) { dk[i] = 0.f; dv[i] = 0.f; }
-  const unsigned hm = head_mask<LPH>();
-  for (int e = beg; e < end; ++e) dkv_edge<T, HN>(b, e, hsafe, off, kf, vf, dk, dv, hm);
-  if (head_ok && !hub) {
-    store_vec<T>(grad_row<T>(b, b.dk, b.ck, row) + off, dk);
-    store_vec<T>(grad_row<T>(b, b.dv, b.cv, row) + off, dv);
-  }
-}
-
-template <typename T, int HN>
-__global__ void __launch_bounds__(256) edge_attn_bwd_kv_hub_kernel(BwdArgs b, int chunks_per_hub) {
-  constexpr int VN = Vec<T>::N;
-  constexpr int LPH = HN / VN;
-  const AttnArgs& a = b.f;
-  const Geo g = make_geo<T, HN>(a.hl);
-  const int w_row = a.hl * HN;
-  const int hub_i = blockIdx.x / chunks_per_hub;
-  const int row = b.t_hub_rows[hub_i];
-  const int rbeg = b.t_rowptr[row], rend = b.t_rowptr[row + 1];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  const int tpw = 32 / g.tl;
-  const int lt = lane % g.tl;
-  const int streams = nwarp * tpw;
-  const int stream = warp * tpw + lane / g.tl;
-  float* scratch = b.hub_scratch_kv + (long long)hub_i * 2 * w_row;
-  for (int chunk = blockIdx.x % chunks_per_hub; (long long)chunk * a.hub_chunk < rend - rbeg; chunk += chunks_per_hub) {
-  const int cbeg = rbeg + chunk * a.hub_chunk;
-  const int cend = min(rend, cbeg + a.hub_chunk);
-  for (int hc = 0; hc < g.n_hc; ++hc) {
-    const int head = hc * g.hpt + lt / LPH;
-    const bool head_ok = head < a.hl;
-    const int hsafe = head_ok ? head : 0;
-    const int off = hsafe * HN + (lt % LPH) * VN;
-    float kf[VN], vf[VN], dk[VN], dv[VN];
-    load_vec<T>(static_cast<const T*>(a.k) + (long long)row * a.ldk + off, kf);
-    load_vec<T>(static_cast<const T*>(a.v) + (long long)row * a.ldv + off, vf);
-#pragma unroll
-    for (int i = 0; i < VN; ++i) { dk[i] = 0.f; dv[i] = 0.f; }
-    const unsigned hm = head_mask<LPH>();
-    if (head_ok)
-      for (int e = cbeg + stream; e < cend; e += streams) dkv_edge<T, HN>(b, e, hsafe, off, kf, vf, dk, dv, hm);
-    if (head_ok) {
-#pragma unroll
-      for (int i = 0; i < VN; ++i) {
-        atomicAdd(scratch + off + i, dk[i]);
-        atomicAdd(scratch + w_row + off + i, dv[i]);
-      }
-    }
-  }
-  }
-}
-
-template <typename T>
-__global__ void hub_scatter_rows(const float* scratch, int scratch_ld, int scratch_off, const int* rows, BwdArgs b, void* local,
-                                 int col0, int width) {
-  const int hub_i = blockIdx.x;
-  const int row = rows[hub_i];
-  T* dst = grad_row<T>(b, local, col0, row);
-  for (int c = threadIdx.x; c < width; c += blockDim.x)
-    dst[c] = from_float<T>(scratch[(long long)hub_i * scratch_ld + scratch_off + c]);
+template <typename T, int MODE>
+void launch_split(const BwdArgs& b, const int4* task, int n_slots, const int* split, int n_split, float* partial, int pitch,
+                  int ncol, int w, int hn, cudaStream_t st) {
+  const size_t smem = sizeof(float) * ncol;
+  split_window_kernel<T, MODE><<<(n_slots + SPLIT_WINDOW - 1) / SPLIT_WINDOW, SPLIT_THREADS, smem, st>>>(b, task, n_slots, partial, pitch, ncol, w, hn);
+  split_cross_kernel<T, MODE><<<n_split < 148 * 8 ? n_split : 148 * 8, SPLIT_THREADS, smem, st>>>(b, split, n_split, partial, pitch, ncol, w, hn);
 }
 
 template <typename T, int HN>
@@ -919,6 +868,13 @@ cudaError_t launch_fwd_t(const AttnArgs& a, int chunks_per_hub, cudaStream_t st)
   const long long warps = (n_task + tpw - 1) / tpw;
   const long long blocks = (warps + 7) / 8;
   if (blocks > 0) edge_attn_fwd_kernel<T, HN><<<(unsigned)blocks, 256, 0, st>>>(a);
+  if (a.n_long_task > 0) {
+    edge_attn_fwd_long_kernel<T, HN><<<(unsigned)(((long long)a.n_long_task * g.n_hc + 7) / 8), 256, 0, st>>>(a);
+    BwdArgs b{};
+    b.f = a;
+    const int w = a.hl * HN, pitch = fwd_pitch(w, a.hl);
+    launch_split<T, SPLIT_FWD>(b, a.long_task, a.n_long_task, a.long_split, a.n_long_split, a.long_partial, pitch, w + a.hl, w, HN, st);
+  }
   if (a.n_hub > 0) {
     edge_attn_fwd_hub_kernel<T, HN><<<a.n_hub * chunks_per_hub, 256, 0, st>>>(a, chunks_per_hub);
     edge_attn_fwd_hub_finalize<T, HN><<<a.n_hub, 256, 0, st>>>(a);
@@ -927,7 +883,7 @@ cudaError_t launch_fwd_t(const AttnArgs& a, int chunks_per_hub, cudaStream_t st)
 }
 
 template <typename T, int HN>
-cudaError_t launch_bwd_t(const BwdArgs& b, int chunks_q, int chunks_kv, cudaStream_t st) {
+cudaError_t launch_bwd_t(const BwdArgs& b, cudaStream_t st) {
   const AttnArgs& a = b.f;
   const Geo g = make_geo<T, HN>(a.hl);
   const long long n_task = (long long)a.n * g.n_hc;
@@ -940,36 +896,27 @@ cudaError_t launch_bwd_t(const BwdArgs& b, int chunks_q, int chunks_kv, cudaStre
     if (a.variant == 2) edge_attn_bwd_q_kernel<T, HN, true><<<(unsigned)blocks, 256, smem, st>>>(b);
     else edge_attn_bwd_q_kernel<T, HN, false><<<(unsigned)blocks, 256, smem, st>>>(b);
   }
-  if (a.n_hub > 0) {
-    edge_attn_bwd_q_hub_kernel<T, HN><<<a.n_hub * chunks_q, 256, 0, st>>>(b, chunks_q);
-    hub_scatter_rows<T><<<a.n_hub, 256, 0, st>>>(b.hub_scratch_q, w_row, 0, a.hub_rows, b, b.dq, b.cq, w_row);
+  if (a.n_long_task > 0) {
+    const unsigned lb = (unsigned)(((long long)a.n_long_task * g.n_hc + 7) / 8);
+    if (a.variant == 2) edge_attn_bwd_q_long_kernel<T, HN, true><<<lb, 256, 0, st>>>(b);
+    else edge_attn_bwd_q_long_kernel<T, HN, false><<<lb, 256, 0, st>>>(b);
+    launch_split<T, SPLIT_DQ>(b, a.long_task, a.n_long_task, a.long_split, a.n_long_split, a.long_partial, w_row, w_row, w_row, HN, st);
   }
-  if (b.kv_task) {
-    const long long kv_tasks = (long long)b.n_kv_task * g.n_hc;
-    const long long kv_warps = (kv_tasks + tpw - 1) / tpw;
-    const long long kv_blocks = (kv_warps + 7) / 8;
-    if (kv_blocks > 0) {
-      if (a.variant == 2) {
-        if (b.qg) edge_attn_bwd_kv_task_kernel<T, HN, true, 3, true><<<(unsigned)kv_blocks, 256, 0, st>>>(b);
-        else edge_attn_bwd_kv_task_kernel<T, HN, true, 3, false><<<(unsigned)kv_blocks, 256, 0, st>>>(b);
-      } else {
-        if (b.qg) edge_attn_bwd_kv_task_kernel<T, HN, false, 4, true><<<(unsigned)kv_blocks, 256, 0, st>>>(b);
-        else edge_attn_bwd_kv_task_kernel<T, HN, false, 4, false><<<(unsigned)kv_blocks, 256, 0, st>>>(b);
-      }
+  const long long kv_tasks = (long long)b.n_kv_task * g.n_hc;
+  const long long kv_warps = (kv_tasks + tpw - 1) / tpw;
+  const long long kv_blocks = (kv_warps + 7) / 8;
+  if (kv_blocks > 0) {
+    if (a.variant == 2) {
+      if (b.qg) edge_attn_bwd_kv_task_kernel<T, HN, true, 3, true><<<(unsigned)kv_blocks, 256, 0, st>>>(b);
+      else edge_attn_bwd_kv_task_kernel<T, HN, true, 3, false><<<(unsigned)kv_blocks, 256, 0, st>>>(b);
+    } else {
+      if (b.qg) edge_attn_bwd_kv_task_kernel<T, HN, false, 4, true><<<(unsigned)kv_blocks, 256, 0, st>>>(b);
+      else edge_attn_bwd_kv_task_kernel<T, HN, false, 4, false><<<(unsigned)kv_blocks, 256, 0, st>>>(b);
     }
-    if (b.n_kv_split > 0) {
-      const int ncol = 2 * w_row;
-      const int G = ncol <= KV_REDUCE_THREADS ? KV_REDUCE_THREADS / ncol : 1;
-      edge_attn_bwd_kv_reduce_kernel<T><<<b.n_kv_split, KV_REDUCE_THREADS, (size_t)G * ncol * sizeof(float), st>>>(b, w_row);
-    }
-    return cudaGetLastError();
   }
-  if (blocks > 0) edge_attn_bwd_kv_kernel<T, HN><<<(unsigned)blocks, 256, 0, st>>>(b);
-  if (b.n_t_hub > 0) {
-    edge_attn_bwd_kv_hub_kernel<T, HN><<<b.n_t_hub * chunks_kv, 256, 0, st>>>(b, chunks_kv);
-    hub_scatter_rows<T><<<b.n_t_hub, 256, 0, st>>>(b.hub_scratch_kv, 2 * w_row, 0, b.t_hub_rows, b, b.dk, b.ck, w_row);
-    hub_scatter_rows<T><<<b.n_t_hub, 256, 0, st>>>(b.hub_scratch_kv, 2 * w_row, w_row, b.t_hub_rows, b, b.dv, b.cv, w_row);
-  }
+  // the items of split keys come first in the list, so item i of them is slot i
+  if (b.n_kv_split > 0)
+    launch_split<T, SPLIT_KV>(b, b.kv_task, b.n_kv_slots, b.kv_split, b.n_kv_split, b.kv_partial, 2 * w_row, 2 * w_row, w_row, HN, st);
   return cudaGetLastError();
 }
 
@@ -987,8 +934,22 @@ AttnArgs to_args(const bf_attn_params& p) {
   a.out_inv_keep = p.out_dropout_p > 0.f ? 1.f / (1.f - p.out_dropout_p) : 1.f;
   a.out_rows_local = p.out_rows_local; a.out_col0 = p.out_col0;
   a.hub_rows = p.hub_rows; a.n_hub = p.n_hub; a.hub_chunk = BF_HUB_CHUNK; a.hub_scratch = p.hub_scratch;
+  a.long_row = p.n_hub > 0 ? BF_HUB_DEGREE : 0;
+  a.long_task = nullptr; a.n_long_task = 0; a.long_split = nullptr; a.n_long_split = 0; a.long_partial = nullptr;
   memset(&a.route_out, 0, sizeof(a.route_out));
   return a;
+}
+
+// A caller's list of long rows (false: reject the call).  It replaces the hub list.
+bool take_long_rows(const bf_long_rows* r, AttnArgs* a) {
+  if (r == nullptr || r->n_task <= 0) return true;
+  if (r->task == nullptr || ((uintptr_t)r->task) % 16 != 0 || r->split == nullptr || r->n_split <= 0 || r->partial == nullptr ||
+      ((uintptr_t)r->partial) % 16 != 0 || r->min_degree <= 0 || a->n_hub > 0)
+    return false;
+  a->long_row = r->min_degree;
+  a->long_task = reinterpret_cast<const int4*>(r->task); a->n_long_task = r->n_task;
+  a->long_split = r->split; a->n_long_split = r->n_split; a->long_partial = r->partial;
+  return true;
 }
 
 // Validated copy of a caller's route for `n` rows of `width` elements each; false = reject the call.
@@ -1025,8 +986,12 @@ bool to_route(const bf_attn_route* r, int n, long long width, Route* out) {
     }                                                                                       \
   } while (0)
 
-extern "C" int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_route* route, cudaStream_t st) {
+extern "C" size_t bf_attn_fwd_long_pitch(int hl, int hn) { return (size_t)fwd_pitch(hl * hn, hl); }
+
+extern "C" int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_route* route, const bf_long_rows* long_rows,
+                                       cudaStream_t st) {
   AttnArgs a = to_args(*p);
+  if (!take_long_rows(long_rows, &a)) return (int)cudaErrorInvalidValue;
   if (!to_route(route, p->n, (long long)p->hl * p->hn, &a.route_out)) return (int)cudaErrorInvalidValue;
   const int chunks = p->max_hub_degree > 0 ? (p->max_hub_degree + BF_HUB_CHUNK - 1) / BF_HUB_CHUNK : 1;
 #define CALL_FWD(T, H) (int)launch_fwd_t<T, H>(a, chunks, st)
@@ -1047,16 +1012,16 @@ extern "C" int bf_edge_attn_fwd(const bf_attn_params* p, cudaStream_t st) {
 extern "C" int bf_edge_attn_bwd(const bf_attn_params* p, const bf_attn_bwd_params* q, cudaStream_t st) {
   BwdArgs b;
   b.f = to_args(*p);
+  if (b.f.n_hub > 0 || !take_long_rows(&q->long_rows, &b.f) || q->kv_task == nullptr) return (int)cudaErrorInvalidValue;
   b.dout = q->dout; b.dq = q->dq; b.dk = q->dk; b.dv = q->dv;
   b.ldg = q->ldg > 0 ? q->ldg : (long long)p->hl * p->hn;
   b.zd = reinterpret_cast<float2*>(q->zd);
   b.t_rowptr = q->t_rowptr; b.t_row = q->t_row; b.t_eid = q->t_eid; b.detab = q->detab;
-  b.t_hub_rows = q->t_hub_rows; b.n_t_hub = q->n_t_hub;
-  b.hub_scratch_q = q->hub_scratch_q; b.hub_scratch_kv = q->hub_scratch_kv;
   b.kv_task = reinterpret_cast<const int4*>(q->kv_task); b.n_kv_task = q->n_kv_task;
-  b.kv_split = q->kv_split; b.n_kv_split = q->n_kv_split; b.kv_partial = q->kv_partial;
-  // the packed records serve the work-list form of the dK/dV pass only
-  b.qg = (q->kv_task != nullptr && q->qg != nullptr && q->cz != nullptr) ? q->qg : nullptr;
+  b.kv_split = q->kv_split; b.n_kv_split = q->n_kv_split; b.n_kv_slots = q->n_kv_slots; b.kv_partial = q->kv_partial;
+  if (b.n_kv_split > 0 && (b.kv_split == nullptr || b.kv_partial == nullptr || b.n_kv_slots <= 0 || b.n_kv_slots > b.n_kv_task))
+    return (int)cudaErrorInvalidValue;
+  b.qg = (q->qg != nullptr && q->cz != nullptr) ? q->qg : nullptr;
   b.cz = b.qg ? q->cz : nullptr;
   b.cq = q->route_cq; b.ck = q->route_ck; b.cv = q->route_cv;
   {
@@ -1067,9 +1032,7 @@ extern "C" int bf_edge_attn_bwd(const bf_attn_params* p, const bf_attn_bwd_param
     if (b.route.n_dest > 0 && (b.cq < 0 || b.ck < 0 || b.cv < 0 || ((b.cq | b.ck | b.cv) % 8) != 0))
       return (int)cudaErrorInvalidValue;
   }
-  const int cq = p->max_hub_degree > 0 ? (p->max_hub_degree + BF_HUB_CHUNK - 1) / BF_HUB_CHUNK : 1;
-  const int ckv = q->max_t_hub_degree > 0 ? (q->max_t_hub_degree + BF_HUB_CHUNK - 1) / BF_HUB_CHUNK : 1;
-#define CALL_BWD(T, H) (int)launch_bwd_t<T, H>(b, cq, ckv, st)
+#define CALL_BWD(T, H) (int)launch_bwd_t<T, H>(b, st)
   BF_DISPATCH(p->dtype, p->hn, CALL_BWD);
 #undef CALL_BWD
   return (int)cudaErrorInvalidValue;

@@ -51,13 +51,14 @@ __global__ void gather_rows_kernel(const int* __restrict__ erow, const int* __re
   if (i < n_edges) t_row[i] = erow[t_eid[i]];
 }
 
-// items per key (at least one, so that keys without edges still get their zero gradient written) and partial slots
-__global__ void task_counts_kernel(const int* __restrict__ t_rowptr, int n, int chunk, int* __restrict__ n_items,
+// items per key (at least one, so that keys without edges still get their zero gradient written) and partial slots; only
+// rows with more than `min_split` edges are cut
+__global__ void task_counts_kernel(const int* __restrict__ t_rowptr, int n, int chunk, int min_split, int* __restrict__ n_items,
                                    int* __restrict__ n_slots, int* __restrict__ is_split) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int deg = t_rowptr[k + 1] - t_rowptr[k];
-  const int c = deg <= chunk ? 1 : (deg + chunk - 1) / chunk;
+  const int c = deg <= min_split ? 1 : (deg + chunk - 1) / chunk;
   n_items[k] = c;
   n_slots[k] = c > 1 ? c : 0;
   is_split[k] = c > 1 ? 1 : 0;
@@ -68,7 +69,7 @@ __global__ void task_counts_kernel(const int* __restrict__ t_rowptr, int n, int 
 // followed by the single item of every other key in key order; an item of a split key sits at its partial-slot index.
 __global__ void task_fill_kernel(const int* __restrict__ t_rowptr, const int* __restrict__ item_first,
                                  const int* __restrict__ slot_first, const int* __restrict__ split_first, int n,
-                                 int chunk, int4* __restrict__ tasks, int* __restrict__ splits) {
+                                 int chunk, int singles, int4* __restrict__ tasks, int* __restrict__ splits) {
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int k = (int)(gt >> 5), lane = (int)(gt & 31);
   if (k >= n) return;
@@ -77,7 +78,7 @@ __global__ void task_fill_kernel(const int* __restrict__ t_rowptr, const int* __
   const int s0 = slot_first[k];
   const int total_slots = slot_first[n];
   if (cnt == 1) {
-    if (lane == 0) tasks[total_slots + (k - split_first[k])] = make_int4(k, beg, end, -1);
+    if (lane == 0 && singles) tasks[total_slots + (k - split_first[k])] = make_int4(k, beg, end, -1);
     return;
   }
   for (int c = lane; c < cnt; c += 32) {
@@ -130,7 +131,7 @@ extern "C" int bf_graph_transpose(const int* rowptr, const int* col, int n, long
 }
 
 // Phase 1 of the work list: per-key counts and their exclusive prefix sums ([n+1] each, last element = total).
-extern "C" int bf_kv_task_counts(const int* t_rowptr, int n, int chunk, int* item_first, int* slot_first,
+extern "C" int bf_kv_task_counts(const int* t_rowptr, int n, int chunk, int min_split, int* item_first, int* slot_first,
                                  int* split_first, void* scratch, size_t scratch_bytes, cudaStream_t st) {
   // scratch: three int[n] count arrays followed by the scan's temporary storage
   int* n_items = static_cast<int*>(scratch);
@@ -139,7 +140,8 @@ extern "C" int bf_kv_task_counts(const int* t_rowptr, int n, int chunk, int* ite
   const size_t head = (3 * (size_t)n * sizeof(int) + 255) & ~(size_t)255;
   void* scan_tmp = static_cast<uint8_t*>(scratch) + head;
   size_t scan_bytes = scratch_bytes - head;
-  task_counts_kernel<<<(n + 255) / 256, 256, 0, st>>>(t_rowptr, n, chunk, n_items, n_slots, is_split);
+  if (chunk < 1 || min_split < chunk) return (int)cudaErrorInvalidValue;
+  task_counts_kernel<<<(n + 255) / 256, 256, 0, st>>>(t_rowptr, n, chunk, min_split, n_items, n_slots, is_split);
   cudaError_t e;
   // exclusive prefix sums with the total appended: out[0] = 0, out[1..n] = inclusive sums
   for (int which = 0; which < 3; ++which) {
@@ -161,11 +163,11 @@ extern "C" size_t bf_kv_task_scratch(int n) {
 
 // Phase 2: write the items and the split list (sizes read back by the caller from the prefix sums).
 extern "C" int bf_kv_task_fill(const int* t_rowptr, const int* item_first, const int* slot_first, const int* split_first,
-                               int n, int chunk, int* tasks, int* splits, cudaStream_t st) {
+                               int n, int chunk, int singles, int* tasks, int* splits, cudaStream_t st) {
   const long long threads = (long long)n * 32;
   const unsigned blocks = (unsigned)((threads + 255) / 256);
   if (blocks > 0)
-    task_fill_kernel<<<blocks, 256, 0, st>>>(t_rowptr, item_first, slot_first, split_first, n, chunk,
+    task_fill_kernel<<<blocks, 256, 0, st>>>(t_rowptr, item_first, slot_first, split_first, n, chunk, singles,
                                              reinterpret_cast<int4*>(tasks), splits);
   return (int)cudaGetLastError();
 }

@@ -20,7 +20,8 @@ from typing import Optional
 
 import torch
 
-HUB_DEGREE = 1024  # rows longer than this take the chunked hub path in the kernels
+LONG_ROW = 128     # query rows with more edges are cut into work items of LONG_CHUNK edges (csrc/bf_kernels.h: BF_LONG_ROW,
+LONG_CHUNK = 64    # BF_LONG_CHUNK)
 KV_TASK_EDGES = 64  # edges per work item of the dK/dV pass (32 and 128 both measured slower on the 2.9 M-node graph)
 
 
@@ -110,6 +111,10 @@ class AttnGraph:
     n_real: int = -1
     n_rw: int = -1
     kv_slots: int = 0                    # number of fp32 partial slots the dK/dV pass needs
+    # work list of the long query rows (device graphs): [T, 4] int32 row, beg, end, slot and [S, 3] int32 row, first slot,
+    # slots; see long_rows
+    q_task: Optional[torch.Tensor] = field(default=None, repr=False)
+    q_split: Optional[torch.Tensor] = field(default=None, repr=False)
 
     @property
     def device(self):
@@ -121,7 +126,8 @@ class AttnGraph:
 
     def nbytes(self) -> int:
         tot = 0
-        for t in (self.rowptr, self.col, self.etype, self.t_rowptr, self.t_row, self.t_eid, self.t_task, self.t_split):
+        for t in (self.rowptr, self.col, self.etype, self.t_rowptr, self.t_row, self.t_eid, self.t_task, self.t_split,
+                  self.q_task, self.q_split):
             if t is not None:
                 tot += int(t.numel()) * t.element_size()
         return tot
@@ -130,12 +136,12 @@ class AttnGraph:
         f = lambda t: None if t is None else t.to(device, non_blocking=non_blocking)
         return AttnGraph(self.num_rows, f(self.rowptr), f(self.col), f(self.etype), f(self.t_rowptr),
                          f(self.t_row), f(self.t_eid), f(self.t_task), f(self.t_split), self.max_degree,
-                         self.n_real, self.n_rw, self.kv_slots)
+                         self.n_real, self.n_rw, self.kv_slots, f(self.q_task), f(self.q_split))
 
     def record_stream(self, stream) -> None:
         """Tell the caching allocator that ``stream`` uses every tensor of the graph (they were allocated on another)."""
         for t in (self.rowptr, self.col, self.etype, self.t_rowptr, self.t_row, self.t_eid, self.t_task, self.t_split,
-                  getattr(self, "_totals", None)):
+                  self.q_task, self.q_split, getattr(self, "_totals", None)):
             if t is not None and t.is_cuda:
                 t.record_stream(stream)
 
@@ -151,6 +157,17 @@ class AttnGraph:
         if self.etype is not None:
             rows.append(self.etype.to(torch.int64))
         return torch.stack(rows, 0)
+
+    def long_rows(self):
+        """``(tasks, splits)`` of the query rows with more than ``LONG_ROW`` edges, for the device kernels; ``(None, None)``
+        when the known degree bound rules them out.  Made once per graph (one host read of the list's length)."""
+        if self.max_degree is not None and self.max_degree <= LONG_ROW:
+            return None, None
+        if self.q_task is None:
+            from ..ops import _ext
+            self.q_task, self.q_split = _ext.load().long_row_tasks(self.rowptr)
+            _ext.count_launches(5)
+        return self.q_task, self.q_split
 
     def ensure_transpose(self) -> "AttnGraph":
         """Build the by-key CSR (deterministic: stable sort keeps query order inside a key's row)."""
@@ -263,5 +280,13 @@ def add_virtual_node(graph: AttnGraph, num_nodes: int, nodes_per_rank: int) -> A
         rows = graph.row_ids()
         pos_in_row = torch.arange(graph.num_edges, device=dev) - graph.rowptr[:-1].to(torch.int64)[rows]
         col[starts[rows] + 1 + pos_in_row] = new_id[graph.col.to(torch.int64)].to(torch.int32)
-    return AttnGraph(total, rowptr.to(torch.int32), col, None, max_degree=None,
-                     n_real=graph.n_real, n_rw=graph.n_rw)
+    g = AttnGraph(total, rowptr.to(torch.int32), col, None, max_degree=None,
+                  n_real=graph.n_real, n_rw=graph.n_rw)
+    if graph.max_degree is not None and graph.max_degree < LONG_ROW:
+        # the virtual node's is the only long row, and its length is known here: no device query
+        m = (n + LONG_CHUNK - 1) // LONG_CHUNK if n > LONG_ROW else 0
+        slot = torch.arange(m, dtype=torch.int32, device=dev)
+        beg = slot * LONG_CHUNK
+        g.q_task = torch.stack([torch.zeros_like(slot), beg, (beg + LONG_CHUNK).clamp_(max=n), slot], 1).contiguous()
+        g.q_split = torch.tensor([[0, 0, m]] if m else [], dtype=torch.int32, device=dev).view(-1, 3)
+    return g

@@ -215,6 +215,7 @@ class EdgeEngine:
             with torch.cuda.stream(self._build_stream):
                 g = self._finalize(self._build_device(seed, state, who="ahead"))
                 g.ensure_transpose()
+                g.long_rows()
                 done = torch.cuda.Event()
                 done.record(self._build_stream)
             return g, done

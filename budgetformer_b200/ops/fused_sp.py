@@ -269,7 +269,7 @@ class _PackedEdgeAttention(torch.autograd.Function):
         # element (row, c) is the one the owner of that row regenerates for (row - its first row, this rank's column)
         out_drop = [float(out_p), int(out_seed), int(sp.rows_local), int(sp.rank * hl)] if out_p > 0 else []
         ext.edge_attn_fwd(q, k, v, out.view(r, hlh, hn), z, graph.rowptr, graph.col, graph.etype, etable,
-                          int(variant_id), float(dropout_p), int(seed), kmax, out_drop, route)
+                          int(variant_id), float(dropout_p), int(seed), kmax, out_drop, route, *graph.long_rows())
         _ext.count_launches(1)
         if sp.token_rows is not None and len(sp.token_rows) > 1:
             out[sp.token_rows[1:]] = out[sp.token_rows[0]].clone()  # copy_global_token0 (gt_sp/utils.py:2365-2386)
@@ -304,7 +304,7 @@ class _PackedEdgeAttention(torch.autograd.Function):
         ext.edge_attn_bwd(q, k, v, out.view(r, hlh, hn), z, dout.view(r, hlh, hn), dq, dk, dv, zd, graph.rowptr, graph.col,
                           graph.etype, graph.t_rowptr, graph.t_row, graph.t_eid, etable if has_tab else None, detab,
                           variant_id, dropout_p, seed, kmax, graph.t_task, graph.t_split, int(graph.kv_slots), ctx.out_drop,
-                          route)
+                          route, *graph.long_rows())
         _ext.count_launches(3)
         if debug.enabled() and dout.data_ptr() == sp.dctx.tensor.data_ptr():
             debug.poison(sp.dctx.tensor)              # d(context) consumed; the next push must overwrite all of it

@@ -62,6 +62,35 @@ def test_edge_attention_hub_rows(variant):
     _run(variant, torch.bfloat16, 1, 16, hub_row=20000, hub_col=3000, n=4500, e=9000)
 
 
+@pytest.mark.parametrize("by_key", [False, True])
+@pytest.mark.parametrize("dtype,hl,hn", [(torch.float32, 3, 8), (torch.bfloat16, 8, 16), (torch.float32, 4, 64), (torch.float16, 5, 128)])
+def test_edge_attention_rows_around_the_work_item_edges(dtype, hl, hn, by_key):
+    """Rows (queries, or keys of the backward pass) of 0 edges up to several reduction windows of 64 slots: one edge below, at
+    and above the length from which a row is cut, whole and ragged last items, rows inside one window, ending at its end and
+    running over several.  Rows wider than a warp (4 x 64 fp32, 5 x 128) take two head chunks.  Bit-equal when repeated."""
+    from budgetformer_b200.graph.attn_graph import AttnGraph
+    gen = torch.Generator().manual_seed(17)
+    lengths = [0, 1, 63, 64, 65, 127, 128, 129, 191, 192, 193, 320, 3000, 4096, 4097, 2, 12289, 130, 9000, 64 * 64 * 3]
+    n = 700
+    long_side = torch.repeat_interleave(torch.arange(len(lengths)), torch.tensor(lengths))
+    other = torch.randint(0, n, (long_side.numel(),), generator=gen)
+    ei = torch.stack([long_side, other] if by_key else [other, long_side])
+    g = AttnGraph.from_edge_index(ei, n).to("cuda")
+    q, k, v = (torch.randn(n, hl, hn, generator=gen).cuda().to(dtype).requires_grad_(True) for _ in range(3))
+    dout = torch.randn(n, hl, hn, generator=gen).cuda().to(dtype)
+    out = edge_attention(q, k, v, g)
+    got = [out] + list(torch.autograd.grad(out, (q, k, v), dout))
+    out2 = edge_attention(q, k, v, g)
+    for a, b in zip(got, [out2] + list(torch.autograd.grad(out2, (q, k, v), dout))):
+        assert torch.equal(a, b)
+    q2, k2, v2 = (t.detach().float().requires_grad_(True) for t in (q, k, v))
+    ref = edge_attention_reference(q2, k2, v2, g)
+    rtol, atol = TOL[dtype]
+    for name, a, b in zip(("out", "dq", "dk", "dv"), got, [ref] + list(torch.autograd.grad(ref, (q2, k2, v2), dout.float()))):
+        scale = max(1.0, float(b.abs().max()))
+        assert float((a.float() - b).abs().max()) <= (atol + rtol) * scale, name
+
+
 @pytest.mark.parametrize("variant,hl,hn", [("plain", 2, 16), ("plain", 1, 16), ("gps", 4, 16), ("exphormer", 2, 32)])
 def test_edge_attention_routed_rows_match_local_rows(variant, hl, hn):
     """Routed stores on one GPU (the "destinations" are local buffers standing in for the peers' mappings): every context
