@@ -77,7 +77,8 @@ typedef struct {
   const void* dout;                 // [n, hl, hn] contiguous
   void *dq, *dk, *dv;               // [n, hl, hn], common row stride ldg (elements; 0 = hl*hn)
   long long ldg;
-  float* zd;                        // [n, hl, 2] fp32 workspace (written by the dQ pass)
+  float* zd;                        // [n, hl, 2] fp32 workspace: 1 / (Z + eps) and <dout, out> of every row
+  float* ds;                        // [E, hl] fp32 workspace: score gradients, from the dK/dV pass to the dQ pass
   const int *t_rowptr, *t_row, *t_eid;  // transposed CSR over keys
   float* detab;                     // zero-filled [2, hl, hn] fp32 or NULL
   bf_long_rows long_rows;           // scratch row: hl*hn floats
@@ -87,7 +88,7 @@ typedef struct {
   const int* kv_split;              // [n_kv_split, 3] int32: key row, first slot, slot count
   int n_kv_split, n_kv_slots;
   float* kv_partial;                // [n_kv_slots, 2*hl*hn] fp32 scratch
-  // Optional workspace for narrow rows (hl*hn elements of 64 bytes or less), used with kv_task: the dQ pass leaves one
+  // Optional workspace for narrow rows (hl*hn elements of 64 bytes or less), used with kv_task: the first kernel leaves one
   // contiguous record [q | dout / (Z + eps)] per (row, head) in qg and D / (Z + eps) in cz, and the dK/dV pass gathers
   // those instead of q, dout and zd separately.
   void* qg;                         // [n, hl, 2, hn] in the operand dtype, or NULL
@@ -266,13 +267,13 @@ size_t bf_graph_transpose_scratch(int n, long long n_edges);
 int bf_graph_transpose(const int* rowptr, const int* col, int n, long long n_edges, int* t_rowptr /* [n+1] */,
                        int* t_row /* [E] */, int* t_eid /* [E] */, void* scratch, size_t scratch_bytes, cudaStream_t st);
 size_t bf_kv_task_scratch(int n);
-// rows with more than min_split (>= chunk) edges become several items of `chunk` edges
+// by_length (optional, [n]): the keys by length of their row, longest first, split keys last
 int bf_kv_task_counts(const int* t_rowptr, int n, int chunk, int min_split, int* item_first /* [n+1] */,
-                      int* slot_first /* [n+1] */, int* split_first /* [n+1] */, void* scratch, size_t scratch_bytes,
-                      cudaStream_t st);
-// singles == 0: only the items of split rows are written ([slots, 4])
-int bf_kv_task_fill(const int* t_rowptr, const int* item_first, const int* slot_first, const int* split_first, int n,
-                    int chunk, int singles, int* tasks /* [T, 4] */, int* splits /* [S, 3] */, cudaStream_t st);
+                      int* slot_first /* [n+1] */, int* split_first /* [n+1] */, int* by_length, void* scratch,
+                      size_t scratch_bytes, cudaStream_t st);
+int bf_kv_task_fill(const int* t_rowptr, const int* item_first, const int* slot_first, const int* split_first,
+                    const int* by_length, int n, int chunk, int n_slots, int n_split, int* tasks /* [T, 4] */,
+                    int* splits /* [S, 3] */, cudaStream_t st);
 
 // ---- row kernels (norm_fused.cu) -----------------------------------------------------------------
 int bf_layernorm_fwd(const void* x, long long ldx, const float* gamma, const float* beta, void* y, long long ldy,

@@ -39,18 +39,20 @@ void check_qkv(const Tensor& t, const char* name) {
 const int* iptr(const Tensor& t) { return t.data_ptr<int>(); }
 
 // Work items of the CSR rows with more than min_split edges: items of `chunk` edges, split rows, and with `singles` one item
-// for every other row behind them.  The totals size the outputs: one host read.
+// for every other row behind them, longest first.  The totals size the outputs: one host read.
 struct RowTasks {
   Tensor tasks, splits, sizes;       // [T, 4], [S, 3], int64 [3] on the host = items, slots, split rows
 };
 RowTasks row_tasks(const Tensor& rowptr, int64_t n, int64_t chunk, int64_t min_split, bool singles, cudaStream_t st) {
   auto iopt = rowptr.options();
   Tensor firsts = torch::empty({3, n + 1}, iopt);
+  Tensor by_length = singles ? torch::empty({n}, iopt) : Tensor();
+  int* by = singles ? by_length.data_ptr<int>() : nullptr;
   {
     const size_t bytes = bf_kv_task_scratch((int)n);
     Tensor scratch = torch::empty({(int64_t)bytes}, iopt.dtype(torch::kUInt8));
     check_cuda(bf_kv_task_counts(rowptr.data_ptr<int>(), (int)n, (int)chunk, (int)min_split, firsts[0].data_ptr<int>(),
-                                 firsts[1].data_ptr<int>(), firsts[2].data_ptr<int>(), scratch.data_ptr(), bytes, st),
+                                 firsts[1].data_ptr<int>(), firsts[2].data_ptr<int>(), by, scratch.data_ptr(), bytes, st),
                "kv_task_counts");
   }
   RowTasks r;
@@ -60,8 +62,8 @@ RowTasks row_tasks(const Tensor& rowptr, int64_t n, int64_t chunk, int64_t min_s
   r.splits = torch::empty({n_splits, 3}, iopt);
   if (n_items > 0)
     check_cuda(bf_kv_task_fill(rowptr.data_ptr<int>(), firsts[0].data_ptr<int>(), firsts[1].data_ptr<int>(),
-                               firsts[2].data_ptr<int>(), (int)n, (int)chunk, singles ? 1 : 0, r.tasks.data_ptr<int>(),
-                               r.splits.data_ptr<int>(), st), "kv_task_fill");
+                               firsts[2].data_ptr<int>(), by, (int)n, (int)chunk, (int)r.sizes[1].item<int64_t>(), (int)n_splits,
+                               r.tasks.data_ptr<int>(), r.splits.data_ptr<int>(), st), "kv_task_fill");
   return r;
 }
 
@@ -171,6 +173,8 @@ void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor do
   LongRows lr = take_long_rows(rowptr, known_max_degree, long_task, long_split, (size_t)w);
   b.long_rows = lr.c;
   Tensor partial, qg, cz;
+  Tensor ds = torch::empty({std::max<int64_t>(col.numel(), 1), (int64_t)p.hl}, q.options().dtype(torch::kFloat));
+  b.ds = ds.data_ptr<float>();
   if (w * q.element_size() <= 64) {
     // narrow rows: one packed record per (query, head) for the dK/dV pass (see bf_attn_bwd_params)
     qg = torch::empty({q.size(0), (int64_t)p.hl, 2, (int64_t)p.hn}, q.options());

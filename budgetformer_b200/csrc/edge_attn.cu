@@ -64,31 +64,72 @@ template <> __device__ __forceinline__ void store_vec<float>(float* p, const flo
   *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
 }
 
-// A gathered row slice kept packed (one 16-byte register quad) and widened element by element where it is used:
-// the dQ pass holds several gathered slices at once, and packed they cost half the registers (four resident
-// blocks per SM instead of three).
-template <typename T> struct Raw;
-template <> struct Raw<__nv_bfloat16> {
-  uint4 u;
-  __device__ __forceinline__ void load(const __nv_bfloat16* p) { u = *reinterpret_cast<const uint4*>(p); }
-  __device__ __forceinline__ float get(int i) const {
-    const uint32_t w = (i >> 1) == 0 ? u.x : (i >> 1) == 1 ? u.y : (i >> 1) == 2 ? u.z : u.w;
-    return (i & 1) ? __uint_as_float(w & 0xFFFF0000u) : __uint_as_float(w << 16);
-  }
-};
-template <> struct Raw<__half> {
-  uint4 u;
-  __device__ __forceinline__ void load(const __half* p) { u = *reinterpret_cast<const uint4*>(p); }
-  __device__ __forceinline__ float get(int i) const {
-    const uint32_t w = (i >> 1) == 0 ? u.x : (i >> 1) == 1 ? u.y : (i >> 1) == 2 ? u.z : u.w;
-    return __half2float(__ushort_as_half((unsigned short)((i & 1) ? (w >> 16) : (w & 0xFFFFu))));
-  }
-};
-template <> struct Raw<float> {
-  float4 f;
-  __device__ __forceinline__ void load(const float* p) { f = *reinterpret_cast<const float4*>(p); }
-  __device__ __forceinline__ float get(int i) const { return i == 0 ? f.x : i == 1 ? f.y : i == 2 ? f.z : f.w; }
-};
+// Pairs of fp32 values in one 64-bit register: sm_100a multiplies and adds them two at a time (fma.rn.f32x2), each half rounded
+// like a plain fp32 fma.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// One 16-byte slice of a row widened to fp32 pairs.
+template <typename T> __device__ __forceinline__ void widen(const uint4& u, f2* p);
+template <> __device__ __forceinline__ void widen<__nv_bfloat16>(const uint4& u, f2* p) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) p[i] = pack2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xFFFF0000u));
+}
+template <> __device__ __forceinline__ void widen<__half>(const uint4& u, f2* p) {
+  const __half2* h = reinterpret_cast<const __half2*>(&u);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { const float2 t = __half22float2(h[i]); p[i] = pack2(t.x, t.y); }
+}
+template <> __device__ __forceinline__ void widen<float>(const uint4& u, f2* p) {
+  p[0] = pack2(__uint_as_float(u.x), __uint_as_float(u.y));
+  p[1] = pack2(__uint_as_float(u.z), __uint_as_float(u.w));
+}
+template <int NP> __device__ __forceinline__ float dot2(const f2* a, const f2* b) {
+  f2 t = mul2(a[0], b[0]);
+#pragma unroll
+  for (int i = 1; i < NP; ++i) t = fma2(a[i], b[i], t);
+  const float2 r = unpack2(t);
+  return r.x + r.y;
+}
+template <typename T, int NP> __device__ __forceinline__ void store_pairs(T* dst, const f2* p) {
+  float f[2 * NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) { const float2 t = unpack2(p[i]); f[2 * i] = t.x; f[2 * i + 1] = t.y; }
+  store_vec<T>(dst, f);
+}
+
+// Asynchronous copies into shared memory (both addresses a multiple of the size).  Every lane copies the bytes that it alone
+// reads back, so waiting for its own groups is enough: no barrier.
+template <int BYTES> __device__ __forceinline__ void copy_async(void* dst, const void* src) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  // .ca: through L1.  A lane's two slices share a 32-byte sector, which L2 would otherwise deliver twice, and rows that
+  // everyone gathers (the virtual node, hubs) would queue at one L2 slice.
+  if constexpr (BYTES == 16) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else if constexpr (BYTES == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 template <typename T> __device__ __forceinline__ T from_float(float x);
 template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
@@ -248,50 +289,221 @@ __device__ __forceinline__ void load_q_scaled(const AttnArgs& a, int row, int he
   }
 }
 
-template <typename T, int HN>
-__global__ void __launch_bounds__(256) edge_attn_fwd_kernel(AttnArgs a) {
-  constexpr int VN = Vec<T>::N;
-  constexpr int LPH = HN / VN;
-  const Geo g = make_geo<T, HN>(a.hl);
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int tpw = 32 / g.tl;
-  const long long task = (long long)warp * tpw + lane / g.tl;
-  const int lt = lane % g.tl;
-  const long long n_task = (long long)a.n * g.n_hc;
-  const bool live = task < n_task;
-  const int row = live ? (int)(task / g.n_hc) : 0;
-  const int hc = live ? (int)(task % g.n_hc) : 0;
-  const int head = hc * g.hpt + lt / LPH;
-  const bool head_ok = live && head < a.hl;
-  const int hsafe = head_ok ? head : 0;
-  const int off = hsafe * HN + (lt % LPH) * VN;
-  int beg = 0, end = 0;
-  if (head_ok) { beg = a.rowptr[row]; end = a.rowptr[row + 1]; }
-  // long rows have kernels of their own when the caller listed them; without a list they are walked here (slow, complete)
-  const bool hub = a.long_row > 0 && (end - beg) > a.long_row;
-  if (hub) end = beg;
-  float qs0[VN], qs1[VN], acc[VN];
-  float zsum = 0.f;
+// ---------------------------------------------------------------------------------------------
+// Streams.  A warp holds 32 / TL lane groups of TL lanes; each group owns one segment (a query row, or a key work item) at a
+// time and `per` of them in all.  The groups of a warp step together: segment r of every group starts at the same step and
+// lasts as long as the longest of them, so all control flow is uniform over the warp.  The rows that the edges name are copied
+// into a shared-memory ring kRing - 1 steps ahead of the arithmetic, across segment ends: a short segment costs no latency of
+// its own, and the gathers in flight take no registers.  A lane holds 32 bytes of a row where the head is wide enough, which
+// halves the scalar work per edge (score, exponential, cursor) against 16 bytes; the arithmetic runs in fp32 pairs.
+// Without this (two 16-byte gathers a step in registers, one row per lane group) issue slots and latency, not memory, bounded
+// the kernels: DRAM stood at 35-42 %.
+// ---------------------------------------------------------------------------------------------
+constexpr int kRing = 4;
+constexpr int kStreamThreads = 128;
+constexpr unsigned kFull = 0xffffffffu;
+
+// elements of a row that one lane holds: 32 bytes, or a whole narrower head
+template <typename T, int HN> constexpr int wide_elems() { return HN < 32 / (int)sizeof(T) ? HN : 32 / (int)sizeof(T); }
+
+// 2^ltl lanes per group, blockIdx.y = head chunk
+struct StreamGeo {
+  int ltl;
+  int per;                     // segments per lane group
+};
+
+// One lane's part of a row in the ring: VN elements as 16-byte slices, slice-major so that a warp's accesses do not collide.
+template <typename T, int VN> struct Slices {
+  static constexpr int N = VN * (int)sizeof(T) / 16;
+  static constexpr int PP = 8 / (int)sizeof(T);             // pairs per slice
+  static __device__ __forceinline__ void copy(uint4 (*dst)[kStreamThreads], int tid, const char* src) {
 #pragma unroll
-  for (int i = 0; i < VN; ++i) acc[i] = 0.f;
-  load_q_scaled<T, HN>(a, row, hsafe, off, qs0, qs1);
-  const unsigned hm = head_mask<LPH>();
-  for (int e = beg; e < end; e += 2) fwd_pair<T, HN>(a, hsafe, off, e, e + 1, e + 1 < end, hm, qs0, qs1, acc, zsum);
-  if (head_ok && !hub) {
-    float inv = 1.f / (zsum + kEps);
-    if (a.variant == 1) inv *= a.inv_keep;
-    float o[VN];
-#pragma unroll
-    for (int i = 0; i < VN; ++i) o[i] = acc[i] * inv;
-    if (a.out_thresh) {
-#pragma unroll
-      for (int i = 0; i < VN; ++i) o[i] = keep_out(a, row, off + i) ? o[i] * a.out_inv_keep : 0.f;
-    }
-    store_vec<T>(static_cast<T*>(a.out) + (long long)row * a.hl * HN + off, o);
-    if (a.route_out.n_dest) store_vec<T>(routed<T>(a.route_out, row, off), o);
-    if ((lt % LPH) == 0) a.z[(long long)row * a.hl + head] = zsum;
+    for (int i = 0; i < N; ++i) copy_async<16>(&dst[i][tid], src + 16 * i);
   }
+  static __device__ __forceinline__ void read(const uint4 (*src)[kStreamThreads], int tid, f2* p) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) widen<T>(src[i][tid], p + PP * i);
+  }
+  static __device__ __forceinline__ void load(const T* src, uint4* u) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) u[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
+  }
+  static __device__ __forceinline__ void spread(const uint4* u, f2* p) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) widen<T>(u[i], p + PP * i);
+  }
+  static __device__ __forceinline__ void store(T* dst, const f2* p) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) store_pairs<T, PP>(dst + 16 / (int)sizeof(T) * i, p + PP * i);
+  }
+};
+
+// the segments of a lane group that are rows of a CSR: row(r) = base + r * stride, long rows and rows past the end are empty
+struct Rows {
+  long long base;
+  int stride, n;
+  bool on;
+  __device__ __forceinline__ bool bounds(const AttnArgs& a, int r, int& beg, int& len) const {
+    beg = len = 0;
+    const long long row = base + (long long)r * stride;
+    if (!on || row >= n) return false;
+    beg = __ldg(a.rowptr + row);
+    len = __ldg(a.rowptr + row + 1) - beg;
+    if (a.long_row > 0 && len > a.long_row) { len = 0; return false; }
+    return true;
+  }
+};
+
+// every segment takes at least one step, so that the ring never runs more than kRing segments ahead
+__device__ __forceinline__ int steps_of(int len) { return max(1, (int)__reduce_max_sync(kFull, (unsigned)len)); }
+
+// The fetching side of a stream over rows, one warp-uniform step at a time: edge i of segment r, its key (and type).  The bounds
+// are read two segments ahead and the first key of a segment one segment ahead (the keys behind it mostly share its sector):
+// a chain of row pointer, key, row would otherwise stall every segment for two trips to memory.
+template <bool TYPED> struct RowFetch {
+  int r, i, m, beg, len, beg1, len1, beg2, len2;
+  int key, key1, type, type1;
+  __device__ __forceinline__ void start(const AttnArgs& a, const Rows& rows, int n_seg) {
+    r = i = 0;
+    rows.bounds(a, 0, beg, len);
+    beg1 = len1 = beg2 = len2 = 0;
+    if (1 < n_seg) rows.bounds(a, 1, beg1, len1);
+    if (2 < n_seg) rows.bounds(a, 2, beg2, len2);
+    m = steps_of(len);
+    key = key1 = type = type1 = 0;
+    if (len > 0) { key = __ldg(a.col + beg); if (TYPED) type = a.etype[beg]; }
+    if (len1 > 0) { key1 = __ldg(a.col + beg1); if (TYPED) type1 = a.etype[beg1]; }
+  }
+  __device__ __forceinline__ bool has() const { return i < len; }
+  __device__ __forceinline__ int edge() const { return beg + i; }
+  __device__ __forceinline__ void advance(const AttnArgs& a, const Rows& rows, int n_seg) {
+    if (r >= n_seg) return;
+    if (++i == m) {
+      i = 0;
+      ++r;
+      beg = beg1; len = len1; key = key1; type = type1;      // empty past the last segment
+      beg1 = beg2; len1 = len2;
+      beg2 = len2 = 0;
+      if (len1 > 0) { key1 = __ldg(a.col + beg1); if (TYPED) type1 = a.etype[beg1]; }
+      if (r + 2 < n_seg) rows.bounds(a, r + 2, beg2, len2);
+      if (r < n_seg) m = steps_of(len);
+    } else if (i < len) {
+      key = __ldg(a.col + beg + i);
+      if (TYPED) type = a.etype[beg + i];
+    }
+  }
+};
+
+template <typename T, int HN, int VAR>
+__global__ void __launch_bounds__(kStreamThreads, 4) edge_attn_fwd_kernel(AttnArgs a, StreamGeo sg) {
+  constexpr int VN = wide_elems<T, HN>(), NP = VN / 2, LPH = HN / VN;
+  using S = Slices<T, VN>;
+  __shared__ uint4 ring[kRing][2][S::N][kStreamThreads];
+  const int tid = threadIdx.x, lane = tid & 31, lt = lane & ((1 << sg.ltl) - 1), groups = 32 >> sg.ltl;
+  const int head = blockIdx.y * ((1 << sg.ltl) / LPH) + lt / LPH;
+  const long long warp0 = ((long long)blockIdx.x * (kStreamThreads / 32) + (tid >> 5)) * groups * sg.per;
+  if (warp0 >= a.n) return;                     // the whole warp
+  const int n_seg = (int)min((long long)sg.per, (a.n - warp0 + groups - 1) / groups);
+  const Rows rows{warp0 + (lane >> sg.ltl), groups, a.n, head < a.hl};
+  const int off = (rows.on ? head * HN : 0) + (lt % LPH) * VN;
+  const char* kb = reinterpret_cast<const char*>(static_cast<const T*>(a.k) + off);
+  const char* vb = reinterpret_cast<const char*>(static_cast<const T*>(a.v) + off);
+  const T* qb = static_cast<const T*>(a.q) + off;
+  const unsigned long long skb = (unsigned long long)a.ldk * sizeof(T), svb = (unsigned long long)a.ldv * sizeof(T);
+
+  RowFetch<VAR == 2> f;
+  f.start(a, rows, n_seg);
+  unsigned types = 0;                           // edge type of every ring slot
+  auto issue = [&](int slot) {
+    if (f.has()) {
+      S::copy(ring[slot][0], tid, kb + (unsigned)f.key * skb);
+      S::copy(ring[slot][1], tid, vb + (unsigned)f.key * svb);
+      if (VAR == 2) types = (types & ~(1u << slot)) | ((f.type ? 1u : 0u) << slot);
+    }
+    copy_commit();
+    f.advance(a, rows, n_seg);
+  };
+#pragma unroll
+  for (int s = 0; s < kRing - 1; ++s) issue(s);
+
+  int beg, len, nbeg = 0, nlen = 0;
+  bool stored = rows.bounds(a, 0, beg, len), nstored = false;
+  uint4 qn[S::N];
+#pragma unroll
+  for (int i = 0; i < S::N; ++i) qn[i] = make_uint4(0, 0, 0, 0);
+  if (stored) S::load(qb + rows.base * a.ldq, qn);
+  int slot = 0;
+  for (int r = 0; r < n_seg; ++r) {
+    const long long row = rows.base + (long long)r * groups;
+    f2 q0[NP], q1[NP], acc[NP];
+    const float scale = inv_sqrt_hn<HN>();
+    const f2 sc = pack2(scale, scale);
+    S::spread(qn, q0);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) { q0[i] = mul2(q0[i], sc); acc[i] = pack2(0.f, 0.f); }
+    if (VAR == 2) {
+      const float* et = a.etab + off;
+      const int w = a.hl * HN;
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        q1[i] = mul2(q0[i], pack2(__ldg(et + w + 2 * i), __ldg(et + w + 2 * i + 1)));
+        q0[i] = mul2(q0[i], pack2(__ldg(et + 2 * i), __ldg(et + 2 * i + 1)));
+      }
+    }
+    if (r + 1 < n_seg) {
+      nstored = rows.bounds(a, r + 1, nbeg, nlen);
+      if (nstored) S::load(qb + (row + groups) * a.ldq, qn);
+    }
+    const int m = steps_of(len);
+    float zsum = 0.f;
+    for (int i = 0; i < m; ++i) {
+      issue((slot + kRing - 1) & (kRing - 1));
+      copy_wait<kRing - 1>();
+      f2 x[NP];
+      S::read(ring[slot][0], tid, x);
+      float d;
+      if (VAR == 2) {
+        const bool t1 = (types >> slot) & 1u;
+        f2 qq[NP];
+#pragma unroll
+        for (int u = 0; u < NP; ++u) qq[u] = t1 ? q1[u] : q0[u];
+        d = dot2<NP>(qq, x);
+      } else {
+        d = dot2<NP>(q0, x);
+      }
+      d = head_sum<LPH>(d, kFull);
+      float w = __expf(fminf(fmaxf(d, -kClamp), kClamp));
+      S::read(ring[slot][1], tid, x);
+      if (i < len) {                            // a group whose segment is over holds a stale slot: nothing of it is added
+        zsum += w;
+        if (VAR == 1 && a.thresh && !keep_edge(a.seed, (uint32_t)(beg + i), (uint32_t)head, a.thresh)) w = 0.f;
+        const f2 ww = pack2(w, w);
+#pragma unroll
+        for (int u = 0; u < NP; ++u) acc[u] = fma2(ww, x[u], acc[u]);
+      }
+      slot = (slot + 1) & (kRing - 1);
+    }
+    if (stored) {
+      float inv = 1.f / (zsum + kEps);
+      if (VAR == 1) inv *= a.inv_keep;
+      const f2 iv = pack2(inv, inv);
+#pragma unroll
+      for (int i = 0; i < NP; ++i) acc[i] = mul2(acc[i], iv);
+      if (a.out_thresh) {
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+          const float2 t = unpack2(acc[i]);
+          acc[i] = pack2(keep_out(a, (int)row, off + 2 * i) ? t.x * a.out_inv_keep : 0.f,
+                         keep_out(a, (int)row, off + 2 * i + 1) ? t.y * a.out_inv_keep : 0.f);
+        }
+      }
+      S::store(static_cast<T*>(a.out) + row * a.hl * HN + off, acc);
+      if (a.route_out.n_dest) S::store(routed<T>(a.route_out, row, off), acc);
+      if ((lt % LPH) == 0) a.z[row * a.hl + head] = zsum;
+    }
+    beg = nbeg; len = nlen; stored = nstored;
+  }
+  copy_wait<0>();
 }
 
 // Long rows.  One warp per (work item, head chunk): the 32 / TL lane groups take consecutive quarters (halves, ...) of the
@@ -416,6 +628,7 @@ struct BwdArgs {
   void *dq, *dk, *dv;          // [n, Hl, HN], row stride ldg (elements)
   long long ldg;
   float2* zd;                  // [n, Hl]: (1/(Z+eps), D = <dout,out>)
+  float* ds;                   // [E, Hl]: score gradient / sqrt(hn), left by the dK/dV pass for the dQ pass
   const int *t_rowptr, *t_row, *t_eid;
   float* detab;                // [T, Hl, HN] fp32 or null
   // balanced dK/dV work list
@@ -424,7 +637,7 @@ struct BwdArgs {
   const int* kv_split;         // [n_kv_split, 3]: key row, first slot, number of slots
   int n_kv_split, n_kv_slots;
   float* kv_partial;           // [n_kv_slots, 2*Hl*HN] fp32
-  // Packed query records for narrow rows (optional): the dQ pass writes, per (row, head), [q | dout / (Z + eps)] next to
+  // Packed query records for narrow rows (optional): the first kernel writes, per (row, head), [q | dout / (Z + eps)] next to
   // each other plus one float D / (Z + eps); the dK/dV pass then gathers one contiguous record per edge instead of
   // three separate short rows (q, dout, (1/Z, D)), which matters when a row of q is only 32 or 64 bytes.
   void* qg;                    // [n, Hl, 2, HN] in the operand dtype, or null
@@ -442,142 +655,327 @@ __device__ __forceinline__ T* grad_row(const BwdArgs& b, void* local, int col0, 
   return routed<T>(b.route, row, col0);
 }
 
-// Four edges of one query at a time (see dkv_edge4).
-template <typename T, int HN, bool EXPH, int NB>
-__device__ __forceinline__ void dq_edge4(const BwdArgs& b, int e, int end, int head, int off, const float* qs0,
-                                         const float* qs1, const float* qraw, const float* dof, float invz, float dterm,
-                                         float* dq, float* de0, float* de1, unsigned hm) {
-  constexpr int VN = Vec<T>::N;
-  constexpr int LPH = HN / VN;
+// What the dK/dV pass needs of every query: 1 / (Z + eps) and D = <dout, out>, or the packed records of narrow rows.
+template <typename T, int HN>
+__global__ void __launch_bounds__(kStreamThreads) edge_attn_bwd_delta_kernel(BwdArgs b, StreamGeo sg) {
+  constexpr int VN = wide_elems<T, HN>(), NP = VN / 2, LPH = HN / VN;
+  using S = Slices<T, VN>;
   const AttnArgs& a = b.f;
-  const float scale = inv_sqrt_hn<HN>();
-  int j[NB], ty[NB];
-  bool ok[NB];
+  const int tid = threadIdx.x, lt = tid & ((1 << sg.ltl) - 1);
+  const int head = blockIdx.y * ((1 << sg.ltl) / LPH) + lt / LPH;
+  const long long row = ((long long)blockIdx.x * kStreamThreads + tid) >> sg.ltl;
+  const bool on = row < a.n && head < a.hl;
+  const int off = (on ? head * HN : 0) + (lt % LPH) * VN;
+  const long long rs = on ? row : 0, at = rs * a.hl * HN + off, hz = rs * a.hl + (on ? head : 0);
+  uint4 gu[S::N], ou[S::N];
+  S::load(static_cast<const T*>(b.dout) + at, gu);
+  S::load(static_cast<const T*>(a.out) + at, ou);
+  const float invz = 1.f / (__ldg(a.z + hz) + kEps);
+  f2 g[NP], o[NP];
+  S::spread(gu, g);
+  S::spread(ou, o);
+  float dterm = head_sum<LPH>(dot2<NP>(g, o), kFull);
+  if (!on) return;
+  if (a.out_thresh) dterm *= a.out_keep;        // the stored output is the dropped one, rescaled by 1 / (1 - p)
+  if (b.qg != nullptr) {
+    T* rec = static_cast<T*>(b.qg) + hz * 2 * HN + (lt % LPH) * VN;
+    S::load(static_cast<const T*>(a.q) + row * a.ldq + off, ou);
+    S::spread(ou, o);
+    S::store(rec, o);
+    const f2 iz = pack2(invz, invz);
 #pragma unroll
-  for (int u = 0; u < NB; ++u) {
-    ok[u] = e + u < end;
-    j[u] = ok[u] ? __ldg(a.col + e + u) : 0;
-    ty[u] = (EXPH && ok[u]) ? a.etype[e + u] : 0;
-  }
-  if constexpr (!EXPH) {
-    // gathered k | v slices stay packed until used (64 registers: four resident blocks per SM)
-    Raw<T> kr[NB], vr[NB];
-#pragma unroll
-    for (int u = 0; u < NB; ++u) {
-      kr[u].load(static_cast<const T*>(a.k) + (long long)j[u] * a.ldk + off);
-      vr[u].load(static_cast<const T*>(a.v) + (long long)j[u] * a.ldv + off);
-    }
-#pragma unroll
-    for (int u = 0; u < NB; ++u) {
-      float d = 0.f, dv = 0.f;
-#pragma unroll
-      for (int i = 0; i < VN; ++i) { d += qs0[i] * kr[u].get(i); dv += dof[i] * vr[u].get(i); }
-      d = head_sum<LPH>(d, hm);
-      dv = head_sum<LPH>(dv, hm);
-      const bool inr = (d > -kClamp) && (d < kClamp);
-      const float w = ok[u] ? __expf(fminf(fmaxf(d, -kClamp), kClamp)) : 0.f;
-      float mf = 1.f;
-      if (a.variant == 1 && a.thresh) mf = keep_edge(a.seed, (uint32_t)(e + u), (uint32_t)head, a.thresh) ? a.inv_keep : 0.f;
-      else if (a.variant == 1) mf = a.inv_keep;
-      const float dss = inr ? (dv * mf - dterm) * invz * w * scale : 0.f;
-#pragma unroll
-      for (int i = 0; i < VN; ++i) dq[i] += dss * kr[u].get(i);
-    }
-  } else {
-    float kf[NB][VN], vf[NB][VN];
-#pragma unroll
-    for (int u = 0; u < NB; ++u) {
-      load_vec<T>(static_cast<const T*>(a.k) + (long long)j[u] * a.ldk + off, kf[u]);
-      load_vec<T>(static_cast<const T*>(a.v) + (long long)j[u] * a.ldv + off, vf[u]);
-    }
-#pragma unroll
-    for (int u = 0; u < NB; ++u) {
-      float d = 0.f, dv = 0.f;
-#pragma unroll
-      for (int i = 0; i < VN; ++i) { d += (ty[u] ? qs1[i] : qs0[i]) * kf[u][i]; dv += dof[i] * vf[u][i]; }
-      d = head_sum<LPH>(d, hm);
-      dv = head_sum<LPH>(dv, hm);
-      const bool inr = (d > -kClamp) && (d < kClamp);
-      const float w = ok[u] ? __expf(fminf(fmaxf(d, -kClamp), kClamp)) : 0.f;
-      float mf = 1.f;
-      if (a.variant == 1 && a.thresh) mf = keep_edge(a.seed, (uint32_t)(e + u), (uint32_t)head, a.thresh) ? a.inv_keep : 0.f;
-      else if (a.variant == 1) mf = a.inv_keep;
-      const float ds = inr ? (dv * mf - dterm) * invz * w : 0.f;
-      const float* et = a.etab + (ty[u] ? a.hl * HN : 0) + off;
-#pragma unroll
-      for (int i = 0; i < VN; ++i) {
-        dq[i] += ds * scale * kf[u][i] * et[i];
-        const float gg = ds * scale * qraw[i] * kf[u][i];
-        de0[i] += ty[u] ? 0.f : gg;
-        de1[i] += ty[u] ? gg : 0.f;
-      }
-    }
+    for (int i = 0; i < NP; ++i) g[i] = mul2(g[i], iz);
+    S::store(rec + HN, g);
+    if ((lt % LPH) == 0) b.cz[hz] = dterm * invz;
+  } else if ((lt % LPH) == 0) {
+    b.zd[hz] = make_float2(invz, dterm);
   }
 }
 
-template <typename T, int HN, bool EXPH>
-__global__ void __launch_bounds__(256, EXPH ? 3 : 4) edge_attn_bwd_q_kernel(BwdArgs b) {
-  constexpr int VN = Vec<T>::N;
-  constexpr int LPH = HN / VN;
+// dK/dV over the balanced work list, first of the two passes over the edges.  It gathers q, dout and (1/Z, D) of each query and
+// leaves the score gradient of every (edge, head) in `ds` (fp32, at the edge's own position), so that the dQ pass gathers k alone.
+// The list holds the items of split keys (64 edges each), then the rest sorted by length.
+template <typename T, int HN, int VAR, bool PACKED>
+__global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bwd_kv_kernel(BwdArgs b, StreamGeo sg) {
+  constexpr bool EXPH = VAR == 2;
+  constexpr int VN = EXPH ? Vec<T>::N : wide_elems<T, HN>(), NP = VN / 2, LPH = HN / VN;
+  using S = Slices<T, VN>;
   const AttnArgs& a = b.f;
-  extern __shared__ float s_detab[];   // [2, Hl*HN] when exphormer
+  __shared__ uint4 ring[kRing][2][S::N][kStreamThreads];
+  __shared__ float2 ring_zd[kRing][kStreamThreads];
+  __shared__ int ring_eid[kRing][kStreamThreads];
+  const int tid = threadIdx.x, lane = tid & 31, lt = lane & ((1 << sg.ltl) - 1), groups = 32 >> sg.ltl;
+  const int head = blockIdx.y * ((1 << sg.ltl) / LPH) + lt / LPH;
+  const bool on = head < a.hl;
+  // the list is sorted by length: a group takes every `stride`-th item, so that every warp gets its share of the long ones, and
+  // the groups of a warp hold neighbours
+  const long long warp = (long long)blockIdx.x * (kStreamThreads / 32) + (tid >> 5);
+  const long long stride = (long long)gridDim.x * (kStreamThreads / 32) * groups;
+  const long long warp0 = warp * groups, item0 = warp0 + (lane >> sg.ltl);
+  if (warp0 >= b.n_kv_task) return;             // the whole warp
+  const int n_seg = (int)((b.n_kv_task - warp0 + stride - 1) / stride);
+  auto item = [&](int r) {                      // key row, first edge, length, partial slot (-2: none)
+    const long long t = item0 + r * stride;
+    if (!on || t >= b.n_kv_task) return make_int4(0, 0, 0, -2);
+    int4 it = __ldg(b.kv_task + t);
+    it.z -= it.y;
+    return it;
+  };
+  const int hsafe = on ? head : 0, off = hsafe * HN + (lt % LPH) * VN, w_row = a.hl * HN;
+  const char *qb, *gb, *zb;
+  unsigned long long sq, sgr, szd;
+  if (PACKED) {
+    qb = reinterpret_cast<const char*>(static_cast<const T*>(b.qg) + (long long)hsafe * 2 * HN + (lt % LPH) * VN);
+    gb = qb + HN * sizeof(T);
+    sq = sgr = (unsigned long long)w_row * 2 * sizeof(T);
+    zb = reinterpret_cast<const char*>(b.cz + hsafe); szd = (unsigned long long)a.hl * sizeof(float);
+  } else {
+    qb = reinterpret_cast<const char*>(static_cast<const T*>(a.q) + off); sq = (unsigned long long)a.ldq * sizeof(T);
+    gb = reinterpret_cast<const char*>(static_cast<const T*>(b.dout) + off); sgr = (unsigned long long)w_row * sizeof(T);
+    zb = reinterpret_cast<const char*>(b.zd + hsafe); szd = (unsigned long long)a.hl * sizeof(float2);
+  }
+  // fetching side: items two segments ahead, the first query of a segment one segment ahead (see RowFetch)
+  int fr = 0, fi = 0, fbeg, flen, beg1, len1, beg2, len2;
+  auto bounds = [&](int r, int& beg, int& len) { const int4 it = item(r); beg = it.y; len = it.z; };
+  bounds(0, fbeg, flen);
+  bounds(1, beg1, len1);
+  bounds(2, beg2, len2);
+  int fm = steps_of(flen);
+  int i_row = 0, eid_n = 0, i_row1 = 0, eid1 = 0;
+  if (flen > 0) { i_row = __ldg(b.t_row + fbeg); eid_n = __ldg(b.t_eid + fbeg); }
+  if (len1 > 0) { i_row1 = __ldg(b.t_row + beg1); eid1 = __ldg(b.t_eid + beg1); }
+  unsigned types = 0;                           // edge type of every ring slot; the newest is still on its way in `ty`
+  int ty = 0;
+  auto issue = [&](int slot) {
+    if (EXPH) {
+      const int prev = (slot + kRing - 1) & (kRing - 1);
+      types = (types & ~(1u << prev)) | ((ty ? 1u : 0u) << prev);
+    }
+    if (fi < flen) {
+      S::copy(ring[slot][0], tid, qb + (unsigned)i_row * sq);
+      S::copy(ring[slot][1], tid, gb + (unsigned)i_row * sgr);
+      if (PACKED) copy_async<4>(&ring_zd[slot][tid].y, zb + (unsigned)i_row * szd);
+      else copy_async<8>(&ring_zd[slot][tid], zb + (unsigned)i_row * szd);
+      ring_eid[slot][tid] = eid_n;
+      if (EXPH) ty = a.etype[eid_n];
+    }
+    copy_commit();
+    if (fr >= n_seg) return;
+    if (++fi == fm) {
+      fi = 0;
+      ++fr;
+      fbeg = beg1; flen = len1; i_row = i_row1; eid_n = eid1;
+      beg1 = beg2; len1 = len2;
+      if (len1 > 0) { i_row1 = __ldg(b.t_row + beg1); eid1 = __ldg(b.t_eid + beg1); }
+      bounds(fr + 2, beg2, len2);
+      if (fr < n_seg) fm = steps_of(flen);
+    } else if (fi < flen) {
+      i_row = __ldg(b.t_row + fbeg + fi);
+      eid_n = __ldg(b.t_eid + fbeg + fi);
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < kRing - 1; ++s) issue(s);
+
+  const T* kb = static_cast<const T*>(a.k) + off;
+  const T* vb = static_cast<const T*>(a.v) + off;
+  int4 it = item(0), itn = item(1);
+  uint4 kn[S::N], vn[S::N];
+#pragma unroll
+  for (int i = 0; i < S::N; ++i) kn[i] = vn[i] = make_uint4(0, 0, 0, 0);
+  if (it.w != -2) { S::load(kb + (long long)it.x * a.ldk, kn); S::load(vb + (long long)it.x * a.ldv, vn); }
+  int slot = 0;
+  for (int r = 0; r < n_seg; ++r) {
+    f2 k0[NP], k1[NP], vf[NP], dk0[NP], dk1[NP], dv[NP];
+    const float scale = inv_sqrt_hn<HN>();
+    const f2 sc = pack2(scale, scale);
+    S::spread(kn, k0);
+    S::spread(vn, vf);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) { k0[i] = mul2(k0[i], sc); dk0[i] = dv[i] = pack2(0.f, 0.f); }
+    if (EXPH) {
+      const float* et = a.etab + off;
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        dk1[i] = pack2(0.f, 0.f);
+        k1[i] = mul2(k0[i], pack2(__ldg(et + w_row + 2 * i), __ldg(et + w_row + 2 * i + 1)));
+        k0[i] = mul2(k0[i], pack2(__ldg(et + 2 * i), __ldg(et + 2 * i + 1)));
+      }
+    }
+    const int4 cur = it;
+    it = itn;
+    itn = item(r + 2);
+    if (it.w != -2) { S::load(kb + (long long)it.x * a.ldk, kn); S::load(vb + (long long)it.x * a.ldv, vn); }
+    const int m = steps_of(cur.z);
+    for (int i = 0; i < m; ++i) {
+      issue((slot + kRing - 1) & (kRing - 1));
+      copy_wait<kRing - 1>();
+      f2 qf[NP], gf[NP];
+      S::read(ring[slot][0], tid, qf);
+      S::read(ring[slot][1], tid, gf);
+      const int eid = ring_eid[slot][tid];
+      float2 zd = ring_zd[slot][tid];
+      if (PACKED) zd.x = 1.f;
+      const bool t1 = EXPH && ((types >> slot) & 1u);
+      float d;
+      if (EXPH) {
+        f2 kk[NP];
+#pragma unroll
+        for (int u = 0; u < NP; ++u) kk[u] = t1 ? k1[u] : k0[u];
+        d = dot2<NP>(qf, kk);
+      } else {
+        d = dot2<NP>(qf, k0);
+      }
+      d = head_sum<LPH>(d, kFull);
+      const float dotv = head_sum<LPH>(dot2<NP>(gf, vf), kFull);
+      if (i < cur.z) {                          // a group whose item is over holds a stale slot: nothing of it is used
+        const bool inr = (d > -kClamp) && (d < kClamp);
+        const float w = __expf(fminf(fmaxf(d, -kClamp), kClamp)) * zd.x;
+        float mf = 1.f;
+        if (VAR == 1) mf = (a.thresh && !keep_edge(a.seed, (uint32_t)eid, (uint32_t)head, a.thresh)) ? 0.f : a.inv_keep;
+        const float dss = inr ? (dotv * mf - zd.y) * w * scale : 0.f;
+        const float wn = w * mf;
+        if ((lt % LPH) == 0) b.ds[(long long)eid * a.hl + head] = dss;
+        const f2 s2 = pack2(dss, dss), w2 = pack2(wn, wn);
+        if (EXPH) {
+          const f2 z2 = pack2(0.f, 0.f), sa = t1 ? z2 : s2, sb = t1 ? s2 : z2;
+#pragma unroll
+          for (int u = 0; u < NP; ++u) { dk0[u] = fma2(sa, qf[u], dk0[u]); dk1[u] = fma2(sb, qf[u], dk1[u]); }
+        } else {
+#pragma unroll
+          for (int u = 0; u < NP; ++u) dk0[u] = fma2(s2, qf[u], dk0[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < NP; ++u) dv[u] = fma2(w2, gf[u], dv[u]);
+      }
+      slot = (slot + 1) & (kRing - 1);
+    }
+    if (EXPH) {
+      const float* et = a.etab + off;
+#pragma unroll
+      for (int i = 0; i < NP; ++i)
+        dk0[i] = fma2(dk0[i], pack2(__ldg(et + 2 * i), __ldg(et + 2 * i + 1)),
+                      mul2(dk1[i], pack2(__ldg(et + w_row + 2 * i), __ldg(et + w_row + 2 * i + 1))));
+    }
+    if (cur.w == -1) {
+      S::store(grad_row<T>(b, b.dk, b.ck, cur.x) + off, dk0);
+      S::store(grad_row<T>(b, b.dv, b.cv, cur.x) + off, dv);
+    } else if (cur.w >= 0) {
+      float* pp = b.kv_partial + (long long)cur.w * 2 * w_row + off;
+#pragma unroll
+      for (int i = 0; i < NP; i += 2) { store_pairs<float, 2>(pp + 2 * i, dk0 + i); store_pairs<float, 2>(pp + w_row + 2 * i, dv + i); }
+    }
+  }
+  copy_wait<0>();
+}
+
+// dQ, the second pass: dq_i = sum over the row's edges of ds * k_j [* E_type].  With the typed sums S_t = sum of ds * k_j over the
+// edges of type t, dq = S_0 * E_0 + S_1 * E_1 and dE_t += q_i * S_t: one product per edge and a few per row.
+template <typename T, int HN, bool EXPH>
+__global__ void __launch_bounds__(kStreamThreads, EXPH ? 4 : 7) edge_attn_bwd_q_kernel(BwdArgs b, StreamGeo sg) {
+  constexpr int VN = EXPH ? Vec<T>::N : wide_elems<T, HN>(), NP = VN / 2, LPH = HN / VN;
+  using S = Slices<T, VN>;
+  const AttnArgs& a = b.f;
+  __shared__ uint4 ring[kRing][S::N][kStreamThreads];
+  __shared__ float ring_ds[kRing][kStreamThreads];
+  extern __shared__ float s_detab[];            // [2, Hl*HN] when exphormer
   const int w_row = a.hl * HN;
   if (EXPH) {
     for (int i = threadIdx.x; i < 2 * w_row; i += blockDim.x) s_detab[i] = 0.f;
     __syncthreads();
   }
-  const Geo g = make_geo<T, HN>(a.hl);
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int tpw = 32 / g.tl;
-  const long long task = (long long)warp * tpw + lane / g.tl;
-  const int lt = lane % g.tl;
-  const long long n_task = (long long)a.n * g.n_hc;
-  const bool live = task < n_task;
-  const int row = live ? (int)(task / g.n_hc) : 0;
-  const int hc = live ? (int)(task % g.n_hc) : 0;
-  const int head = hc * g.hpt + lt / LPH;
-  const bool head_ok = live && head < a.hl;
-  const int hsafe = head_ok ? head : 0;
-  const int off = hsafe * HN + (lt % LPH) * VN;
-  int beg = 0, end = 0;
-  if (head_ok) { beg = a.rowptr[row]; end = a.rowptr[row + 1]; }
-  const bool hub = a.long_row > 0 && (end - beg) > a.long_row;
-  float qs0[VN], qs1[VN], qraw[VN], dof[VN], of[VN], dq[VN], de0[VN], de1[VN];
-  load_q_scaled<T, HN>(a, row, hsafe, off, qs0, qs1);
-  load_vec<T>(static_cast<const T*>(a.q) + (long long)row * a.ldq + off, qraw);
-  load_vec<T>(static_cast<const T*>(b.dout) + (long long)row * w_row + off, dof);
-  load_vec<T>(static_cast<const T*>(a.out) + (long long)row * w_row + off, of);
-  float dterm = 0.f;
+  const int tid = threadIdx.x, lane = tid & 31, lt = lane & ((1 << sg.ltl) - 1), groups = 32 >> sg.ltl;
+  const int head = blockIdx.y * ((1 << sg.ltl) / LPH) + lt / LPH;
+  const long long warp0 = ((long long)blockIdx.x * (kStreamThreads / 32) + (tid >> 5)) * groups * sg.per;
+  const int n_seg = warp0 >= a.n ? 0 : (int)min((long long)sg.per, (a.n - warp0 + groups - 1) / groups);
+  const Rows rows{warp0 + (lane >> sg.ltl), groups, a.n, head < a.hl};
+  const int hsafe = rows.on ? head : 0, off = hsafe * HN + (lt % LPH) * VN;
+  const char* kb = reinterpret_cast<const char*>(static_cast<const T*>(a.k) + off);
+  const T* qb = static_cast<const T*>(a.q) + off;
+  const unsigned long long skb = (unsigned long long)a.ldk * sizeof(T);
+  const float* dsb = b.ds + hsafe;
+  if (n_seg > 0) {
+    RowFetch<EXPH> f;
+    f.start(a, rows, n_seg);
+    unsigned types = 0;
+    auto issue = [&](int slot) {
+      if (f.has()) {
+        S::copy(ring[slot], tid, kb + (unsigned)f.key * skb);
+        copy_async<4>(&ring_ds[slot][tid], dsb + (long long)f.edge() * a.hl);
+        if (EXPH) types = (types & ~(1u << slot)) | ((f.type ? 1u : 0u) << slot);
+      }
+      copy_commit();
+      f.advance(a, rows, n_seg);
+    };
 #pragma unroll
-  for (int i = 0; i < VN; ++i) { dterm += dof[i] * of[i]; dq[i] = 0.f; de0[i] = 0.f; de1[i] = 0.f; }
-  const unsigned hm = head_mask<LPH>();
-  dterm = head_sum<LPH>(dterm, hm);
-  if (a.out_thresh) dterm *= a.out_keep;        // the stored output is the dropped one, rescaled by 1 / (1 - p)
-  float zsum = head_ok ? a.z[(long long)row * a.hl + hsafe] : 1.f;
-  const float invz = 1.f / (zsum + kEps);
-  if (head_ok && (lt % LPH) == 0) b.zd[(long long)row * a.hl + head] = make_float2(invz, dterm);
-  if (b.qg != nullptr && head_ok) {
-    T* rec = static_cast<T*>(b.qg) + ((long long)row * a.hl + head) * 2 * HN + (lt % LPH) * VN;
-    float gz[VN];
+    for (int s = 0; s < kRing - 1; ++s) issue(s);
+    int beg, len, nbeg = 0, nlen = 0;
+    bool stored = rows.bounds(a, 0, beg, len), nstored = false;
+    f2 de0[NP], de1[NP];
+    uint4 qn[S::N];
 #pragma unroll
-    for (int i = 0; i < VN; ++i) gz[i] = dof[i] * invz;
-    store_vec<T>(rec, qraw);
-    store_vec<T>(rec + HN, gz);
-    if ((lt % LPH) == 0) b.cz[(long long)row * a.hl + head] = dterm * invz;
-  }
-  if (hub) end = beg;
-  for (int e = beg; e < end; e += 2)
-    dq_edge4<T, HN, EXPH, 2>(b, e, end, hsafe, off, qs0, qs1, qraw, dof, invz, dterm, dq, de0, de1, hm);
-  if (head_ok && !hub) store_vec<T>(grad_row<T>(b, b.dq, b.cq, row) + off, dq);
-  if (EXPH) {
-    if (head_ok) {
+    for (int i = 0; i < NP; ++i) de0[i] = de1[i] = pack2(0.f, 0.f);
 #pragma unroll
-      for (int i = 0; i < VN; ++i) {
-        atomicAdd(&s_detab[off + i], de0[i]);
-        atomicAdd(&s_detab[w_row + off + i], de1[i]);
+    for (int i = 0; i < S::N; ++i) qn[i] = make_uint4(0, 0, 0, 0);
+    if (EXPH && stored) S::load(qb + rows.base * a.ldq, qn);
+    int slot = 0;
+    for (int r = 0; r < n_seg; ++r) {
+      const long long row = rows.base + (long long)r * groups;
+      f2 s0[NP], s1[NP], qf[NP];
+      if (EXPH) S::spread(qn, qf);
+#pragma unroll
+      for (int i = 0; i < NP; ++i) { s0[i] = pack2(0.f, 0.f); s1[i] = pack2(0.f, 0.f); }
+      if (r + 1 < n_seg) {
+        nstored = rows.bounds(a, r + 1, nbeg, nlen);
+        if (EXPH && nstored) S::load(qb + (row + groups) * a.ldq, qn);
+      }
+      const int m = steps_of(len);
+      for (int i = 0; i < m; ++i) {
+        issue((slot + kRing - 1) & (kRing - 1));
+        copy_wait<kRing - 1>();
+        if (i < len) {
+          f2 kf[NP];
+          S::read(ring[slot], tid, kf);
+          const float dss = ring_ds[slot][tid];
+          const f2 d2 = pack2(dss, dss);
+          if (EXPH) {
+            const bool t1 = (types >> slot) & 1u;
+            const f2 z2 = pack2(0.f, 0.f), sa = t1 ? z2 : d2, sb = t1 ? d2 : z2;
+#pragma unroll
+            for (int u = 0; u < NP; ++u) { s0[u] = fma2(sa, kf[u], s0[u]); s1[u] = fma2(sb, kf[u], s1[u]); }
+          } else {
+#pragma unroll
+            for (int u = 0; u < NP; ++u) s0[u] = fma2(d2, kf[u], s0[u]);
+          }
+        }
+        slot = (slot + 1) & (kRing - 1);
+      }
+      if (stored) {
+        if (EXPH) {
+          const float* et = a.etab + off;
+#pragma unroll
+          for (int i = 0; i < NP; ++i) {
+            de0[i] = fma2(qf[i], s0[i], de0[i]);
+            de1[i] = fma2(qf[i], s1[i], de1[i]);
+            s0[i] = fma2(s0[i], pack2(__ldg(et + 2 * i), __ldg(et + 2 * i + 1)),
+                         mul2(s1[i], pack2(__ldg(et + w_row + 2 * i), __ldg(et + w_row + 2 * i + 1))));
+          }
+        }
+        S::store(grad_row<T>(b, b.dq, b.cq, row) + off, s0);
+      }
+      beg = nbeg; len = nlen; stored = nstored;
+    }
+    copy_wait<0>();
+    if (EXPH && rows.on) {
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        const float2 x = unpack2(de0[i]), y = unpack2(de1[i]);
+        atomicAdd(&s_detab[off + 2 * i], x.x); atomicAdd(&s_detab[off + 2 * i + 1], x.y);
+        atomicAdd(&s_detab[w_row + off + 2 * i], y.x); atomicAdd(&s_detab[w_row + off + 2 * i + 1], y.y);
       }
     }
+  }
+  if (EXPH) {
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * w_row; i += blockDim.x)
       if (s_detab[i] != 0.f) atomicAdd(b.detab + i, s_detab[i]);
@@ -586,9 +984,8 @@ __global__ void __launch_bounds__(256, EXPH ? 3 : 4) edge_attn_bwd_q_kernel(BwdA
 
 // Long rows of the dQ pass: work items as in edge_attn_fwd_long_kernel, partial dQ rows to the scratch.
 template <typename T, int HN, bool EXPH>
-__global__ void __launch_bounds__(256, EXPH ? 2 : 3) edge_attn_bwd_q_long_kernel(BwdArgs b) {
-  constexpr int VN = Vec<T>::N;
-  constexpr int LPH = HN / VN;
+__global__ void __launch_bounds__(256, EXPH ? 3 : 4) edge_attn_bwd_q_long_kernel(BwdArgs b) {
+  constexpr int VN = Vec<T>::N, NP = VN / 2, LPH = HN / VN, NB = 4;
   const AttnArgs& a = b.f;
   const Geo g = make_geo<T, HN>(a.hl);
   const int w_row = a.hl * HN;
@@ -602,146 +999,65 @@ __global__ void __launch_bounds__(256, EXPH ? 2 : 3) edge_attn_bwd_q_long_kernel
   const int hsafe = head_ok ? head : 0;
   const int off = hsafe * HN + (lt % LPH) * VN;
   const int4 it = __ldg(a.long_task + item);
-  const int row = it.x;
   const int per = (it.z - it.y + tpw - 1) / tpw;
   const int beg = it.y + sub * per, end = min(it.z, beg + per);
-  float qs0[VN], qs1[VN], qraw[VN], dof[VN], of[VN], dq[VN], de0[VN], de1[VN];
-  load_q_scaled<T, HN>(a, row, hsafe, off, qs0, qs1);
-  load_vec<T>(static_cast<const T*>(a.q) + (long long)row * a.ldq + off, qraw);
-  load_vec<T>(static_cast<const T*>(b.dout) + (long long)row * w_row + off, dof);
-  load_vec<T>(static_cast<const T*>(a.out) + (long long)row * w_row + off, of);
-  float dterm = 0.f;
+  f2 s0[NP], s1[NP];
 #pragma unroll
-  for (int i = 0; i < VN; ++i) { dterm += dof[i] * of[i]; dq[i] = 0.f; de0[i] = 0.f; de1[i] = 0.f; }
-  const unsigned hm = head_mask<LPH>();
-  dterm = head_sum<LPH>(dterm, hm);
-  if (a.out_thresh) dterm *= a.out_keep;
-  const float invz = 1.f / (a.z[(long long)row * a.hl + hsafe] + kEps);
-  for (int e = beg; e < end; e += 2)
-    dq_edge4<T, HN, EXPH, 2>(b, e, end, hsafe, off, qs0, qs1, qraw, dof, invz, dterm, dq, de0, de1, hm);
-  __syncwarp();
+  for (int i = 0; i < NP; ++i) { s0[i] = pack2(0.f, 0.f); s1[i] = pack2(0.f, 0.f); }
+  for (int e = beg; e < end; e += NB) {
+    uint4 kr[NB];
+    float ds[NB];
+    bool t1[NB];
 #pragma unroll
-  for (int i = 0; i < VN; ++i) dq[i] = group_total(dq[i], g.tl);
-  if (EXPH) {
+    for (int u = 0; u < NB; ++u) {
+      const bool ok = e + u < end;
+      const int j = ok ? __ldg(a.col + e + u) : 0;
+      kr[u] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(a.k) + (long long)j * a.ldk + off));
+      ds[u] = ok ? __ldg(b.ds + (long long)(e + u) * a.hl + hsafe) : 0.f;
+      t1[u] = EXPH && ok && a.etype[e + u] != 0;
+    }
 #pragma unroll
-    for (int i = 0; i < VN; ++i) { de0[i] = group_total(de0[i], g.tl); de1[i] = group_total(de1[i], g.tl); }
-  }
-  if (sub == 0 && head_ok) {
-    float* pp = a.long_partial + (long long)it.w * w_row;
+    for (int u = 0; u < NB; ++u) {
+      // an absent edge reads key 0 with weight 0: nothing may be added from it, not even 0 * inf
+      if (e + u >= end) break;
+      f2 kf[NP];
+      widen<T>(kr[u], kf);
+      const f2 z2 = pack2(0.f, 0.f), d2 = pack2(ds[u], ds[u]);
+      const f2 sa = t1[u] ? z2 : d2;
 #pragma unroll
-    for (int i = 0; i < VN; i += 4) *reinterpret_cast<float4*>(pp + off + i) = make_float4(dq[i], dq[i + 1], dq[i + 2], dq[i + 3]);
-    if (EXPH) {
+      for (int i = 0; i < NP; ++i) s0[i] = fma2(sa, kf[i], s0[i]);
+      if (EXPH) {
+        const f2 sb = t1[u] ? d2 : z2;
 #pragma unroll
-      for (int i = 0; i < VN; ++i) {
-        atomicAdd(b.detab + off + i, de0[i]);
-        atomicAdd(b.detab + w_row + off + i, de1[i]);
+        for (int i = 0; i < NP; ++i) s1[i] = fma2(sb, kf[i], s1[i]);
       }
     }
   }
-}
-
-// Four transposed edges at a time: all index and row loads are issued before any arithmetic so that a lane group
-// keeps 8 independent 16-byte gathers in flight (the pass is bound by gather latency, not by math).
-template <typename T, int HN, bool EXPH, int NB, bool PACKED>
-__device__ __forceinline__ void dkv_edge4(const BwdArgs& b, int te, int end, int head, int off, const Raw<T>& kf,
-                                          const Raw<T>& vf, float* dk, float* dv, unsigned hm) {
-  constexpr int VN = Vec<T>::N;
-  constexpr int LPH = HN / VN;
-  const AttnArgs& a = b.f;
-  const float scale = inv_sqrt_hn<HN>();
-  const int w_row = a.hl * HN;
-  int i_row[NB], eid[NB];
-  bool ok[NB];
+  __syncwarp();
+  float x0[VN], x1[VN];
 #pragma unroll
-  for (int u = 0; u < NB; ++u) {
-    ok[u] = te + u < end;
-    i_row[u] = ok[u] ? __ldg(b.t_row + te + u) : 0;
-    eid[u] = ok[u] ? __ldg(b.t_eid + te + u) : 0;
-  }
-  Raw<T> qr[NB], dr[NB];                      // gathered slices stay packed until used
-  float2 zd[NB];
-  int ty[NB];
-#pragma unroll
-  for (int u = 0; u < NB; ++u) {
-    if constexpr (PACKED) {
-      // one contiguous record per (query, head): q, then dout already divided by the normaliser; zd = (1, D / (Z + eps))
-      const T* rec = static_cast<const T*>(b.qg) + ((long long)i_row[u] * a.hl + head) * 2 * HN + (off - head * HN);
-      qr[u].load(rec);
-      dr[u].load(rec + HN);
-      zd[u] = make_float2(1.f, __ldg(b.cz + (long long)i_row[u] * a.hl + head));
-    } else {
-      qr[u].load(static_cast<const T*>(a.q) + (long long)i_row[u] * a.ldq + off);
-      dr[u].load(static_cast<const T*>(b.dout) + (long long)i_row[u] * w_row + off);
-      zd[u] = __ldg(b.zd + (long long)i_row[u] * a.hl + head);
-    }
-    ty[u] = (EXPH && ok[u]) ? a.etype[eid[u]] : 0;
-  }
-#pragma unroll
-  for (int u = 0; u < NB; ++u) {
-    float et[VN];
-#pragma unroll
-    for (int i = 0; i < VN; ++i) et[i] = EXPH ? a.etab[(ty[u] ? w_row : 0) + off + i] : 1.f;
-    float d = 0.f, dotv = 0.f;
-#pragma unroll
-    for (int i = 0; i < VN; ++i) { d += qr[u].get(i) * kf.get(i) * et[i]; dotv += dr[u].get(i) * vf.get(i); }
-    d = head_sum<LPH>(d, hm) * scale;
-    dotv = head_sum<LPH>(dotv, hm);
-    const bool inr = (d > -kClamp) && (d < kClamp);
-    const float w = ok[u] ? __expf(fminf(fmaxf(d, -kClamp), kClamp)) : 0.f;
-    float mf = 1.f;
-    if (a.variant == 1 && a.thresh) mf = keep_edge(a.seed, (uint32_t)eid[u], (uint32_t)head, a.thresh) ? a.inv_keep : 0.f;
-    else if (a.variant == 1) mf = a.inv_keep;
-    const float ds = inr ? (dotv * mf - zd[u].y) * zd[u].x * w : 0.f;
-    const float wn = w * mf * zd[u].x;
-#pragma unroll
-    const float dss = ds * scale;
-#pragma unroll
-    for (int i = 0; i < VN; ++i) {
-      dk[i] += dss * qr[u].get(i) * et[i];
-      dv[i] += wn * dr[u].get(i);
+  for (int i = 0; i < NP; ++i) {
+    const float2 t = unpack2(s0[i]);
+    x0[2 * i] = group_total(t.x, g.tl); x0[2 * i + 1] = group_total(t.y, g.tl);
+    if (EXPH) {
+      const float2 y = unpack2(s1[i]);
+      x1[2 * i] = group_total(y.x, g.tl); x1[2 * i + 1] = group_total(y.y, g.tl);
     }
   }
-}
-
-// dK/dV over the balanced work list: one lane group per (work item, head chunk).  (Letting two lane groups share an
-// item and split its edges was measured slower: most items are short, and the shared form halves the items in flight.)
-template <typename T, int HN, bool EXPH, int MINB, bool PACKED>
-__global__ void __launch_bounds__(256, MINB) edge_attn_bwd_kv_task_kernel(BwdArgs b) {
-  constexpr int VN = Vec<T>::N;
-  constexpr int LPH = HN / VN;
-  const AttnArgs& a = b.f;
-  const Geo g = make_geo<T, HN>(a.hl);
-  const int w_row = a.hl * HN;
-  const int lane = threadIdx.x & 31;
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int tpw = 32 / g.tl;
-  const long long task = warp * tpw + lane / g.tl;
-  const int lt = lane % g.tl;
-  const long long n_task = (long long)b.n_kv_task * g.n_hc;
-  const bool live = task < n_task;
-  const int item = live ? (int)(task / g.n_hc) : 0;
-  const int hc = live ? (int)(task % g.n_hc) : 0;
-  const int head = hc * g.hpt + lt / LPH;
-  const bool head_ok = live && head < a.hl;
-  if (!head_ok) return;                       // whole head groups leave together; shuffles use head masks
-  const int off = head * HN + (lt % LPH) * VN;
-  const int4 it = __ldg(b.kv_task + item);
-  const int row = it.x, beg = it.y, end = it.z, slot = it.w;
-  Raw<T> kf, vf;                              // this key's k | v slice stays packed for the whole task
-  float dk[VN], dv[VN];
-  kf.load(static_cast<const T*>(a.k) + (long long)row * a.ldk + off);
-  vf.load(static_cast<const T*>(a.v) + (long long)row * a.ldv + off);
+  if (sub == 0 && head_ok) {
+    float* pp = a.long_partial + (long long)it.w * w_row;
+    if (EXPH) {
+      float qf[VN];
+      load_vec<T>(static_cast<const T*>(a.q) + (long long)it.x * a.ldq + off, qf);
 #pragma unroll
-  for (int i = 0; i < VN; ++i) { dk[i] = 0.f; dv[i] = 0.f; }
-  const unsigned hm = head_mask<LPH>();
-  for (int e = beg; e < end; e += 2) dkv_edge4<T, HN, EXPH, 2, PACKED>(b, e, end, head, off, kf, vf, dk, dv, hm);
-  if (slot < 0) {
-    store_vec<T>(grad_row<T>(b, b.dk, b.ck, row) + off, dk);
-    store_vec<T>(grad_row<T>(b, b.dv, b.cv, row) + off, dv);
-  } else {
-    float* pp = b.kv_partial + (long long)slot * 2 * w_row;
+      for (int i = 0; i < VN; ++i) {
+        atomicAdd(b.detab + off + i, qf[i] * x0[i]);
+        atomicAdd(b.detab + w_row + off + i, qf[i] * x1[i]);
+        x0[i] = x0[i] * __ldg(a.etab + off + i) + x1[i] * __ldg(a.etab + w_row + off + i);
+      }
+    }
 #pragma unroll
-    for (int i = 0; i < VN; ++i) { pp[off + i] = dk[i]; pp[w_row + off + i] = dv[i]; }
+    for (int i = 0; i < VN; i += 4) *reinterpret_cast<float4*>(pp + off + i) = make_float4(x0[i], x0[i + 1], x0[i + 2], x0[i + 3]);
   }
 }
 
@@ -860,14 +1176,53 @@ void launch_split(const BwdArgs& b, const int4* task, int n_slots, const int* sp
   split_cross_kernel<T, MODE><<<n_split < 148 * 8 ? n_split : 148 * 8, SPLIT_THREADS, smem, st>>>(b, split, n_split, partial, pitch, ncol, w, hn);
 }
 
+// Lanes of a group (VN elements each, whole heads, at most a warp), and how many segments each group takes: as many as leave two
+// full loads of the chip (every SM holding `blocks_per_sm` blocks), at most `most`.
+template <int HN, int VN>
+StreamGeo stream_geo(int hl, long long segments, int blocks_per_sm, int most) {
+  constexpr int lph = HN / VN;
+  StreamGeo s;
+  int tl = lph;
+  while (tl * 2 <= 32 && tl / lph * 2 <= hl) tl *= 2;
+  s.ltl = 0;
+  while ((1 << s.ltl) < tl) ++s.ltl;
+  const int chunks = (hl + tl / lph - 1) / (tl / lph);
+  const long long resident = 148ll * blocks_per_sm * (kStreamThreads >> s.ltl);
+  const long long per = segments * chunks / (2 * resident);
+  s.per = (int)(per < 1 ? 1 : per > most ? most : per);
+  return s;
+}
+template <int HN, int VN>
+dim3 stream_grid(int hl, long long warps, const StreamGeo& s) {
+  const int heads = (1 << s.ltl) / (HN / VN);
+  return dim3((unsigned)((warps + kStreamThreads / 32 - 1) / (kStreamThreads / 32)), (unsigned)((hl + heads - 1) / heads));
+}
+// warps over n segments
+inline long long stream_warps(long long n, const StreamGeo& s, int per) {
+  const long long each = (32ll >> s.ltl) * per;
+  return (n + each - 1) / each;
+}
+
+template <typename T, int HN, int VAR>
+void launch_kv(const BwdArgs& b, cudaStream_t st) {
+  constexpr int VN = VAR == 2 ? Vec<T>::N : wide_elems<T, HN>();
+  const StreamGeo s = stream_geo<HN, VN>(b.f.hl, b.n_kv_task, VAR == 2 ? 4 : 3, 8);
+  const dim3 grid = stream_grid<HN, VN>(b.f.hl, stream_warps(b.n_kv_task, s, s.per), s);
+  if (b.qg) edge_attn_bwd_kv_kernel<T, HN, VAR, true><<<grid, kStreamThreads, 0, st>>>(b, s);
+  else edge_attn_bwd_kv_kernel<T, HN, VAR, false><<<grid, kStreamThreads, 0, st>>>(b, s);
+}
+
 template <typename T, int HN>
 cudaError_t launch_fwd_t(const AttnArgs& a, int chunks_per_hub, cudaStream_t st) {
   const Geo g = make_geo<T, HN>(a.hl);
-  const long long n_task = (long long)a.n * g.n_hc;
-  const int tpw = 32 / g.tl;
-  const long long warps = (n_task + tpw - 1) / tpw;
-  const long long blocks = (warps + 7) / 8;
-  if (blocks > 0) edge_attn_fwd_kernel<T, HN><<<(unsigned)blocks, 256, 0, st>>>(a);
+  if (a.n > 0) {
+    constexpr int VN = wide_elems<T, HN>();
+    const StreamGeo s = stream_geo<HN, VN>(a.hl, a.n, 4, 8);
+    const dim3 grid = stream_grid<HN, VN>(a.hl, stream_warps(a.n, s, s.per), s);
+    if (a.variant == 2) edge_attn_fwd_kernel<T, HN, 2><<<grid, kStreamThreads, 0, st>>>(a, s);
+    else if (a.variant == 1) edge_attn_fwd_kernel<T, HN, 1><<<grid, kStreamThreads, 0, st>>>(a, s);
+    else edge_attn_fwd_kernel<T, HN, 0><<<grid, kStreamThreads, 0, st>>>(a, s);
+  }
   if (a.n_long_task > 0) {
     edge_attn_fwd_long_kernel<T, HN><<<(unsigned)(((long long)a.n_long_task * g.n_hc + 7) / 8), 256, 0, st>>>(a);
     BwdArgs b{};
@@ -886,15 +1241,31 @@ template <typename T, int HN>
 cudaError_t launch_bwd_t(const BwdArgs& b, cudaStream_t st) {
   const AttnArgs& a = b.f;
   const Geo g = make_geo<T, HN>(a.hl);
-  const long long n_task = (long long)a.n * g.n_hc;
-  const int tpw = 32 / g.tl;
-  const long long warps = (n_task + tpw - 1) / tpw;
-  const long long blocks = (warps + 7) / 8;
   const int w_row = a.hl * HN;
-  const size_t smem = a.variant == 2 ? sizeof(float) * 2 * w_row : 0;
-  if (blocks > 0) {
-    if (a.variant == 2) edge_attn_bwd_q_kernel<T, HN, true><<<(unsigned)blocks, 256, smem, st>>>(b);
-    else edge_attn_bwd_q_kernel<T, HN, false><<<(unsigned)blocks, 256, smem, st>>>(b);
+  if (a.n > 0) {
+    constexpr int VN = wide_elems<T, HN>();
+    const StreamGeo s = stream_geo<HN, VN>(a.hl, 0, 1, 1);
+    edge_attn_bwd_delta_kernel<T, HN><<<stream_grid<HN, VN>(a.hl, stream_warps(a.n, s, 1), s), kStreamThreads, 0, st>>>(b, s);
+  }
+  if (b.n_kv_task > 0) {
+    if (a.variant == 2) launch_kv<T, HN, 2>(b, st);
+    else if (a.variant == 1) launch_kv<T, HN, 1>(b, st);
+    else launch_kv<T, HN, 0>(b, st);
+  }
+  // the items of split keys come first in the list, so item i of them is slot i
+  if (b.n_kv_split > 0)
+    launch_split<T, SPLIT_KV>(b, b.kv_task, b.n_kv_slots, b.kv_split, b.n_kv_split, b.kv_partial, 2 * w_row, 2 * w_row, w_row, HN, st);
+  if (a.n > 0) {
+    if (a.variant == 2) {
+      // every block ends in 2 * Hl * HN atomics: longer streams where the rows allow it
+      constexpr int VN = Vec<T>::N;
+      const StreamGeo s = stream_geo<HN, VN>(a.hl, a.n, 4, 32);
+      edge_attn_bwd_q_kernel<T, HN, true><<<stream_grid<HN, VN>(a.hl, stream_warps(a.n, s, s.per), s), kStreamThreads, sizeof(float) * 2 * w_row, st>>>(b, s);
+    } else {
+      constexpr int VN = wide_elems<T, HN>();
+      const StreamGeo s = stream_geo<HN, VN>(a.hl, a.n, 7, 8);
+      edge_attn_bwd_q_kernel<T, HN, false><<<stream_grid<HN, VN>(a.hl, stream_warps(a.n, s, s.per), s), kStreamThreads, 0, st>>>(b, s);
+    }
   }
   if (a.n_long_task > 0) {
     const unsigned lb = (unsigned)(((long long)a.n_long_task * g.n_hc + 7) / 8);
@@ -902,21 +1273,6 @@ cudaError_t launch_bwd_t(const BwdArgs& b, cudaStream_t st) {
     else edge_attn_bwd_q_long_kernel<T, HN, false><<<lb, 256, 0, st>>>(b);
     launch_split<T, SPLIT_DQ>(b, a.long_task, a.n_long_task, a.long_split, a.n_long_split, a.long_partial, w_row, w_row, w_row, HN, st);
   }
-  const long long kv_tasks = (long long)b.n_kv_task * g.n_hc;
-  const long long kv_warps = (kv_tasks + tpw - 1) / tpw;
-  const long long kv_blocks = (kv_warps + 7) / 8;
-  if (kv_blocks > 0) {
-    if (a.variant == 2) {
-      if (b.qg) edge_attn_bwd_kv_task_kernel<T, HN, true, 3, true><<<(unsigned)kv_blocks, 256, 0, st>>>(b);
-      else edge_attn_bwd_kv_task_kernel<T, HN, true, 3, false><<<(unsigned)kv_blocks, 256, 0, st>>>(b);
-    } else {
-      if (b.qg) edge_attn_bwd_kv_task_kernel<T, HN, false, 4, true><<<(unsigned)kv_blocks, 256, 0, st>>>(b);
-      else edge_attn_bwd_kv_task_kernel<T, HN, false, 4, false><<<(unsigned)kv_blocks, 256, 0, st>>>(b);
-    }
-  }
-  // the items of split keys come first in the list, so item i of them is slot i
-  if (b.n_kv_split > 0)
-    launch_split<T, SPLIT_KV>(b, b.kv_task, b.n_kv_slots, b.kv_split, b.n_kv_split, b.kv_partial, 2 * w_row, 2 * w_row, w_row, HN, st);
   return cudaGetLastError();
 }
 
@@ -1012,13 +1368,14 @@ extern "C" int bf_edge_attn_fwd(const bf_attn_params* p, cudaStream_t st) {
 extern "C" int bf_edge_attn_bwd(const bf_attn_params* p, const bf_attn_bwd_params* q, cudaStream_t st) {
   BwdArgs b;
   b.f = to_args(*p);
-  if (b.f.n_hub > 0 || !take_long_rows(&q->long_rows, &b.f) || q->kv_task == nullptr) return (int)cudaErrorInvalidValue;
+  if (b.f.n_hub > 0 || !take_long_rows(&q->long_rows, &b.f) || q->kv_task == nullptr || q->ds == nullptr) return (int)cudaErrorInvalidValue;
   b.dout = q->dout; b.dq = q->dq; b.dk = q->dk; b.dv = q->dv;
   b.ldg = q->ldg > 0 ? q->ldg : (long long)p->hl * p->hn;
   b.zd = reinterpret_cast<float2*>(q->zd);
+  b.ds = q->ds;
   b.t_rowptr = q->t_rowptr; b.t_row = q->t_row; b.t_eid = q->t_eid; b.detab = q->detab;
   b.kv_task = reinterpret_cast<const int4*>(q->kv_task); b.n_kv_task = q->n_kv_task;
-  b.kv_split = q->kv_split; b.n_kv_split = q->n_kv_split; b.n_kv_slots = q->n_kv_slots; b.kv_partial = q->kv_partial;
+  b.kv_split = q->kv_split; b.n_kv_split = q->n_kv_split; b.n_kv_slots = q->n_kv_split > 0 ? q->n_kv_slots : 0; b.kv_partial = q->kv_partial;
   if (b.n_kv_split > 0 && (b.kv_split == nullptr || b.kv_partial == nullptr || b.n_kv_slots <= 0 || b.n_kv_slots > b.n_kv_task))
     return (int)cudaErrorInvalidValue;
   b.qg = (q->qg != nullptr && q->cz != nullptr) ? q->qg : nullptr;

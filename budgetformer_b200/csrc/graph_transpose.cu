@@ -54,7 +54,8 @@ __global__ void gather_rows_kernel(const int* __restrict__ erow, const int* __re
 // items per key (at least one, so that keys without edges still get their zero gradient written) and partial slots; only
 // rows with more than `min_split` edges are cut
 __global__ void task_counts_kernel(const int* __restrict__ t_rowptr, int n, int chunk, int min_split, int* __restrict__ n_items,
-                                   int* __restrict__ n_slots, int* __restrict__ is_split) {
+                                   int* __restrict__ n_slots, int* __restrict__ is_split, int* __restrict__ length_key,
+                                   int* __restrict__ ids) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int deg = t_rowptr[k + 1] - t_rowptr[k];
@@ -62,35 +63,46 @@ __global__ void task_counts_kernel(const int* __restrict__ t_rowptr, int n, int 
   n_items[k] = c;
   n_slots[k] = c > 1 ? c : 0;
   is_split[k] = c > 1 ? 1 : 0;
+  if (length_key != nullptr) {
+    length_key[k] = c > 1 ? min_split + 1 : min_split - deg;
+    ids[k] = k;
+  }
 }
 
-// One warp per key: lane l writes items l, l+32, ... (hub keys own thousands of items).  The list starts with the
-// items of all split keys (full-length items: the long work is scheduled first and runs side by side in a warp),
-// followed by the single item of every other key in key order; an item of a split key sits at its partial-slot index.
+// The list starts with the items of all split keys in key order (full-length items: the long work is scheduled first and runs
+// side by side in a warp); an item of a split key sits at its partial-slot index.  One warp per key: lane l writes items l, l+32,
+// ... (hub keys own thousands of items).  `keys` lists the split keys; without it all n keys are looked through.
 __global__ void task_fill_kernel(const int* __restrict__ t_rowptr, const int* __restrict__ item_first,
-                                 const int* __restrict__ slot_first, const int* __restrict__ split_first, int n,
-                                 int chunk, int singles, int4* __restrict__ tasks, int* __restrict__ splits) {
+                                 const int* __restrict__ slot_first, const int* __restrict__ split_first,
+                                 const int* __restrict__ keys, int n, int chunk, int4* __restrict__ tasks, int* __restrict__ splits) {
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = (int)(gt >> 5), lane = (int)(gt & 31);
-  if (k >= n) return;
-  const int beg = t_rowptr[k], end = t_rowptr[k + 1];
+  const int i = (int)(gt >> 5), lane = (int)(gt & 31);
+  if (i >= n) return;
+  const int k = keys != nullptr ? keys[i] : i;
   const int cnt = item_first[k + 1] - item_first[k];
-  const int s0 = slot_first[k];
-  const int total_slots = slot_first[n];
-  if (cnt == 1) {
-    if (lane == 0 && singles) tasks[total_slots + (k - split_first[k])] = make_int4(k, beg, end, -1);
-    return;
-  }
+  if (cnt <= 1) return;
+  const int beg = t_rowptr[k], end = t_rowptr[k + 1], s0 = slot_first[k];
   for (int c = lane; c < cnt; c += 32) {
     const int b = beg + c * chunk;
     int e = b + chunk;
     if (e > end) e = end;
     tasks[s0 + c] = make_int4(k, b, e, s0 + c);
   }
-  if (lane == 0 && cnt > 1) {
+  if (lane == 0) {
     const int s = split_first[k];
     splits[3 * s] = k; splits[3 * s + 1] = s0; splits[3 * s + 2] = cnt;
   }
+}
+
+// Behind them the single item of every other key, longest first (key order among equals): the lane groups of a warp that work
+// on neighbouring items finish together.  Sorting 2.9 M keys by their 7-bit length is one radix pass; a thread per key instead
+// of a warp writes the list in a tenth of the time.
+__global__ void task_singles_kernel(const int* __restrict__ t_rowptr, const int* __restrict__ keys, int n_single,
+                                    int4* __restrict__ tasks) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_single) return;
+  const int k = keys[i];
+  tasks[i] = make_int4(k, t_rowptr[k], t_rowptr[k + 1], -1);
 }
 
 int bits_for(int n) {
@@ -130,18 +142,23 @@ extern "C" int bf_graph_transpose(const int* rowptr, const int* col, int n, long
   return (int)cudaGetLastError();
 }
 
-// Phase 1 of the work list: per-key counts and their exclusive prefix sums ([n+1] each, last element = total).
+// Phase 1 of the work list: per-key counts and their exclusive prefix sums ([n+1] each, last element = total), and with
+// `by_length` the keys sorted by the length of their row, longest first, split keys behind all others ([n]).
 extern "C" int bf_kv_task_counts(const int* t_rowptr, int n, int chunk, int min_split, int* item_first, int* slot_first,
-                                 int* split_first, void* scratch, size_t scratch_bytes, cudaStream_t st) {
-  // scratch: three int[n] count arrays followed by the scan's temporary storage
+                                 int* split_first, int* by_length, void* scratch, size_t scratch_bytes, cudaStream_t st) {
+  // scratch: six int[n] arrays (three counts; length keys, their sorted copy, ids) followed by the temporary storage of CUB
   int* n_items = static_cast<int*>(scratch);
   int* n_slots = n_items + n;
   int* is_split = n_slots + n;
-  const size_t head = (3 * (size_t)n * sizeof(int) + 255) & ~(size_t)255;
-  void* scan_tmp = static_cast<uint8_t*>(scratch) + head;
-  size_t scan_bytes = scratch_bytes - head;
+  int* key_in = is_split + n;
+  int* key_out = key_in + n;
+  int* ids = key_out + n;
+  const size_t head = (6 * (size_t)n * sizeof(int) + 255) & ~(size_t)255;
+  void* tmp = static_cast<uint8_t*>(scratch) + head;
+  size_t tmp_bytes = scratch_bytes - head;
   if (chunk < 1 || min_split < chunk) return (int)cudaErrorInvalidValue;
-  task_counts_kernel<<<(n + 255) / 256, 256, 0, st>>>(t_rowptr, n, chunk, min_split, n_items, n_slots, is_split);
+  task_counts_kernel<<<(n + 255) / 256, 256, 0, st>>>(t_rowptr, n, chunk, min_split, n_items, n_slots, is_split,
+                                                      by_length != nullptr ? key_in : nullptr, ids);
   cudaError_t e;
   // exclusive prefix sums with the total appended: out[0] = 0, out[1..n] = inclusive sums
   for (int which = 0; which < 3; ++which) {
@@ -149,25 +166,39 @@ extern "C" int bf_kv_task_counts(const int* t_rowptr, int n, int chunk, int min_
     int* out = which == 0 ? item_first : which == 1 ? slot_first : split_first;
     e = cudaMemsetAsync(out, 0, sizeof(int), st);
     if (e != cudaSuccess) return (int)e;
-    e = cub::DeviceScan::InclusiveSum(scan_tmp, scan_bytes, in, out + 1, n, st);
+    size_t bytes = tmp_bytes;
+    e = cub::DeviceScan::InclusiveSum(tmp, bytes, in, out + 1, n, st);
+    if (e != cudaSuccess) return (int)e;
+  }
+  if (by_length != nullptr) {
+    size_t bytes = tmp_bytes;
+    e = cub::DeviceRadixSort::SortPairs(tmp, bytes, key_in, key_out, ids, by_length, n, 0, bits_for(min_split + 2), st);
     if (e != cudaSuccess) return (int)e;
   }
   return (int)cudaGetLastError();
 }
 
 extern "C" size_t bf_kv_task_scratch(int n) {
-  size_t scan_bytes = 0;
+  size_t scan_bytes = 0, sort_bytes = 0;
   cub::DeviceScan::InclusiveSum(nullptr, scan_bytes, (const int*)nullptr, (int*)nullptr, n);
-  return ((3 * (size_t)n * sizeof(int) + 255) & ~(size_t)255) + ((scan_bytes + 255) & ~(size_t)255) + 256;
+  cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (const int*)nullptr, (int*)nullptr, (const int*)nullptr, (int*)nullptr, n);
+  const size_t tmp = scan_bytes > sort_bytes ? scan_bytes : sort_bytes;
+  return ((6 * (size_t)n * sizeof(int) + 255) & ~(size_t)255) + ((tmp + 255) & ~(size_t)255) + 256;
 }
 
-// Phase 2: write the items and the split list (sizes read back by the caller from the prefix sums).
+// Phase 2: write the items and the split list (n_split and n_slots read back by the caller from the prefix sums).  With
+// `by_length` (of phase 1) the keys that are not split get their single items; without it they get none.
 extern "C" int bf_kv_task_fill(const int* t_rowptr, const int* item_first, const int* slot_first, const int* split_first,
-                               int n, int chunk, int singles, int* tasks, int* splits, cudaStream_t st) {
-  const long long threads = (long long)n * 32;
-  const unsigned blocks = (unsigned)((threads + 255) / 256);
-  if (blocks > 0)
-    task_fill_kernel<<<blocks, 256, 0, st>>>(t_rowptr, item_first, slot_first, split_first, n, chunk, singles,
-                                             reinterpret_cast<int4*>(tasks), splits);
+                               const int* by_length, int n, int chunk, int n_slots, int n_split, int* tasks, int* splits,
+                               cudaStream_t st) {
+  int4* out = reinterpret_cast<int4*>(tasks);
+  const int n_single = n - n_split;
+  if (n_split > 0) {
+    const int rows = by_length != nullptr ? n_split : n;
+    task_fill_kernel<<<(unsigned)(((long long)rows * 32 + 255) / 256), 256, 0, st>>>(
+        t_rowptr, item_first, slot_first, split_first, by_length != nullptr ? by_length + n_single : nullptr, rows, chunk, out, splits);
+  }
+  if (by_length != nullptr && n_single > 0)
+    task_singles_kernel<<<(n_single + 255) / 256, 256, 0, st>>>(t_rowptr, by_length, n_single, out + n_slots);
   return (int)cudaGetLastError();
 }

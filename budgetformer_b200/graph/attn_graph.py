@@ -214,8 +214,11 @@ class AttnGraph:
         slot = torch.cumsum(is_split.to(torch.int64), 0) - 1
         slot = torch.where(is_split, slot, torch.full_like(slot, -1))
         tasks = torch.stack([rows, beg, end, slot], 1)
-        # items of split keys first (long work is scheduled first), then one item per remaining key, both in key order
-        tasks = torch.cat([tasks[is_split], tasks[~is_split]], 0)
+        # items of split keys first (long work is scheduled first), in key order; then one item per remaining key, longest first
+        # (the lane groups of a warp finish together), in key order among equals
+        single = tasks[~is_split]
+        single = single[torch.sort(single[:, 2] - single[:, 1], descending=True, stable=True).indices]
+        tasks = torch.cat([tasks[is_split], single], 0)
         self.t_task = tasks.to(torch.int32).contiguous()
         srows = torch.nonzero(split_row).flatten()
         nsl = n_chunks[srows]
