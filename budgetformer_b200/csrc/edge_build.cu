@@ -48,6 +48,38 @@ __device__ __forceinline__ void group_insert(uint64_t& list, int K, bool valid, 
   }
 }
 
+// Keep the WIDTH smallest of the sorted list and one candidate per lane (kInf: none).  A bitonic sort of the candidates and one
+// bitonic merge: the same instructions for every group of the warp, where insertion takes a round per candidate and the groups'
+// rounds follow one another.  With eight lanes that is 10 exchanges; a full warp would need 21, and rows that long mostly carry
+// few candidates that still matter, so the 32-lane kernels insert (group_take).
+template <int WIDTH>
+__device__ __forceinline__ uint64_t exchange(uint64_t v, int j, bool want_min, unsigned gm) {
+  const uint64_t o = __shfl_xor_sync(gm, v, j);
+  return ((o < v) == want_min) ? o : v;
+}
+template <int WIDTH>
+__device__ __forceinline__ void group_merge(uint64_t& list, uint64_t comp, int gl, unsigned gm) {
+#pragma unroll
+  for (int k = 2; k <= WIDTH; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) comp = exchange<WIDTH>(comp, j, ((gl & j) == 0) == ((gl & k) != 0 && k < WIDTH ? false : true), gm);
+  const uint64_t rev = __shfl_sync(gm, comp, WIDTH - 1 - gl, WIDTH);
+  uint64_t v = rev < list ? rev : list;         // the WIDTH smallest of both, bitonic
+#pragma unroll
+  for (int j = WIDTH >> 1; j > 0; j >>= 1) v = exchange<WIDTH>(v, j, (gl & j) == 0, gm);
+  list = v;
+}
+// candidates (valid, comp) of the group's lanes into the list
+template <int WIDTH>
+__device__ __forceinline__ void group_take(uint64_t& list, int K, bool valid, uint64_t comp, int gl, unsigned gm, int lane) {
+  if (WIDTH == 8) {
+    const uint64_t kth = __shfl_sync(gm, list, K - 1, WIDTH);
+    if (group_ballot<WIDTH>(gm, lane, valid && comp < kth) != 0) group_merge<WIDTH>(list, valid ? comp : kInf, gl, gm);
+  } else {
+    group_insert<WIDTH>(list, K, valid, comp, gl, gm, lane);
+  }
+}
+
 struct BuildArgs {
   const int *in_rowptr, *in_src, *out_rowptr, *out_col;
   int n;
@@ -128,7 +160,7 @@ __global__ void __launch_bounds__(256) budget_select_kernel(BuildArgs a) {
           const int e = base + gl;
           const bool valid = e < end;
           const uint32_t s = valid ? (uint32_t)__ldg(a.in_src + e) : 0u;
-          group_insert<WIDTH>(rlist, a.b_real, valid, valid ? bf_edge_composite(s, q, rs) : kInf, gl, gm, lane);
+          group_take<WIDTH>(rlist, a.b_real, valid, valid ? bf_edge_composite(s, q, rs) : kInf, gl, gm, lane);
         }
       }
       r_cnt = min(end - beg, a.b_real);
@@ -139,11 +171,16 @@ __global__ void __launch_bounds__(256) budget_select_kernel(BuildArgs a) {
     if (a.b_rw > 0 && a.walks > 0 && a.walk_len > 0) {
       const int64_t ws = a.seed + BF_RW_SEED_OFFSET;
       int n_cand = 0;
+      // with fewer walks than half the lanes, the candidates of several steps are collected before they are ranked: lane
+      // t * walks + w takes walk w's candidate of step t
+      const int batch = WIDTH == 8 ? max(1, min(a.walk_len, WIDTH / a.walks)) : 1;
       for (int wbase = 0; wbase < a.walks; wbase += WIDTH) {
         const int w = wbase + gl;
         const bool active = w < a.walks;
         const uint64_t walk_id = (uint64_t)v * (uint64_t)a.walks + (uint64_t)w;
-        int cur = (int)v, prev = (int)v;
+        const int slot_step = batch > 1 ? gl / a.walks : 0, slot_lane = batch > 1 ? gl - slot_step * a.walks : gl;
+        uint64_t held = kInf;
+        int cur = (int)v, prev = (int)v, in_batch = 0;
         for (int d = 1; d <= a.walk_len; ++d) {
           bool emit = false;
           if (active) {
@@ -157,7 +194,18 @@ __global__ void __launch_bounds__(256) budget_select_kernel(BuildArgs a) {
             emit = (d == 1) || (cur != prev);
           }
           n_cand += __popc(group_ballot<WIDTH>(gm, lane, emit));
-          group_insert<WIDTH>(wlist, a.b_rw, emit, emit ? bf_edge_composite((uint32_t)cur, q, ws) : kInf, gl, gm, lane);
+          uint64_t comp = emit ? bf_edge_composite((uint32_t)cur, q, ws) : kInf;
+          if (batch > 1) {
+            comp = __shfl_sync(gm, comp, slot_lane, WIDTH);
+            if (slot_step == in_batch) held = comp;
+            if (++in_batch == batch || d == a.walk_len) {
+              group_take<WIDTH>(wlist, a.b_rw, held != kInf, held, gl, gm, lane);
+              held = kInf;
+              in_batch = 0;
+            }
+          } else {
+            group_take<WIDTH>(wlist, a.b_rw, emit, comp, gl, gm, lane);
+          }
         }
       }
       w_cnt = min(n_cand, a.b_rw);

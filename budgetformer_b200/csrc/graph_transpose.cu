@@ -7,7 +7,7 @@
 //   t_row    [E]     the query of each of those edges,
 //   tasks    [T, 4]  (key, first, end, partial slot) work items of at most `chunk` edges,
 //   splits   [S, 3]  (key, first slot, number of slots) for keys cut into several items.
-// Steps: row id per edge (one warp per query), LSD radix sort of (key, edge id) pairs over only the bits a node id
+// Steps: row id per edge, LSD radix sort of (key, edge id) pairs over only the bits a node id
 // needs (cub::DeviceRadixSort: 3 passes for 2.9 M nodes instead of 8 for 64-bit keys), key boundaries read off the
 // sorted keys, and two compaction kernels driven by prefix sums.  The reference has no
 // counterpart (its attention runs on COO with scatter reductions, e.g. models/gt_dist_node_level.py:224-262).
@@ -21,18 +21,25 @@
 
 namespace {
 
-// one warp per query row (a virtual-node row holds every node: its lanes stride over it)
-__global__ void edge_rows_kernel(const int* __restrict__ rowptr, int n, int* __restrict__ erow) {
+// erow[e] = row of edge e, iota[e] = e.  Eight lanes per row (an attention graph holds 5 to 30 edges a row); rows above 64 edges
+// (the virtual node's holds every node) are left to the whole warp, one after the other.
+__global__ void edge_rows_kernel(const int* __restrict__ rowptr, int n, int* __restrict__ erow, int* __restrict__ iota) {
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int row = (int)(gt >> 5), lane = (int)(gt & 31);
-  if (row >= n) return;
-  const int beg = rowptr[row], end = rowptr[row + 1];
-  for (int e = beg + lane; e < end; e += 32) erow[e] = row;
-}
-
-__global__ void iota_kernel(int* __restrict__ p, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = (int)i;
+  const long long row = gt >> 3;
+  const int lane = threadIdx.x & 31;
+  int beg = 0, end = 0;
+  if (row < n) { beg = rowptr[row]; end = rowptr[row + 1]; }
+  const bool wide = end - beg > 64;
+  if (!wide)
+    for (int e = beg + (lane & 7); e < end; e += 8) { erow[e] = (int)row; iota[e] = e; }
+  unsigned left = __ballot_sync(0xffffffffu, wide && (lane & 7) == 0);
+  while (left != 0) {
+    const int src = __ffs(left) - 1;
+    left &= left - 1;
+    const int b = __shfl_sync(0xffffffffu, beg, src), e1 = __shfl_sync(0xffffffffu, end, src);
+    const int r = (int)((gt >> 5) * 4 + (src >> 3));
+    for (int e = b + lane; e < e1; e += 32) { erow[e] = r; iota[e] = e; }
+  }
 }
 
 // t_rowptr[k] = first position in the sorted key array whose key is >= k: position i is that boundary for every key
@@ -132,8 +139,7 @@ extern "C" int bf_graph_transpose(const int* rowptr, const int* col, int n, long
   void* sort_tmp = static_cast<uint8_t*>(scratch) + head;
   size_t sort_bytes = scratch_bytes - head;
   const unsigned eb = (unsigned)((n_edges + 255) / 256);
-  iota_kernel<<<eb, 256, 0, st>>>(iota, n_edges);
-  edge_rows_kernel<<<(unsigned)(((long long)n * 32 + 255) / 256), 256, 0, st>>>(rowptr, n, erow);
+  edge_rows_kernel<<<(unsigned)(((long long)n * 8 + 255) / 256), 256, 0, st>>>(rowptr, n, erow, iota);
   cudaError_t e = cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, col, keys_out, iota, t_eid, n_edges, 0,
                                                   bits_for(n), st);
   if (e != cudaSuccess) return (int)e;
