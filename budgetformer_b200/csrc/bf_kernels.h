@@ -275,6 +275,12 @@ int bf_kv_task_fill(const int* t_rowptr, const int* item_first, const int* slot_
                     const int* by_length, int n, int chunk, int n_slots, int n_split, int* tasks /* [T, 4] */,
                     int* splits /* [S, 3] */, cudaStream_t st);
 
+// ---- weight and bias gradient of an fp32 linear layer (linear_f32.cu) -------------------------------------
+// out = [dW (N*K) | db (N, with want_bias)]; partial: bf_f32_dw_slices(M, N, K) times as many floats as out
+int bf_f32_dw_slices(long long M, int N, int K);
+int bf_f32_dw(const float* dy, long long lddy, const float* x, long long ldx, long long M, int N, int K, int want_bias,
+              float* partial, float* out, cudaStream_t st);
+
 // ---- row kernels (norm_fused.cu) -----------------------------------------------------------------
 int bf_layernorm_fwd(const void* x, long long ldx, const float* gamma, const float* beta, void* y, long long ldy,
                      float* stats /* [rows, 2] mean, rstd or NULL */, long long rows, int h, float eps, int dtype,

@@ -667,6 +667,20 @@ std::vector<Tensor> layernorm_bwd(Tensor dy, Tensor x, Tensor stats, Tensor gamm
   return {dx, dgamma, dbeta};
 }
 
+// [dY^T X flattened | column sums of dY] of fp32 matrices, one flat tensor
+Tensor f32_weight_grad(Tensor dy, Tensor x, bool want_bias) {
+  TORCH_CHECK(dy.is_cuda() && dy.dim() == 2 && x.dim() == 2 && dy.device() == x.device() && dy.scalar_type() == torch::kFloat &&
+              x.scalar_type() == torch::kFloat && dy.stride(1) == 1 && x.stride(1) == 1 && dy.size(0) == x.size(0) && dy.size(0) > 0 &&
+              dy.size(1) > 0 && x.size(1) > 0, "f32_weight_grad: fp32 [M, N] and [M, K]");
+  c10::cuda::CUDAGuard guard(dy.device());
+  const int64_t m = dy.size(0), n = dy.size(1), k = x.size(1), size = n * k + (want_bias ? n : 0);
+  Tensor out = torch::empty({size}, dy.options());
+  Tensor partial = torch::empty({bf_f32_dw_slices(m, (int)n, (int)k), size}, dy.options());
+  check_cuda(bf_f32_dw(dy.data_ptr<float>(), dy.stride(0), x.data_ptr<float>(), x.stride(0), m, (int)n, (int)k, want_bias ? 1 : 0,
+                       partial.data_ptr<float>(), out.data_ptr<float>(), at::cuda::getCurrentCUDAStream()), "f32_weight_grad");
+  return out;
+}
+
 Tensor colsum(Tensor x) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.stride(1) == 1);
   c10::cuda::CUDAGuard guard(x.device());
@@ -817,6 +831,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bn_stats", &bn_stats);
   m.def("bn_bwd_reduce", &bn_bwd_reduce);
   m.def("col_affine", &col_affine);
+  m.def("f32_weight_grad", &f32_weight_grad);
   m.def("colsum", &colsum);
   m.def("nll_fwd_bwd", &nll_fwd_bwd);
   m.def("grad_sumsq", &grad_sumsq);

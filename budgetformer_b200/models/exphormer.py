@@ -13,7 +13,7 @@ from torch.utils.checkpoint import checkpoint
 
 from ..parallel.initialize import get_sequence_parallel_group, get_sequence_parallel_rank
 from ..parallel.sp_ops import DistributedAttentionNodeLevel
-from .common import NodeModelBase, SparseCoreAttention, encode_features, init_params
+from .common import Linear, NodeModelBase, SparseCoreAttention, encode_features, init_params
 
 
 class ExphormerCoreAttention(SparseCoreAttention):
@@ -24,7 +24,7 @@ class ExphormerCoreAttention(SparseCoreAttention):
         super().__init__(hidden_size, attention_dropout_rate, num_heads)
         hidden = num_heads * self.hidden_size_per_attention_head
         self.edge_type_emb = nn.Embedding(self.N_EDGE_TYPES, hidden)
-        self.edge_proj = nn.Linear(hidden, hidden, bias=False)
+        self.edge_proj = Linear(hidden, hidden, bias=False)
 
     def edge_table(self):
         hl = self.num_attention_heads_per_partition
@@ -44,9 +44,9 @@ class MultiHeadAttention(nn.Module):
         super().__init__()
         self.num_heads = num_heads
         self.att_size = hidden_size // num_heads
-        self.linear_q = nn.Linear(hidden_size, num_heads * self.att_size, bias=False)
-        self.linear_k = nn.Linear(hidden_size, num_heads * self.att_size, bias=False)
-        self.linear_v = nn.Linear(hidden_size, num_heads * self.att_size, bias=False)
+        self.linear_q = Linear(hidden_size, num_heads * self.att_size, bias=False)
+        self.linear_k = Linear(hidden_size, num_heads * self.att_size, bias=False)
+        self.linear_v = Linear(hidden_size, num_heads * self.att_size, bias=False)
         self.dist_attn = DistributedAttentionNodeLevel(
             ExphormerCoreAttention(hidden_size, attention_dropout_rate, num_heads), get_sequence_parallel_group())
 
@@ -64,8 +64,8 @@ class EncoderLayer(nn.Module):
         self.self_attention = MultiHeadAttention(hidden_size, attention_dropout_rate, num_heads)
         self.dropout1 = nn.Dropout(dropout_rate)
         self.norm1 = nn.BatchNorm1d(hidden_size)
-        self.ffn1 = nn.Linear(hidden_size, hidden_size * 2)
-        self.ffn2 = nn.Linear(hidden_size * 2, hidden_size)
+        self.ffn1 = Linear(hidden_size, hidden_size * 2)
+        self.ffn2 = Linear(hidden_size * 2, hidden_size)
         self.ff_dropout1 = nn.Dropout(dropout_rate)
         self.ff_dropout2 = nn.Dropout(dropout_rate)
         self.norm2 = nn.BatchNorm1d(hidden_size)
@@ -99,11 +99,11 @@ class Exphormer(NodeModelBase):
     def __init__(self, n_layers, num_heads, input_dim, hidden_dim, output_dim, attn_bias_dim, dropout_rate,
                  input_dropout_rate, attention_dropout_rate, ffn_dim, num_global_node, **kwargs):
         super().__init__()
-        self.node_encoder = nn.Linear(input_dim, hidden_dim)
+        self.node_encoder = Linear(input_dim, hidden_dim)
         self.input_dropout = nn.Dropout(input_dropout_rate)
         self.layers = nn.ModuleList([
             EncoderLayer(hidden_dim, dropout_rate, attention_dropout_rate, num_heads) for _ in range(n_layers)])
-        self.output_proj = nn.Linear(hidden_dim, output_dim)
+        self.output_proj = Linear(hidden_dim, output_dim)
         self.apply(lambda m: init_params(m, n_layers=n_layers))
         self._init_ckpt_state()
 

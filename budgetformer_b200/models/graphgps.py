@@ -16,7 +16,7 @@ from torch.utils.checkpoint import checkpoint
 
 from ..parallel.initialize import get_sequence_parallel_group
 from ..parallel.sp_ops import DistributedAttentionNodeLevel
-from .common import NodeModelBase, SparseCoreAttention, encode_features
+from .common import Linear, NodeModelBase, SparseCoreAttention, encode_features
 
 
 def _gaussian_orthogonal_random_matrix(nb_rows, nb_columns, device=None):
@@ -96,10 +96,10 @@ class MultiHeadAttention(nn.Module):
         self.num_heads = num_heads
         self.att_size = hidden_size // num_heads
         qkv_bias = str(attn_type).lower() == "full"
-        self.linear_q = nn.Linear(hidden_size, num_heads * self.att_size, bias=qkv_bias)
-        self.linear_k = nn.Linear(hidden_size, num_heads * self.att_size, bias=qkv_bias)
-        self.linear_v = nn.Linear(hidden_size, num_heads * self.att_size, bias=qkv_bias)
-        self.out_proj = nn.Linear(hidden_size, hidden_size)
+        self.linear_q = Linear(hidden_size, num_heads * self.att_size, bias=qkv_bias)
+        self.linear_k = Linear(hidden_size, num_heads * self.att_size, bias=qkv_bias)
+        self.linear_v = Linear(hidden_size, num_heads * self.att_size, bias=qkv_bias)
+        self.out_proj = Linear(hidden_size, hidden_size)
         self.dist_attn = DistributedAttentionNodeLevel(
             GPSCoreAttention(hidden_size, attention_dropout_rate, num_heads), get_sequence_parallel_group())
 
@@ -117,8 +117,8 @@ class EncoderLayer(nn.Module):
         self.self_attention = MultiHeadAttention(hidden_size, attention_dropout_rate, num_heads, attn_type=attn_type)
         self.dropout1 = nn.Dropout(dropout_rate)
         self.norm1 = nn.BatchNorm1d(hidden_size)
-        self.ffn1 = nn.Linear(hidden_size, hidden_size * 2)
-        self.ffn2 = nn.Linear(hidden_size * 2, hidden_size)
+        self.ffn1 = Linear(hidden_size, hidden_size * 2)
+        self.ffn2 = Linear(hidden_size * 2, hidden_size)
         self.ff_dropout1 = nn.Dropout(dropout_rate)
         self.ff_dropout2 = nn.Dropout(dropout_rate)
         self.norm2 = nn.BatchNorm1d(hidden_size)
@@ -152,11 +152,11 @@ class GraphGPS(NodeModelBase):
     def __init__(self, n_layers, num_heads, input_dim, hidden_dim, output_dim, attn_bias_dim, dropout_rate,
                  input_dropout_rate, attention_dropout_rate, ffn_dim, num_global_node, attn_type="sparse", **kwargs):
         super().__init__()
-        self.node_encoder = nn.Linear(input_dim, hidden_dim)
+        self.node_encoder = Linear(input_dim, hidden_dim)
         self.layers = nn.ModuleList([
             EncoderLayer(hidden_dim, dropout_rate, attention_dropout_rate, num_heads, attn_type=attn_type)
             for _ in range(n_layers)])
-        self.output_proj = nn.Linear(hidden_dim, output_dim)
+        self.output_proj = Linear(hidden_dim, output_dim)
         self._init_ckpt_state()
 
     def redraw_performer_projections(self, device=None):

@@ -12,17 +12,18 @@ from torch import nn
 from torch.nn import functional as F
 from torch.utils.checkpoint import checkpoint
 
+from ..ops.norm import layer_norm
 from ..parallel.initialize import get_sequence_parallel_group
 from ..parallel.sp_ops import DistributedAttentionNoMerge
-from .common import NodeModelBase, SparseCoreAttention, encode_features, init_params
+from .common import LayerNorm, Linear, NodeModelBase, SparseCoreAttention, encode_features, init_params
 
 
 class FeedForwardNetwork(nn.Module):
     def __init__(self, hidden_size, ffn_size, dropout_rate):
         super().__init__()
-        self.layer1 = nn.Linear(hidden_size, ffn_size)
+        self.layer1 = Linear(hidden_size, ffn_size)
         self.gelu = nn.GELU()
-        self.layer2 = nn.Linear(ffn_size, hidden_size)
+        self.layer2 = Linear(ffn_size, hidden_size)
 
     def forward(self, x):
         return self.layer2(self.gelu(self.layer1(x)))
@@ -66,12 +67,12 @@ class MultiHeadAttention(nn.Module):
         super().__init__()
         self.num_heads = num_heads
         self.att_size = hidden_size // num_heads
-        self.linear_q = nn.Linear(hidden_size, num_heads * self.att_size)
-        self.linear_k = nn.Linear(hidden_size, num_heads * self.att_size)
-        self.linear_v = nn.Linear(hidden_size, num_heads * self.att_size)
+        self.linear_q = Linear(hidden_size, num_heads * self.att_size)
+        self.linear_k = Linear(hidden_size, num_heads * self.att_size)
+        self.linear_v = Linear(hidden_size, num_heads * self.att_size)
         self.dist_attn = DistributedAttentionNoMerge(
             CoreAttention(hidden_size, attention_dropout_rate, num_heads, attn_bias_dim), get_sequence_parallel_group())
-        self.output_layer = nn.Linear(num_heads * self.att_size, hidden_size)
+        self.output_layer = Linear(num_heads * self.att_size, hidden_size)
 
     def forward(self, x, attn_bias=None, edge_index=None, attn_type=None):
         b = x.size(0)
@@ -84,10 +85,10 @@ class MultiHeadAttention(nn.Module):
 class EncoderLayer(nn.Module):
     def __init__(self, hidden_size, ffn_size, dropout_rate, attention_dropout_rate, num_heads, attn_bias_dim):
         super().__init__()
-        self.self_attention_norm = nn.LayerNorm(hidden_size)
+        self.self_attention_norm = LayerNorm(hidden_size)
         self.self_attention = MultiHeadAttention(hidden_size, attention_dropout_rate, num_heads, attn_bias_dim)
         self.self_attention_dropout = nn.Dropout(dropout_rate)
-        self.ffn_norm = nn.LayerNorm(hidden_size)
+        self.ffn_norm = LayerNorm(hidden_size)
         self.ffn = FeedForwardNetwork(hidden_size, ffn_size, dropout_rate)
         self.ffn_dropout = nn.Dropout(dropout_rate)
 
@@ -110,19 +111,19 @@ class Graphormer(NodeModelBase):
                  input_dropout_rate, attention_dropout_rate, ffn_dim, num_global_node, **kwargs):
         super().__init__()
         self.num_heads = num_heads
-        self.node_encoder = nn.Linear(input_dim, hidden_dim)
+        self.node_encoder = Linear(input_dim, hidden_dim)
         self.input_dropout = nn.Dropout(input_dropout_rate)
         self.layers = nn.ModuleList([
             EncoderLayer(hidden_dim, ffn_dim, dropout_rate, attention_dropout_rate, num_heads, attn_bias_dim)
             for _ in range(n_layers)])
         self.n_layers = n_layers
-        self.final_ln = nn.LayerNorm(hidden_dim)
-        self.downstream_out_proj = nn.Linear(hidden_dim, output_dim)
+        self.final_ln = LayerNorm(hidden_dim)
+        self.downstream_out_proj = Linear(hidden_dim, output_dim)
         self.hidden_dim = hidden_dim
         self.num_global_node = num_global_node
         self.graph_token = nn.Embedding(self.num_global_node, hidden_dim)
         self.graph_token_virtual_distance = nn.Embedding(self.num_global_node, attn_bias_dim)
-        self.attn_bias_proj = nn.Linear(attn_bias_dim, num_heads, bias=False)
+        self.attn_bias_proj = Linear(attn_bias_dim, num_heads, bias=False)
         self._init_ckpt_state()
         self.apply(lambda m: init_params(m, n_layers=n_layers))
 
@@ -149,9 +150,14 @@ class Graphormer(NodeModelBase):
         x = self.input_dropout(x)
         bias = self._graph_attn_bias(attn_bias, x.device)
         x = self._run_layers(x, attn_bias=bias, edge_index=edge_index, attn_type=attn_type)
-        x = self.final_ln(x)
         from ..ops.gemm import readout_linear
-        return readout_linear(x[0, int(self.num_global_node):, :], self.downstream_out_proj.weight, self.downstream_out_proj.bias)
+        x = x[0, int(self.num_global_node):, :]
+        if x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and torch.is_autocast_enabled("cuda"):
+            # autocast would normalise an fp32 copy and round the result for the projection: the row kernel rounds once as well
+            x = layer_norm(x, self.final_ln.weight, self.final_ln.bias, self.final_ln.eps)
+        else:
+            x = self.final_ln(x)
+        return readout_linear(x, self.downstream_out_proj.weight, self.downstream_out_proj.bias)
 
     def forward(self, x, attn_bias, edge_index, perturb=None, attn_type=None):
         return F.log_softmax(self.forward_logits(x, attn_bias, edge_index, perturb, attn_type), dim=1)

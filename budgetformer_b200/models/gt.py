@@ -12,7 +12,7 @@ from torch.utils.checkpoint import checkpoint
 
 from ..parallel.initialize import get_sequence_parallel_group
 from ..parallel.sp_ops import DistributedAttentionNodeLevel
-from .common import NodeModelBase, SparseCoreAttention, encode_features, init_params
+from .common import LayerNorm, Linear, NodeModelBase, SparseCoreAttention, encode_features, init_params
 
 
 class CoreAttention(SparseCoreAttention):
@@ -28,9 +28,9 @@ class MultiHeadAttention(nn.Module):
         super().__init__()
         self.num_heads = num_heads
         self.att_size = hidden_size // num_heads
-        self.linear_q = nn.Linear(hidden_size, num_heads * self.att_size)
-        self.linear_k = nn.Linear(hidden_size, num_heads * self.att_size)
-        self.linear_v = nn.Linear(hidden_size, num_heads * self.att_size)
+        self.linear_q = Linear(hidden_size, num_heads * self.att_size)
+        self.linear_k = Linear(hidden_size, num_heads * self.att_size)
+        self.linear_v = Linear(hidden_size, num_heads * self.att_size)
         self.dist_attn = DistributedAttentionNodeLevel(
             CoreAttention(hidden_size, attention_dropout_rate, num_heads), get_sequence_parallel_group())
 
@@ -49,11 +49,11 @@ class EncoderLayer(nn.Module):
         super().__init__()
         self.self_attention = MultiHeadAttention(hidden_size, attention_dropout_rate, num_heads)
         self.self_attention_dropout = nn.Dropout(dropout_rate)
-        self.O = nn.Linear(hidden_size, hidden_size)
-        self.layer_norm1 = nn.LayerNorm(hidden_size)
-        self.FFN_layer1 = nn.Linear(hidden_size, hidden_size * 2)
-        self.FFN_layer2 = nn.Linear(hidden_size * 2, hidden_size)
-        self.layer_norm2 = nn.LayerNorm(hidden_size)
+        self.O = Linear(hidden_size, hidden_size)
+        self.layer_norm1 = LayerNorm(hidden_size)
+        self.FFN_layer1 = Linear(hidden_size, hidden_size * 2)
+        self.FFN_layer2 = Linear(hidden_size * 2, hidden_size)
+        self.layer_norm2 = LayerNorm(hidden_size)
 
     def _ffn(self, h):
         y = self.FFN_layer1(h)
@@ -78,8 +78,8 @@ class EncoderLayer(nn.Module):
 class MLPReadout(nn.Module):
     def __init__(self, input_dim, output_dim, L=2):
         super().__init__()
-        layers = [nn.Linear(input_dim // 2 ** l, input_dim // 2 ** (l + 1), bias=True) for l in range(L)]
-        layers.append(nn.Linear(input_dim // 2 ** L, output_dim, bias=True))
+        layers = [Linear(input_dim // 2 ** l, input_dim // 2 ** (l + 1), bias=True) for l in range(L)]
+        layers.append(Linear(input_dim // 2 ** L, output_dim, bias=True))
         self.FC_layers = nn.ModuleList(layers)
         self.L = L
 
@@ -95,7 +95,7 @@ class GT(NodeModelBase):
     def __init__(self, n_layers, num_heads, input_dim, hidden_dim, output_dim, attn_bias_dim, dropout_rate,
                  input_dropout_rate, attention_dropout_rate, ffn_dim, num_global_node, **kwargs):
         super().__init__()
-        self.node_encoder = nn.Linear(input_dim, hidden_dim)
+        self.node_encoder = Linear(input_dim, hidden_dim)
         self.input_dropout = nn.Dropout(input_dropout_rate)
         self.layers = nn.ModuleList([
             EncoderLayer(hidden_dim, ffn_dim, dropout_rate, attention_dropout_rate, num_heads) for _ in range(n_layers)])

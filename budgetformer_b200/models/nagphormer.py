@@ -12,15 +12,15 @@ from torch import nn
 from torch.nn import functional as F
 from torch.utils.checkpoint import checkpoint
 
-from .common import NodeModelBase, init_params
+from .common import LayerNorm, Linear, NodeModelBase, init_params
 
 
 class FeedForwardNetwork(nn.Module):
     def __init__(self, hidden_size, ffn_size):
         super().__init__()
-        self.layer1 = nn.Linear(hidden_size, ffn_size)
+        self.layer1 = Linear(hidden_size, ffn_size)
         self.gelu = nn.GELU()
-        self.layer2 = nn.Linear(ffn_size, hidden_size)
+        self.layer2 = Linear(ffn_size, hidden_size)
 
     def forward(self, x):
         return self.layer2(self.gelu(self.layer1(x)))
@@ -32,11 +32,11 @@ class MultiHeadAttention(nn.Module):
         self.num_heads = num_heads
         self.att_size = hidden_size // num_heads
         self.scale = self.att_size ** -0.5
-        self.linear_q = nn.Linear(hidden_size, num_heads * self.att_size)
-        self.linear_k = nn.Linear(hidden_size, num_heads * self.att_size)
-        self.linear_v = nn.Linear(hidden_size, num_heads * self.att_size)
+        self.linear_q = Linear(hidden_size, num_heads * self.att_size)
+        self.linear_k = Linear(hidden_size, num_heads * self.att_size)
+        self.linear_v = Linear(hidden_size, num_heads * self.att_size)
         self.att_dropout = nn.Dropout(attention_dropout_rate)
-        self.output_layer = nn.Linear(num_heads * self.att_size, hidden_size)
+        self.output_layer = Linear(num_heads * self.att_size, hidden_size)
 
     def forward(self, q, k, v):
         bsz, seq_len, _ = q.size()
@@ -52,10 +52,10 @@ class MultiHeadAttention(nn.Module):
 class EncoderLayer(nn.Module):
     def __init__(self, hidden_size, ffn_size, dropout_rate, attention_dropout_rate, num_heads):
         super().__init__()
-        self.self_attention_norm = nn.LayerNorm(hidden_size)
+        self.self_attention_norm = LayerNorm(hidden_size)
         self.self_attention = MultiHeadAttention(hidden_size, attention_dropout_rate, num_heads)
         self.self_attention_dropout = nn.Dropout(dropout_rate)
-        self.ffn_norm = nn.LayerNorm(hidden_size)
+        self.ffn_norm = LayerNorm(hidden_size)
         self.ffn = FeedForwardNetwork(hidden_size, ffn_size)
         self.ffn_dropout = nn.Dropout(dropout_rate)
 
@@ -82,13 +82,13 @@ class NAGphormer(NodeModelBase):
         self.n_layers = n_layers
         if ffn_dim is None or ffn_dim <= 0:
             ffn_dim = 2 * hidden_dim
-        self.att_embeddings_nope = nn.Linear(input_dim, hidden_dim)
+        self.att_embeddings_nope = Linear(input_dim, hidden_dim)
         self.layers = nn.ModuleList([
             EncoderLayer(hidden_dim, ffn_dim, dropout_rate, attention_dropout_rate, num_heads) for _ in range(n_layers)])
-        self.final_ln = nn.LayerNorm(hidden_dim)
-        self.out_proj = nn.Linear(hidden_dim, hidden_dim // 2)
-        self.attn_layer = nn.Linear(2 * hidden_dim, 1)
-        self.Linear1 = nn.Linear(hidden_dim // 2, n_class)
+        self.final_ln = LayerNorm(hidden_dim)
+        self.out_proj = Linear(hidden_dim, hidden_dim // 2)
+        self.attn_layer = Linear(2 * hidden_dim, 1)
+        self.Linear1 = Linear(hidden_dim // 2, n_class)
         self.scaling = nn.Parameter(torch.ones(1) * 0.5)
         self.apply(lambda m: init_params(m, n_layers=n_layers))
         self._init_ckpt_state()

@@ -43,13 +43,20 @@ class _LayerNorm(torch.autograd.Function):
         _ext.count_launches(1)
         ctx.save_for_backward(x, stats, g32)
         ctx.pdtype = gamma.dtype
-        ctx.slot = slot
+        ctx.slot, ctx.eps = slot, float(eps)
         return y
 
     @staticmethod
     def backward(ctx, dy):
         ext = _ext.load()
         x, stats, g32 = ctx.saved_tensors
+        if torch.is_grad_enabled():                        # a second derivative is wanted: differentiable operators
+            xf, d = x.float(), dy.float()
+            xc = xf - xf.mean(1, keepdim=True)
+            rstd = torch.rsqrt((xc * xc).mean(1, keepdim=True) + ctx.eps)
+            xhat, gd = xc * rstd, d * g32
+            dx = rstd * (gd - gd.mean(1, keepdim=True) - xhat * (gd * xhat).mean(1, keepdim=True))
+            return dx.to(x.dtype), (d * xhat).sum(0).to(ctx.pdtype), d.sum(0).to(ctx.pdtype), None, None
         dy = dy if dy.stride(-1) == 1 else dy.contiguous()
         if ctx.slot is not None:
             dx, dg, db, dxsum = ext.layernorm_bwd(dy.to(x.dtype), x, stats, g32, True)

@@ -1,5 +1,5 @@
-"""Edge attention as streams of segments, at the sizes where the split ends: one row, partial warps, heads that do not fill a
-lane group, several segments per lane group, empty rows."""
+"""Edge attention as streams of segments, the fp32 weight gradient and the row-wise element kernels, at the sizes where their
+splits end: one row, partial warps, heads that do not fill a lane group, several segments per lane group, empty rows."""
 import pytest
 import torch
 
@@ -74,3 +74,67 @@ def test_attention_streams_keep_other_rows_finite():
     keys = torch.ones(n, dtype=torch.bool, device="cuda")
     keys[9] = False
     assert torch.isfinite(dk[keys]).all() and torch.isfinite(dv[keys]).all()
+
+
+@pytest.mark.parametrize("m,n,k,pad", [(1, 1, 1, 0), (63, 64, 64, 0), (65, 60, 68, 0), (1000, 47, 101, 0), (4097, 256, 64, 4),
+                                       (20011, 64, 256, 0), (300, 130, 70, 1)])
+def test_f32_weight_grad(m, n, k, pad):
+    from budgetformer_b200.ops import _ext
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    dy = torch.randn(m, n + pad, generator=gen, device="cuda")[:, :n]
+    x = torch.randn(m, k + pad, generator=gen, device="cuda")[:, :k]
+    for bias in (True, False):
+        flat = _ext.load().f32_weight_grad(dy, x, bias)
+        want, size = dy.double().t() @ x.double(), dy.double().abs().t() @ x.double().abs()
+        # any order of m products and additions: |error| <= m * 2^-24 * sum |dy| |x|
+        assert bool(((flat[:n * k].view(n, k).double() - want).abs() <= m * 2.0 ** -24 * size + 1e-30).all())
+        if bias:
+            db = dy.double().sum(0)
+            assert bool(((flat[n * k:].double() - db).abs() <= m * 2.0 ** -24 * dy.double().abs().sum(0) + 1e-30).all())
+
+
+def test_fp32_modules_match_torch():
+    """Linear and LayerNorm of the models against torch's, first and second derivative, rows above and below the split."""
+    from budgetformer_b200.models.common import LayerNorm, Linear
+    for rows in (7, 3000):
+        for cls, ref, args in ((Linear, torch.nn.Linear, (24, 40)), (LayerNorm, torch.nn.LayerNorm, (24,))):
+            torch.manual_seed(rows)
+            a, b = cls(*args).cuda(), ref(*args).cuda()
+            b.load_state_dict(a.state_dict())
+            x = torch.randn(1, rows, 24, device="cuda")
+            res = []
+            weights = torch.randn_like(a(x)).detach()                      # sum(y^2) alone is constant behind a LayerNorm
+            for mod in (a, b):
+                xi = x.clone().requires_grad_()
+                y = mod(xi)
+                g1 = torch.autograd.grad((y * y * weights).sum(), [xi] + list(mod.parameters()), retain_graph=True)
+                g2 = torch.autograd.grad((y * y * y * weights).sum(), xi, create_graph=True)[0]
+                g2 = torch.autograd.grad((g2 * g2).sum(), [xi] + list(mod.parameters()), allow_unused=True)
+                res.append([y] + list(g1) + [g for g in g2 if g is not None])
+            assert len(res[0]) == len(res[1])
+            for u, w in zip(*res):
+                assert float((u - w).norm()) <= 2e-5 * float(w.norm()) + 1e-6
+
+
+@pytest.mark.parametrize("rows,cols,dtype", [(1, 8, torch.bfloat16), (37, 24, torch.float16), (4099, 256, torch.bfloat16),
+                                             (515, 2048, torch.bfloat16), (700, 136, torch.float32)])
+def test_row_element_kernels(rows, cols, dtype):
+    """BatchNorm's affine passes and the hashed dropout: fp32 arithmetic, one rounding."""
+    from budgetformer_b200.ops import _ext
+    from budgetformer_b200.ops.gemm import hash_keep_mask
+    from budgetformer_b200.ops.norm import gelu_dropout, hash_dropout
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, cols + 8, generator=gen, device="cuda").to(dtype)[:, :cols]      # row pitch wider than the row
+    z = torch.randn(rows, cols, generator=gen, device="cuda").to(dtype)
+    a, b, c = (torch.randn(cols, generator=gen, device="cuda") for _ in range(3))
+    unit = {torch.float32: 2.0 ** -23, torch.float16: 2.0 ** -10, torch.bfloat16: 2.0 ** -7}[dtype]
+    ext = _ext.load()
+    for got, want, size in ((ext.col_affine(x, None, a, b, None), x.double() * a + b, (x.double() * a).abs() + b.abs()),
+                            (ext.col_affine(x, z, a, b, c), z.double() * a + x.double() * b + c,
+                             (z.double() * a).abs() + (x.double() * b).abs() + c.abs())):
+        assert bool(((got.double() - want).abs() <= unit * size + 1e-7).all())
+    keep = hash_keep_mask(5, rows, cols, 0.25, "cuda")
+    want = torch.where(keep, x.float() * (1.0 / 0.75), torch.zeros((), device="cuda"))
+    assert bool(((hash_dropout(x, 5, 0.25).float() - want).abs() <= unit * want.abs() + 1e-7).all())
+    want = torch.where(keep, torch.nn.functional.gelu(x.float()) * (1.0 / 0.75), torch.zeros((), device="cuda"))
+    assert bool(((gelu_dropout(x, 5, 0.25).float() - want).abs() <= unit * want.abs() + 1e-6).all())
