@@ -388,6 +388,40 @@ __global__ void __launch_bounds__(256) hash_dropout_kernel(const T* __restrict__
   }
 }
 
+// The same for 16-bit rows of whole, aligned 16-byte chunks (at most 2048 columns): a thread keeps its chunk and walks the rows
+// four at a time, so that four loads are in flight while the masks are hashed (612 k x 256: 107 us, 130 us with one).
+template <typename T, bool GELU>
+__global__ void __launch_bounds__(256) hash_dropout_rows_kernel(const T* __restrict__ x, long long ldx, T* __restrict__ y,
+                                                                long long ldy, long long rows, int cols, uint32_t seed,
+                                                                uint32_t thresh, float scale) {
+  constexpr int U = 4;
+  const int chunks = cols / 8, row_lanes = blockDim.x / chunks;
+  const int rl = threadIdx.x / chunks, c = (threadIdx.x - rl * chunks) * 8;
+  if (rl >= row_lanes) return;
+  const long long step = (long long)gridDim.x * row_lanes;
+  for (long long r0 = (long long)blockIdx.x * row_lanes + rl; r0 < rows; r0 += U * step) {
+    uint4 u[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+      if (r0 + q * step < rows) u[q] = *reinterpret_cast<const uint4*>(x + (r0 + q * step) * ldx + c);
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const long long r = r0 + q * step;
+      if (r >= rows) break;
+      const uint32_t rh = (uint32_t)r * 0x9E3779B1u + seed;
+      float f[8];
+      unpack8<T>(u[q], f);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const bool keep = mix32(rh + (uint32_t)(c + k) * 0x85EBCA77u) >= thresh;
+        const float val = GELU ? gelu_erf_f(f[k]) : f[k];
+        f[k] = keep ? val * scale : 0.f;
+      }
+      *reinterpret_cast<uint4*>(y + r * ldy + c) = pack8<T>(f);
+    }
+  }
+}
+
 // out[c] += sum_r x[r, c] (fp32 accumulation): bias gradients without an fp32 copy of the activation gradient.
 // Each thread owns 8 consecutive columns and strides over rows; partials meet in shared memory, then one atomic
 // per column and block.
@@ -526,23 +560,41 @@ __global__ void __launch_bounds__(256) colstats_kernel(const T* __restrict__ x, 
 }
 
 // TWO = false: y = x*a + b;  TWO = true: y = in2*a + x*b + c0
+// A thread keeps one chunk of 8 columns, with its coefficients in registers, and walks the rows U at a time: U (or 2 U)
+// independent 16-byte loads in flight and no index division.  612 k x 256 bf16: 117 us (y = x*a + b) and 223 us (three matrices),
+// 5.4 and 4.2 TB/s; with one load per thread and the coefficients read again for every chunk 307 and 452 us.
 template <typename T, bool TWO>
 __global__ void __launch_bounds__(256) col_affine_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ in2,
                                                          long long ld2, const float* __restrict__ a,
                                                          const float* __restrict__ b, const float* __restrict__ c0,
                                                          T* __restrict__ y, long long ldy, long long rows, int cols) {
-  const int chunks = cols / 8;
-  const long long total = rows * chunks;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const long long r = i / chunks;
-    const int c = (int)(i - r * chunks) * 8;
-    float u[8], w[8], o[8];
-    load8<T>(x + r * ldx + c, u);
-    if (TWO) load8<T>(in2 + r * ld2 + c, w);
+  constexpr int U = sizeof(T) == 2 ? 4 : 2;
+  const int chunks = cols / 8, row_lanes = blockDim.x / chunks;
+  const int rl = threadIdx.x / chunks, c = (threadIdx.x - rl * chunks) * 8;
+  if (rl >= row_lanes) return;
+  float fa[8], fb[8], fc[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = TWO ? w[k] * a[c + k] + u[k] * b[c + k] + c0[c + k] : u[k] * a[c + k] + b[c + k];
-    store8<T>(y + r * ldy + c, o);
+  for (int k = 0; k < 8; ++k) { fa[k] = __ldg(a + c + k); fb[k] = __ldg(b + c + k); fc[k] = TWO ? __ldg(c0 + c + k) : 0.f; }
+  const long long step = (long long)gridDim.x * row_lanes;
+  for (long long r0 = (long long)blockIdx.x * row_lanes + rl; r0 < rows; r0 += U * step) {
+    float u[U][8], w[U][8];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const long long r = r0 + q * step;
+      if (r < rows) {
+        load8<T>(x + r * ldx + c, u[q]);
+        if (TWO) load8<T>(in2 + r * ld2 + c, w[q]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const long long r = r0 + q * step;
+      if (r >= rows) break;
+      float o[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) o[k] = TWO ? w[q][k] * fa[k] + u[q][k] * fb[k] + fc[k] : u[q][k] * fa[k] + fb[k];
+      store8<T>(y + r * ldy + c, o);
+    }
   }
 }
 
@@ -553,6 +605,11 @@ __global__ void __launch_bounds__(256) col_affine_kernel(const T* __restrict__ x
   else if (DT == BF_FP16) { CALL(__half); }                             \
   else if (DT == BF_FP32) { CALL(float); }                              \
   else return (int)cudaErrorInvalidValue;
+
+static bool cols8_ok(int cols, int dtype, const void* p, long long ld) {
+  const int esz = dtype == BF_FP32 ? 4 : 2;
+  return cols % 8 == 0 && cols >= 8 && cols <= 2048 && ((uintptr_t)p) % 16 == 0 && (ld * esz) % 16 == 0;
+}
 
 static bool ln_packed_ok(int h, int dtype, const void* a, long long lda, const void* b2, long long ldb) {
   const int esz = dtype == BF_FP32 ? 4 : 2;
@@ -640,6 +697,14 @@ extern "C" int bf_hash_dropout(const void* x, long long ldx, void* y, long long 
   if (rows * cols == 0) return 0;
   const uint32_t thresh = (uint32_t)(p * 4294967296.0);
   const float scale = 1.f / (1.f - p);
+  if (dtype != BF_FP32 && cols8_ok(cols, dtype, x, ldx) && cols8_ok(cols, dtype, y, ldy)) {
+    const int row_lanes = 256 / (cols / 8);
+    long long rb = (rows + 4 * row_lanes - 1) / (4 * row_lanes);
+    if (rb > 148 * 8) rb = 148 * 8;
+    if (dtype == BF_BF16) hash_dropout_rows_kernel<__nv_bfloat16, false><<<(unsigned)rb, 256, 0, st>>>((const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)y, ldy, rows, cols, seed, thresh, scale);
+    else hash_dropout_rows_kernel<__half, false><<<(unsigned)rb, 256, 0, st>>>((const __half*)x, ldx, (__half*)y, ldy, rows, cols, seed, thresh, scale);
+    return (int)cudaGetLastError();
+  }
   long long blocks = (rows * ((cols + 7) / 8) + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
 #define CALL(T) hash_dropout_kernel<T, false><<<(unsigned)blocks, 256, 0, st>>>((const T*)x, ldx, (T*)y, ldy, rows, cols, seed, thresh, scale)
@@ -655,6 +720,14 @@ extern "C" int bf_gelu_dropout(const void* x, long long ldx, void* y, long long 
   if (p < 0.f || p >= 1.f) return (int)cudaErrorInvalidValue;
   const uint32_t thresh = (uint32_t)(p * 4294967296.0);
   const float scale = 1.f / (1.f - p);
+  if (dtype != BF_FP32 && cols8_ok(cols, dtype, x, ldx) && cols8_ok(cols, dtype, y, ldy)) {
+    const int row_lanes = 256 / (cols / 8);
+    long long rb = (rows + 4 * row_lanes - 1) / (4 * row_lanes);
+    if (rb > 148 * 8) rb = 148 * 8;
+    if (dtype == BF_BF16) hash_dropout_rows_kernel<__nv_bfloat16, true><<<(unsigned)rb, 256, 0, st>>>((const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)y, ldy, rows, cols, seed, thresh, scale);
+    else hash_dropout_rows_kernel<__half, true><<<(unsigned)rb, 256, 0, st>>>((const __half*)x, ldx, (__half*)y, ldy, rows, cols, seed, thresh, scale);
+    return (int)cudaGetLastError();
+  }
   long long blocks = (rows * ((cols + 7) / 8) + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
 #define CALL(T) hash_dropout_kernel<T, true><<<(unsigned)blocks, 256, 0, st>>>((const T*)x, ldx, (T*)y, ldy, rows, cols, seed, thresh, scale)
@@ -679,11 +752,6 @@ extern "C" int bf_colsum(const void* x, long long ldx, long long rows, int cols,
   BF_DT_SWITCH(dtype, CALL)
 #undef CALL
   return (int)cudaGetLastError();
-}
-
-static bool cols8_ok(int cols, int dtype, const void* p, long long ld) {
-  const int esz = dtype == BF_FP32 ? 4 : 2;
-  return cols % 8 == 0 && cols >= 8 && cols <= 2048 && ((uintptr_t)p) % 16 == 0 && (ld * esz) % 16 == 0;
 }
 
 extern "C" int bf_bn_stats(const void* x, long long ldx, const float* shift, long long rows, int cols, float* s1,
@@ -723,8 +791,9 @@ extern "C" int bf_col_affine(const void* x, long long ldx, const void* in2, long
   if (!cols8_ok(cols, dtype, x, ldx) || !cols8_ok(cols, dtype, y, ldy) || (in2 && !cols8_ok(cols, dtype, in2, ld2)))
     return (int)cudaErrorInvalidValue;
   if (rows == 0) return 0;
-  long long blocks = (rows * (cols / 8) + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
+  const int row_lanes = 256 / (cols / 8);
+  long long blocks = (rows + 4 * row_lanes - 1) / (4 * row_lanes);
+  if (blocks > 148 * 8) blocks = 148 * 8;
   if (in2) {
 #define CALL(T) col_affine_kernel<T, true><<<(unsigned)blocks, 256, 0, st>>>((const T*)x, ldx, (const T*)in2, ld2, a, b, c0, (T*)y, ldy, rows, cols)
     BF_DT_SWITCH(dtype, CALL)
