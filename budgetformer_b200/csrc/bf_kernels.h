@@ -17,8 +17,8 @@ extern "C" {
 #define BF_FLAG_CHANNELS 64      // barrier channels per flag page (uint32[BF_FLAG_CHANNELS][BF_MAX_PEERS])
 
 // Edge attention: query rows with more than BF_LONG_ROW edges are cut into work items of BF_LONG_CHUNK edges.  A row below
-// the line is one lane group's serial walk, two gathers at a time: 64 rounds of roughly 0.7 us at 128 edges, about what an
-// item, its scratch and the two reduction launches cost.
+// the line is one lane group's serial walk, a step of roughly 0.3 us per edge while the warp's other groups wait: at 128 edges
+// about what an item, its scratch and the two reduction launches cost.
 #define BF_LONG_ROW 128
 #define BF_LONG_CHUNK 64
 // allocation-free forward entry point (bf_noalloc.h): its callers list the rows with more than BF_HUB_DEGREE edges
