@@ -12,8 +12,7 @@ from torch.utils.checkpoint import checkpoint
 
 from ..graph.attn_graph import AttnGraph, as_attn_graph
 from ..ops.edge_attention import edge_attention
-from ..ops.gemm import linear_f32, plain_eager
-from ..ops.norm import layer_norm
+from ..ops.gemm import linear_f32
 from ..parallel.initialize import get_sequence_parallel_world_size
 
 
@@ -33,19 +32,6 @@ class Linear(nn.Linear):
 
     def forward(self, x):
         return linear_f32(x, self.weight, self.bias)
-
-
-class LayerNorm(nn.LayerNorm):
-    """``nn.LayerNorm`` over the last dimension; fp32 CUDA tensors outside autocast take the row kernels of
-    ``csrc/norm_fused.cu`` (PyTorch's gamma / beta gradient alone takes 180 us at 40 k rows of 64)."""
-
-    def forward(self, x):
-        h = x.size(-1)
-        if (x.is_cuda and x.dtype == torch.float32 and type(x) is torch.Tensor and self.bias is not None
-                and self.weight.dtype == torch.float32 and self.normalized_shape == (h,) and h <= 512 and x.numel() > 0
-                and not torch.is_autocast_enabled("cuda") and plain_eager()):
-            return layer_norm(x.reshape(-1, h), self.weight, self.bias, self.eps).view(x.shape)
-        return super().forward(x)
 
 
 class SparseCoreAttention(nn.Module):

@@ -15,7 +15,7 @@ from torch.utils.checkpoint import checkpoint
 from ..ops.norm import layer_norm
 from ..parallel.initialize import get_sequence_parallel_group
 from ..parallel.sp_ops import DistributedAttentionNoMerge
-from .common import LayerNorm, Linear, NodeModelBase, SparseCoreAttention, encode_features, init_params
+from .common import Linear, NodeModelBase, SparseCoreAttention, encode_features, init_params
 
 
 class FeedForwardNetwork(nn.Module):
@@ -85,10 +85,10 @@ class MultiHeadAttention(nn.Module):
 class EncoderLayer(nn.Module):
     def __init__(self, hidden_size, ffn_size, dropout_rate, attention_dropout_rate, num_heads, attn_bias_dim):
         super().__init__()
-        self.self_attention_norm = LayerNorm(hidden_size)
+        self.self_attention_norm = nn.LayerNorm(hidden_size)
         self.self_attention = MultiHeadAttention(hidden_size, attention_dropout_rate, num_heads, attn_bias_dim)
         self.self_attention_dropout = nn.Dropout(dropout_rate)
-        self.ffn_norm = LayerNorm(hidden_size)
+        self.ffn_norm = nn.LayerNorm(hidden_size)
         self.ffn = FeedForwardNetwork(hidden_size, ffn_size, dropout_rate)
         self.ffn_dropout = nn.Dropout(dropout_rate)
 
@@ -117,7 +117,7 @@ class Graphormer(NodeModelBase):
             EncoderLayer(hidden_dim, ffn_dim, dropout_rate, attention_dropout_rate, num_heads, attn_bias_dim)
             for _ in range(n_layers)])
         self.n_layers = n_layers
-        self.final_ln = LayerNorm(hidden_dim)
+        self.final_ln = nn.LayerNorm(hidden_dim)
         self.downstream_out_proj = Linear(hidden_dim, output_dim)
         self.hidden_dim = hidden_dim
         self.num_global_node = num_global_node

@@ -12,7 +12,7 @@ from torch.utils.checkpoint import checkpoint
 
 from ..parallel.initialize import get_sequence_parallel_group
 from ..parallel.sp_ops import DistributedAttentionNodeLevel
-from .common import LayerNorm, Linear, NodeModelBase, SparseCoreAttention, encode_features, init_params
+from .common import Linear, NodeModelBase, SparseCoreAttention, encode_features, init_params
 
 
 class CoreAttention(SparseCoreAttention):
@@ -50,10 +50,10 @@ class EncoderLayer(nn.Module):
         self.self_attention = MultiHeadAttention(hidden_size, attention_dropout_rate, num_heads)
         self.self_attention_dropout = nn.Dropout(dropout_rate)
         self.O = Linear(hidden_size, hidden_size)
-        self.layer_norm1 = LayerNorm(hidden_size)
+        self.layer_norm1 = nn.LayerNorm(hidden_size)
         self.FFN_layer1 = Linear(hidden_size, hidden_size * 2)
         self.FFN_layer2 = Linear(hidden_size * 2, hidden_size)
-        self.layer_norm2 = LayerNorm(hidden_size)
+        self.layer_norm2 = nn.LayerNorm(hidden_size)
 
     def _ffn(self, h):
         y = self.FFN_layer1(h)

@@ -12,7 +12,7 @@ from torch import nn
 from torch.nn import functional as F
 from torch.utils.checkpoint import checkpoint
 
-from .common import LayerNorm, Linear, NodeModelBase, init_params
+from .common import Linear, NodeModelBase, init_params
 
 
 class FeedForwardNetwork(nn.Module):
@@ -52,10 +52,10 @@ class MultiHeadAttention(nn.Module):
 class EncoderLayer(nn.Module):
     def __init__(self, hidden_size, ffn_size, dropout_rate, attention_dropout_rate, num_heads):
         super().__init__()
-        self.self_attention_norm = LayerNorm(hidden_size)
+        self.self_attention_norm = nn.LayerNorm(hidden_size)
         self.self_attention = MultiHeadAttention(hidden_size, attention_dropout_rate, num_heads)
         self.self_attention_dropout = nn.Dropout(dropout_rate)
-        self.ffn_norm = LayerNorm(hidden_size)
+        self.ffn_norm = nn.LayerNorm(hidden_size)
         self.ffn = FeedForwardNetwork(hidden_size, ffn_size)
         self.ffn_dropout = nn.Dropout(dropout_rate)
 
@@ -85,7 +85,7 @@ class NAGphormer(NodeModelBase):
         self.att_embeddings_nope = Linear(input_dim, hidden_dim)
         self.layers = nn.ModuleList([
             EncoderLayer(hidden_dim, ffn_dim, dropout_rate, attention_dropout_rate, num_heads) for _ in range(n_layers)])
-        self.final_ln = LayerNorm(hidden_dim)
+        self.final_ln = nn.LayerNorm(hidden_dim)
         self.out_proj = Linear(hidden_dim, hidden_dim // 2)
         self.attn_layer = Linear(2 * hidden_dim, 1)
         self.Linear1 = Linear(hidden_dim // 2, n_class)

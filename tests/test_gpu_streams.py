@@ -94,8 +94,14 @@ def test_f32_weight_grad(m, n, k, pad):
 
 
 def test_fp32_modules_match_torch():
-    """Linear and LayerNorm of the models against torch's, first and second derivative, rows above and below the split."""
-    from budgetformer_b200.models.common import LayerNorm, Linear
+    """The models' Linear and the row-kernel LayerNorm against torch's, first and second derivative, few and many rows."""
+    from budgetformer_b200.models.common import Linear
+    from budgetformer_b200.ops.norm import layer_norm
+
+    class LayerNorm(torch.nn.LayerNorm):
+        def forward(self, x):
+            return layer_norm(x[0], self.weight, self.bias, self.eps)[None]
+
     for rows in (7, 3000):
         for cls, ref, args in ((Linear, torch.nn.Linear, (24, 40)), (LayerNorm, torch.nn.LayerNorm, (24,))):
             torch.manual_seed(rows)
