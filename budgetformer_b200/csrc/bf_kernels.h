@@ -88,11 +88,9 @@ typedef struct {
   const int* kv_split;              // [n_kv_split, 3] int32: key row, first slot, slot count
   int n_kv_split, n_kv_slots;
   float* kv_partial;                // [n_kv_slots, 2*hl*hn] fp32 scratch
-  // Optional workspace for narrow rows (hl*hn elements of 64 bytes or less), used with kv_task: the first kernel leaves one
-  // contiguous record [q | dout / (Z + eps)] per (row, head) in qg and D / (Z + eps) in cz, and the dK/dV pass gathers
-  // those instead of q, dout and zd separately.
-  void* qg;                         // [n, hl, 2, hn] in the operand dtype, or NULL
-  float* cz;                        // [n, hl] fp32, or NULL
+  // Optional workspace for narrow rows (hl*hn elements of 64 bytes or less): the first kernel leaves one contiguous record
+  // [q | dout] per (row, head), and the dK/dV pass gathers those instead of q and dout separately.
+  void* qg;                         // [n, hl, 2, hn] in the operand dtype, 16-byte aligned, or NULL
   // Optional: dq / dk / dv rows go to the owner of each row (route.n_dest > 0) at column offsets route_cq / _ck / _cv
   // (multiples of 8) of the destination's row, instead of into dq / dk / dv
   bf_attn_route route;

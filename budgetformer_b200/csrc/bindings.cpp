@@ -172,14 +172,13 @@ void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor do
   const int64_t w = (int64_t)p.hl * p.hn;
   LongRows lr = take_long_rows(rowptr, known_max_degree, long_task, long_split, (size_t)w);
   b.long_rows = lr.c;
-  Tensor partial, qg, cz;
+  Tensor partial, qg;
   Tensor ds = torch::empty({std::max<int64_t>(col.numel(), 1), (int64_t)p.hl}, q.options().dtype(torch::kFloat));
   b.ds = ds.data_ptr<float>();
   if (w * q.element_size() <= 64) {
     // narrow rows: one packed record per (query, head) for the dK/dV pass (see bf_attn_bwd_params)
     qg = torch::empty({q.size(0), (int64_t)p.hl, 2, (int64_t)p.hn}, q.options());
-    cz = torch::empty({q.size(0), (int64_t)p.hl}, q.options().dtype(torch::kFloat));
-    b.qg = qg.data_ptr(); b.cz = cz.data_ptr<float>();
+    b.qg = qg.data_ptr();
   }
   TORCH_CHECK(kv_task.has_value() && kv_task->scalar_type() == torch::kInt && kv_task->is_contiguous() && kv_task->size(1) == 4 &&
               ((uintptr_t)kv_task->data_ptr()) % 16 == 0, "kv_task must be contiguous int32 [T, 4]");

@@ -331,6 +331,10 @@ template <typename T, int VN> struct Slices {
 #pragma unroll
     for (int i = 0; i < N; ++i) u[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
   }
+  static __device__ __forceinline__ void put(T* dst, const uint4* u) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) reinterpret_cast<uint4*>(dst)[i] = u[i];
+  }
   static __device__ __forceinline__ void spread(const uint4* u, f2* p) {
 #pragma unroll
     for (int i = 0; i < N; ++i) widen<T>(u[i], p + PP * i);
@@ -640,11 +644,11 @@ struct BwdArgs {
   const int* kv_split;         // [n_kv_split, 3]: key row, first slot, number of slots
   int n_kv_split, n_kv_slots;
   float* kv_partial;           // [n_kv_slots, 2*Hl*HN] fp32
-  // Packed query records for narrow rows (optional): the first kernel writes, per (row, head), [q | dout / (Z + eps)] next to
-  // each other plus one float D / (Z + eps); the dK/dV pass then gathers one contiguous record per edge instead of
-  // three separate short rows (q, dout, (1/Z, D)), which matters when a row of q is only 32 or 64 bytes.
+  // Packed query records for narrow rows (optional): the first kernel writes q and dout of every (row, head) next to each other
+  // and the dK/dV pass gathers one contiguous record per edge instead of two short rows, which matters when a row of q is only 32
+  // or 64 bytes.  dout goes in as it is: dout / (Z + eps) rounded to 16 bits would enter <dout, v> but not D, and the score
+  // gradient is a difference of the two (1.5 times the error in dQ).
   void* qg;                    // [n, Hl, 2, HN] in the operand dtype, or null
-  float* cz;                   // [n, Hl]
   // Routed gradients (route.n_dest > 0): dq / dk / dv rows go to the owner of the row instead of the local buffers, at
   // column offsets cq / ck / cv of the destination's packed row
   Route route;
@@ -658,7 +662,7 @@ __device__ __forceinline__ T* grad_row(const BwdArgs& b, void* local, int col0, 
   return routed<T>(b.route, row, col0);
 }
 
-// What the dK/dV pass needs of every query: 1 / (Z + eps) and D = <dout, out>, or the packed records of narrow rows.
+// What the dK/dV pass needs of every query: 1 / (Z + eps) and D = <dout, out>, and the packed records of narrow rows.
 template <typename T, int HN>
 __global__ void __launch_bounds__(kStreamThreads) edge_attn_bwd_delta_kernel(BwdArgs b, StreamGeo sg) {
   constexpr int VN = wide_elems<T, HN>(), NP = VN / 2, LPH = HN / VN;
@@ -683,22 +687,16 @@ __global__ void __launch_bounds__(kStreamThreads) edge_attn_bwd_delta_kernel(Bwd
   if (b.qg != nullptr) {
     T* rec = static_cast<T*>(b.qg) + hz * 2 * HN + (lt % LPH) * VN;
     S::load(static_cast<const T*>(a.q) + row * a.ldq + off, ou);
-    S::spread(ou, o);
-    S::store(rec, o);
-    const f2 iz = pack2(invz, invz);
-#pragma unroll
-    for (int i = 0; i < NP; ++i) g[i] = mul2(g[i], iz);
-    S::store(rec + HN, g);
-    if ((lt % LPH) == 0) b.cz[hz] = dterm * invz;
-  } else if ((lt % LPH) == 0) {
-    b.zd[hz] = make_float2(invz, dterm);
+    S::put(rec, ou);
+    S::put(rec + HN, gu);
   }
+  if ((lt % LPH) == 0) b.zd[hz] = make_float2(invz, dterm);
 }
 
 // dK/dV over the balanced work list, first of the two passes over the edges.  It gathers q, dout and (1/Z, D) of each query and
 // leaves the score gradient of every (edge, head) in `ds` (fp32, at the edge's own position), so that the dQ pass gathers k alone.
 // The list holds the items of split keys (64 edges each), then the rest sorted by length.
-template <typename T, int HN, int VAR, bool PACKED>
+template <typename T, int HN, int VAR>
 __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bwd_kv_kernel(BwdArgs b, StreamGeo sg) {
   constexpr bool EXPH = VAR == 2;
   constexpr int VN = EXPH ? Vec<T>::N : wide_elems<T, HN>(), NP = VN / 2, LPH = HN / VN;
@@ -725,17 +723,15 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
     return it;
   };
   const int hsafe = on ? head : 0, off = hsafe * HN + (lt % LPH) * VN, w_row = a.hl * HN;
-  const char *qb, *gb, *zb;
-  unsigned long long sq, sgr, szd;
-  if (PACKED) {
+  const char* qb = reinterpret_cast<const char*>(static_cast<const T*>(a.q) + off);
+  const char* gb = reinterpret_cast<const char*>(static_cast<const T*>(b.dout) + off);
+  const char* zb = reinterpret_cast<const char*>(b.zd + hsafe);
+  unsigned long long sq = (unsigned long long)a.ldq * sizeof(T), sgr = (unsigned long long)w_row * sizeof(T);
+  const unsigned long long szd = (unsigned long long)a.hl * sizeof(float2);
+  if (b.qg != nullptr) {
     qb = reinterpret_cast<const char*>(static_cast<const T*>(b.qg) + (long long)hsafe * 2 * HN + (lt % LPH) * VN);
     gb = qb + HN * sizeof(T);
     sq = sgr = (unsigned long long)w_row * 2 * sizeof(T);
-    zb = reinterpret_cast<const char*>(b.cz + hsafe); szd = (unsigned long long)a.hl * sizeof(float);
-  } else {
-    qb = reinterpret_cast<const char*>(static_cast<const T*>(a.q) + off); sq = (unsigned long long)a.ldq * sizeof(T);
-    gb = reinterpret_cast<const char*>(static_cast<const T*>(b.dout) + off); sgr = (unsigned long long)w_row * sizeof(T);
-    zb = reinterpret_cast<const char*>(b.zd + hsafe); szd = (unsigned long long)a.hl * sizeof(float2);
   }
   // fetching side: items two segments ahead, the first query of a segment one segment ahead (see RowFetch)
   int fr = 0, fi = 0, fbeg, flen, beg1, len1, beg2, len2;
@@ -757,8 +753,7 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
     if (fi < flen) {
       S::copy(ring[slot][0], tid, qb + (unsigned)i_row * sq);
       S::copy(ring[slot][1], tid, gb + (unsigned)i_row * sgr);
-      if (PACKED) copy_async<4>(&ring_zd[slot][tid].y, zb + (unsigned)i_row * szd);
-      else copy_async<8>(&ring_zd[slot][tid], zb + (unsigned)i_row * szd);
+      copy_async<8>(&ring_zd[slot][tid], zb + (unsigned)i_row * szd);
       ring_eid[slot][tid] = eid_n;
       if (EXPH) ty = a.etype[eid_n];
     }
@@ -816,8 +811,7 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
       S::read(ring[slot][0], tid, qf);
       S::read(ring[slot][1], tid, gf);
       const int eid = ring_eid[slot][tid];
-      float2 zd = ring_zd[slot][tid];
-      if (PACKED) zd.x = 1.f;
+      const float2 zd = ring_zd[slot][tid];
       const bool t1 = EXPH && ((types >> slot) & 1u);
       float d;
       if (EXPH) {
@@ -1210,8 +1204,7 @@ void launch_kv(const BwdArgs& b, cudaStream_t st) {
   constexpr int VN = VAR == 2 ? Vec<T>::N : wide_elems<T, HN>();
   const StreamGeo s = stream_geo<HN, VN>(b.f.hl, b.n_kv_task, VAR == 2 ? 4 : 3, 8);
   const dim3 grid = stream_grid<HN, VN>(b.f.hl, stream_warps(b.n_kv_task, s, s.per), s);
-  if (b.qg) edge_attn_bwd_kv_kernel<T, HN, VAR, true><<<grid, kStreamThreads, 0, st>>>(b, s);
-  else edge_attn_bwd_kv_kernel<T, HN, VAR, false><<<grid, kStreamThreads, 0, st>>>(b, s);
+  edge_attn_bwd_kv_kernel<T, HN, VAR><<<grid, kStreamThreads, 0, st>>>(b, s);
 }
 
 template <typename T, int HN>
@@ -1380,8 +1373,7 @@ extern "C" int bf_edge_attn_bwd(const bf_attn_params* p, const bf_attn_bwd_param
   b.kv_split = q->kv_split; b.n_kv_split = q->n_kv_split; b.n_kv_slots = q->n_kv_split > 0 ? q->n_kv_slots : 0; b.kv_partial = q->kv_partial;
   if (b.n_kv_split > 0 && (b.kv_split == nullptr || b.kv_partial == nullptr || b.n_kv_slots <= 0 || b.n_kv_slots > b.n_kv_task))
     return (int)cudaErrorInvalidValue;
-  b.qg = (q->qg != nullptr && q->cz != nullptr) ? q->qg : nullptr;
-  b.cz = b.qg ? q->cz : nullptr;
+  b.qg = q->qg;
   b.cq = q->route_cq; b.ck = q->route_ck; b.cv = q->route_cv;
   {
     // a routed row is [.. ck: dk .. cv: dv .. cq: dq ..]: every part must fit the destination's row stride

@@ -54,6 +54,38 @@ def test_attention_streams(n, heads, hn, max_deg, dtype, variant):
         assert float((a.double() - b.double()).norm()) <= tol * scale + 1e-6, (float((a.double() - b.double()).norm()), scale)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("heads,hn", [(1, 8), (1, 16), (1, 32), (2, 16), (4, 8)])
+def test_narrow_rows_keep_the_precision_of_dq(heads, hn, dtype):
+    """Rows of 16 to 64 bytes: dQ against 64 bits is as far off as storing the context and the result in 16 bits makes it (D takes
+    the rounded context), and no further.  dout / (Z + eps) rounded to 16 bits instead of dout gives 1.5 times that."""
+    from budgetformer_b200.graph.attn_graph import AttnGraph
+    from budgetformer_b200.ops.edge_attention import edge_attention
+    n, deg = 6007, 6
+    gen = torch.Generator(device="cuda").manual_seed(hn + heads)
+    dst = torch.arange(n, device="cuda").repeat_interleave(deg)
+    src = torch.randint(0, n, (n * deg,), generator=gen, device="cuda")
+    graph = AttnGraph.from_edge_index(torch.stack([src, dst]), n)
+    q, k, v, dout = (torch.randn(n, heads, hn, generator=gen, device="cuda").to(dtype) for _ in range(4))
+    args = [t.requires_grad_() for t in (q, k, v)]
+    out = edge_attention(*args, graph)
+    dq = torch.autograd.grad(out, q, dout)[0].double()
+
+    kd, vd, g = k.detach().double()[src].view(n, deg, heads, hn), v.detach().double()[src].view(n, deg, heads, hn), dout.double()
+    s = torch.einsum("nhd,nehd->neh", q.detach().double(), kd) / hn ** 0.5
+    w = s.clamp(-5, 5).exp()
+    p = w / (w.sum(1, keepdim=True) + 1e-6)
+    ctx = torch.einsum("neh,nehd->nhd", p, vd)
+
+    def grad(c):
+        ds = p * (torch.einsum("nhd,nehd->neh", g, vd) - (g * c).sum(-1)[:, None]) * (s.abs() < 5)
+        return torch.einsum("neh,nehd->nhd", ds, kd) / hn ** 0.5
+
+    want = grad(ctx)
+    least = float((grad(ctx.to(dtype).double()).to(dtype).double() - want).norm())
+    assert float((dq - want).norm()) <= 1.2 * least, (float((dq - want).norm()) / least, least / float(want.norm()))
+
+
 def test_attention_streams_keep_other_rows_finite():
     """An infinite key / value row reaches the queries that name it and nobody else: stale ring slots are never added."""
     from budgetformer_b200.graph.attn_graph import AttnGraph
