@@ -269,9 +269,9 @@ size_t bf_kv_task_scratch(int n);
 int bf_kv_task_counts(const int* t_rowptr, int n, int chunk, int min_split, int* item_first /* [n+1] */,
                       int* slot_first /* [n+1] */, int* split_first /* [n+1] */, int* by_length, void* scratch,
                       size_t scratch_bytes, cudaStream_t st);
-int bf_kv_task_fill(const int* t_rowptr, const int* item_first, const int* slot_first, const int* split_first,
-                    const int* by_length, int n, int chunk, int n_slots, int n_split, int* tasks /* [T, 4] */,
-                    int* splits /* [S, 3] */, cudaStream_t st);
+// max_tasks / max_splits: rows of `tasks` and `splits`, which may be upper bounds of the totals; nothing is written behind them
+int bf_kv_task_fill(const int* t_rowptr, const int* slot_first, const int* split_first, const int* by_length, int n, int chunk,
+                    int max_tasks, int max_splits, int* tasks /* [T, 4] */, int* splits /* [S, 3] */, cudaStream_t st);
 
 // ---- weight and bias gradient of an fp32 linear layer (linear_f32.cu) -------------------------------------
 // out = [dW (N*K) | db (N, with want_bias)]; partial: bf_f32_dw_slices(M, N, K) times as many floats as out

@@ -39,11 +39,13 @@ void check_qkv(const Tensor& t, const char* name) {
 const int* iptr(const Tensor& t) { return t.data_ptr<int>(); }
 
 // Work items of the CSR rows with more than min_split edges: items of `chunk` edges, split rows, and with `singles` one item
-// for every other row behind them, longest first.  The totals size the outputs: one host read.
+// for every other row behind them, longest first.  The outputs are cut from buffers of the most items that n_edges edges can
+// make, so that the one host read (of the totals) comes last: what is returned is complete, whatever stream uses it next.
 struct RowTasks {
   Tensor tasks, splits, sizes;       // [T, 4], [S, 3], int64 [3] on the host = items, slots, split rows
 };
-RowTasks row_tasks(const Tensor& rowptr, int64_t n, int64_t chunk, int64_t min_split, bool singles, cudaStream_t st) {
+RowTasks row_tasks(const Tensor& rowptr, int64_t n, int64_t n_edges, int64_t chunk, int64_t min_split, bool singles,
+                   cudaStream_t st) {
   auto iopt = rowptr.options();
   Tensor firsts = torch::empty({3, n + 1}, iopt);
   Tensor by_length = singles ? torch::empty({n}, iopt) : Tensor();
@@ -55,24 +57,28 @@ RowTasks row_tasks(const Tensor& rowptr, int64_t n, int64_t chunk, int64_t min_s
                                  firsts[1].data_ptr<int>(), firsts[2].data_ptr<int>(), by, scratch.data_ptr(), bytes, st),
                "kv_task_counts");
   }
+  const int64_t max_splits = std::min(n, n_edges / (min_split + 1)), max_slots = max_splits > 0 ? n_edges / chunk + max_splits : 0;
+  const int64_t max_items = singles ? n + max_slots : max_slots;
+  TORCH_CHECK(max_items < (int64_t)INT32_MAX, "too many work items: ", max_items);
   RowTasks r;
+  r.tasks = torch::empty({max_items, 4}, iopt);
+  r.splits = torch::empty({max_splits, 3}, iopt);
+  check_cuda(bf_kv_task_fill(rowptr.data_ptr<int>(), firsts[1].data_ptr<int>(), firsts[2].data_ptr<int>(), by, (int)n, (int)chunk,
+                             (int)max_items, (int)max_splits, r.tasks.data_ptr<int>(), r.splits.data_ptr<int>(), st), "kv_task_fill");
   r.sizes = firsts.select(1, n).to(torch::kCPU).to(torch::kLong);
   const int64_t n_items = r.sizes[singles ? 0 : 1].item<int64_t>(), n_splits = r.sizes[2].item<int64_t>();
-  r.tasks = torch::empty({n_items, 4}, iopt);
-  r.splits = torch::empty({n_splits, 3}, iopt);
-  if (n_items > 0)
-    check_cuda(bf_kv_task_fill(rowptr.data_ptr<int>(), firsts[0].data_ptr<int>(), firsts[1].data_ptr<int>(),
-                               firsts[2].data_ptr<int>(), by, (int)n, (int)chunk, (int)r.sizes[1].item<int64_t>(), (int)n_splits,
-                               r.tasks.data_ptr<int>(), r.splits.data_ptr<int>(), st), "kv_task_fill");
+  TORCH_CHECK(n_items <= max_items && n_splits <= max_splits, "the row pointer names more than the ", n_edges, " edges of the list");
+  r.tasks = r.tasks.narrow(0, 0, n_items);
+  r.splits = r.splits.narrow(0, 0, n_splits);
   return r;
 }
 
-// (tasks, splits) of the query rows with more than BF_LONG_ROW edges (empty tensors: none)
-std::vector<Tensor> long_row_tasks(Tensor rowptr) {
+// (tasks, splits) of the query rows with more than BF_LONG_ROW of the n_edges edges (empty tensors: none)
+std::vector<Tensor> long_row_tasks(Tensor rowptr, int64_t n_edges) {
   TORCH_CHECK(rowptr.is_cuda() && rowptr.scalar_type() == torch::kInt && rowptr.is_contiguous() && rowptr.numel() >= 1);
   c10::cuda::CUDAGuard guard(rowptr.device());
   if (rowptr.numel() == 1) return {torch::empty({0, 4}, rowptr.options()), torch::empty({0, 3}, rowptr.options())};
-  RowTasks r = row_tasks(rowptr, rowptr.numel() - 1, BF_LONG_CHUNK, BF_LONG_ROW, false, at::cuda::getCurrentCUDAStream());
+  RowTasks r = row_tasks(rowptr, rowptr.numel() - 1, n_edges, BF_LONG_CHUNK, BF_LONG_ROW, false, at::cuda::getCurrentCUDAStream());
   return {r.tasks, r.splits};
 }
 
@@ -82,7 +88,7 @@ struct LongRows {
   Tensor tasks, splits, partial;
   bf_long_rows c{};
 };
-LongRows take_long_rows(const Tensor& rowptr, int64_t known_max, const OptTensor& tasks, const OptTensor& splits, size_t pitch) {
+LongRows take_long_rows(const Tensor& rowptr, int64_t n_edges, int64_t known_max, const OptTensor& tasks, const OptTensor& splits, size_t pitch) {
   LongRows r;
   if (known_max >= 0 && known_max <= BF_LONG_ROW) return r;
   if (tasks.has_value() && splits.has_value()) {
@@ -92,7 +98,7 @@ LongRows take_long_rows(const Tensor& rowptr, int64_t known_max, const OptTensor
     TORCH_CHECK(r.splits.is_cuda() && r.splits.scalar_type() == torch::kInt && r.splits.is_contiguous() && r.splits.dim() == 2 &&
                 r.splits.size(1) == 3, "long rows: splits int32 [S, 3]");
   } else {
-    auto v = long_row_tasks(rowptr);
+    auto v = long_row_tasks(rowptr, n_edges);
     r.tasks = v[0]; r.splits = v[1];
   }
   if (r.tasks.size(0) == 0) return r;
@@ -146,7 +152,7 @@ void edge_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor ro
   c10::cuda::CUDAGuard guard(q.device());
   bf_attn_params p{};
   fill_common(p, q, k, v, out, z, rowptr, col, etype, etab, variant, dropout_p, seed, out_drop);
-  LongRows lr = take_long_rows(rowptr, known_max_degree, long_task, long_split, bf_attn_fwd_long_pitch(p.hl, p.hn));
+  LongRows lr = take_long_rows(rowptr, col.numel(), known_max_degree, long_task, long_split, bf_attn_fwd_long_pitch(p.hl, p.hn));
   const bf_attn_route r = parse_route(route, 3);
   check_cuda(bf_edge_attn_fwd_routed(&p, &r, &lr.c, at::cuda::getCurrentCUDAStream()), "edge_attn_fwd");
 }
@@ -170,7 +176,7 @@ void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor do
   b.t_rowptr = iptr(t_rowptr); b.t_row = iptr(t_row); b.t_eid = iptr(t_eid);
   b.detab = detab.has_value() ? detab->data_ptr<float>() : nullptr;
   const int64_t w = (int64_t)p.hl * p.hn;
-  LongRows lr = take_long_rows(rowptr, known_max_degree, long_task, long_split, (size_t)w);
+  LongRows lr = take_long_rows(rowptr, col.numel(), known_max_degree, long_task, long_split, (size_t)w);
   b.long_rows = lr.c;
   Tensor partial, qg;
   Tensor ds = torch::empty({std::max<int64_t>(col.numel(), 1), (int64_t)p.hl}, q.options().dtype(torch::kFloat));
@@ -409,7 +415,7 @@ std::vector<Tensor> graph_transpose(Tensor rowptr, Tensor col, int64_t n, int64_
                                   t_row.data_ptr<int>(), t_eid.data_ptr<int>(), scratch.data_ptr(), bytes, st),
                "graph_transpose");
   }
-  RowTasks r = row_tasks(t_rowptr, n, chunk, chunk, true, st);
+  RowTasks r = row_tasks(t_rowptr, n, n_edges, chunk, chunk, true, st);
   return {t_rowptr, t_row, t_eid, r.tasks, r.splits, r.sizes};
 }
 

@@ -77,39 +77,41 @@ __global__ void task_counts_kernel(const int* __restrict__ t_rowptr, int n, int 
 }
 
 // The list starts with the items of all split keys in key order (full-length items: the long work is scheduled first and runs
-// side by side in a warp); an item of a split key sits at its partial-slot index.  One warp per key: lane l writes items l, l+32,
-// ... (hub keys own thousands of items).  `keys` lists the split keys; without it all n keys are looked through.
-__global__ void task_fill_kernel(const int* __restrict__ t_rowptr, const int* __restrict__ item_first,
-                                 const int* __restrict__ slot_first, const int* __restrict__ split_first,
-                                 const int* __restrict__ keys, int n, int chunk, int4* __restrict__ tasks, int* __restrict__ splits) {
+// side by side in a warp); an item of a split key sits at its partial-slot index.  A lane looks at one key, and the warp writes the
+// items of those that are split one key after the other, 32 items at a time (hub keys own thousands).
+__global__ void task_fill_kernel(const int* __restrict__ t_rowptr, const int* __restrict__ slot_first,
+                                 const int* __restrict__ split_first, int n, int chunk, int max_tasks, int max_splits,
+                                 int4* __restrict__ tasks, int* __restrict__ splits) {
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = (int)(gt >> 5), lane = (int)(gt & 31);
-  if (i >= n) return;
-  const int k = keys != nullptr ? keys[i] : i;
-  const int cnt = item_first[k + 1] - item_first[k];
-  if (cnt <= 1) return;
-  const int beg = t_rowptr[k], end = t_rowptr[k + 1], s0 = slot_first[k];
-  for (int c = lane; c < cnt; c += 32) {
-    const int b = beg + c * chunk;
-    int e = b + chunk;
-    if (e > end) e = end;
-    tasks[s0 + c] = make_int4(k, b, e, s0 + c);
-  }
-  if (lane == 0) {
+  const int lane = threadIdx.x & 31;
+  int s0 = 0, cnt = 0;
+  if (gt < n) { s0 = slot_first[gt]; cnt = slot_first[gt + 1] - s0; }
+  unsigned left = __ballot_sync(0xffffffffu, cnt > 0);
+  while (left != 0) {
+    const int src = __ffs(left) - 1;
+    left &= left - 1;
+    const int first = __shfl_sync(0xffffffffu, s0, src), m = __shfl_sync(0xffffffffu, cnt, src);
+    const int k = (int)(gt - lane) + src;
+    const int beg = t_rowptr[k], end = t_rowptr[k + 1];
+    for (int c = lane; c < m && first + c < max_tasks; c += 32) {
+      const int b = beg + c * chunk;
+      tasks[first + c] = make_int4(k, b, min(b + chunk, end), first + c);
+    }
     const int s = split_first[k];
-    splits[3 * s] = k; splits[3 * s + 1] = s0; splits[3 * s + 2] = cnt;
+    if (lane == 0 && s < max_splits) { splits[3 * s] = k; splits[3 * s + 1] = first; splits[3 * s + 2] = m; }
   }
 }
 
 // Behind them the single item of every other key, longest first (key order among equals): the lane groups of a warp that work
 // on neighbouring items finish together.  Sorting 2.9 M keys by their 7-bit length is one radix pass; a thread per key instead
 // of a warp writes the list in a tenth of the time.
-__global__ void task_singles_kernel(const int* __restrict__ t_rowptr, const int* __restrict__ keys, int n_single,
+__global__ void task_singles_kernel(const int* __restrict__ t_rowptr, const int* __restrict__ slot_first,
+                                    const int* __restrict__ split_first, const int* __restrict__ keys, int n, int max_tasks,
                                     int4* __restrict__ tasks) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_single) return;
-  const int k = keys[i];
-  tasks[i] = make_int4(k, t_rowptr[k], t_rowptr[k + 1], -1);
+  if (i >= n - split_first[n]) return;
+  const int k = keys[i], at = slot_first[n] + i;
+  if (at < max_tasks) tasks[at] = make_int4(k, t_rowptr[k], t_rowptr[k + 1], -1);
 }
 
 int bits_for(int n) {
@@ -192,19 +194,15 @@ extern "C" size_t bf_kv_task_scratch(int n) {
   return ((6 * (size_t)n * sizeof(int) + 255) & ~(size_t)255) + ((tmp + 255) & ~(size_t)255) + 256;
 }
 
-// Phase 2: write the items and the split list (n_split and n_slots read back by the caller from the prefix sums).  With
-// `by_length` (of phase 1) the keys that are not split get their single items; without it they get none.
-extern "C" int bf_kv_task_fill(const int* t_rowptr, const int* item_first, const int* slot_first, const int* split_first,
-                               const int* by_length, int n, int chunk, int n_slots, int n_split, int* tasks, int* splits,
-                               cudaStream_t st) {
+// Phase 2: write the items and the split list.  The totals are read on the device, so the caller can read them back last: then
+// the list is complete when the host knows its length, whatever stream uses it.  With `by_length` (of phase 1) the keys that are
+// not split get their single items; without it they get none.
+extern "C" int bf_kv_task_fill(const int* t_rowptr, const int* slot_first, const int* split_first, const int* by_length, int n,
+                               int chunk, int max_tasks, int max_splits, int* tasks, int* splits, cudaStream_t st) {
+  if (n <= 0) return 0;
   int4* out = reinterpret_cast<int4*>(tasks);
-  const int n_single = n - n_split;
-  if (n_split > 0) {
-    const int rows = by_length != nullptr ? n_split : n;
-    task_fill_kernel<<<(unsigned)(((long long)rows * 32 + 255) / 256), 256, 0, st>>>(
-        t_rowptr, item_first, slot_first, split_first, by_length != nullptr ? by_length + n_single : nullptr, rows, chunk, out, splits);
-  }
-  if (by_length != nullptr && n_single > 0)
-    task_singles_kernel<<<(n_single + 255) / 256, 256, 0, st>>>(t_rowptr, by_length, n_single, out + n_slots);
+  const unsigned blocks = (unsigned)(((long long)n + 255) / 256);
+  if (max_splits > 0) task_fill_kernel<<<blocks, 256, 0, st>>>(t_rowptr, slot_first, split_first, n, chunk, max_tasks, max_splits, out, splits);
+  if (by_length != nullptr) task_singles_kernel<<<blocks, 256, 0, st>>>(t_rowptr, slot_first, split_first, by_length, n, max_tasks, out);
   return (int)cudaGetLastError();
 }

@@ -15,6 +15,7 @@ reference's COO form so both representations are accepted by every model.
 """
 from __future__ import annotations
 
+import threading
 from dataclasses import dataclass, field
 from typing import Optional
 
@@ -22,6 +23,7 @@ import torch
 
 LONG_ROW = 128     # query rows with more edges are cut into work items of LONG_CHUNK edges (csrc/bf_kernels.h: BF_LONG_ROW,
 LONG_CHUNK = 64    # BF_LONG_CHUNK)
+_LIST_LOCKS = tuple(threading.Lock() for _ in range(64))   # one thread makes a graph's lists, the others wait for it
 KV_TASK_EDGES = 64  # edges per work item of the dK/dV pass (32 and 128 both measured slower on the 2.9 M-node graph)
 
 
@@ -144,6 +146,24 @@ class AttnGraph:
                   self.q_task, self.q_split, getattr(self, "_totals", None)):
             if t is not None and t.is_cuda:
                 t.record_stream(stream)
+        self.__dict__.setdefault("_list_users", set()).update(
+            (kind, stream.cuda_stream) for kind, made in (("long", self.q_task), ("by key", self.t_rowptr)) if made is not None)
+
+    def _use_lists(self, kind: str, tensors) -> None:
+        """The lists that the graph makes of itself on first use are complete by then, so any stream may read them; the caching
+        allocator learns here which streams do (the one that made them is the first)."""
+        if not self.col.is_cuda:
+            return
+        stream = torch.cuda.current_stream(self.col.device)
+        users = self.__dict__.setdefault("_list_users", set())
+        if (kind, stream.cuda_stream) not in users:
+            for t in tensors:
+                if t is not None and t.is_cuda:
+                    t.record_stream(stream)
+            users.add((kind, stream.cuda_stream))
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_list_users"}     # streams of this process
 
     def row_ids(self) -> torch.Tensor:
         """Query id of every edge (int64), i.e. ``edge_index[1]`` of the COO form."""
@@ -160,28 +180,41 @@ class AttnGraph:
 
     def long_rows(self):
         """``(tasks, splits)`` of the query rows with more than ``LONG_ROW`` edges, for the device kernels; ``(None, None)``
-        when the known degree bound rules them out.  Made once per graph (one host read of the list's length)."""
+        when the known degree bound rules them out.  Made once per graph; one host read, behind the kernels that write the list:
+        it is complete for every stream by the time the graph holds it."""
         if self.max_degree is not None and self.max_degree <= LONG_ROW:
             return None, None
         if self.q_task is None:
             from ..ops import _ext
-            self.q_task, self.q_split = _ext.load().long_row_tasks(self.rowptr)
-            _ext.count_launches(5)
+            with _LIST_LOCKS[id(self) // 64 % 64]:
+                if self.q_task is None:
+                    task, self.q_split = _ext.load().long_row_tasks(self.rowptr, self.num_edges)
+                    _ext.count_launches(5)
+                    self.q_task = task                     # last: whoever finds it finds the other
+        self._use_lists("long", (self.q_task, self.q_split))
         return self.q_task, self.q_split
 
     def ensure_transpose(self) -> "AttnGraph":
-        """Build the by-key CSR (deterministic: stable sort keeps query order inside a key's row)."""
-        if self.t_rowptr is not None:
-            return self
+        """Build the by-key CSR (deterministic: stable sort keeps query order inside a key's row).  Complete for every stream
+        when this returns (the host read of the work list's length comes last)."""
+        if self.t_rowptr is None:
+            with _LIST_LOCKS[id(self) // 64 % 64]:
+                if self.t_rowptr is None:
+                    self._build_transpose()
+        self._use_lists("by key", (self.t_rowptr, self.t_row, self.t_eid, self.t_task, self.t_split))
+        return self
+
+    def _build_transpose(self) -> None:
         if self.col.is_cuda and self.col.dtype == torch.int32 and self.rowptr.dtype == torch.int32:
             # device graphs: radix sort over the node-id bits + compaction kernels (csrc/graph_transpose.cu)
             from ..ops import _ext
             t_rowptr, t_row, t_eid, tasks, splits, sizes = _ext.load().graph_transpose(
                 self.rowptr.contiguous(), self.col.contiguous(), int(self.num_rows), int(KV_TASK_EDGES))
             _ext.count_launches(9)
-            self.t_rowptr, self.t_row, self.t_eid = t_rowptr, t_row, t_eid
+            self.t_row, self.t_eid = t_row, t_eid
             self.t_task, self.t_split, self.kv_slots = tasks, splits, int(sizes[1])
-            return self
+            self.t_rowptr = t_rowptr                       # last: whoever finds it finds the others
+            return
         col64 = self.col.to(torch.int64)
         _, perm = torch.sort(col64, stable=True)
         rows = self.row_ids()
@@ -190,9 +223,9 @@ class AttnGraph:
         t_rowptr = torch.zeros(self.num_rows + 1, dtype=torch.int64, device=self.device)
         if self.num_edges:
             t_rowptr[1:] = torch.cumsum(torch.bincount(col64, minlength=self.num_rows), 0)
-        self.t_rowptr = t_rowptr.to(torch.int32)
-        self._build_kv_tasks(t_rowptr)
-        return self
+        t_rowptr32 = t_rowptr.to(torch.int32)
+        self._build_kv_tasks(t_rowptr)                     # ends in a host read of what it made
+        self.t_rowptr = t_rowptr32
 
     def _build_kv_tasks(self, t_rowptr: torch.Tensor) -> None:
         """Work list of the dK/dV pass.  Key popularity is heavy-tailed (a hub is the key of 10^4-10^5 edges), so a

@@ -86,6 +86,39 @@ def test_narrow_rows_keep_the_precision_of_dq(heads, hn, dtype):
     assert float((dq - want).norm()) <= 1.2 * least, (float((dq - want).norm()) / least, least / float(want.norm()))
 
 
+@pytest.mark.parametrize("virtual_node", [False, True])
+def test_lists_of_a_graph_serve_every_stream(virtual_node):
+    """The lists that a graph makes of itself on first use are complete when the host gets them (nothing is queued behind the read
+    of their length), so another stream may use them at once; forward and backward on two streams, one after the other."""
+    from budgetformer_b200.graph.attn_graph import AttnGraph, add_virtual_node
+    from budgetformer_b200.ops.edge_attention import edge_attention
+    graph = _graph(4001, 300, 5, False)
+    if virtual_node:
+        graph.max_degree = 300
+        graph = add_virtual_node(graph, 4001, 4001)
+    fresh = AttnGraph(graph.num_rows, graph.rowptr, graph.col)
+    torch.cuda.synchronize()
+    fresh.long_rows()
+    assert torch.cuda.current_stream().query()
+    fresh.ensure_transpose()
+    assert torch.cuda.current_stream().query()
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v, dout = (torch.randn(graph.num_rows, 4, 16, generator=gen, device="cuda") for _ in range(4))
+    want = _reference(q, k, v, dout, graph, None, "plain", 0.0, 0)
+    args = [t.requires_grad_() for t in (q, k, v)]
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(2):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            out = edge_attention(*args, graph)
+            got.append([out] + list(torch.autograd.grad(out, args, dout)))
+    torch.cuda.synchronize()
+    assert len({s for kind, s in graph._list_users if kind == "long"}) == 2
+    for res in got:
+        for a, b in zip(res, want):
+            assert float((a.double() - b.double()).norm()) <= 2e-5 * (float(b.double().norm()) + float(dout.norm()))
+
+
 def test_attention_streams_keep_other_rows_finite():
     """An infinite key / value row reaches the queries that name it and nobody else: stale ring slots are never added."""
     from budgetformer_b200.graph.attn_graph import AttnGraph
