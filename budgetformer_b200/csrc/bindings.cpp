@@ -675,8 +675,8 @@ std::vector<Tensor> layernorm_bwd(Tensor dy, Tensor x, Tensor stats, Tensor gamm
 // [dY^T X flattened | column sums of dY] of fp32 matrices, one flat tensor
 Tensor f32_weight_grad(Tensor dy, Tensor x, bool want_bias) {
   TORCH_CHECK(dy.is_cuda() && dy.dim() == 2 && x.dim() == 2 && dy.device() == x.device() && dy.scalar_type() == torch::kFloat &&
-              x.scalar_type() == torch::kFloat && dy.stride(1) == 1 && x.stride(1) == 1 && dy.size(0) == x.size(0) && dy.size(0) > 0 &&
-              dy.size(1) > 0 && x.size(1) > 0, "f32_weight_grad: fp32 [M, N] and [M, K]");
+              x.scalar_type() == torch::kFloat && (dy.stride(1) == 1 || dy.size(1) == 1) && (x.stride(1) == 1 || x.size(1) == 1) &&
+              dy.size(0) == x.size(0) && dy.size(0) > 0 && dy.size(1) > 0 && x.size(1) > 0, "f32_weight_grad: fp32 [M, N] and [M, K]");
   c10::cuda::CUDAGuard guard(dy.device());
   const int64_t m = dy.size(0), n = dy.size(1), k = x.size(1), size = n * k + (want_bias ? n : 0);
   Tensor out = torch::empty({size}, dy.options());

@@ -206,6 +206,12 @@ def plain_eager() -> bool:
                 or torch.autograd.forward_ad._current_level >= 0)
 
 
+def _unit_columns(t: torch.Tensor) -> torch.Tensor:
+    """``t`` with neighbouring columns next to each other.  One column has no neighbour: its stride is arbitrary (a transposed
+    row), and ``contiguous()`` would leave it as it is."""
+    return t if t.stride(1) == 1 or t.size(1) == 1 else t.contiguous()
+
+
 class _LinearF32(torch.autograd.Function):
     """``torch.nn.functional.linear`` on fp32 with weight and bias gradient from ``csrc/linear_f32.cu``."""
 
@@ -226,8 +232,7 @@ class _LinearF32(torch.autograd.Function):
             g, a = dy.reshape(-1, n), x.reshape(-1, k)
             if torch.is_grad_enabled():                    # a second derivative is wanted: differentiable operators
                 return dx, g.t() @ a, g.sum(0) if ctx.has_bias else None
-            flat = _ext.load().f32_weight_grad(g if g.stride(1) == 1 else g.contiguous(), a if a.stride(1) == 1 else a.contiguous(),
-                                               ctx.has_bias)
+            flat = _ext.load().f32_weight_grad(_unit_columns(g), _unit_columns(a), ctx.has_bias)
             _ext.count_launches(2)
             dw, db = flat[:n * k].view(n, k), flat[n * k:] if ctx.has_bias else None
         return dx, dw, db

@@ -158,6 +158,26 @@ def test_f32_weight_grad(m, n, k, pad):
             assert bool(((flat[n * k:].double() - db).abs() <= m * 2.0 ** -24 * dy.double().abs().sum(0) + 1e-30).all())
 
 
+@pytest.mark.parametrize("out_features,in_features", [(1, 24), (24, 1), (1, 1)])
+@pytest.mark.parametrize("rows", [128, 1003])
+def test_fp32_linear_of_one_column(out_features, in_features, rows):
+    """One output or one feature whose matrix is a transposed row: its column stride is not 1 and means nothing."""
+    from budgetformer_b200.ops.gemm import linear_f32
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(in_features, rows, generator=gen, device="cuda").t() if in_features == 1 else torch.randn(rows, in_features, device="cuda")
+    w = torch.randn(out_features, in_features, generator=gen, device="cuda", requires_grad=True)
+    b = torch.randn(out_features, generator=gen, device="cuda", requires_grad=True)
+    probe = torch.randn(out_features, rows, generator=gen, device="cuda")
+    for loss in (lambda y: (y.t() * probe).sum(), lambda y: torch.softmax(y.t(), 1).pow(2).sum(), lambda y: y.sum()):
+        got = torch.autograd.grad(loss(linear_f32(x, w, b)), (w, b))
+        wd, bd = w.detach().double().requires_grad_(), b.detach().double().requires_grad_()
+        y = torch.nn.functional.linear(x.double(), wd, bd)
+        want = torch.autograd.grad(loss(y), (wd, bd))
+        for u, v in zip(got, want):
+            # sums of `rows` products of values of order 1 in any order, and fp32 rounding of dy itself
+            assert u.shape == v.shape and float((u.double() - v).abs().max()) <= rows * 2.0 ** -23
+
+
 def test_fp32_modules_match_torch():
     """The models' Linear and the row-kernel LayerNorm against torch's, first and second derivative, few and many rows."""
     from budgetformer_b200.models.common import Linear
