@@ -206,6 +206,13 @@ def plain_eager() -> bool:
                 or torch.autograd.forward_ad._current_level >= 0)
 
 
+def plain_gradient(dy: torch.Tensor) -> bool:
+    """False for the gradients of ``is_grads_batched`` (which set no transform that ``plain_eager`` could see), of transforms and
+    of subclasses: a kernel would take their storage for the matrix they stand for."""
+    return (type(dy) is torch.Tensor and not torch._C._functorch.is_legacy_batchedtensor(dy)
+            and not torch._C._functorch.is_functorch_wrapped_tensor(dy) and plain_eager())
+
+
 def _unit_columns(t: torch.Tensor) -> torch.Tensor:
     """``t`` with neighbouring columns next to each other.  One column has no neighbour: its stride is arbitrary (a transposed
     row), and ``contiguous()`` would leave it as it is."""
@@ -230,7 +237,7 @@ class _LinearF32(torch.autograd.Function):
         dw = db = None
         if need_w or need_b:
             g, a = dy.reshape(-1, n), x.reshape(-1, k)
-            if torch.is_grad_enabled():                    # a second derivative is wanted: differentiable operators
+            if torch.is_grad_enabled() or not plain_gradient(dy):      # a second derivative, or many at once: PyTorch's operators
                 return dx, g.t() @ a, g.sum(0) if ctx.has_bias else None
             flat = _ext.load().f32_weight_grad(_unit_columns(g), _unit_columns(a), ctx.has_bias)
             _ext.count_launches(2)

@@ -209,3 +209,18 @@ def test_two_phase_sparse_attention_equals_one_pass():
     two = core.sparse_aggregate_phase(ctx, v).reshape(1, n, -1)
     one = core(q, k, v, None, ei, "sparse")
     assert torch.allclose(one, two, atol=1e-5)
+
+
+def test_linear_gradient_under_batched_gradients():
+    """The fp32 linear function's own backward pass, given several gradients at once (``is_grads_batched``, a vectorised
+    Jacobian), returns what PyTorch's linear layer does."""
+    from budgetformer_b200.ops.gemm import _LinearF32
+    gen = torch.Generator().manual_seed(5)
+    x, w, b = (torch.randn(*size, generator=gen, requires_grad=True) for size in ((1, 9, 4), (3, 4), (3,)))
+    dys = torch.randn(5, 1, 9, 3, generator=gen)
+    got = torch.autograd.grad(_LinearF32.apply(x, w, b), (x, w, b), dys, is_grads_batched=True)
+    want = torch.autograd.grad(torch.nn.functional.linear(x, w, b), (x, w, b), dys, is_grads_batched=True)
+    for u, v in zip(got, want):
+        assert u.shape == v.shape and torch.allclose(u, v, rtol=1e-5, atol=1e-5)
+    jac = lambda f: torch.autograd.functional.jacobian(lambda t: f(x, t, b).sum(1), w, vectorize=True)
+    assert torch.allclose(jac(_LinearF32.apply), jac(torch.nn.functional.linear), rtol=1e-5, atol=1e-5)
