@@ -256,7 +256,7 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     weight and bias gradients come from this package's kernel."""
     if (x.is_cuda and x.dtype == weight.dtype == torch.float32 and (bias is None or bias.dtype == torch.float32)
             and type(x) is torch.Tensor and x.dim() >= 2 and weight.device == x.device
-            and x.numel() >= LINEAR_F32_MIN_ROWS * weight.size(1) and torch.is_grad_enabled() and weight.requires_grad
+            and weight.numel() > 0 and x.numel() >= LINEAR_F32_MIN_ROWS * weight.size(1) and torch.is_grad_enabled() and weight.requires_grad
             and not torch.is_autocast_enabled("cuda") and plain_eager()):
         return _LinearF32.apply(x, weight, bias)
     return torch.nn.functional.linear(x, weight, bias)

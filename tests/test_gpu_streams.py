@@ -178,6 +178,21 @@ def test_fp32_linear_of_one_column(out_features, in_features, rows):
             assert u.shape == v.shape and float((u.double() - v).abs().max()) <= rows * 2.0 ** -23
 
 
+@pytest.mark.parametrize("out_features,in_features", [(0, 8), (8, 0), (0, 0)])
+def test_fp32_linear_of_no_width(out_features, in_features):
+    """No outputs or no features: zeros and empty tensors, as PyTorch's linear layer gives."""
+    from budgetformer_b200.ops.gemm import linear_f32
+    x = torch.randn(300, in_features, device="cuda", requires_grad=True)
+    w = torch.randn(out_features, in_features, device="cuda", requires_grad=True)
+    b = torch.randn(out_features, device="cuda", requires_grad=True)
+    res = []
+    for f in (linear_f32, torch.nn.functional.linear):
+        y = f(x, w, b)
+        res.append([y] + list(torch.autograd.grad(y.sum(), (x, w, b))))
+    for u, v in zip(*res):
+        assert u.shape == v.shape and torch.equal(u, v)
+
+
 def test_fp32_modules_match_torch():
     """The models' Linear and the row-kernel LayerNorm against torch's, first and second derivative, few and many rows."""
     from budgetformer_b200.models.common import Linear
