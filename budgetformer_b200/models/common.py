@@ -27,11 +27,20 @@ def init_params(module: nn.Module, n_layers: int) -> None:
         module.weight.data.normal_(mean=0.0, std=0.02)
 
 
-class Linear(nn.Linear):
-    """``nn.Linear`` whose fp32 gradients run on this package's kernel (see ``ops.gemm.linear_f32``)."""
+def plain_module(module: nn.Module, cls) -> bool:
+    """``module`` is a ``cls`` and calling it does no more than its ``forward``: no hooks, its own or global ones, no subclass or
+    parametrisation, no ``forward`` put on the instance.  Only then may its parameters be used in its place."""
+    return (type(module) is cls and "forward" not in module.__dict__
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
+                     or nn.modules.module._has_any_global_hook()))
 
-    def forward(self, x):
-        return linear_f32(x, self.weight, self.bias)
+
+def linear(module: nn.Linear, x: torch.Tensor) -> torch.Tensor:
+    """``module(x)``; on fp32 CUDA tensors with the gradients of ``ops.gemm.linear_f32``.  The modules stay ``nn.Linear``: scripting,
+    symbolic tracing and dynamic quantisation go by that class."""
+    if type(x) is torch.Tensor and x.is_cuda and x.dtype == torch.float32 and plain_module(module, nn.Linear):
+        return linear_f32(x, module.weight, module.bias)
+    return module(x)
 
 
 class SparseCoreAttention(nn.Module):

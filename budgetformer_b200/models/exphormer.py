@@ -13,7 +13,7 @@ from torch.utils.checkpoint import checkpoint
 
 from ..parallel.initialize import get_sequence_parallel_group, get_sequence_parallel_rank
 from ..parallel.sp_ops import DistributedAttentionNodeLevel
-from .common import Linear, NodeModelBase, SparseCoreAttention, encode_features, init_params
+from .common import NodeModelBase, SparseCoreAttention, encode_features, init_params, linear
 
 
 class ExphormerCoreAttention(SparseCoreAttention):
@@ -24,11 +24,11 @@ class ExphormerCoreAttention(SparseCoreAttention):
         super().__init__(hidden_size, attention_dropout_rate, num_heads)
         hidden = num_heads * self.hidden_size_per_attention_head
         self.edge_type_emb = nn.Embedding(self.N_EDGE_TYPES, hidden)
-        self.edge_proj = Linear(hidden, hidden, bias=False)
+        self.edge_proj = nn.Linear(hidden, hidden, bias=False)
 
     def edge_table(self):
         hl = self.num_attention_heads_per_partition
-        tab = self.edge_proj(self.edge_type_emb.weight).view(self.N_EDGE_TYPES, self.num_heads,
+        tab = linear(self.edge_proj, self.edge_type_emb.weight).view(self.N_EDGE_TYPES, self.num_heads,
                                                              self.hidden_size_per_attention_head)
         if hl != self.num_heads:
             r = get_sequence_parallel_rank()
@@ -44,17 +44,17 @@ class MultiHeadAttention(nn.Module):
         super().__init__()
         self.num_heads = num_heads
         self.att_size = hidden_size // num_heads
-        self.linear_q = Linear(hidden_size, num_heads * self.att_size, bias=False)
-        self.linear_k = Linear(hidden_size, num_heads * self.att_size, bias=False)
-        self.linear_v = Linear(hidden_size, num_heads * self.att_size, bias=False)
+        self.linear_q = nn.Linear(hidden_size, num_heads * self.att_size, bias=False)
+        self.linear_k = nn.Linear(hidden_size, num_heads * self.att_size, bias=False)
+        self.linear_v = nn.Linear(hidden_size, num_heads * self.att_size, bias=False)
         self.dist_attn = DistributedAttentionNodeLevel(
             ExphormerCoreAttention(hidden_size, attention_dropout_rate, num_heads), get_sequence_parallel_group())
 
     def forward(self, x, attn_bias=None, edge_index=None, attn_type=None):
         b = x.size(0)
-        q = self.linear_q(x).view(b, -1, self.num_heads, self.att_size)
-        k = self.linear_k(x).view(b, -1, self.num_heads, self.att_size)
-        v = self.linear_v(x).view(b, -1, self.num_heads, self.att_size)
+        q = linear(self.linear_q, x).view(b, -1, self.num_heads, self.att_size)
+        k = linear(self.linear_k, x).view(b, -1, self.num_heads, self.att_size)
+        v = linear(self.linear_v, x).view(b, -1, self.num_heads, self.att_size)
         return self.dist_attn(q, k, v, attn_bias, edge_index, attn_type)
 
 
@@ -64,8 +64,8 @@ class EncoderLayer(nn.Module):
         self.self_attention = MultiHeadAttention(hidden_size, attention_dropout_rate, num_heads)
         self.dropout1 = nn.Dropout(dropout_rate)
         self.norm1 = nn.BatchNorm1d(hidden_size)
-        self.ffn1 = Linear(hidden_size, hidden_size * 2)
-        self.ffn2 = Linear(hidden_size * 2, hidden_size)
+        self.ffn1 = nn.Linear(hidden_size, hidden_size * 2)
+        self.ffn2 = nn.Linear(hidden_size * 2, hidden_size)
         self.ff_dropout1 = nn.Dropout(dropout_rate)
         self.ff_dropout2 = nn.Dropout(dropout_rate)
         self.norm2 = nn.BatchNorm1d(hidden_size)
@@ -80,8 +80,8 @@ class EncoderLayer(nn.Module):
         return norm(x.reshape(b * n, c)).view(b, n, c)
 
     def _ffn(self, h):
-        out = self.ff_dropout1(F.relu(self.ffn1(h)))
-        out = self.ff_dropout2(self.ffn2(out))
+        out = self.ff_dropout1(F.relu(linear(self.ffn1, h)))
+        out = self.ff_dropout2(linear(self.ffn2, out))
         return self._bn(self.norm2, h + out)
 
     def forward_attn_only(self, x, attn_bias=None, edge_index=None, attn_type=None, **kwargs):
@@ -99,11 +99,11 @@ class Exphormer(NodeModelBase):
     def __init__(self, n_layers, num_heads, input_dim, hidden_dim, output_dim, attn_bias_dim, dropout_rate,
                  input_dropout_rate, attention_dropout_rate, ffn_dim, num_global_node, **kwargs):
         super().__init__()
-        self.node_encoder = Linear(input_dim, hidden_dim)
+        self.node_encoder = nn.Linear(input_dim, hidden_dim)
         self.input_dropout = nn.Dropout(input_dropout_rate)
         self.layers = nn.ModuleList([
             EncoderLayer(hidden_dim, dropout_rate, attention_dropout_rate, num_heads) for _ in range(n_layers)])
-        self.output_proj = Linear(hidden_dim, output_dim)
+        self.output_proj = nn.Linear(hidden_dim, output_dim)
         self.apply(lambda m: init_params(m, n_layers=n_layers))
         self._init_ckpt_state()
 

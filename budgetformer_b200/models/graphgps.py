@@ -16,7 +16,7 @@ from torch.utils.checkpoint import checkpoint
 
 from ..parallel.initialize import get_sequence_parallel_group
 from ..parallel.sp_ops import DistributedAttentionNodeLevel
-from .common import Linear, NodeModelBase, SparseCoreAttention, encode_features
+from .common import NodeModelBase, SparseCoreAttention, encode_features, linear
 
 
 def _gaussian_orthogonal_random_matrix(nb_rows, nb_columns, device=None):
@@ -96,19 +96,19 @@ class MultiHeadAttention(nn.Module):
         self.num_heads = num_heads
         self.att_size = hidden_size // num_heads
         qkv_bias = str(attn_type).lower() == "full"
-        self.linear_q = Linear(hidden_size, num_heads * self.att_size, bias=qkv_bias)
-        self.linear_k = Linear(hidden_size, num_heads * self.att_size, bias=qkv_bias)
-        self.linear_v = Linear(hidden_size, num_heads * self.att_size, bias=qkv_bias)
-        self.out_proj = Linear(hidden_size, hidden_size)
+        self.linear_q = nn.Linear(hidden_size, num_heads * self.att_size, bias=qkv_bias)
+        self.linear_k = nn.Linear(hidden_size, num_heads * self.att_size, bias=qkv_bias)
+        self.linear_v = nn.Linear(hidden_size, num_heads * self.att_size, bias=qkv_bias)
+        self.out_proj = nn.Linear(hidden_size, hidden_size)
         self.dist_attn = DistributedAttentionNodeLevel(
             GPSCoreAttention(hidden_size, attention_dropout_rate, num_heads), get_sequence_parallel_group())
 
     def forward(self, x, attn_bias=None, edge_index=None, attn_type=None):
         b = x.size(0)
-        q = self.linear_q(x).view(b, -1, self.num_heads, self.att_size)
-        k = self.linear_k(x).view(b, -1, self.num_heads, self.att_size)
-        v = self.linear_v(x).view(b, -1, self.num_heads, self.att_size)
-        return self.out_proj(self.dist_attn(q, k, v, attn_bias, edge_index, attn_type))
+        q = linear(self.linear_q, x).view(b, -1, self.num_heads, self.att_size)
+        k = linear(self.linear_k, x).view(b, -1, self.num_heads, self.att_size)
+        v = linear(self.linear_v, x).view(b, -1, self.num_heads, self.att_size)
+        return linear(self.out_proj, self.dist_attn(q, k, v, attn_bias, edge_index, attn_type))
 
 
 class EncoderLayer(nn.Module):
@@ -117,8 +117,8 @@ class EncoderLayer(nn.Module):
         self.self_attention = MultiHeadAttention(hidden_size, attention_dropout_rate, num_heads, attn_type=attn_type)
         self.dropout1 = nn.Dropout(dropout_rate)
         self.norm1 = nn.BatchNorm1d(hidden_size)
-        self.ffn1 = Linear(hidden_size, hidden_size * 2)
-        self.ffn2 = Linear(hidden_size * 2, hidden_size)
+        self.ffn1 = nn.Linear(hidden_size, hidden_size * 2)
+        self.ffn2 = nn.Linear(hidden_size * 2, hidden_size)
         self.ff_dropout1 = nn.Dropout(dropout_rate)
         self.ff_dropout2 = nn.Dropout(dropout_rate)
         self.norm2 = nn.BatchNorm1d(hidden_size)
@@ -133,8 +133,8 @@ class EncoderLayer(nn.Module):
         return norm(x.reshape(b * n, c)).view(b, n, c)
 
     def _ffn(self, h):
-        out = self.ff_dropout1(F.relu(self.ffn1(h)))
-        out = self.ff_dropout2(self.ffn2(out))
+        out = self.ff_dropout1(F.relu(linear(self.ffn1, h)))
+        out = self.ff_dropout2(linear(self.ffn2, out))
         return self._bn(self.norm2, h + out)
 
     def forward_attn_only(self, x, attn_bias=None, edge_index=None, attn_type=None, **kwargs):
@@ -152,11 +152,11 @@ class GraphGPS(NodeModelBase):
     def __init__(self, n_layers, num_heads, input_dim, hidden_dim, output_dim, attn_bias_dim, dropout_rate,
                  input_dropout_rate, attention_dropout_rate, ffn_dim, num_global_node, attn_type="sparse", **kwargs):
         super().__init__()
-        self.node_encoder = Linear(input_dim, hidden_dim)
+        self.node_encoder = nn.Linear(input_dim, hidden_dim)
         self.layers = nn.ModuleList([
             EncoderLayer(hidden_dim, dropout_rate, attention_dropout_rate, num_heads, attn_type=attn_type)
             for _ in range(n_layers)])
-        self.output_proj = Linear(hidden_dim, output_dim)
+        self.output_proj = nn.Linear(hidden_dim, output_dim)
         self._init_ckpt_state()
 
     def redraw_performer_projections(self, device=None):

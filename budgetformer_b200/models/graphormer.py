@@ -15,18 +15,21 @@ from torch.utils.checkpoint import checkpoint
 from ..ops.norm import layer_norm
 from ..parallel.initialize import get_sequence_parallel_group
 from ..parallel.sp_ops import DistributedAttentionNoMerge
-from .common import Linear, NodeModelBase, SparseCoreAttention, encode_features, init_params
+from .common import NodeModelBase, SparseCoreAttention, encode_features, init_params, linear
 
 
 class FeedForwardNetwork(nn.Module):
     def __init__(self, hidden_size, ffn_size, dropout_rate):
         super().__init__()
-        self.layer1 = Linear(hidden_size, ffn_size)
+        self.layer1 = nn.Linear(hidden_size, ffn_size)
         self.gelu = nn.GELU()
-        self.layer2 = Linear(ffn_size, hidden_size)
+        self.layer2 = nn.Linear(ffn_size, hidden_size)
 
     def forward(self, x):
-        return self.layer2(self.gelu(self.layer1(x)))
+        if torch.jit.is_scripting():
+            return self.layer2(self.gelu(self.layer1(x)))
+        else:
+            return linear(self.layer2, self.gelu(linear(self.layer1, x)))
 
 
 class CoreAttention(SparseCoreAttention):
@@ -67,19 +70,19 @@ class MultiHeadAttention(nn.Module):
         super().__init__()
         self.num_heads = num_heads
         self.att_size = hidden_size // num_heads
-        self.linear_q = Linear(hidden_size, num_heads * self.att_size)
-        self.linear_k = Linear(hidden_size, num_heads * self.att_size)
-        self.linear_v = Linear(hidden_size, num_heads * self.att_size)
+        self.linear_q = nn.Linear(hidden_size, num_heads * self.att_size)
+        self.linear_k = nn.Linear(hidden_size, num_heads * self.att_size)
+        self.linear_v = nn.Linear(hidden_size, num_heads * self.att_size)
         self.dist_attn = DistributedAttentionNoMerge(
             CoreAttention(hidden_size, attention_dropout_rate, num_heads, attn_bias_dim), get_sequence_parallel_group())
-        self.output_layer = Linear(num_heads * self.att_size, hidden_size)
+        self.output_layer = nn.Linear(num_heads * self.att_size, hidden_size)
 
     def forward(self, x, attn_bias=None, edge_index=None, attn_type=None):
         b = x.size(0)
-        q = self.linear_q(x).view(b, -1, self.num_heads, self.att_size)
-        k = self.linear_k(x).view(b, -1, self.num_heads, self.att_size)
-        v = self.linear_v(x).view(b, -1, self.num_heads, self.att_size)
-        return self.output_layer(self.dist_attn(q, k, v, attn_bias, edge_index, attn_type))
+        q = linear(self.linear_q, x).view(b, -1, self.num_heads, self.att_size)
+        k = linear(self.linear_k, x).view(b, -1, self.num_heads, self.att_size)
+        v = linear(self.linear_v, x).view(b, -1, self.num_heads, self.att_size)
+        return linear(self.output_layer, self.dist_attn(q, k, v, attn_bias, edge_index, attn_type))
 
 
 class EncoderLayer(nn.Module):
@@ -111,29 +114,29 @@ class Graphormer(NodeModelBase):
                  input_dropout_rate, attention_dropout_rate, ffn_dim, num_global_node, **kwargs):
         super().__init__()
         self.num_heads = num_heads
-        self.node_encoder = Linear(input_dim, hidden_dim)
+        self.node_encoder = nn.Linear(input_dim, hidden_dim)
         self.input_dropout = nn.Dropout(input_dropout_rate)
         self.layers = nn.ModuleList([
             EncoderLayer(hidden_dim, ffn_dim, dropout_rate, attention_dropout_rate, num_heads, attn_bias_dim)
             for _ in range(n_layers)])
         self.n_layers = n_layers
         self.final_ln = nn.LayerNorm(hidden_dim)
-        self.downstream_out_proj = Linear(hidden_dim, output_dim)
+        self.downstream_out_proj = nn.Linear(hidden_dim, output_dim)
         self.hidden_dim = hidden_dim
         self.num_global_node = num_global_node
         self.graph_token = nn.Embedding(self.num_global_node, hidden_dim)
         self.graph_token_virtual_distance = nn.Embedding(self.num_global_node, attn_bias_dim)
-        self.attn_bias_proj = Linear(attn_bias_dim, num_heads, bias=False)
+        self.attn_bias_proj = nn.Linear(attn_bias_dim, num_heads, bias=False)
         self._init_ckpt_state()
         self.apply(lambda m: init_params(m, n_layers=n_layers))
 
     def _graph_attn_bias(self, attn_bias, device):
         if attn_bias is None:
             return None
-        proj = self.attn_bias_proj(attn_bias.to(device))                     # [sub_s, full_s, H]
+        proj = linear(self.attn_bias_proj, attn_bias.to(device))                     # [sub_s, full_s, H]
         if self.num_global_node > 0:
             g = self.num_global_node
-            vd = self.attn_bias_proj(self.graph_token_virtual_distance.weight)  # [g, H]
+            vd = linear(self.attn_bias_proj, self.graph_token_virtual_distance.weight)  # [g, H]
             sub_s, full_s = proj.size(0), proj.size(1)
             row = vd.unsqueeze(1).expand(g, full_s + g, self.num_heads)
             colb = vd.unsqueeze(0).expand(sub_s, g, self.num_heads)

@@ -12,7 +12,7 @@ from torch.utils.checkpoint import checkpoint
 
 from ..parallel.initialize import get_sequence_parallel_group
 from ..parallel.sp_ops import DistributedAttentionNodeLevel
-from .common import Linear, NodeModelBase, SparseCoreAttention, encode_features, init_params
+from .common import NodeModelBase, SparseCoreAttention, encode_features, init_params, linear
 
 
 class CoreAttention(SparseCoreAttention):
@@ -28,17 +28,17 @@ class MultiHeadAttention(nn.Module):
         super().__init__()
         self.num_heads = num_heads
         self.att_size = hidden_size // num_heads
-        self.linear_q = Linear(hidden_size, num_heads * self.att_size)
-        self.linear_k = Linear(hidden_size, num_heads * self.att_size)
-        self.linear_v = Linear(hidden_size, num_heads * self.att_size)
+        self.linear_q = nn.Linear(hidden_size, num_heads * self.att_size)
+        self.linear_k = nn.Linear(hidden_size, num_heads * self.att_size)
+        self.linear_v = nn.Linear(hidden_size, num_heads * self.att_size)
         self.dist_attn = DistributedAttentionNodeLevel(
             CoreAttention(hidden_size, attention_dropout_rate, num_heads), get_sequence_parallel_group())
 
     def forward(self, x, attn_bias=None, edge_index=None, attn_type=None):
         b = x.size(0)
-        q = self.linear_q(x).view(b, -1, self.num_heads, self.att_size)
-        k = self.linear_k(x).view(b, -1, self.num_heads, self.att_size)
-        v = self.linear_v(x).view(b, -1, self.num_heads, self.att_size)
+        q = linear(self.linear_q, x).view(b, -1, self.num_heads, self.att_size)
+        k = linear(self.linear_k, x).view(b, -1, self.num_heads, self.att_size)
+        v = linear(self.linear_v, x).view(b, -1, self.num_heads, self.att_size)
         out = self.dist_attn(q, k, v, attn_bias, edge_index, attn_type)
         assert out.size() == x.size()
         return out
@@ -49,23 +49,23 @@ class EncoderLayer(nn.Module):
         super().__init__()
         self.self_attention = MultiHeadAttention(hidden_size, attention_dropout_rate, num_heads)
         self.self_attention_dropout = nn.Dropout(dropout_rate)
-        self.O = Linear(hidden_size, hidden_size)
+        self.O = nn.Linear(hidden_size, hidden_size)
         self.layer_norm1 = nn.LayerNorm(hidden_size)
-        self.FFN_layer1 = Linear(hidden_size, hidden_size * 2)
-        self.FFN_layer2 = Linear(hidden_size * 2, hidden_size)
+        self.FFN_layer1 = nn.Linear(hidden_size, hidden_size * 2)
+        self.FFN_layer2 = nn.Linear(hidden_size * 2, hidden_size)
         self.layer_norm2 = nn.LayerNorm(hidden_size)
 
     def _ffn(self, h):
-        y = self.FFN_layer1(h)
+        y = linear(self.FFN_layer1, h)
         y = F.relu(y)
         y = self.self_attention_dropout(y)
-        y = self.FFN_layer2(y)
+        y = linear(self.FFN_layer2, y)
         return self.layer_norm2(h + y)
 
     def forward_attn_only(self, x, attn_bias=None, edge_index=None, attn_type=None, **kwargs):
         y = self.self_attention(x, attn_bias, edge_index=edge_index, attn_type=attn_type)
         y = self.self_attention_dropout(y)
-        y = self.O(y)
+        y = linear(self.O, y)
         return self.layer_norm1(x + y)
 
     def forward_ffn_checkpointed(self, x_ln):
@@ -78,8 +78,8 @@ class EncoderLayer(nn.Module):
 class MLPReadout(nn.Module):
     def __init__(self, input_dim, output_dim, L=2):
         super().__init__()
-        layers = [Linear(input_dim // 2 ** l, input_dim // 2 ** (l + 1), bias=True) for l in range(L)]
-        layers.append(Linear(input_dim // 2 ** L, output_dim, bias=True))
+        layers = [nn.Linear(input_dim // 2 ** l, input_dim // 2 ** (l + 1), bias=True) for l in range(L)]
+        layers.append(nn.Linear(input_dim // 2 ** L, output_dim, bias=True))
         self.FC_layers = nn.ModuleList(layers)
         self.L = L
 
@@ -95,7 +95,7 @@ class GT(NodeModelBase):
     def __init__(self, n_layers, num_heads, input_dim, hidden_dim, output_dim, attn_bias_dim, dropout_rate,
                  input_dropout_rate, attention_dropout_rate, ffn_dim, num_global_node, **kwargs):
         super().__init__()
-        self.node_encoder = Linear(input_dim, hidden_dim)
+        self.node_encoder = nn.Linear(input_dim, hidden_dim)
         self.input_dropout = nn.Dropout(input_dropout_rate)
         self.layers = nn.ModuleList([
             EncoderLayer(hidden_dim, ffn_dim, dropout_rate, attention_dropout_rate, num_heads) for _ in range(n_layers)])

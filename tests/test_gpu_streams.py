@@ -194,9 +194,20 @@ def test_fp32_linear_of_no_width(out_features, in_features):
 
 
 def test_fp32_modules_match_torch():
-    """The models' Linear and the row-kernel LayerNorm against torch's, first and second derivative, few and many rows."""
-    from budgetformer_b200.models.common import Linear
+    """The models' call of a linear layer and the row-kernel LayerNorm against torch's, first and second derivative, few and many
+    rows."""
+    from budgetformer_b200.models.common import linear
     from budgetformer_b200.ops.norm import layer_norm
+
+    class Linear(torch.nn.Module):
+        def __init__(self, k, n):
+            super().__init__()
+            self.weight, self.bias = (torch.nn.Parameter(torch.randn(*size) * k ** -0.5) for size in ((n, k), (n,)))
+
+        def forward(self, x):
+            inner = torch.nn.Linear(self.weight.size(1), self.weight.size(0), device="meta")
+            inner.weight, inner.bias = self.weight, self.bias
+            return linear(inner, x)
 
     class LayerNorm(torch.nn.LayerNorm):
         def forward(self, x):

@@ -224,3 +224,25 @@ def test_linear_gradient_under_batched_gradients():
         assert u.shape == v.shape and torch.allclose(u, v, rtol=1e-5, atol=1e-5)
     jac = lambda f: torch.autograd.functional.jacobian(lambda t: f(x, t, b).sum(1), w, vectorize=True)
     assert torch.allclose(jac(_LinearF32.apply), jac(torch.nn.functional.linear), rtol=1e-5, atol=1e-5)
+
+
+def test_model_parts_stay_torch_linear_modules():
+    """What goes by the class of a linear layer keeps working on the models' parts: scripting, symbolic tracing, dynamic
+    quantisation; and hooks on a layer run."""
+    from budgetformer_b200.models import graphormer, nagphormer
+    x = torch.randn(2, 5, 16)
+    for part, args in ((graphormer.FeedForwardNetwork(16, 32, 0.0), (x,)), (nagphormer.FeedForwardNetwork(16, 32), (x,)),
+                       (nagphormer.MultiHeadAttention(16, 0.0, 4), (x, x, x))):
+        part.eval()
+        want = part(*args)
+        assert torch.allclose(torch.jit.script(part)(*args), want, atol=1e-6)
+    ffn = nagphormer.FeedForwardNetwork(16, 32)
+    layer = nagphormer.EncoderLayer(16, 32, 0.0, 0.0, 4)
+    assert torch.allclose(torch.fx.symbolic_trace(ffn)(x), ffn(x), atol=1e-6)
+    assert torch.allclose(torch.fx.symbolic_trace(layer)(x), layer(x), atol=1e-5)
+    quantised = torch.ao.quantization.quantize_dynamic(ffn, {torch.nn.Linear})
+    assert "quantized" in type(quantised.layer1).__module__
+    seen = []
+    ffn.layer1.register_forward_hook(lambda m, i, o: seen.append(tuple(o.shape)))
+    ffn(x)
+    assert seen == [(2, 5, 32)]
