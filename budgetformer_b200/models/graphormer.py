@@ -15,7 +15,7 @@ from torch.utils.checkpoint import checkpoint
 from ..ops.norm import layer_norm
 from ..parallel.initialize import get_sequence_parallel_group
 from ..parallel.sp_ops import DistributedAttentionNoMerge
-from .common import NodeModelBase, SparseCoreAttention, encode_features, init_params, linear
+from .common import NodeModelBase, SparseCoreAttention, encode_features, init_params, linear, plain_module
 
 
 class FeedForwardNetwork(nn.Module):
@@ -153,13 +153,14 @@ class Graphormer(NodeModelBase):
         x = self.input_dropout(x)
         bias = self._graph_attn_bias(attn_bias, x.device)
         x = self._run_layers(x, attn_bias=bias, edge_index=edge_index, attn_type=attn_type)
-        from ..ops.gemm import readout_linear
-        x = x[0, int(self.num_global_node):, :]
-        if x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and torch.is_autocast_enabled("cuda"):
+        from ..ops.gemm import plain_eager, readout_linear
+        first, ln = int(self.num_global_node), self.final_ln
+        if (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and torch.is_autocast_enabled("cuda")
+                and x.dtype == torch.get_autocast_dtype("cuda") and plain_module(ln, nn.LayerNorm) and plain_eager()):
             # autocast would normalise an fp32 copy and round the result for the projection: the row kernel rounds once as well
-            x = layer_norm(x, self.final_ln.weight, self.final_ln.bias, self.final_ln.eps)
+            x = layer_norm(x[0, first:, :], ln.weight, ln.bias, ln.eps)
         else:
-            x = self.final_ln(x)
+            x = ln(x)[0, first:, :]
         return readout_linear(x, self.downstream_out_proj.weight, self.downstream_out_proj.bias)
 
     def forward(self, x, attn_bias, edge_index, perturb=None, attn_type=None):

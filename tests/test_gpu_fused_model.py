@@ -183,3 +183,19 @@ def test_fused_gradients_against_fp32_portable_run(model):
         worst = max(worst, rel)
         assert rel < 0.05, f"{model}: {na}: relative gradient error {rel:.4f}"
     assert worst > 0.0
+
+
+def test_hooks_on_the_last_norm_run_under_autocast():
+    """Graphormer's last norm runs on the row kernel under 16-bit autocast; with a hook on the module the module is called, on the
+    whole sequence, and the logits are those of the row kernel up to one 16-bit rounding."""
+    t = _trainer("graphormer", fused=True)
+    graph = t.build_edges(1)
+    t.model.eval()
+    with torch.no_grad():
+        plain = t._loss(graph, t.local_idx["train"])[1].float()
+        seen = []
+        handle = t.model.final_ln.register_forward_hook(lambda m, i, o: seen.append(tuple(o.shape)))
+        hooked = t._loss(graph, t.local_idx["train"])[1].float()
+        handle.remove()
+    assert seen and seen[0][-2:] == (1537, 128)
+    assert float((plain - hooked).norm()) <= 1e-2 * float(plain.norm())
