@@ -186,6 +186,12 @@ void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor do
     qg = torch::empty({q.size(0), (int64_t)p.hl, 2, (int64_t)p.hn}, q.options());
     b.qg = qg.data_ptr();
   }
+  if (p.n > 0 && (!kv_task.has_value() || kv_task->numel() == 0)) {
+    // a by-key view without its work list
+    RowTasks r = row_tasks(t_rowptr, p.n, t_row.numel(), BF_LONG_CHUNK, BF_LONG_CHUNK, true, at::cuda::getCurrentCUDAStream());
+    kv_task = r.tasks; kv_split = r.splits;
+    kv_slots = r.sizes[1].item<int64_t>();
+  }
   TORCH_CHECK(kv_task.has_value() && kv_task->scalar_type() == torch::kInt && kv_task->is_contiguous() && kv_task->size(1) == 4 &&
               ((uintptr_t)kv_task->data_ptr()) % 16 == 0, "kv_task must be contiguous int32 [T, 4]");
   b.kv_task = kv_task->data_ptr<int>(); b.n_kv_task = (int)kv_task->size(0);

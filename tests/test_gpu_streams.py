@@ -119,6 +119,21 @@ def test_lists_of_a_graph_serve_every_stream(virtual_node):
             assert float((a.double() - b.double()).norm()) <= 2e-5 * (float(b.double().norm()) + float(dout.norm()))
 
 
+def test_by_key_view_without_its_work_list():
+    """A graph that was given t_rowptr, t_row and t_eid alone: the backward pass makes the work list, and the gradients are those
+    of the graph's own."""
+    from budgetformer_b200.graph.attn_graph import AttnGraph
+    from budgetformer_b200.ops.edge_attention import edge_attention
+    whole = _graph(900, 60, 3, False).ensure_transpose()
+    assert whole.kv_slots > 0
+    part = AttnGraph(whole.num_rows, whole.rowptr, whole.col, None, whole.t_rowptr, whole.t_row, whole.t_eid)
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    q, k, v, dout = (torch.randn(900, 4, 16, generator=gen, device="cuda") for _ in range(4))
+    args = [t.requires_grad_() for t in (q, k, v)]
+    for a, b in zip(*(torch.autograd.grad(edge_attention(*args, g), args, dout) for g in (whole, part))):
+        assert torch.equal(a, b)
+
+
 def test_attention_streams_keep_other_rows_finite():
     """An infinite key / value row reaches the queries that name it and nobody else: stale ring slots are never added."""
     from budgetformer_b200.graph.attn_graph import AttnGraph
