@@ -1069,38 +1069,48 @@ __global__ void __launch_bounds__(256, EXPH ? 3 : 4) edge_attn_bwd_q_long_kernel
 // ---------------------------------------------------------------------------------------------
 constexpr int SPLIT_WINDOW = 64;
 constexpr int SPLIT_THREADS = 256;
+constexpr int SPLIT_COLS = 4096;            // columns and normalisers of the forward pass that a block holds at a time
 constexpr int SPLIT_FWD = 0, SPLIT_DQ = 1, SPLIT_KV = 2;
 
-// s[0 .. ncol) holds the finished sums of row `row`
-template <typename T, int MODE>
-__device__ __forceinline__ void split_finish(const BwdArgs& b, int row, int w, int hn, const float* s) {
+// Writes row `row` from the finished column sums sum(c), c < Hl*HN (forward: the numerators, and Hl normalisers behind them) or
+// 2*Hl*HN (dK | dV).  The whole block takes part.  The forward pass needs a head's normaliser beside its columns: heads go through
+// shared memory as many at a time as fit, so rows may be of any width.
+template <typename T, int MODE, typename F>
+__device__ __forceinline__ void split_finish(const BwdArgs& b, int row, int w, int hn, F sum) {
   const AttnArgs& a = b.f;
   if (MODE == SPLIT_FWD) {
-    for (int c = threadIdx.x; c < w; c += blockDim.x) {
-      const int head = c / hn;
-      const float zs = s[w + head];
-      float inv = 1.f / (zs + kEps);
-      if (a.variant == 1) inv *= a.inv_keep;
-      float ov = s[c] * inv;
-      if (a.out_thresh) ov = keep_out(a, row, c) ? ov * a.out_inv_keep : 0.f;
-      static_cast<T*>(a.out)[(long long)row * w + c] = from_float<T>(ov);
-      if (a.route_out.n_dest) *routed<T>(a.route_out, row, c) = from_float<T>(ov);
-      if (c % hn == 0) a.z[(long long)row * a.hl + head] = zs;
+    __shared__ float s_sum[SPLIT_COLS];
+    const int fit = SPLIT_COLS / (hn + 1);
+    for (int h0 = 0; h0 < a.hl; h0 += fit) {
+      const int heads = min(fit, a.hl - h0), nc = heads * hn;
+      for (int c = threadIdx.x; c < nc + heads; c += blockDim.x) s_sum[c] = sum(c < nc ? h0 * hn + c : w + h0 + (c - nc));
+      __syncthreads();
+      for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+        const int head = h0 + c / hn, col = h0 * hn + c;
+        const float zs = s_sum[nc + c / hn];
+        float inv = 1.f / (zs + kEps);
+        if (a.variant == 1) inv *= a.inv_keep;
+        float ov = s_sum[c] * inv;
+        if (a.out_thresh) ov = keep_out(a, row, col) ? ov * a.out_inv_keep : 0.f;
+        static_cast<T*>(a.out)[(long long)row * w + col] = from_float<T>(ov);
+        if (a.route_out.n_dest) *routed<T>(a.route_out, row, col) = from_float<T>(ov);
+        if (c % hn == 0) a.z[(long long)row * a.hl + head] = zs;
+      }
+      __syncthreads();
     }
   } else if (MODE == SPLIT_DQ) {
     T* dst = grad_row<T>(b, b.dq, b.cq, row);
-    for (int c = threadIdx.x; c < w; c += blockDim.x) dst[c] = from_float<T>(s[c]);
+    for (int c = threadIdx.x; c < w; c += blockDim.x) dst[c] = from_float<T>(sum(c));
   } else {
     T* dk = grad_row<T>(b, b.dk, b.ck, row);
     T* dv = grad_row<T>(b, b.dv, b.cv, row);
-    for (int c = threadIdx.x; c < 2 * w; c += blockDim.x) (c < w ? dk + c : dv + (c - w))[0] = from_float<T>(s[c]);
+    for (int c = threadIdx.x; c < 2 * w; c += blockDim.x) (c < w ? dk + c : dv + (c - w))[0] = from_float<T>(sum(c));
   }
 }
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(SPLIT_THREADS) split_window_kernel(BwdArgs b, const int4* __restrict__ task, int n_slots,
                                                                      float* partial, int pitch, int ncol, int w, int hn) {
-  extern __shared__ float s_sum[];            // [ncol]
   __shared__ int s_key[SPLIT_WINDOW];
   const int s0 = blockIdx.x * SPLIT_WINDOW, s1 = min(s0 + SPLIT_WINDOW, n_slots);
   for (int i = threadIdx.x; i < s1 - s0; i += blockDim.x) s_key[i] = task[s0 + i].x;
@@ -1111,7 +1121,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_window_kernel(BwdArgs b, 
     int j = i + 1;
     while (j < s1 && s_key[j - s0] == key) ++j;
     const bool whole = !(i == s0 && before == key) && !(j == s1 && after == key);
-    for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
+    auto sum = [&](int c) {
       const float* pp = partial + (long long)i * pitch + c;
       float acc[8];
 #pragma unroll
@@ -1124,28 +1134,23 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_window_kernel(BwdArgs b, 
 #pragma unroll
       for (int u = 0; u < 7; ++u)
         if (u < n) acc[u] += pp[u * (long long)pitch];
-      const float sum = ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
-      if (whole) s_sum[c] = sum;
-      else partial[(long long)i * pitch + c] = sum;
-    }
-    if (whole) {
-      __syncthreads();
-      split_finish<T, MODE>(b, key, w, hn, s_sum);
-      __syncthreads();
-    }
+      return ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
+    };
+    if (whole) split_finish<T, MODE>(b, key, w, hn, sum);
+    else
+      for (int c = threadIdx.x; c < ncol; c += blockDim.x) partial[(long long)i * pitch + c] = sum(c);
     i = j;
   }
 }
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(SPLIT_THREADS) split_cross_kernel(BwdArgs b, const int* __restrict__ split, int n_split,
-                                                                    const float* partial, int pitch, int ncol, int w, int hn) {
-  extern __shared__ float s_sum[];            // [ncol]
+                                                                    const float* partial, int pitch, int w, int hn) {
   for (int s = blockIdx.x; s < n_split; s += gridDim.x) {
     const int first = split[3 * s + 1];
     const int w0 = first / SPLIT_WINDOW, w1 = (first + split[3 * s + 2] - 1) / SPLIT_WINDOW;
     if (w0 == w1) continue;                   // finished by its window
-    for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
+    split_finish<T, MODE>(b, split[3 * s], w, hn, [&](int c) {
       float acc[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) acc[u] = 0.f;
@@ -1156,20 +1161,16 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_cross_kernel(BwdArgs b, c
         for (int u = 0; u < 8; ++u) acc[u] += pp[(long long)(k + u) * SPLIT_WINDOW * pitch];
       }
       for (; k <= w1; ++k) acc[0] += pp[(long long)k * SPLIT_WINDOW * pitch];
-      s_sum[c] = pp[(long long)first * pitch] + ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
-    }
-    __syncthreads();
-    split_finish<T, MODE>(b, split[3 * s], w, hn, s_sum);
-    __syncthreads();
+      return pp[(long long)first * pitch] + ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
+    });
   }
 }
 
 template <typename T, int MODE>
 void launch_split(const BwdArgs& b, const int4* task, int n_slots, const int* split, int n_split, float* partial, int pitch,
                   int ncol, int w, int hn, cudaStream_t st) {
-  const size_t smem = sizeof(float) * ncol;
-  split_window_kernel<T, MODE><<<(n_slots + SPLIT_WINDOW - 1) / SPLIT_WINDOW, SPLIT_THREADS, smem, st>>>(b, task, n_slots, partial, pitch, ncol, w, hn);
-  split_cross_kernel<T, MODE><<<n_split < 148 * 8 ? n_split : 148 * 8, SPLIT_THREADS, smem, st>>>(b, split, n_split, partial, pitch, ncol, w, hn);
+  split_window_kernel<T, MODE><<<(n_slots + SPLIT_WINDOW - 1) / SPLIT_WINDOW, SPLIT_THREADS, 0, st>>>(b, task, n_slots, partial, pitch, ncol, w, hn);
+  split_cross_kernel<T, MODE><<<n_split < 148 * 8 ? n_split : 148 * 8, SPLIT_THREADS, 0, st>>>(b, split, n_split, partial, pitch, w, hn);
 }
 
 // Lanes of a group (VN elements each, whole heads, at most a warp), and how many segments each group takes: as many as leave two
@@ -1232,6 +1233,9 @@ cudaError_t launch_fwd_t(const AttnArgs& a, int chunks_per_hub, cudaStream_t st)
   return cudaGetLastError();
 }
 
+// shared memory for the gradient of the two rows of the type table
+inline size_t type_table_bytes(int w_row) { return sizeof(float) * 2 * (size_t)w_row; }
+
 template <typename T, int HN>
 cudaError_t launch_bwd_t(const BwdArgs& b, cudaStream_t st) {
   const AttnArgs& a = b.f;
@@ -1255,7 +1259,12 @@ cudaError_t launch_bwd_t(const BwdArgs& b, cudaStream_t st) {
       // every block ends in 2 * Hl * HN atomics: longer streams where the rows allow it
       constexpr int VN = Vec<T>::N;
       const StreamGeo s = stream_geo<HN, VN>(a.hl, a.n, 4, 32);
-      edge_attn_bwd_q_kernel<T, HN, true><<<stream_grid<HN, VN>(a.hl, stream_warps(a.n, s, s.per), s), kStreamThreads, sizeof(float) * 2 * w_row, st>>>(b, s);
+      if (type_table_bytes(w_row) + kRing * kStreamThreads * (sizeof(uint4) + sizeof(float)) > 48 * 1024 && type_table_bytes(w_row) <= 48 * 1024) {
+        // beside the ring (10 KB) the type table's gradient of rows above 4,864 elements goes over the default 48 KB of a block
+        const cudaError_t e = cudaFuncSetAttribute(edge_attn_bwd_q_kernel<T, HN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
+        if (e != cudaSuccess) return e;
+      }
+      edge_attn_bwd_q_kernel<T, HN, true><<<stream_grid<HN, VN>(a.hl, stream_warps(a.n, s, s.per), s), kStreamThreads, type_table_bytes(w_row), st>>>(b, s);
     } else {
       constexpr int VN = wide_elems<T, HN>();
       const StreamGeo s = stream_geo<HN, VN>(a.hl, a.n, 7, 8);

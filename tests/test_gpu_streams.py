@@ -134,6 +134,29 @@ def test_by_key_view_without_its_work_list():
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("heads,variant,dtype", [(40, "exphormer", torch.bfloat16), (48, "exphormer", torch.float32), (48, "plain", torch.bfloat16)])
+def test_attention_of_wide_rows(heads, variant, dtype):
+    """Rows of 5,120 and 6,144 elements with long queries and split keys: the type table's gradient and the sums of split rows
+    need more shared memory than a block gets by default, or have to do without."""
+    from budgetformer_b200.graph.attn_graph import AttnGraph
+    from budgetformer_b200.ops.edge_attention import edge_attention
+    gen = torch.Generator().manual_seed(heads)
+    n, hn = 61, 128
+    dst = torch.cat([torch.zeros(200, dtype=torch.long), torch.arange(n).repeat_interleave(4)])
+    src = torch.randint(0, n, (dst.numel(),), generator=gen)
+    src[200:300] = 7                                                       # a split key
+    graph = AttnGraph.from_edge_index(torch.stack([src, dst, torch.randint(0, 2, (dst.numel(),), generator=gen)]), n).to("cuda")
+    q, k, v, dout = (torch.randn(n, heads, hn, generator=gen).cuda().to(dtype) for _ in range(4))
+    tab = torch.randn(2, heads, hn, generator=gen).cuda() if variant == "exphormer" else None
+    want = _reference(q, k, v, dout, graph, tab, variant, 0.0, 0)
+    args = [x.requires_grad_() for x in (q, k, v)] + ([tab.requires_grad_()] if tab is not None else [])
+    out = edge_attention(q, k, v, graph, variant=variant, etable=tab)
+    got = [out] + list(torch.autograd.grad(out, args, dout))
+    tol = {torch.float32: 2e-5, torch.bfloat16: 2.5e-2}[dtype]             # as in test_attention_streams
+    for a, b in zip(got, want):
+        assert float((a.double() - b.double()).norm()) <= tol * (float(b.double().norm()) + float(dout.double().norm()))
+
+
 def test_attention_streams_keep_other_rows_finite():
     """An infinite key / value row reaches the queries that name it and nobody else: stale ring slots are never added."""
     from budgetformer_b200.graph.attn_graph import AttnGraph
