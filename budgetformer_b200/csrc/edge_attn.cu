@@ -693,6 +693,18 @@ __global__ void __launch_bounds__(kStreamThreads) edge_attn_bwd_delta_kernel(Bwd
   if ((lt % LPH) == 0) b.zd[hz] = make_float2(invz, dterm);
 }
 
+// s0 * E_0 + s1 * E_1 into s0, of the edge types that were met (bit t of `seen`)
+template <int NP> __device__ __forceinline__ void typed_sum(const float* et, int w_row, unsigned seen, f2* s0, const f2* s1) {
+  if (seen & 1u) {
+#pragma unroll
+    for (int i = 0; i < NP; ++i) s0[i] = mul2(s0[i], pack2(__ldg(et + 2 * i), __ldg(et + 2 * i + 1)));
+  }
+  if (seen & 2u) {
+#pragma unroll
+    for (int i = 0; i < NP; ++i) s0[i] = fma2(s1[i], pack2(__ldg(et + w_row + 2 * i), __ldg(et + w_row + 2 * i + 1)), s0[i]);
+  }
+}
+
 // dK/dV over the balanced work list, first of the two passes over the edges.  It gathers q, dout and (1/Z, D) of each query and
 // leaves the score gradient of every (edge, head) in `ds` (fp32, at the edge's own position), so that the dQ pass gathers k alone.
 // The list holds the items of split keys (64 edges each), then the rest sorted by length.
@@ -804,6 +816,7 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
     itn = item(r + 2);
     if (it.w != -2) { S::load(kb + (long long)it.x * a.ldk, kn); S::load(vb + (long long)it.x * a.ldv, vn); }
     const int m = steps_of(cur.z);
+    unsigned seen = 0;                          // edge types of the item: only their products count (0 * inf is not 0)
     for (int i = 0; i < m; ++i) {
       issue((slot + kRing - 1) & (kRing - 1));
       copy_wait<kRing - 1>();
@@ -834,9 +847,14 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
         if ((lt % LPH) == 0) b.ds[(long long)eid * a.hl + head] = dss;
         const f2 s2 = pack2(dss, dss), w2 = pack2(wn, wn);
         if (EXPH) {
-          const f2 z2 = pack2(0.f, 0.f), sa = t1 ? z2 : s2, sb = t1 ? s2 : z2;
+          seen |= t1 ? 2u : 1u;
+          if (t1) {
 #pragma unroll
-          for (int u = 0; u < NP; ++u) { dk0[u] = fma2(sa, qf[u], dk0[u]); dk1[u] = fma2(sb, qf[u], dk1[u]); }
+            for (int u = 0; u < NP; ++u) dk1[u] = fma2(s2, qf[u], dk1[u]);
+          } else {
+#pragma unroll
+            for (int u = 0; u < NP; ++u) dk0[u] = fma2(s2, qf[u], dk0[u]);
+          }
         } else {
 #pragma unroll
           for (int u = 0; u < NP; ++u) dk0[u] = fma2(s2, qf[u], dk0[u]);
@@ -847,11 +865,7 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
       slot = (slot + 1) & (kRing - 1);
     }
     if (EXPH) {
-      const float* et = a.etab + off;
-#pragma unroll
-      for (int i = 0; i < NP; ++i)
-        dk0[i] = fma2(dk0[i], pack2(__ldg(et + 2 * i), __ldg(et + 2 * i + 1)),
-                      mul2(dk1[i], pack2(__ldg(et + w_row + 2 * i), __ldg(et + w_row + 2 * i + 1))));
+      typed_sum<NP>(a.etab + off, w_row, seen, dk0, dk1);
     }
     if (cur.w == -1) {
       S::store(grad_row<T>(b, b.dk, b.ck, cur.x) + off, dk0);
@@ -926,6 +940,7 @@ __global__ void __launch_bounds__(kStreamThreads, EXPH ? 4 : 7) edge_attn_bwd_q_
         if (EXPH && nstored) S::load(qb + (row + groups) * a.ldq, qn);
       }
       const int m = steps_of(len);
+      unsigned seen = 0;                        // edge types of the row (see the dK/dV pass)
       for (int i = 0; i < m; ++i) {
         issue((slot + kRing - 1) & (kRing - 1));
         copy_wait<kRing - 1>();
@@ -936,9 +951,14 @@ __global__ void __launch_bounds__(kStreamThreads, EXPH ? 4 : 7) edge_attn_bwd_q_
           const f2 d2 = pack2(dss, dss);
           if (EXPH) {
             const bool t1 = (types >> slot) & 1u;
-            const f2 z2 = pack2(0.f, 0.f), sa = t1 ? z2 : d2, sb = t1 ? d2 : z2;
+            seen |= t1 ? 2u : 1u;
+            if (t1) {
 #pragma unroll
-            for (int u = 0; u < NP; ++u) { s0[u] = fma2(sa, kf[u], s0[u]); s1[u] = fma2(sb, kf[u], s1[u]); }
+              for (int u = 0; u < NP; ++u) s1[u] = fma2(d2, kf[u], s1[u]);
+            } else {
+#pragma unroll
+              for (int u = 0; u < NP; ++u) s0[u] = fma2(d2, kf[u], s0[u]);
+            }
           } else {
 #pragma unroll
             for (int u = 0; u < NP; ++u) s0[u] = fma2(d2, kf[u], s0[u]);
@@ -948,14 +968,15 @@ __global__ void __launch_bounds__(kStreamThreads, EXPH ? 4 : 7) edge_attn_bwd_q_
       }
       if (stored) {
         if (EXPH) {
-          const float* et = a.etab + off;
+          if (seen & 1u) {
 #pragma unroll
-          for (int i = 0; i < NP; ++i) {
-            de0[i] = fma2(qf[i], s0[i], de0[i]);
-            de1[i] = fma2(qf[i], s1[i], de1[i]);
-            s0[i] = fma2(s0[i], pack2(__ldg(et + 2 * i), __ldg(et + 2 * i + 1)),
-                         mul2(s1[i], pack2(__ldg(et + w_row + 2 * i), __ldg(et + w_row + 2 * i + 1))));
+            for (int i = 0; i < NP; ++i) de0[i] = fma2(qf[i], s0[i], de0[i]);
           }
+          if (seen & 2u) {
+#pragma unroll
+            for (int i = 0; i < NP; ++i) de1[i] = fma2(qf[i], s1[i], de1[i]);
+          }
+          typed_sum<NP>(a.etab + off, w_row, seen, s0, s1);
         }
         S::store(grad_row<T>(b, b.dq, b.cq, row) + off, s0);
       }
@@ -998,6 +1019,7 @@ __global__ void __launch_bounds__(256, EXPH ? 3 : 4) edge_attn_bwd_q_long_kernel
   const int per = (it.z - it.y + tpw - 1) / tpw;
   const int beg = it.y + sub * per, end = min(it.z, beg + per);
   f2 s0[NP], s1[NP];
+  unsigned seen = 0;                            // edge types of the item (see the dK/dV pass)
 #pragma unroll
   for (int i = 0; i < NP; ++i) { s0[i] = pack2(0.f, 0.f); s1[i] = pack2(0.f, 0.f); }
   for (int e = beg; e < end; e += NB) {
@@ -1018,18 +1040,19 @@ __global__ void __launch_bounds__(256, EXPH ? 3 : 4) edge_attn_bwd_q_long_kernel
       if (e + u >= end) break;
       f2 kf[NP];
       widen<T>(kr[u], kf);
-      const f2 z2 = pack2(0.f, 0.f), d2 = pack2(ds[u], ds[u]);
-      const f2 sa = t1[u] ? z2 : d2;
+      const f2 d2 = pack2(ds[u], ds[u]);
+      if (EXPH) seen |= t1[u] ? 2u : 1u;
+      if (EXPH && t1[u]) {
 #pragma unroll
-      for (int i = 0; i < NP; ++i) s0[i] = fma2(sa, kf[i], s0[i]);
-      if (EXPH) {
-        const f2 sb = t1[u] ? d2 : z2;
+        for (int i = 0; i < NP; ++i) s1[i] = fma2(d2, kf[i], s1[i]);
+      } else {
 #pragma unroll
-        for (int i = 0; i < NP; ++i) s1[i] = fma2(sb, kf[i], s1[i]);
+        for (int i = 0; i < NP; ++i) s0[i] = fma2(d2, kf[i], s0[i]);
       }
     }
   }
   __syncwarp();
+  if (EXPH) seen = __reduce_or_sync(kFull, seen);
   float x0[VN], x1[VN];
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
@@ -1047,9 +1070,9 @@ __global__ void __launch_bounds__(256, EXPH ? 3 : 4) edge_attn_bwd_q_long_kernel
       load_vec<T>(static_cast<const T*>(a.q) + (long long)it.x * a.ldq + off, qf);
 #pragma unroll
       for (int i = 0; i < VN; ++i) {
-        atomicAdd(b.detab + off + i, qf[i] * x0[i]);
-        atomicAdd(b.detab + w_row + off + i, qf[i] * x1[i]);
-        x0[i] = x0[i] * __ldg(a.etab + off + i) + x1[i] * __ldg(a.etab + w_row + off + i);
+        if (seen & 1u) atomicAdd(b.detab + off + i, qf[i] * x0[i]);
+        if (seen & 2u) atomicAdd(b.detab + w_row + off + i, qf[i] * x1[i]);
+        x0[i] = ((seen & 1u) ? x0[i] * __ldg(a.etab + off + i) : 0.f) + ((seen & 2u) ? x1[i] * __ldg(a.etab + w_row + off + i) : 0.f);
       }
     }
 #pragma unroll

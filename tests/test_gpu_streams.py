@@ -179,6 +179,37 @@ def test_attention_streams_keep_other_rows_finite():
     assert torch.isfinite(dk[keys]).all() and torch.isfinite(dv[keys]).all()
 
 
+@pytest.mark.parametrize("long_row", [False, True])
+def test_typed_attention_keeps_the_other_type_finite(long_row):
+    """A row of the type table that no edge carries, and an infinite key that only edges of one type name, leave the gradients of the
+    other type as they are: nothing is multiplied by an absent type."""
+    from budgetformer_b200.graph.attn_graph import AttnGraph
+    from budgetformer_b200.ops.edge_attention import edge_attention
+    n, deg = 301, 5
+    dst = torch.arange(n).repeat_interleave(deg)
+    if long_row:
+        dst = torch.cat([torch.zeros(300, dtype=torch.long), dst])
+    src = (torch.arange(dst.numel()) * 7 + 3) % n
+    typ = (dst % 2 == 1).long()                                            # odd queries: type 1 alone
+    src[src == 9] = 10
+    src[dst == 51] = 9                                                     # only query 51 (type 1) names key 9
+    graph = AttnGraph.from_edge_index(torch.stack([src, dst, typ]), n).to("cuda")
+    q, k, v, dout = (torch.randn(n, 4, 16, device="cuda") for _ in range(4))
+    k[9] = float("inf")
+    tab = torch.randn(2, 4, 16, device="cuda")
+    args = [t.requires_grad_() for t in (q, k, v, tab)]
+    grads = torch.autograd.grad(edge_attention(q, k, v, graph, variant="exphormer", etable=tab), args, dout)
+    assert torch.isfinite(grads[3][0]).all() and torch.isfinite(grads[0][::2]).all()
+    with torch.no_grad():
+        k[9] = 0.0
+        tab[1] = float("inf")
+    grads = torch.autograd.grad(edge_attention(q, k, v, graph, variant="exphormer", etable=tab), args, dout)
+    assert torch.isfinite(grads[0][::2]).all() and torch.isfinite(grads[3][0]).all()
+    even = torch.ones(n, dtype=torch.bool, device="cuda")
+    even[src[typ == 1].cuda()] = False                                     # keys that no edge of type 1 names
+    assert even.any() and torch.isfinite(grads[1][even]).all()
+
+
 @pytest.mark.parametrize("m,n,k,pad", [(1, 1, 1, 0), (63, 64, 64, 0), (65, 60, 68, 0), (1000, 47, 101, 0), (4097, 256, 64, 4),
                                        (20011, 64, 256, 0), (300, 130, 70, 1)])
 def test_f32_weight_grad(m, n, k, pad):
