@@ -82,17 +82,20 @@ std::vector<Tensor> long_row_tasks(Tensor rowptr, int64_t n_edges) {
   return {r.tasks, r.splits};
 }
 
-// The long rows of a call: the caller's list, or a list made here.  A known bound on the row length of at most BF_LONG_ROW
-// means that there are none.
+// The long rows of a call: the caller's list, which holds every row with more than list_min edges, or a list made here.  A known
+// bound on the row length of at most BF_LONG_ROW means that there are none, and list_min = 0 that every row is walked whole.
 struct LongRows {
   Tensor tasks, splits, partial;
   bf_long_rows c{};
 };
-LongRows take_long_rows(const Tensor& rowptr, int64_t n_edges, int64_t known_max, const OptTensor& tasks, const OptTensor& splits, size_t pitch) {
+LongRows take_long_rows(const Tensor& rowptr, int64_t n_edges, int64_t known_max, const OptTensor& tasks, const OptTensor& splits,
+                        int64_t list_min, size_t pitch) {
   LongRows r;
-  if (known_max >= 0 && known_max <= BF_LONG_ROW) return r;
+  if ((known_max >= 0 && known_max <= BF_LONG_ROW) || list_min == 0) return r;
+  r.c.min_degree = BF_LONG_ROW;
   if (tasks.has_value() && splits.has_value()) {
     r.tasks = *tasks; r.splits = *splits;
+    if (list_min > 0) r.c.min_degree = (int)list_min;
     TORCH_CHECK(r.tasks.is_cuda() && r.tasks.scalar_type() == torch::kInt && r.tasks.is_contiguous() && r.tasks.dim() == 2 &&
                 r.tasks.size(1) == 4 && ((uintptr_t)r.tasks.data_ptr()) % 16 == 0, "long rows: tasks int32 [T, 4]");
     TORCH_CHECK(r.splits.is_cuda() && r.splits.scalar_type() == torch::kInt && r.splits.is_contiguous() && r.splits.dim() == 2 &&
@@ -105,7 +108,7 @@ LongRows take_long_rows(const Tensor& rowptr, int64_t n_edges, int64_t known_max
   r.partial = torch::empty({r.tasks.size(0), (int64_t)pitch}, rowptr.options().dtype(torch::kFloat));
   r.c.task = r.tasks.data_ptr<int>(); r.c.n_task = (int)r.tasks.size(0);
   r.c.split = r.splits.data_ptr<int>(); r.c.n_split = (int)r.splits.size(0);
-  r.c.partial = r.partial.data_ptr<float>(); r.c.min_degree = BF_LONG_ROW;
+  r.c.partial = r.partial.data_ptr<float>();
   return r;
 }
 
@@ -148,11 +151,12 @@ bf_attn_route parse_route(const std::vector<int64_t>& route, size_t header) {
 
 void edge_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor rowptr, Tensor col, OptTensor etype,
                    OptTensor etab, int64_t variant, double dropout_p, int64_t seed, int64_t known_max_degree,
-                   std::vector<double> out_drop, std::vector<int64_t> route, OptTensor long_task, OptTensor long_split) {
+                   std::vector<double> out_drop, std::vector<int64_t> route, OptTensor long_task, OptTensor long_split,
+                   int64_t long_min) {
   c10::cuda::CUDAGuard guard(q.device());
   bf_attn_params p{};
   fill_common(p, q, k, v, out, z, rowptr, col, etype, etab, variant, dropout_p, seed, out_drop);
-  LongRows lr = take_long_rows(rowptr, col.numel(), known_max_degree, long_task, long_split, bf_attn_fwd_long_pitch(p.hl, p.hn));
+  LongRows lr = take_long_rows(rowptr, col.numel(), known_max_degree, long_task, long_split, long_min, bf_attn_fwd_long_pitch(p.hl, p.hn));
   const bf_attn_route r = parse_route(route, 3);
   check_cuda(bf_edge_attn_fwd_routed(&p, &r, &lr.c, at::cuda::getCurrentCUDAStream()), "edge_attn_fwd");
 }
@@ -161,7 +165,8 @@ void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor do
                    Tensor zd, Tensor rowptr, Tensor col, OptTensor etype, Tensor t_rowptr, Tensor t_row, Tensor t_eid,
                    OptTensor etab, OptTensor detab, int64_t variant, double dropout_p, int64_t seed,
                    int64_t known_max_degree, OptTensor kv_task, OptTensor kv_split, int64_t kv_slots,
-                   std::vector<double> out_drop, std::vector<int64_t> route, OptTensor long_task, OptTensor long_split) {
+                   std::vector<double> out_drop, std::vector<int64_t> route, OptTensor long_task, OptTensor long_split,
+                   int64_t long_min) {
   c10::cuda::CUDAGuard guard(q.device());
   bf_attn_params p{};
   fill_common(p, q, k, v, out, z, rowptr, col, etype, etab, variant, dropout_p, seed, out_drop);
@@ -176,7 +181,7 @@ void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor do
   b.t_rowptr = iptr(t_rowptr); b.t_row = iptr(t_row); b.t_eid = iptr(t_eid);
   b.detab = detab.has_value() ? detab->data_ptr<float>() : nullptr;
   const int64_t w = (int64_t)p.hl * p.hn;
-  LongRows lr = take_long_rows(rowptr, col.numel(), known_max_degree, long_task, long_split, (size_t)w);
+  LongRows lr = take_long_rows(rowptr, col.numel(), known_max_degree, long_task, long_split, long_min, (size_t)w);
   b.long_rows = lr.c;
   Tensor partial, qg;
   Tensor ds = torch::empty({std::max<int64_t>(col.numel(), 1), (int64_t)p.hl}, q.options().dtype(torch::kFloat));
@@ -810,15 +815,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("edge_attn_fwd", &edge_attn_fwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("out"), py::arg("z"), py::arg("rowptr"),
         py::arg("col"), py::arg("etype"), py::arg("etab"), py::arg("variant"), py::arg("dropout_p"), py::arg("seed"),
         py::arg("known_max_degree"), py::arg("out_drop"), py::arg("route"), py::arg("long_task") = py::none(),
-        py::arg("long_split") = py::none());
+        py::arg("long_split") = py::none(), py::arg("long_min") = -1);
   m.def("edge_attn_bwd", &edge_attn_bwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("out"), py::arg("z"), py::arg("dout"),
         py::arg("dq"), py::arg("dk"), py::arg("dv"), py::arg("zd"), py::arg("rowptr"), py::arg("col"), py::arg("etype"),
         py::arg("t_rowptr"), py::arg("t_row"), py::arg("t_eid"), py::arg("etab"), py::arg("detab"), py::arg("variant"),
         py::arg("dropout_p"), py::arg("seed"), py::arg("known_max_degree"), py::arg("kv_task"), py::arg("kv_split"),
         py::arg("kv_slots"), py::arg("out_drop"), py::arg("route"), py::arg("long_task") = py::none(),
-        py::arg("long_split") = py::none());
+        py::arg("long_split") = py::none(), py::arg("long_min") = -1);
   m.def("long_row_tasks", &long_row_tasks);
   m.attr("LONG_ROW") = (int64_t)BF_LONG_ROW;
+  m.attr("LONG_CHUNK") = (int64_t)BF_LONG_CHUNK;
   m.attr("BUILD_HUB_DEGREE") = (int64_t)BF_BUILD_HUB_DEGREE;
   m.def("build_attn_graph", &build_attn_graph);
   m.def("budget_select_rows", &budget_select_rows);

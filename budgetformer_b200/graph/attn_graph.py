@@ -117,6 +117,7 @@ class AttnGraph:
     # slots; see long_rows
     q_task: Optional[torch.Tensor] = field(default=None, repr=False)
     q_split: Optional[torch.Tensor] = field(default=None, repr=False)
+    q_min: int = LONG_ROW                # the list holds every row with more edges than this; the kernels walk all others
 
     @property
     def device(self):
@@ -138,7 +139,7 @@ class AttnGraph:
         f = lambda t: None if t is None else t.to(device, non_blocking=non_blocking)
         return AttnGraph(self.num_rows, f(self.rowptr), f(self.col), f(self.etype), f(self.t_rowptr),
                          f(self.t_row), f(self.t_eid), f(self.t_task), f(self.t_split), self.max_degree,
-                         self.n_real, self.n_rw, self.kv_slots, f(self.q_task), f(self.q_split))
+                         self.n_real, self.n_rw, self.kv_slots, f(self.q_task), f(self.q_split), self.q_min)
 
     def record_stream(self, stream) -> None:
         """Tell the caching allocator that ``stream`` uses every tensor of the graph (they were allocated on another)."""
@@ -179,11 +180,11 @@ class AttnGraph:
         return torch.stack(rows, 0)
 
     def long_rows(self):
-        """``(tasks, splits)`` of the query rows with more than ``LONG_ROW`` edges, for the device kernels; ``(None, None)``
-        when the known degree bound rules them out.  Made once per graph; one host read, behind the kernels that write the list:
+        """``(tasks, splits, n)``: work list of all query rows with more than ``n`` edges, for the device kernels; ``(None, None, 0)``
+        when the known degree bound rules out rows above ``LONG_ROW`` edges.  Made once per graph; one host read, behind the kernels that write the list:
         it is complete for every stream by the time the graph holds it."""
         if self.max_degree is not None and self.max_degree <= LONG_ROW:
-            return None, None
+            return None, None, 0
         if self.q_task is None:
             from ..ops import _ext
             with _LIST_LOCKS[id(self) // 64 % 64]:
@@ -192,7 +193,7 @@ class AttnGraph:
                     _ext.count_launches(5)
                     self.q_task = task                     # last: whoever finds it finds the other
         self._use_lists("long", (self.q_task, self.q_split))
-        return self.q_task, self.q_split
+        return self.q_task, self.q_split, self.q_min
 
     def ensure_transpose(self) -> "AttnGraph":
         """Build the by-key CSR (deterministic: stable sort keeps query order inside a key's row).  Complete for every stream
@@ -319,10 +320,13 @@ def add_virtual_node(graph: AttnGraph, num_nodes: int, nodes_per_rank: int) -> A
     g = AttnGraph(total, rowptr.to(torch.int32), col, None, max_degree=None,
                   n_real=graph.n_real, n_rw=graph.n_rw)
     if graph.max_degree is not None and graph.max_degree < LONG_ROW:
-        # the virtual node's is the only long row, and its length is known here: no device query
+        # the virtual node's is the only long row, and its length is known here: no device query.  The list holds the rows of n and
+        # more edges, whatever the bound of the others is worth.
         m = (n + LONG_CHUNK - 1) // LONG_CHUNK if n > LONG_ROW else 0
         slot = torch.arange(m, dtype=torch.int32, device=dev)
         beg = slot * LONG_CHUNK
         g.q_task = torch.stack([torch.zeros_like(slot), beg, (beg + LONG_CHUNK).clamp_(max=n), slot], 1).contiguous()
-        g.q_split = torch.tensor([[0, 0, m]] if m else [], dtype=torch.int32, device=dev).view(-1, 3)
+        g.q_split = torch.zeros((1 if m else 0, 3), dtype=torch.int32, device=dev)
+        g.q_split[:, 2] = m
+        g.q_min = max(n - 1, LONG_ROW)
     return g

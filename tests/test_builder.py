@@ -198,3 +198,12 @@ def test_general_native_build_equals_spec(b_real, b_rw, walks, length, fanout, u
     via_dispatch = builder.build_attn_graph(topo, b_real, b_rw, walks, length, 31, use_real=use_real, use_rw=use_rw,
                                             exphormer=exphormer, fanout=fanout)
     assert torch.equal(via_dispatch.col, want.col)
+
+
+def test_work_list_constants_match_the_kernels():
+    """The Python side writes work lists with its own copies of the kernels' line and chunk."""
+    from budgetformer_b200.graph import attn_graph
+    from budgetformer_b200.ops import _ext
+    ext = _ext.load()
+    assert (attn_graph.LONG_ROW, attn_graph.LONG_CHUNK) == (ext.LONG_ROW, ext.LONG_CHUNK)
+    assert attn_graph.KV_TASK_EDGES == ext.LONG_CHUNK

@@ -119,6 +119,24 @@ def test_lists_of_a_graph_serve_every_stream(virtual_node):
             assert float((a.double() - b.double()).norm()) <= 2e-5 * (float(b.double().norm()) + float(dout.norm()))
 
 
+def test_virtual_node_beside_a_row_above_its_declared_bound():
+    """add_virtual_node lists the virtual node's row without looking at the others; a row that is longer than the graph's degree
+    bound says is walked all the same."""
+    from budgetformer_b200.graph.attn_graph import add_virtual_node
+    from budgetformer_b200.ops.edge_attention import edge_attention
+    graph = _graph(1500, 300, 9, False)
+    graph.max_degree = 8
+    graph = add_virtual_node(graph, 1500, 1500)
+    assert graph.q_task is not None and int(graph.q_task.size(0)) == 24 and graph.q_split.tolist() == [[0, 0, 24]]
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v, dout = (torch.randn(1501, 2, 16, generator=gen, device="cuda") for _ in range(4))
+    want = _reference(q, k, v, dout, graph, None, "plain", 0.0, 0)
+    args = [t.requires_grad_() for t in (q, k, v)]
+    out = edge_attention(*args, graph)
+    for a, b in zip([out] + list(torch.autograd.grad(out, args, dout)), want):
+        assert float((a.double() - b.double()).norm()) <= 2e-5 * (float(b.double().norm()) + float(dout.norm()))
+
+
 def test_by_key_view_without_its_work_list():
     """A graph that was given t_rowptr, t_row and t_eid alone: the backward pass makes the work list, and the gradients are those
     of the graph's own."""
