@@ -24,6 +24,7 @@ import torch
 LONG_ROW = 128     # query rows with more edges are cut into work items of LONG_CHUNK edges (csrc/bf_kernels.h: BF_LONG_ROW,
 LONG_CHUNK = 64    # BF_LONG_CHUNK)
 _LIST_LOCKS = tuple(threading.Lock() for _ in range(64))   # one thread makes a graph's lists, the others wait for it
+CAPTURE_ROW = 1024  # longest rows that a forward recorded into a CUDA graph walks whole when their list was not made before
 KV_TASK_EDGES = 64  # edges per work item of the dK/dV pass (32 and 128 both measured slower on the 2.9 M-node graph)
 
 
@@ -187,6 +188,9 @@ class AttnGraph:
             return None, None, 0
         if self.q_task is None:
             from ..ops import _ext
+            if (self.max_degree is not None and self.max_degree <= CAPTURE_ROW and self.col.is_cuda
+                    and torch.cuda.is_current_stream_capturing()):
+                return None, None, 0                       # no host read while launches are recorded: all rows are walked
             with _LIST_LOCKS[id(self) // 64 % 64]:
                 if self.q_task is None:
                     task, self.q_split = _ext.load().long_row_tasks(self.rowptr, self.num_edges)

@@ -137,6 +137,30 @@ def test_virtual_node_beside_a_row_above_its_declared_bound():
         assert float((a.double() - b.double()).norm()) <= 2e-5 * (float(b.double().norm()) + float(dout.norm()))
 
 
+@pytest.mark.parametrize("listed_before", [False, True])
+def test_forward_with_long_rows_is_captured(listed_before):
+    """Rows of 129 to 1,024 edges under a known bound: a forward recorded into a CUDA graph needs no host read, whether or not the
+    graph's work list was made before."""
+    from budgetformer_b200.ops.edge_attention import edge_attention, edge_attention_reference
+    graph = _graph(700, 400, 21, False)
+    graph.max_degree = 400
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    q, k, v = (torch.randn(700, 4, 16, generator=gen, device="cuda") for _ in range(3))
+    with torch.no_grad():
+        edge_attention(q, k, v, _graph(700, 5, 1, False))                  # the kernels are loaded
+        if listed_before:
+            edge_attention(q, k, v, graph)
+        torch.cuda.synchronize()
+        rec = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(rec):
+            out = edge_attention(q, k, v, graph)
+        out.zero_()
+        rec.replay()
+        torch.cuda.synchronize()
+    ref = edge_attention_reference(q, k, v, graph)
+    assert float((out - ref).norm()) <= 2e-5 * float(ref.norm())
+
+
 def test_by_key_view_without_its_work_list():
     """A graph that was given t_rowptr, t_row and t_eid alone: the backward pass makes the work list, and the gradients are those
     of the graph's own."""
