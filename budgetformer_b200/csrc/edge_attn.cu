@@ -4,7 +4,8 @@
 // numerator / normaliser in registers.  Rows longer than BF_LONG_ROW (the Graphormer virtual node,
 // hubs of a graph without a budget, popular keys in the transposed graph) are cut into work items of
 // BF_LONG_CHUNK edges, one warp each, whose fp32 partial sums are added in a fixed order by two small
-// kernels: no atomics, bit-reproducible.
+// kernels: no atomics, bit-reproducible.  (The gradient of the edge-type table, a sum over all edges, does meet in atomics, one
+// set per thread block.)
 //
 // Math (reference: models/graphormer_dist_node_level.py:231-263, models/gt_dist_node_level.py:
 // 224-262, models/graphgps_dist_node_level.py:151-177, models/exphormer_dist_node_level.py:92-121):
@@ -999,7 +1000,9 @@ __global__ void __launch_bounds__(kStreamThreads, EXPH ? 4 : 7) edge_attn_bwd_q_
   }
 }
 
-// Long rows of the dQ pass: work items as in edge_attn_fwd_long_kernel, partial dQ rows to the scratch.
+// Long rows of the dQ pass: work items as in edge_attn_fwd_long_kernel, partial dQ rows to the scratch.  The type table's gradient
+// of a block's eight items meets in shared memory first, as in the regular kernel: every item would otherwise add 2 * Hl * HN
+// values to the same addresses.
 template <typename T, int HN, bool EXPH>
 __global__ void __launch_bounds__(256, EXPH ? 3 : 4) edge_attn_bwd_q_long_kernel(BwdArgs b) {
   constexpr int VN = Vec<T>::N, NP = VN / 2, LPH = HN / VN, NB = 4;
@@ -1008,75 +1011,89 @@ __global__ void __launch_bounds__(256, EXPH ? 3 : 4) edge_attn_bwd_q_long_kernel
   const int w_row = a.hl * HN;
   const int lane = threadIdx.x & 31;
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (warp >= (long long)a.n_long_task * g.n_hc) return;
-  const int tpw = 32 / g.tl, sub = lane / g.tl, lt = lane % g.tl;
-  const int item = (int)(warp / g.n_hc), hc = (int)(warp % g.n_hc);
-  const int head = hc * g.hpt + lt / LPH;
-  const bool head_ok = head < a.hl;
-  const int hsafe = head_ok ? head : 0;
-  const int off = hsafe * HN + (lt % LPH) * VN;
-  const int4 it = __ldg(a.long_task + item);
-  const int per = (it.z - it.y + tpw - 1) / tpw;
-  const int beg = it.y + sub * per, end = min(it.z, beg + per);
-  f2 s0[NP], s1[NP];
-  unsigned seen = 0;                            // edge types of the item (see the dK/dV pass)
+  const bool work = warp < (long long)a.n_long_task * g.n_hc;         // the whole warp
+  extern __shared__ float s_detab[];            // [2, Hl*HN] when exphormer
+  if (EXPH) {
+    for (int i = threadIdx.x; i < 2 * w_row; i += blockDim.x) s_detab[i] = 0.f;
+    __syncthreads();
+  } else if (!work) {
+    return;
+  }
+  if (work) {
+    const int tpw = 32 / g.tl, sub = lane / g.tl, lt = lane % g.tl;
+    const int item = (int)(warp / g.n_hc), hc = (int)(warp % g.n_hc);
+    const int head = hc * g.hpt + lt / LPH;
+    const bool head_ok = head < a.hl;
+    const int hsafe = head_ok ? head : 0;
+    const int off = hsafe * HN + (lt % LPH) * VN;
+    const int4 it = __ldg(a.long_task + item);
+    const int per = (it.z - it.y + tpw - 1) / tpw;
+    const int beg = it.y + sub * per, end = min(it.z, beg + per);
+    f2 s0[NP], s1[NP];
+    unsigned seen = 0;                            // edge types of the item (see the dK/dV pass)
 #pragma unroll
-  for (int i = 0; i < NP; ++i) { s0[i] = pack2(0.f, 0.f); s1[i] = pack2(0.f, 0.f); }
-  for (int e = beg; e < end; e += NB) {
-    uint4 kr[NB];
-    float ds[NB];
-    bool t1[NB];
+    for (int i = 0; i < NP; ++i) { s0[i] = pack2(0.f, 0.f); s1[i] = pack2(0.f, 0.f); }
+    for (int e = beg; e < end; e += NB) {
+      uint4 kr[NB];
+      float ds[NB];
+      bool t1[NB];
 #pragma unroll
-    for (int u = 0; u < NB; ++u) {
-      const bool ok = e + u < end;
-      const int j = ok ? __ldg(a.col + e + u) : 0;
-      kr[u] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(a.k) + (long long)j * a.ldk + off));
-      ds[u] = ok ? __ldg(b.ds + (long long)(e + u) * a.hl + hsafe) : 0.f;
-      t1[u] = EXPH && ok && a.etype[e + u] != 0;
-    }
+      for (int u = 0; u < NB; ++u) {
+        const bool ok = e + u < end;
+        const int j = ok ? __ldg(a.col + e + u) : 0;
+        kr[u] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(a.k) + (long long)j * a.ldk + off));
+        ds[u] = ok ? __ldg(b.ds + (long long)(e + u) * a.hl + hsafe) : 0.f;
+        t1[u] = EXPH && ok && a.etype[e + u] != 0;
+      }
 #pragma unroll
-    for (int u = 0; u < NB; ++u) {
-      // an absent edge reads key 0 with weight 0: nothing may be added from it, not even 0 * inf
-      if (e + u >= end) break;
-      f2 kf[NP];
-      widen<T>(kr[u], kf);
-      const f2 d2 = pack2(ds[u], ds[u]);
-      if (EXPH) seen |= t1[u] ? 2u : 1u;
-      if (EXPH && t1[u]) {
+      for (int u = 0; u < NB; ++u) {
+        // an absent edge reads key 0 with weight 0: nothing may be added from it, not even 0 * inf
+        if (e + u >= end) break;
+        f2 kf[NP];
+        widen<T>(kr[u], kf);
+        const f2 d2 = pack2(ds[u], ds[u]);
+        if (EXPH) seen |= t1[u] ? 2u : 1u;
+        if (EXPH && t1[u]) {
 #pragma unroll
-        for (int i = 0; i < NP; ++i) s1[i] = fma2(d2, kf[i], s1[i]);
-      } else {
+          for (int i = 0; i < NP; ++i) s1[i] = fma2(d2, kf[i], s1[i]);
+        } else {
 #pragma unroll
-        for (int i = 0; i < NP; ++i) s0[i] = fma2(d2, kf[i], s0[i]);
+          for (int i = 0; i < NP; ++i) s0[i] = fma2(d2, kf[i], s0[i]);
+        }
       }
     }
-  }
-  __syncwarp();
-  if (EXPH) seen = __reduce_or_sync(kFull, seen);
-  float x0[VN], x1[VN];
+    __syncwarp();
+    if (EXPH) seen = __reduce_or_sync(kFull, seen);
+    float x0[VN], x1[VN];
 #pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    const float2 t = unpack2(s0[i]);
-    x0[2 * i] = group_total(t.x, g.tl); x0[2 * i + 1] = group_total(t.y, g.tl);
-    if (EXPH) {
-      const float2 y = unpack2(s1[i]);
-      x1[2 * i] = group_total(y.x, g.tl); x1[2 * i + 1] = group_total(y.y, g.tl);
-    }
-  }
-  if (sub == 0 && head_ok) {
-    float* pp = a.long_partial + (long long)it.w * w_row;
-    if (EXPH) {
-      float qf[VN];
-      load_vec<T>(static_cast<const T*>(a.q) + (long long)it.x * a.ldq + off, qf);
-#pragma unroll
-      for (int i = 0; i < VN; ++i) {
-        if (seen & 1u) atomicAdd(b.detab + off + i, qf[i] * x0[i]);
-        if (seen & 2u) atomicAdd(b.detab + w_row + off + i, qf[i] * x1[i]);
-        x0[i] = ((seen & 1u) ? x0[i] * __ldg(a.etab + off + i) : 0.f) + ((seen & 2u) ? x1[i] * __ldg(a.etab + w_row + off + i) : 0.f);
+    for (int i = 0; i < NP; ++i) {
+      const float2 t = unpack2(s0[i]);
+      x0[2 * i] = group_total(t.x, g.tl); x0[2 * i + 1] = group_total(t.y, g.tl);
+      if (EXPH) {
+        const float2 y = unpack2(s1[i]);
+        x1[2 * i] = group_total(y.x, g.tl); x1[2 * i + 1] = group_total(y.y, g.tl);
       }
     }
+    if (sub == 0 && head_ok) {
+      float* pp = a.long_partial + (long long)it.w * w_row;
+      if (EXPH) {
+        float qf[VN];
+        load_vec<T>(static_cast<const T*>(a.q) + (long long)it.x * a.ldq + off, qf);
 #pragma unroll
-    for (int i = 0; i < VN; i += 4) *reinterpret_cast<float4*>(pp + off + i) = make_float4(x0[i], x0[i + 1], x0[i + 2], x0[i + 3]);
+        for (int i = 0; i < VN; ++i) {
+          if (seen & 1u) atomicAdd(&s_detab[off + i], qf[i] * x0[i]);
+          if (seen & 2u) atomicAdd(&s_detab[w_row + off + i], qf[i] * x1[i]);
+          x0[i] = ((seen & 1u) ? x0[i] * __ldg(a.etab + off + i) : 0.f) + ((seen & 2u) ? x1[i] * __ldg(a.etab + w_row + off + i) : 0.f);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < VN; i += 4) *reinterpret_cast<float4*>(pp + off + i) = make_float4(x0[i], x0[i + 1], x0[i + 2], x0[i + 3]);
+    }
+  }
+  if (EXPH) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * w_row; i += blockDim.x)
+      if (s_detab[i] != 0.f) atomicAdd(b.detab + i, s_detab[i]);
   }
 }
 
@@ -1296,7 +1313,7 @@ cudaError_t launch_bwd_t(const BwdArgs& b, cudaStream_t st) {
   }
   if (a.n_long_task > 0) {
     const unsigned lb = (unsigned)(((long long)a.n_long_task * g.n_hc + 7) / 8);
-    if (a.variant == 2) edge_attn_bwd_q_long_kernel<T, HN, true><<<lb, 256, 0, st>>>(b);
+    if (a.variant == 2) edge_attn_bwd_q_long_kernel<T, HN, true><<<lb, 256, type_table_bytes(w_row), st>>>(b);
     else edge_attn_bwd_q_long_kernel<T, HN, false><<<lb, 256, 0, st>>>(b);
     launch_split<T, SPLIT_DQ>(b, a.long_task, a.n_long_task, a.long_split, a.n_long_split, a.long_partial, w_row, w_row, w_row, HN, st);
   }
