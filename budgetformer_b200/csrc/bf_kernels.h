@@ -79,7 +79,7 @@ typedef struct {
   long long ldg;
   float* zd;                        // [n, hl, 2] fp32 workspace: 1 / (Z + eps) and <dout, out> of every row
   float* ds;                        // [E, hl] fp32 workspace: score gradients, from the dK/dV pass to the dQ pass
-  const int *t_rowptr, *t_row, *t_eid;  // transposed CSR over keys
+  const int *t_row, *t_eid;         // edges grouped by key: query, and position in the query-grouped list
   float* detab;                     // zero-filled [2, hl, hn] fp32 or NULL
   bf_long_rows long_rows;           // scratch row: hl*hn floats
   // balanced dK/dV work list; the n_kv_slots items of split keys come first, in slot order

@@ -178,7 +178,7 @@ void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor do
   b.dout = dout.data_ptr(); b.dq = dq.data_ptr(); b.dk = dk.data_ptr(); b.dv = dv.data_ptr();
   b.ldg = dq.stride(0);
   b.zd = zd.data_ptr<float>();
-  b.t_rowptr = iptr(t_rowptr); b.t_row = iptr(t_row); b.t_eid = iptr(t_eid);
+  b.t_row = iptr(t_row); b.t_eid = iptr(t_eid);
   b.detab = detab.has_value() ? detab->data_ptr<float>() : nullptr;
   const int64_t w = (int64_t)p.hl * p.hn;
   LongRows lr = take_long_rows(rowptr, col.numel(), known_max_degree, long_task, long_split, long_min, (size_t)w);

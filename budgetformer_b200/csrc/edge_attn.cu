@@ -637,7 +637,7 @@ struct BwdArgs {
   long long ldg;
   float2* zd;                  // [n, Hl]: (1/(Z+eps), D = <dout,out>)
   float* ds;                   // [E, Hl]: score gradient / sqrt(hn), left by the dK/dV pass for the dQ pass
-  const int *t_rowptr, *t_row, *t_eid;
+  const int *t_row, *t_eid;    // by key: query and position of every edge
   float* detab;                // [T, Hl, HN] fp32 or null
   // balanced dK/dV work list
   const int4* kv_task;         // [n_kv_task]: key row, first edge, end edge, partial slot (-1 = direct store)
@@ -1417,7 +1417,7 @@ extern "C" int bf_edge_attn_bwd(const bf_attn_params* p, const bf_attn_bwd_param
   b.ldg = q->ldg > 0 ? q->ldg : (long long)p->hl * p->hn;
   b.zd = reinterpret_cast<float2*>(q->zd);
   b.ds = q->ds;
-  b.t_rowptr = q->t_rowptr; b.t_row = q->t_row; b.t_eid = q->t_eid; b.detab = q->detab;
+  b.t_row = q->t_row; b.t_eid = q->t_eid; b.detab = q->detab;
   b.kv_task = reinterpret_cast<const int4*>(q->kv_task); b.n_kv_task = q->n_kv_task;
   b.kv_split = q->kv_split; b.n_kv_split = q->n_kv_split; b.n_kv_slots = q->n_kv_split > 0 ? q->n_kv_slots : 0; b.kv_partial = q->kv_partial;
   if (b.n_kv_split > 0 && (b.kv_split == nullptr || b.kv_partial == nullptr || b.n_kv_slots <= 0 || b.n_kv_slots > b.n_kv_task))

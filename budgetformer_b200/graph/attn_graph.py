@@ -194,7 +194,7 @@ class AttnGraph:
             with _LIST_LOCKS[id(self) // 64 % 64]:
                 if self.q_task is None:
                     task, self.q_split = _ext.load().long_row_tasks(self.rowptr, self.num_edges)
-                    _ext.count_launches(5)
+                    _ext.count_launches(2)                 # counts, fill (and the library's prefix sums between them)
                     self.q_task = task                     # last: whoever finds it finds the other
         self._use_lists("long", (self.q_task, self.q_split))
         return self.q_task, self.q_split, self.q_min
@@ -215,7 +215,7 @@ class AttnGraph:
             from ..ops import _ext
             t_rowptr, t_row, t_eid, tasks, splits, sizes = _ext.load().graph_transpose(
                 self.rowptr.contiguous(), self.col.contiguous(), int(self.num_rows), int(KV_TASK_EDGES))
-            _ext.count_launches(9)
+            _ext.count_launches(6)                         # rows, key offsets, gather, counts, two fills (and the library's sorts)
             self.t_row, self.t_eid = t_row, t_eid
             self.t_task, self.t_split, self.kv_slots = tasks, splits, int(sizes[1])
             self.t_rowptr = t_rowptr                       # last: whoever finds it finds the others

@@ -57,7 +57,7 @@ def test_edge_attention_gps_dropout():
 
 @pytest.mark.parametrize("variant", ["plain", "gps", "exphormer"])
 def test_edge_attention_hub_rows(variant):
-    """A query with 5000 in-edges and a key used by 4000 queries take the chunked hub kernels."""
+    """A query with 5000 in-edges and a key used by 4000 queries are cut into work items of 64 edges."""
     _run(variant, torch.float32, 4, 16, hub_row=5000, hub_col=4000, n=4500, e=9000)
     _run(variant, torch.bfloat16, 1, 16, hub_row=20000, hub_col=3000, n=4500, e=9000)
 
