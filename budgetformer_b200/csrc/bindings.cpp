@@ -822,18 +822,21 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("dropout_p"), py::arg("seed"), py::arg("known_max_degree"), py::arg("kv_task"), py::arg("kv_split"),
         py::arg("kv_slots"), py::arg("out_drop"), py::arg("route"), py::arg("long_task") = py::none(),
         py::arg("long_split") = py::none(), py::arg("long_min") = -1);
-  m.def("long_row_tasks", &long_row_tasks);
+  // These wait for the device (the sizes of what they return).  The interpreter lock is free meanwhile: the look-ahead build runs
+  // on a thread of its own beside the one that launches the step.
+  using unlocked = py::call_guard<py::gil_scoped_release>;
+  m.def("long_row_tasks", &long_row_tasks, unlocked());
   m.attr("LONG_ROW") = (int64_t)BF_LONG_ROW;
   m.attr("LONG_CHUNK") = (int64_t)BF_LONG_CHUNK;
   m.attr("BUILD_HUB_DEGREE") = (int64_t)BF_BUILD_HUB_DEGREE;
-  m.def("build_attn_graph", &build_attn_graph);
+  m.def("build_attn_graph", &build_attn_graph, unlocked());
   m.def("budget_select_rows", &budget_select_rows);
-  m.def("ell_rows_to_csr", &ell_rows_to_csr);
+  m.def("ell_rows_to_csr", &ell_rows_to_csr, unlocked());
   m.def("peer_concat", &peer_concat);
   m.def("khop_candidates_cpu", &khop_candidates_cpu);
   m.def("partition_cpu", &partition_cpu);
   m.def("build_attn_graph_rows_cpu", &build_attn_graph_rows_cpu);
-  m.def("graph_transpose", &graph_transpose);
+  m.def("graph_transpose", &graph_transpose, unlocked());
   m.def("gemm_tn", &gemm_tn);
   m.def("gemm_tn_pull", &gemm_tn_pull);
   m.def("gemm_dw", &gemm_dw);
