@@ -99,8 +99,9 @@ typedef struct {
 
 int bf_edge_attn_fwd(const bf_attn_params* p, cudaStream_t st);
 // as above; additionally every output row is stored into its owner's buffer (route may be NULL), and long rows come as
-// work items (long_rows may be NULL; its scratch has bf_attn_fwd_long_pitch floats per item)
-int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_route* route, const bf_long_rows* long_rows, cudaStream_t st);
+// work items (long_rows may be NULL; its scratch has bf_attn_fwd_long_pitch floats per item); n_edges chooses between two kernels
+int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_route* route, const bf_long_rows* long_rows, long long n_edges,
+                            cudaStream_t st);
 size_t bf_attn_fwd_long_pitch(int hl, int hn);
 int bf_edge_attn_bwd(const bf_attn_params* p, const bf_attn_bwd_params* q, cudaStream_t st);
 

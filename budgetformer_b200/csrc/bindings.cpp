@@ -158,7 +158,7 @@ void edge_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor ro
   fill_common(p, q, k, v, out, z, rowptr, col, etype, etab, variant, dropout_p, seed, out_drop);
   LongRows lr = take_long_rows(rowptr, col.numel(), known_max_degree, long_task, long_split, long_min, bf_attn_fwd_long_pitch(p.hl, p.hn));
   const bf_attn_route r = parse_route(route, 3);
-  check_cuda(bf_edge_attn_fwd_routed(&p, &r, &lr.c, at::cuda::getCurrentCUDAStream()), "edge_attn_fwd");
+  check_cuda(bf_edge_attn_fwd_routed(&p, &r, &lr.c, col.numel(), at::cuda::getCurrentCUDAStream()), "edge_attn_fwd");
 }
 
 void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor dout, Tensor dq, Tensor dk, Tensor dv,

@@ -290,6 +290,51 @@ __device__ __forceinline__ void load_q_scaled(const AttnArgs& a, int row, int he
   }
 }
 
+// Forward over the rows, one lane group (16 bytes a lane) per (row, head chunk), two edges' gathers in flight in registers.  Many
+// small lane groups and few registers: the better form where the gathered rows come out of L2 (see rows_forward).
+template <typename T, int HN>
+__global__ void __launch_bounds__(256) edge_attn_fwd_rows_kernel(AttnArgs a) {
+  constexpr int VN = Vec<T>::N;
+  constexpr int LPH = HN / VN;
+  const Geo g = make_geo<T, HN>(a.hl);
+  const int lane = threadIdx.x & 31;
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long task = warp * (32 / g.tl) + lane / g.tl;
+  const int lt = lane % g.tl;
+  const bool live = task < (long long)a.n * g.n_hc;
+  const int row = live ? (int)(task / g.n_hc) : 0;
+  const int hc = live ? (int)(task % g.n_hc) : 0;
+  const int head = hc * g.hpt + lt / LPH;
+  const bool head_ok = live && head < a.hl;
+  const int hsafe = head_ok ? head : 0;
+  const int off = hsafe * HN + (lt % LPH) * VN;
+  int beg = 0, end = 0;
+  if (head_ok) { beg = a.rowptr[row]; end = a.rowptr[row + 1]; }
+  const bool cut = a.long_row > 0 && end - beg > a.long_row;          // left to the long-row kernels
+  if (cut) end = beg;
+  float qs0[VN], qs1[VN], acc[VN];
+  float zsum = 0.f;
+#pragma unroll
+  for (int i = 0; i < VN; ++i) acc[i] = 0.f;
+  load_q_scaled<T, HN>(a, row, hsafe, off, qs0, qs1);
+  const unsigned hm = head_mask<LPH>();
+  for (int e = beg; e < end; e += 2) fwd_pair<T, HN>(a, hsafe, off, e, e + 1, e + 1 < end, hm, qs0, qs1, acc, zsum);
+  if (head_ok && !cut) {
+    float inv = 1.f / (zsum + kEps);
+    if (a.variant == 1) inv *= a.inv_keep;
+    float o[VN];
+#pragma unroll
+    for (int i = 0; i < VN; ++i) o[i] = acc[i] * inv;
+    if (a.out_thresh) {
+#pragma unroll
+      for (int i = 0; i < VN; ++i) o[i] = keep_out(a, row, off + i) ? o[i] * a.out_inv_keep : 0.f;
+    }
+    store_vec<T>(static_cast<T*>(a.out) + (long long)row * a.hl * HN + off, o);
+    if (a.route_out.n_dest) store_vec<T>(routed<T>(a.route_out, row, off), o);
+    if ((lt % LPH) == 0) a.z[(long long)row * a.hl + head] = zsum;
+  }
+}
+
 // ---------------------------------------------------------------------------------------------
 // Streams.  A warp holds 32 / TL lane groups of TL lanes; each group owns one segment (a query row, or a key work item) at a
 // time and `per` of them in all.  The groups of a warp step together: segment r of every group starts at the same step and
@@ -402,7 +447,7 @@ template <bool TYPED> struct RowFetch {
   }
 };
 
-template <typename T, int HN, int VAR>
+template <typename T, int HN, bool GPS>
 __global__ void __launch_bounds__(kStreamThreads, 4) edge_attn_fwd_kernel(AttnArgs a, StreamGeo sg) {
   constexpr int VN = wide_elems<T, HN>(), NP = VN / 2, LPH = HN / VN;
   using S = Slices<T, VN>;
@@ -419,14 +464,12 @@ __global__ void __launch_bounds__(kStreamThreads, 4) edge_attn_fwd_kernel(AttnAr
   const T* qb = static_cast<const T*>(a.q) + off;
   const unsigned long long skb = (unsigned long long)a.ldk * sizeof(T), svb = (unsigned long long)a.ldv * sizeof(T);
 
-  RowFetch<VAR == 2> f;
+  RowFetch<false> f;
   f.start(a, rows, n_seg);
-  unsigned types = 0;                           // edge type of every ring slot
   auto issue = [&](int slot) {
     if (f.has()) {
       S::copy(ring[slot][0], tid, kb + (unsigned)f.key * skb);
       S::copy(ring[slot][1], tid, vb + (unsigned)f.key * svb);
-      if (VAR == 2) types = (types & ~(1u << slot)) | ((f.type ? 1u : 0u) << slot);
     }
     copy_commit();
     f.advance(a, rows, n_seg);
@@ -443,21 +486,12 @@ __global__ void __launch_bounds__(kStreamThreads, 4) edge_attn_fwd_kernel(AttnAr
   int slot = 0;
   for (int r = 0; r < n_seg; ++r) {
     const long long row = rows.base + (long long)r * groups;
-    f2 q0[NP], q1[NP], acc[NP];
+    f2 q0[NP], acc[NP];
     const float scale = inv_sqrt_hn<HN>();
     const f2 sc = pack2(scale, scale);
     S::spread(qn, q0);
 #pragma unroll
     for (int i = 0; i < NP; ++i) { q0[i] = mul2(q0[i], sc); acc[i] = pack2(0.f, 0.f); }
-    if (VAR == 2) {
-      const float* et = a.etab + off;
-      const int w = a.hl * HN;
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        q1[i] = mul2(q0[i], pack2(__ldg(et + w + 2 * i), __ldg(et + w + 2 * i + 1)));
-        q0[i] = mul2(q0[i], pack2(__ldg(et + 2 * i), __ldg(et + 2 * i + 1)));
-      }
-    }
     if (r + 1 < n_seg) {
       nstored = rows.bounds(a, r + 1, nbeg, nlen);
       if (nstored) S::load(qb + (row + groups) * a.ldq, qn);
@@ -469,22 +503,12 @@ __global__ void __launch_bounds__(kStreamThreads, 4) edge_attn_fwd_kernel(AttnAr
       copy_wait<kRing - 1>();
       f2 x[NP];
       S::read(ring[slot][0], tid, x);
-      float d;
-      if (VAR == 2) {
-        const bool t1 = (types >> slot) & 1u;
-        f2 qq[NP];
-#pragma unroll
-        for (int u = 0; u < NP; ++u) qq[u] = t1 ? q1[u] : q0[u];
-        d = dot2<NP>(qq, x);
-      } else {
-        d = dot2<NP>(q0, x);
-      }
-      d = head_sum<LPH>(d, kFull);
+      const float d = head_sum<LPH>(dot2<NP>(q0, x), kFull);
       float w = __expf(fminf(fmaxf(d, -kClamp), kClamp));
       S::read(ring[slot][1], tid, x);
       if (i < len) {                            // a group whose segment is over holds a stale slot: nothing of it is added
         zsum += w;
-        if (VAR == 1 && a.thresh && !keep_edge(a.seed, (uint32_t)(beg + i), (uint32_t)head, a.thresh)) w = 0.f;
+        if (GPS && a.thresh && !keep_edge(a.seed, (uint32_t)(beg + i), (uint32_t)head, a.thresh)) w = 0.f;
         const f2 ww = pack2(w, w);
 #pragma unroll
         for (int u = 0; u < NP; ++u) acc[u] = fma2(ww, x[u], acc[u]);
@@ -493,7 +517,7 @@ __global__ void __launch_bounds__(kStreamThreads, 4) edge_attn_fwd_kernel(AttnAr
     }
     if (stored) {
       float inv = 1.f / (zsum + kEps);
-      if (VAR == 1) inv *= a.inv_keep;
+      if (GPS) inv *= a.inv_keep;
       const f2 iv = pack2(inv, inv);
 #pragma unroll
       for (int i = 0; i < NP; ++i) acc[i] = mul2(acc[i], iv);
@@ -1248,16 +1272,38 @@ void launch_kv(const BwdArgs& b, cudaStream_t st) {
   edge_attn_bwd_kv_kernel<T, HN, VAR><<<grid, kStreamThreads, 0, st>>>(b, s);
 }
 
+// Whether the forward pass takes edge_attn_fwd_rows_kernel.  Streams hide the latency of DRAM; where the gathered rows stay in L2
+// (126 MB, shared with everything else) they cost more instructions per edge than they save.  Measured, us, rows against streams:
+// - fp32, 8 x 16: 10 k nodes 14 / 18, 50 k (51 MB of k and v) 76 / 117, 170 k (174 MB) 297 / 354, 300 k 406 / 410, 2 M 2155 / 1975;
+//   8 x 8: 300 k (154 MB) 225 / 232, 600 k 472 / 453; 4 x 64: 60 k (123 MB) 189 / 224, 170 k (348 MB) 450 / 418
+// - 16 bits, rows of up to 64 bytes (little work per lane): 1 x 16 600 k (38 MB) 60 / 96, 2.9 M (186 MB) 339 / 363; 2 x 16 600 k
+//   (77 MB) 118 / 138, 2.9 M (371 MB) 681 / 624
+// - 16 bits, heads of 8 (a head is one lane's 16 bytes): 8 x 8 170 k (44 MB) 83 / 98, 300 k (77 MB) 151 / 159, 600 k 222 / 206
+// - 16 bits otherwise, 16 edges a row: 4 x 16 170 k (44 MB) 95 / 105, 8 x 32 50 k (51 MB) with dropout 153 / 178, 8 x 16 170 k (87 MB)
+//   198 / 186; 5 to 8 edges a row: 4 x 16 110 k 57 / 49, 8 x 16 50 k 36 / 31, 8 x 32 50 k 63 / 58 (longer rows pay the streams' cost
+//   per edge, short ones the other kernel's cost per row)
+// - typed edges (two scaled queries, a select per element): 8 x 32, 25 edges, 50 k 167 / 201, 390 k (400 MB) 1879 / 1893
+inline bool rows_forward(int dtype, long long n, int hl, int hn, int variant, long long n_edges) {
+  const long long row = (long long)hl * hn * (dtype == BF_FP32 ? 4 : 2), gathered = 2 * n * row;
+  if (variant == 2) return true;
+  if (dtype == BF_FP32 || row <= 64) return gathered <= 200'000'000;
+  if (hn == 8) return gathered <= 100'000'000;
+  return n_edges >= 12 * n && gathered <= 64'000'000;
+}
+
 template <typename T, int HN>
-cudaError_t launch_fwd_t(const AttnArgs& a, int chunks_per_hub, cudaStream_t st) {
+cudaError_t launch_fwd_t(const AttnArgs& a, bool rows, int chunks_per_hub, cudaStream_t st) {
   const Geo g = make_geo<T, HN>(a.hl);
-  if (a.n > 0) {
+  if (a.n > 0 && rows) {
+    const int tpw = 32 / g.tl;
+    const long long warps = ((long long)a.n * g.n_hc + tpw - 1) / tpw;
+    edge_attn_fwd_rows_kernel<T, HN><<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(a);
+  } else if (a.n > 0) {
     constexpr int VN = wide_elems<T, HN>();
     const StreamGeo s = stream_geo<HN, VN>(a.hl, a.n, 4, 8);
     const dim3 grid = stream_grid<HN, VN>(a.hl, stream_warps(a.n, s, s.per), s);
-    if (a.variant == 2) edge_attn_fwd_kernel<T, HN, 2><<<grid, kStreamThreads, 0, st>>>(a, s);
-    else if (a.variant == 1) edge_attn_fwd_kernel<T, HN, 1><<<grid, kStreamThreads, 0, st>>>(a, s);
-    else edge_attn_fwd_kernel<T, HN, 0><<<grid, kStreamThreads, 0, st>>>(a, s);
+    if (a.variant == 1) edge_attn_fwd_kernel<T, HN, true><<<grid, kStreamThreads, 0, st>>>(a, s);
+    else edge_attn_fwd_kernel<T, HN, false><<<grid, kStreamThreads, 0, st>>>(a, s);
   }
   if (a.n_long_task > 0) {
     edge_attn_fwd_long_kernel<T, HN><<<(unsigned)(((long long)a.n_long_task * g.n_hc + 7) / 8), 256, 0, st>>>(a);
@@ -1389,12 +1435,13 @@ bool to_route(const bf_attn_route* r, int n, long long width, Route* out) {
 extern "C" size_t bf_attn_fwd_long_pitch(int hl, int hn) { return (size_t)fwd_pitch(hl * hn, hl); }
 
 extern "C" int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_route* route, const bf_long_rows* long_rows,
-                                       cudaStream_t st) {
+                                       long long n_edges, cudaStream_t st) {
   AttnArgs a = to_args(*p);
   if (!take_long_rows(long_rows, &a)) return (int)cudaErrorInvalidValue;
   if (!to_route(route, p->n, (long long)p->hl * p->hn, &a.route_out)) return (int)cudaErrorInvalidValue;
   const int chunks = p->max_hub_degree > 0 ? (p->max_hub_degree + BF_HUB_CHUNK - 1) / BF_HUB_CHUNK : 1;
-#define CALL_FWD(T, H) (int)launch_fwd_t<T, H>(a, chunks, st)
+  const bool rows = rows_forward(p->dtype, p->n, p->hl, p->hn, p->variant, n_edges);
+#define CALL_FWD(T, H) (int)launch_fwd_t<T, H>(a, rows, chunks, st)
   BF_DISPATCH(p->dtype, p->hn, CALL_FWD);
 #undef CALL_FWD
   return (int)cudaErrorInvalidValue;
@@ -1403,7 +1450,8 @@ extern "C" int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_ro
 extern "C" int bf_edge_attn_fwd(const bf_attn_params* p, cudaStream_t st) {
   AttnArgs a = to_args(*p);
   const int chunks = p->max_hub_degree > 0 ? (p->max_hub_degree + BF_HUB_CHUNK - 1) / BF_HUB_CHUNK : 1;
-#define CALL_FWD(T, H) (int)launch_fwd_t<T, H>(a, chunks, st)
+  const bool rows = rows_forward(p->dtype, p->n, p->hl, p->hn, p->variant, -1);       // the number of edges is not known here
+#define CALL_FWD(T, H) (int)launch_fwd_t<T, H>(a, rows, chunks, st)
   BF_DISPATCH(p->dtype, p->hn, CALL_FWD);
 #undef CALL_FWD
   return (int)cudaErrorInvalidValue;

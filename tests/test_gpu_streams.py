@@ -33,7 +33,9 @@ def _reference(q, k, v, dout, graph, tab, variant, p, seed):
     (30011, 8, 32, 8, torch.bfloat16), (30011, 8, 8, 6, torch.float16), (9001, 4, 64, 8, torch.float32),
     # two and three segments a lane group in every pass, and the most that one takes (8; 32 in the typed dQ pass)
     (35003, 8, 32, 5, torch.bfloat16), (25013, 4, 64, 5, torch.float32), (134999, 8, 32, 4, torch.bfloat16),
-    (310007, 4, 64, 3, torch.float16)])
+    (310007, 4, 64, 3, torch.float16),
+    # behind the lines up to which the forward pass walks rows without a stream (k and v of 200 MB; 100 MB with heads of 8)
+    (101021, 4, 64, 3, torch.float32), (1600007, 2, 16, 3, torch.bfloat16), (410003, 8, 8, 3, torch.float16)])
 def test_attention_streams(n, heads, hn, max_deg, dtype, variant):
     from budgetformer_b200.ops.edge_attention import edge_attention
     if variant == "exphormer" and max_deg == 0:
