@@ -149,7 +149,8 @@ bf_attn_route parse_route(const std::vector<int64_t>& route, size_t header) {
   return r;
 }
 
-void edge_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor rowptr, Tensor col, OptTensor etype,
+// returns the number of kernels launched
+int64_t edge_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor rowptr, Tensor col, OptTensor etype,
                    OptTensor etab, int64_t variant, double dropout_p, int64_t seed, int64_t known_max_degree,
                    std::vector<double> out_drop, std::vector<int64_t> route, OptTensor long_task, OptTensor long_split,
                    int64_t long_min) {
@@ -159,9 +160,11 @@ void edge_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor ro
   LongRows lr = take_long_rows(rowptr, col.numel(), known_max_degree, long_task, long_split, long_min, bf_attn_fwd_long_pitch(p.hl, p.hn));
   const bf_attn_route r = parse_route(route, 3);
   check_cuda(bf_edge_attn_fwd_routed(&p, &r, &lr.c, col.numel(), at::cuda::getCurrentCUDAStream()), "edge_attn_fwd");
+  return 1 + (lr.c.n_task > 0 ? 3 : 0);
 }
 
-void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor dout, Tensor dq, Tensor dk, Tensor dv,
+// returns the number of kernels launched
+int64_t edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor dout, Tensor dq, Tensor dk, Tensor dv,
                    Tensor zd, Tensor rowptr, Tensor col, OptTensor etype, Tensor t_rowptr, Tensor t_row, Tensor t_eid,
                    OptTensor etab, OptTensor detab, int64_t variant, double dropout_p, int64_t seed,
                    int64_t known_max_degree, OptTensor kv_task, OptTensor kv_split, int64_t kv_slots,
@@ -184,8 +187,12 @@ void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor do
   LongRows lr = take_long_rows(rowptr, col.numel(), known_max_degree, long_task, long_split, long_min, (size_t)w);
   b.long_rows = lr.c;
   Tensor partial, qg;
-  Tensor ds = torch::empty({std::max<int64_t>(col.numel(), 1), (int64_t)p.hl}, q.options().dtype(torch::kFloat));
-  b.ds = ds.data_ptr<float>();
+  const bool keeps = bf_attn_bwd_keeps_scores(p.dtype, p.n, p.hl, p.hn, p.variant) != 0;
+  Tensor ds;
+  if (keeps) {
+    ds = torch::empty({std::max<int64_t>(col.numel(), 1), (int64_t)p.hl}, q.options().dtype(torch::kFloat));
+    b.ds = ds.data_ptr<float>();
+  }
   if (w * q.element_size() <= 64) {
     // narrow rows: one packed record per (query, head) for the dK/dV pass (see bf_attn_bwd_params)
     qg = torch::empty({q.size(0), (int64_t)p.hl, 2, (int64_t)p.hn}, q.options());
@@ -212,6 +219,7 @@ void edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor do
     b.route_cq = (int)route[3]; b.route_ck = (int)route[4]; b.route_cv = (int)route[5];
   }
   check_cuda(bf_edge_attn_bwd(&p, &b, at::cuda::getCurrentCUDAStream()), "edge_attn_bwd");
+  return (keeps ? 3 : 2) + (b.n_kv_split > 0 ? 2 : 0) + (lr.c.n_task > 0 ? 3 : 0);
 }
 
 // Returns (rowptr int32 [n+1], col int32 [E], etype uint8 [E] or empty, totals int64 [2]).

@@ -65,6 +65,30 @@ template <> __device__ __forceinline__ void store_vec<float>(float* p, const flo
   *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
 }
 
+// One 16-byte slice of a row, kept packed until used.
+template <typename T> struct Raw;
+template <> struct Raw<__nv_bfloat16> {
+  uint4 u;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { u = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ float get(int i) const {
+    const uint32_t w = (i >> 1) == 0 ? u.x : (i >> 1) == 1 ? u.y : (i >> 1) == 2 ? u.z : u.w;
+    return (i & 1) ? __uint_as_float(w & 0xFFFF0000u) : __uint_as_float(w << 16);
+  }
+};
+template <> struct Raw<__half> {
+  uint4 u;
+  __device__ __forceinline__ void load(const __half* p) { u = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ float get(int i) const {
+    const uint32_t w = (i >> 1) == 0 ? u.x : (i >> 1) == 1 ? u.y : (i >> 1) == 2 ? u.z : u.w;
+    return __half2float(__ushort_as_half((unsigned short)((i & 1) ? (w >> 16) : (w & 0xFFFFu))));
+  }
+};
+template <> struct Raw<float> {
+  float4 f;
+  __device__ __forceinline__ void load(const float* p) { f = *reinterpret_cast<const float4*>(p); }
+  __device__ __forceinline__ float get(int i) const { return i == 0 ? f.x : i == 1 ? f.y : i == 2 ? f.z : f.w; }
+};
+
 // Pairs of fp32 values in one 64-bit register: sm_100a multiplies and adds them two at a time (fma.rn.f32x2), each half rounded
 // like a plain fp32 fma.
 typedef unsigned long long f2;
@@ -660,7 +684,7 @@ struct BwdArgs {
   void *dq, *dk, *dv;          // [n, Hl, HN], row stride ldg (elements)
   long long ldg;
   float2* zd;                  // [n, Hl]: (1/(Z+eps), D = <dout,out>)
-  float* ds;                   // [E, Hl]: score gradient / sqrt(hn), left by the dK/dV pass for the dQ pass
+  float* ds;                   // [E, Hl]: score gradient / sqrt(hn), left by the dK/dV pass for the dQ pass; null: computed twice
   const int *t_row, *t_eid;    // by key: query and position of every edge
   float* detab;                // [T, Hl, HN] fp32 or null
   // balanced dK/dV work list
@@ -1122,6 +1146,203 @@ __global__ void __launch_bounds__(256, EXPH ? 3 : 4) edge_attn_bwd_q_long_kernel
 }
 
 // ---------------------------------------------------------------------------------------------
+// The backward pass without streams (untyped edges; see recomputed_backward): dQ first, over the queries, which also leaves the row
+// terms and records, then dK/dV over the work list.  Both compute the score gradients, so none are kept: `ds` is not used.
+// ---------------------------------------------------------------------------------------------
+// what a query's gradient needs beside its edges
+template <typename T, int HN> struct QueryTerms {
+  float qs[Vec<T>::N], dof[Vec<T>::N], invz, dterm;
+  __device__ __forceinline__ void load(const BwdArgs& b, int row, int head, int off, unsigned hm) {
+    constexpr int VN = Vec<T>::N;
+    const AttnArgs& a = b.f;
+    const long long at = (long long)row * a.hl * HN + off;
+    float of[VN], unused[VN];
+    load_q_scaled<T, HN>(a, row, head, off, qs, unused);
+    load_vec<T>(static_cast<const T*>(b.dout) + at, dof);
+    load_vec<T>(static_cast<const T*>(a.out) + at, of);
+    dterm = 0.f;
+#pragma unroll
+    for (int i = 0; i < VN; ++i) dterm += dof[i] * of[i];
+    dterm = head_sum<HN / VN>(dterm, hm);
+    if (a.out_thresh) dterm *= a.out_keep;      // the stored output is the dropped one, rescaled by 1 / (1 - p)
+    invz = 1.f / (a.z[(long long)row * a.hl + head] + kEps);
+  }
+};
+
+// two edges of one query
+template <typename T, int HN>
+__device__ __forceinline__ void dq_pair(const BwdArgs& b, int e, int end, int head, int off, const QueryTerms<T, HN>& t, float* dq,
+                                        unsigned hm) {
+  constexpr int VN = Vec<T>::N, LPH = HN / VN;
+  const AttnArgs& a = b.f;
+  const int j0 = __ldg(a.col + e), j1 = e + 1 < end ? __ldg(a.col + e + 1) : j0;
+  Raw<T> kr[2], vr[2];
+  kr[0].load(static_cast<const T*>(a.k) + (long long)j0 * a.ldk + off);
+  vr[0].load(static_cast<const T*>(a.v) + (long long)j0 * a.ldv + off);
+  kr[1].load(static_cast<const T*>(a.k) + (long long)j1 * a.ldk + off);
+  vr[1].load(static_cast<const T*>(a.v) + (long long)j1 * a.ldv + off);
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    if (u == 1 && e + 1 >= end) break;
+    float d = 0.f, dv = 0.f;
+#pragma unroll
+    for (int i = 0; i < VN; ++i) { d += t.qs[i] * kr[u].get(i); dv += t.dof[i] * vr[u].get(i); }
+    d = head_sum<LPH>(d, hm);
+    dv = head_sum<LPH>(dv, hm);
+    const bool inr = (d > -kClamp) && (d < kClamp);
+    const float w = __expf(fminf(fmaxf(d, -kClamp), kClamp));
+    float mf = 1.f;
+    if (a.variant == 1) mf = (a.thresh && !keep_edge(a.seed, (uint32_t)(e + u), (uint32_t)head, a.thresh)) ? 0.f : a.inv_keep;
+    const float dss = inr ? (dv * mf - t.dterm) * t.invz * w * inv_sqrt_hn<HN>() : 0.f;
+#pragma unroll
+    for (int i = 0; i < VN; ++i) dq[i] += dss * kr[u].get(i);
+  }
+}
+
+template <typename T, int HN>
+__global__ void __launch_bounds__(256, 4) edge_attn_bwd_q_rows_kernel(BwdArgs b) {
+  constexpr int VN = Vec<T>::N, LPH = HN / VN;
+  const AttnArgs& a = b.f;
+  const Geo g = make_geo<T, HN>(a.hl);
+  const int lane = threadIdx.x & 31, lt = lane % g.tl;
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long task = warp * (32 / g.tl) + lane / g.tl;
+  const bool live = task < (long long)a.n * g.n_hc;
+  const int row = live ? (int)(task / g.n_hc) : 0, hc = live ? (int)(task % g.n_hc) : 0;
+  const int head = hc * g.hpt + lt / LPH;
+  if (!live || head >= a.hl) return;            // whole heads leave together; shuffles use head masks
+  const int off = head * HN + (lt % LPH) * VN;
+  const int beg = a.rowptr[row];
+  int end = a.rowptr[row + 1];
+  const bool cut = a.long_row > 0 && end - beg > a.long_row;
+  if (cut) end = beg;
+  const unsigned hm = head_mask<LPH>();
+  QueryTerms<T, HN> t;
+  t.load(b, row, head, off, hm);
+  if ((lt % LPH) == 0) b.zd[(long long)row * a.hl + head] = make_float2(t.invz, t.dterm);
+  if (b.qg != nullptr) {
+    T* rec = static_cast<T*>(b.qg) + ((long long)row * a.hl + head) * 2 * HN + (lt % LPH) * VN;
+    *reinterpret_cast<uint4*>(rec) = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(a.q) + (long long)row * a.ldq + off));
+    store_vec<T>(rec + HN, t.dof);
+  }
+  float dq[VN];
+#pragma unroll
+  for (int i = 0; i < VN; ++i) dq[i] = 0.f;
+  for (int e = beg; e < end; e += 2) dq_pair<T, HN>(b, e, end, head, off, t, dq, hm);
+  if (!cut) store_vec<T>(grad_row<T>(b, b.dq, b.cq, row) + off, dq);
+}
+
+// its long rows: work items as in edge_attn_fwd_long_kernel
+template <typename T, int HN>
+__global__ void __launch_bounds__(256, 3) edge_attn_bwd_q_items_kernel(BwdArgs b) {
+  constexpr int VN = Vec<T>::N, LPH = HN / VN;
+  const AttnArgs& a = b.f;
+  const Geo g = make_geo<T, HN>(a.hl);
+  const int lane = threadIdx.x & 31;
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (warp >= (long long)a.n_long_task * g.n_hc) return;
+  const int tpw = 32 / g.tl, sub = lane / g.tl, lt = lane % g.tl;
+  const int head = (int)(warp % g.n_hc) * g.hpt + lt / LPH;
+  const bool head_ok = head < a.hl;
+  const int hsafe = head_ok ? head : 0, off = hsafe * HN + (lt % LPH) * VN;
+  const int4 it = __ldg(a.long_task + warp / g.n_hc);
+  const int per = (it.z - it.y + tpw - 1) / tpw;
+  const int beg = it.y + sub * per, end = min(it.z, beg + per);
+  const unsigned hm = head_mask<LPH>();
+  QueryTerms<T, HN> t;
+  t.load(b, it.x, hsafe, off, hm);
+  float dq[VN];
+#pragma unroll
+  for (int i = 0; i < VN; ++i) dq[i] = 0.f;
+  for (int e = beg; e < end; e += 2) dq_pair<T, HN>(b, e, end, hsafe, off, t, dq, hm);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < VN; ++i) dq[i] = group_total(dq[i], g.tl);
+  if (sub == 0 && head_ok) {
+    float* pp = a.long_partial + (long long)it.w * a.hl * HN + off;
+#pragma unroll
+    for (int i = 0; i < VN; i += 4) *reinterpret_cast<float4*>(pp + i) = make_float4(dq[i], dq[i + 1], dq[i + 2], dq[i + 3]);
+  }
+}
+
+// one lane group per (work item, head chunk), two edges at a time: four 16-byte gathers in flight
+template <typename T, int HN>
+__global__ void __launch_bounds__(256, 4) edge_attn_bwd_kv_rows_kernel(BwdArgs b) {
+  constexpr int VN = Vec<T>::N, LPH = HN / VN;
+  const AttnArgs& a = b.f;
+  const Geo g = make_geo<T, HN>(a.hl);
+  const int w_row = a.hl * HN;
+  const int lane = threadIdx.x & 31, lt = lane % g.tl;
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long task = warp * (32 / g.tl) + lane / g.tl;
+  const bool live = task < (long long)b.n_kv_task * g.n_hc;
+  const int item = live ? (int)(task / g.n_hc) : 0, hc = live ? (int)(task % g.n_hc) : 0;
+  const int head = hc * g.hpt + lt / LPH;
+  if (!live || head >= a.hl) return;            // whole heads leave together; shuffles use head masks
+  const int off = head * HN + (lt % LPH) * VN;
+  const int4 it = __ldg(b.kv_task + item);
+  const T *qb = static_cast<const T*>(a.q) + off, *gb = static_cast<const T*>(b.dout) + off;
+  long long sq = a.ldq, sg = w_row;
+  if (b.qg != nullptr) {
+    qb = static_cast<const T*>(b.qg) + (long long)head * 2 * HN + (lt % LPH) * VN;
+    gb = qb + HN;
+    sq = sg = 2 * (long long)w_row;
+  }
+  Raw<T> kf, vf;                                // this key's k | v slice stays packed for the whole item
+  kf.load(static_cast<const T*>(a.k) + (long long)it.x * a.ldk + off);
+  vf.load(static_cast<const T*>(a.v) + (long long)it.x * a.ldv + off);
+  float dk[VN], dv[VN];
+#pragma unroll
+  for (int i = 0; i < VN; ++i) { dk[i] = 0.f; dv[i] = 0.f; }
+  const unsigned hm = head_mask<LPH>();
+  const float scale = inv_sqrt_hn<HN>();
+  for (int e = it.y; e < it.z; e += 2) {
+    int row[2], eid[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int at = min(e + u, it.z - 1);
+      row[u] = __ldg(b.t_row + at);
+      eid[u] = a.variant == 1 ? __ldg(b.t_eid + at) : 0;
+    }
+    Raw<T> qr[2], gr[2];
+    float2 zd[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      qr[u].load(qb + row[u] * sq);
+      gr[u].load(gb + row[u] * sg);
+      zd[u] = __ldg(b.zd + (long long)row[u] * a.hl + head);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (u == 1 && e + 1 >= it.z) break;
+      float d = 0.f, dotv = 0.f;
+#pragma unroll
+      for (int i = 0; i < VN; ++i) { d += qr[u].get(i) * kf.get(i); dotv += gr[u].get(i) * vf.get(i); }
+      d = head_sum<LPH>(d, hm) * scale;
+      dotv = head_sum<LPH>(dotv, hm);
+      const bool inr = (d > -kClamp) && (d < kClamp);
+      const float w = __expf(fminf(fmaxf(d, -kClamp), kClamp)) * zd[u].x;
+      float mf = 1.f;
+      if (a.variant == 1) mf = (a.thresh && !keep_edge(a.seed, (uint32_t)eid[u], (uint32_t)head, a.thresh)) ? 0.f : a.inv_keep;
+      const float dss = inr ? (dotv * mf - zd[u].y) * w * scale : 0.f, wn = w * mf;
+#pragma unroll
+      for (int i = 0; i < VN; ++i) { dk[i] += dss * qr[u].get(i); dv[i] += wn * gr[u].get(i); }
+    }
+  }
+  if (it.w < 0) {
+    store_vec<T>(grad_row<T>(b, b.dk, b.ck, it.x) + off, dk);
+    store_vec<T>(grad_row<T>(b, b.dv, b.cv, it.x) + off, dv);
+  } else {
+    float* pp = b.kv_partial + (long long)it.w * 2 * w_row + off;
+#pragma unroll
+    for (int i = 0; i < VN; i += 4) {
+      *reinterpret_cast<float4*>(pp + i) = make_float4(dk[i], dk[i + 1], dk[i + 2], dk[i + 3]);
+      *reinterpret_cast<float4*>(pp + w_row + i) = make_float4(dv[i], dv[i + 1], dv[i + 2], dv[i + 3]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 // Rows cut into work items: their partial sums lie side by side in slot order.  Pass 1 gives every window of SPLIT_WINDOW
 // slots to a block, which adds the slots of each row inside its window (threads run along the columns, so every slot is one
 // coalesced read) and finishes the rows that lie in the window whole; of a row that goes on, the window's sum replaces its
@@ -1322,11 +1543,45 @@ cudaError_t launch_fwd_t(const AttnArgs& a, bool rows, int chunks_per_hub, cudaS
 // shared memory for the gradient of the two rows of the type table
 inline size_t type_table_bytes(int w_row) { return sizeof(float) * 2 * (size_t)w_row; }
 
+// Whether the backward pass computes the score gradients twice instead of keeping them in `ds` (untyped edges).  `ds` holds 4 bytes
+// per edge and head, and the dK/dV pass writes them edge by edge in another order than they lie in: with one or two heads every
+// write is a sector of its own.  Measured, us, dQ and dK/dV of this form against row terms, dK/dV and dQ of the streams:
+// - rows of 32 bytes: 1 x 16 bf16, 50 k 44 / 47, 170 k 78 / 84, 600 k 217 / 274, 2.9 M 963 / 1233
+// - rows of 64 bytes: 2 x 16 bf16, 170 k (22 MB of k and v) 104 / 98, 300 k (38 MB) 205 / 188, 600 k (77 MB) 375 / 400, 2.9 M 1557 / 1654
+// - fp32, rows of 512 bytes and more that stay in L2 (the dK/dV stream holds 12 warps an SM, this form 32): 8 x 16, 2 k 26 / 32, 10 k
+//   41 / 43, 50 k (51 MB) with 16 edges a row 219 / 253 and with five 121 / 111, 110 k (113 MB) 356 / 311; 4 x 64, 10 k (20 MB) 61 / 66,
+//   50 k (102 MB) 248 / 190; 8 x 8, 10 k 37 / 32, 50 k 136 / 117
+inline bool recomputed_backward(int dtype, long long n, int hl, int hn, int variant) {
+  const long long row = (long long)hl * hn * (dtype == BF_FP32 ? 4 : 2), gathered = 2 * n * row;
+  if (variant == 2) return false;
+  if (row <= 32) return true;
+  if (row <= 64) return gathered > 64'000'000;
+  return dtype == BF_FP32 && row >= 512 && gathered <= 64'000'000;
+}
+
+template <typename T, int HN>
+cudaError_t launch_recomputed_bwd_t(const BwdArgs& b, cudaStream_t st) {
+  const AttnArgs& a = b.f;
+  const Geo g = make_geo<T, HN>(a.hl);
+  const int w_row = a.hl * HN, tpw = 32 / g.tl;
+  auto blocks = [&](long long rows) { return (unsigned)(((rows * g.n_hc + tpw - 1) / tpw + 7) / 8); };
+  if (a.n > 0) edge_attn_bwd_q_rows_kernel<T, HN><<<blocks(a.n), 256, 0, st>>>(b);
+  if (a.n_long_task > 0) {
+    edge_attn_bwd_q_items_kernel<T, HN><<<(unsigned)(((long long)a.n_long_task * g.n_hc + 7) / 8), 256, 0, st>>>(b);
+    launch_split<T, SPLIT_DQ>(b, a.long_task, a.n_long_task, a.long_split, a.n_long_split, a.long_partial, w_row, w_row, w_row, HN, st);
+  }
+  if (b.n_kv_task > 0) edge_attn_bwd_kv_rows_kernel<T, HN><<<blocks(b.n_kv_task), 256, 0, st>>>(b);
+  if (b.n_kv_split > 0)
+    launch_split<T, SPLIT_KV>(b, b.kv_task, b.n_kv_slots, b.kv_split, b.n_kv_split, b.kv_partial, 2 * w_row, 2 * w_row, w_row, HN, st);
+  return cudaGetLastError();
+}
+
 template <typename T, int HN>
 cudaError_t launch_bwd_t(const BwdArgs& b, cudaStream_t st) {
   const AttnArgs& a = b.f;
   const Geo g = make_geo<T, HN>(a.hl);
   const int w_row = a.hl * HN;
+  if (b.ds == nullptr) return launch_recomputed_bwd_t<T, HN>(b, st);
   if (a.n > 0) {
     constexpr int VN = wide_elems<T, HN>();
     const StreamGeo s = stream_geo<HN, VN>(a.hl, 0, 1, 1);
@@ -1457,14 +1712,20 @@ extern "C" int bf_edge_attn_fwd(const bf_attn_params* p, cudaStream_t st) {
   return (int)cudaErrorInvalidValue;
 }
 
+extern "C" int bf_attn_bwd_keeps_scores(int dtype, long long n, int hl, int hn, int variant) {
+  return recomputed_backward(dtype, n, hl, hn, variant) ? 0 : 1;
+}
+
 extern "C" int bf_edge_attn_bwd(const bf_attn_params* p, const bf_attn_bwd_params* q, cudaStream_t st) {
   BwdArgs b;
   b.f = to_args(*p);
-  if (b.f.n_hub > 0 || !take_long_rows(&q->long_rows, &b.f) || q->kv_task == nullptr || q->ds == nullptr) return (int)cudaErrorInvalidValue;
+  if (b.f.n_hub > 0 || !take_long_rows(&q->long_rows, &b.f) || q->kv_task == nullptr) return (int)cudaErrorInvalidValue;
+  const bool keeps = bf_attn_bwd_keeps_scores(p->dtype, p->n, p->hl, p->hn, p->variant) != 0;
+  if (keeps && q->ds == nullptr) return (int)cudaErrorInvalidValue;
   b.dout = q->dout; b.dq = q->dq; b.dk = q->dk; b.dv = q->dv;
   b.ldg = q->ldg > 0 ? q->ldg : (long long)p->hl * p->hn;
   b.zd = reinterpret_cast<float2*>(q->zd);
-  b.ds = q->ds;
+  b.ds = keeps ? q->ds : nullptr;
   b.t_row = q->t_row; b.t_eid = q->t_eid; b.detab = q->detab;
   b.kv_task = reinterpret_cast<const int4*>(q->kv_task); b.n_kv_task = q->n_kv_task;
   b.kv_split = q->kv_split; b.n_kv_split = q->n_kv_split; b.n_kv_slots = q->n_kv_split > 0 ? q->n_kv_slots : 0; b.kv_partial = q->kv_partial;

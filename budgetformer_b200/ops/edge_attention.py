@@ -87,12 +87,6 @@ def edge_attention_reference(
     return (out, z) if return_z else out
 
 
-def launches(graph: AttnGraph, backward: bool) -> int:
-    """Kernels of one pass: the rows (and, backward, row terms and keys), then items and two reductions where rows are cut."""
-    cut = 3 if graph.q_task is not None and graph.q_task.size(0) > 0 else 0
-    return cut + (3 + (2 if graph.kv_slots > 0 else 0) if backward else 1)
-
-
 class _EdgeAttentionCUDA(torch.autograd.Function):
     """sm_100a kernels; see csrc/edge_attn.cu."""
 
@@ -104,9 +98,9 @@ class _EdgeAttentionCUDA(torch.autograd.Function):
         out = torch.empty((n, hl, hn), dtype=q.dtype, device=q.device)
         z = torch.empty((n, hl), dtype=torch.float32, device=q.device)
         kmax = -1 if graph.max_degree is None else int(graph.max_degree)
-        ext.edge_attn_fwd(q, k, v, out, z, graph.rowptr, graph.col, graph.etype,
-                          etable, int(variant_id), float(dropout_p), int(dropout_seed), kmax, [], [], *graph.long_rows())
-        _ext.count_launches(launches(graph, False))
+        made = ext.edge_attn_fwd(q, k, v, out, z, graph.rowptr, graph.col, graph.etype,
+                                 etable, int(variant_id), float(dropout_p), int(dropout_seed), kmax, [], [], *graph.long_rows())
+        _ext.count_launches(made)
         ctx.save_for_backward(q, k, v, out, z, etable if etable is not None else q.new_empty(0))
         ctx.graph = graph
         ctx.cfg = (int(variant_id), float(dropout_p), int(dropout_seed), etable is not None)
@@ -126,13 +120,13 @@ class _EdgeAttentionCUDA(torch.autograd.Function):
         zd = torch.empty(z.shape + (2,), dtype=torch.float32, device=q.device)
         detab = torch.zeros(etable.shape, dtype=torch.float32, device=q.device) if has_tab else None
         kmax = -1 if graph.max_degree is None else int(graph.max_degree)
-        ext.edge_attn_bwd(q, k, v, out, z, dout, dq, dk, dv, zd,
-                          graph.rowptr, graph.col, graph.etype,
-                          graph.t_rowptr, graph.t_row, graph.t_eid,
-                          etable if has_tab else None, detab,
-                          variant_id, dropout_p, dropout_seed, kmax, graph.t_task, graph.t_split, int(graph.kv_slots), [], [],
-                          *graph.long_rows())
-        _ext.count_launches(launches(graph, True))
+        made = ext.edge_attn_bwd(q, k, v, out, z, dout, dq, dk, dv, zd,
+                                 graph.rowptr, graph.col, graph.etype,
+                                 graph.t_rowptr, graph.t_row, graph.t_eid,
+                                 etable if has_tab else None, detab,
+                                 variant_id, dropout_p, dropout_seed, kmax, graph.t_task, graph.t_split, int(graph.kv_slots), [], [],
+                                 *graph.long_rows())
+        _ext.count_launches(made)
         return dq, dk, dv, (detab.to(etable.dtype) if has_tab else None), None, None, None, None
 
 

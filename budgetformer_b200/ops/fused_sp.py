@@ -39,7 +39,7 @@ from ..graph.attn_graph import AttnGraph, as_attn_graph
 from ..parallel import symm
 from . import _ext, gemm
 from ..utils import debug
-from .edge_attention import _VARIANTS, launches
+from .edge_attention import _VARIANTS
 from .ffn import fused_ffn
 from .norm import ColsumSlot, batch_norm, hash_dropout, layer_norm, new_seed
 
@@ -268,9 +268,9 @@ class _PackedEdgeAttention(torch.autograd.Function):
         # dropout on the context (GT applies it before the output projection) is fused into the store: the mask of
         # element (row, c) is the one the owner of that row regenerates for (row - its first row, this rank's column)
         out_drop = [float(out_p), int(out_seed), int(sp.rows_local), int(sp.rank * hl)] if out_p > 0 else []
-        ext.edge_attn_fwd(q, k, v, out.view(r, hlh, hn), z, graph.rowptr, graph.col, graph.etype, etable,
-                          int(variant_id), float(dropout_p), int(seed), kmax, out_drop, route, *graph.long_rows())
-        _ext.count_launches(launches(graph, False))
+        made = ext.edge_attn_fwd(q, k, v, out.view(r, hlh, hn), z, graph.rowptr, graph.col, graph.etype, etable,
+                                 int(variant_id), float(dropout_p), int(seed), kmax, out_drop, route, *graph.long_rows())
+        _ext.count_launches(made)
         if sp.token_rows is not None and len(sp.token_rows) > 1:
             out[sp.token_rows[1:]] = out[sp.token_rows[0]].clone()  # copy_global_token0 (gt_sp/utils.py:2365-2386)
         ctx.sp, ctx.graph, ctx.layer = sp, graph, layer
@@ -301,11 +301,11 @@ class _PackedEdgeAttention(torch.autograd.Function):
         route = sp.route(sp.dqkv, sp.qkv_ld, extra=(2 * hl, 0, hl)) if sp.routed else []
         zd = torch.empty((r, hlh, 2), dtype=torch.float32, device=qkv.device)
         detab = torch.zeros(etable.shape, dtype=torch.float32, device=qkv.device) if has_tab else None
-        ext.edge_attn_bwd(q, k, v, out.view(r, hlh, hn), z, dout.view(r, hlh, hn), dq, dk, dv, zd, graph.rowptr, graph.col,
-                          graph.etype, graph.t_rowptr, graph.t_row, graph.t_eid, etable if has_tab else None, detab,
-                          variant_id, dropout_p, seed, kmax, graph.t_task, graph.t_split, int(graph.kv_slots), ctx.out_drop,
-                          route, *graph.long_rows())
-        _ext.count_launches(launches(graph, True))
+        made = ext.edge_attn_bwd(q, k, v, out.view(r, hlh, hn), z, dout.view(r, hlh, hn), dq, dk, dv, zd, graph.rowptr,
+                                 graph.col, graph.etype, graph.t_rowptr, graph.t_row, graph.t_eid, etable if has_tab else None, detab,
+                                 variant_id, dropout_p, seed, kmax, graph.t_task, graph.t_split, int(graph.kv_slots), ctx.out_drop,
+                                 route, *graph.long_rows())
+        _ext.count_launches(made)
         if debug.enabled() and dout.data_ptr() == sp.dctx.tensor.data_ptr():
             debug.poison(sp.dctx.tensor)              # d(context) consumed; the next push must overwrite all of it
         return dbuf, (detab.to(etable.dtype) if has_tab else None), None, None, None, None, None, None, None, None

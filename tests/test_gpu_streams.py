@@ -35,7 +35,8 @@ def _reference(q, k, v, dout, graph, tab, variant, p, seed):
     (35003, 8, 32, 5, torch.bfloat16), (25013, 4, 64, 5, torch.float32), (134999, 8, 32, 4, torch.bfloat16),
     (310007, 4, 64, 3, torch.float16),
     # behind the lines up to which the forward pass walks rows without a stream (k and v of 200 MB; 100 MB with heads of 8)
-    (101021, 4, 64, 3, torch.float32), (1600007, 2, 16, 3, torch.bfloat16), (410003, 8, 8, 3, torch.float16)])
+    (101021, 4, 64, 3, torch.float32), (1600007, 2, 16, 3, torch.bfloat16), (410003, 8, 8, 3, torch.float16),
+    (5003, 8, 8, 9, torch.float32)])
 def test_attention_streams(n, heads, hn, max_deg, dtype, variant):
     from budgetformer_b200.ops.edge_attention import edge_attention
     if variant == "exphormer" and max_deg == 0:
