@@ -1,12 +1,13 @@
 // Weight and bias gradient of a linear layer in fp32: dW[N, K] = dY[M, N]^T X[M, K], db[N] = column sums of dY.
 //
-// M (rows of the activation) is 10^4 to 10^6, N and K are layer widths (64 .. 512): the output is a few 64 x 64 tiles, so one
-// tile per block leaves the chip empty, and a library GEMM that splits no further takes one block's walk over all rows.  Here
-// the rows are cut into slices until every SM has two blocks; each block leaves its 64 x 64 partial sum, and a second kernel
+// M (rows of the activation) is 10^2 to 10^6, N and K are layer widths: the output is a few 64 x 64 tiles (for many, the library's
+// GEMM is faster: ops/gemm.py::f32_gradient_pays), so one tile per block leaves the chip empty, and a library GEMM that splits no
+// further takes one block's walk over all rows.  Here the rows are cut into slices until every SM has two blocks; each block
+// leaves its 64 x 64 partial sum, and a second kernel
 // adds the slices in a fixed order (no atomics: the gradients are bit-reproducible).  The bias gradient rides on the blocks of
 // the first column of tiles, which hold dY in shared memory anyway.  All sums are plain fp32 multiply-adds, two per instruction;
 // cutting the rows shortens the chains: against 64 bits dW is 1.7e-7 off at 40 k rows of 64 x 64 (one long sum: 8.3e-7).
-// 40,009 rows, dW and db, us: 64 x 64 19.5 (library GEMM and column sum 135), 256 x 64 45 (168).  Bound by the shared-memory reads
+// 40,009 rows, dW and db, us: 64 x 64 23 (library GEMM and column sum 137), 128 x 128 50 (172).  Bound by the shared-memory reads
 // and issue of the 64 multiply-adds per thread and row.
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -245,18 +245,40 @@ class _LinearF32(torch.autograd.Function):
         return dx, dw, db
 
 
-# Rows from which the gradient kernel is used.  Weight and bias gradient together, us, this kernel against the library's GEMM
-# and column sum, 64 x 64: 6.5 / 7.7 at 128 rows, 7.2 / 19.7 at 1,024, 19.5 / 135 at 40 k.  Below, launches are all there is and
-# both take two.
+# Rows from which the gradient kernel is used; below, launches are all there is and both sides take two.
 LINEAR_F32_MIN_ROWS = 128
 
 
+def f32_gradient_pays(rows: int, n: int, k: int) -> bool:
+    """Whether ``csrc/linear_f32.cu`` is the faster way to weight and bias gradient.  It adds 64 x 64 tiles with plain multiply-adds and
+    splits the rows; the library splits its rows too little for few tiles, and has the better tile for many.  us, this kernel
+    against the library's GEMM and column sum (outputs x features, rows):
+
+    * up to 8 tiles: 64 x 64 13 / 28 at 128, 23 / 137 at 40 k, 63 / 307 at 200 k; 128 x 256 43 / 111 at 16 k, 525 / 677 at 262 k; 64 x 500
+      394 / 503 at 200 k.  Widths that are no multiple of 4 take 4-byte copies: 64 x 269 647 / 710 at 262 k, 128 x 269 (10 tiles) 330 / 357
+      at 66 k, 1279 / 828 at 262 k
+    * 9 to 16 tiles: 192 x 192 839 / 1079 at 262 k; 256 x 256 17 / 32 at 1 k, 103 / 129 at 16 k, 372 / 376 at 66 k, 1448 / 926 at 262 k; 64 x 1000
+      36 / 56 at 4 k, 103 / 100 at 16 k
+    * up to 32 tiles: 64 x 1433 25 / 32 at 1 k, 58 / 58 at 4 k, 198 / 151 at 16 k; 320 x 320 157 / 189 at 16 k, 582 / 492 at 66 k; 512 x 256 56 / 68
+      at 4 k, 188 / 159 at 16 k
+    * more: 512 x 512 38 / 33 at 1 k, 864 / 510 at 40 k; 1024 x 1024 100 / 57 at 1 k
+    * one output or feature (the library has a matrix-vector product): 1 x 64 13 / 19 at 4 k, 34 / 26 at 66 k; 1 x 256 21 / 18 at 8 k
+    """
+    if min(n, k) < 2:
+        return rows <= 4096
+    tiles = -(-n // 64) * -(-k // 64)
+    return rows <= (1 << 40 if tiles <= 8 else 65536 if tiles <= 12 else 12288 if tiles <= 16 else 4096 if tiles <= 32 else 0)
+
+
 def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``torch.nn.functional.linear``; on fp32 CUDA tensors outside autocast with ``LINEAR_F32_MIN_ROWS`` rows or more the
-    weight and bias gradients come from this package's kernel."""
+    """``torch.nn.functional.linear``; on fp32 CUDA tensors outside autocast, where the kernel is the faster way
+    (``f32_gradient_pays``), the weight and bias gradients come from this package's kernel.  Whoever lets fp32 products run in TF32
+    gets the library's."""
     if (x.is_cuda and x.dtype == weight.dtype == torch.float32 and (bias is None or bias.dtype == torch.float32)
             and type(x) is torch.Tensor and x.dim() >= 2 and weight.device == x.device
-            and weight.numel() > 0 and x.numel() >= LINEAR_F32_MIN_ROWS * weight.size(1) and torch.is_grad_enabled() and weight.requires_grad
+            and weight.numel() > 0 and x.numel() >= LINEAR_F32_MIN_ROWS * weight.size(1)
+            and f32_gradient_pays(x.numel() // weight.size(1), weight.size(0), weight.size(1))
+            and torch.backends.cuda.matmul.fp32_precision != "tf32" and torch.is_grad_enabled() and weight.requires_grad
             and not torch.is_autocast_enabled("cuda") and plain_eager()):
         return _LinearF32.apply(x, weight, bias)
     return torch.nn.functional.linear(x, weight, bias)

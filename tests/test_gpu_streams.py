@@ -315,6 +315,21 @@ def test_fp32_linear_of_no_width(out_features, in_features):
         assert u.shape == v.shape and torch.equal(u, v)
 
 
+def test_fp32_linear_leaves_wide_layers_and_tf32_to_the_library(monkeypatch):
+    from budgetformer_b200.ops import gemm
+    calls = []
+    monkeypatch.setattr(gemm._LinearF32, "apply", lambda *a: calls.append(1) or torch.nn.functional.linear(*a))
+    for rows, n, k, kernel in ((4096, 64, 64, True), (4096, 512, 512, False), (9000, 64, 1433, False), (9000, 1, 256, False), (300, 1, 256, True)):
+        x, w = torch.randn(rows, k, device="cuda"), torch.randn(n, k, device="cuda", requires_grad=True)
+        calls.clear()
+        gemm.linear_f32(x, w)
+        assert bool(calls) == kernel, (rows, n, k)
+    monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", True)
+    calls.clear()
+    gemm.linear_f32(torch.randn(4096, 64, device="cuda"), torch.randn(64, 64, device="cuda", requires_grad=True))
+    assert not calls
+
+
 def test_fp32_modules_match_torch():
     """The models' call of a linear layer and the row-kernel LayerNorm against torch's, first and second derivative, few and many
     rows."""

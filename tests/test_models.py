@@ -246,3 +246,13 @@ def test_model_parts_stay_torch_linear_modules():
     ffn.layer1.register_forward_hook(lambda m, i, o: seen.append(tuple(o.shape)))
     ffn(x)
     assert seen == [(2, 5, 32)]
+
+
+def test_widths_of_the_fp32_gradient_kernel():
+    """The layer widths that the kernel was made for stay with it; wide layers and long thin ones go to the library."""
+    from budgetformer_b200.ops.gemm import f32_gradient_pays
+    assert all(f32_gradient_pays(m, n, k) for m in (128, 40009, 1 << 20) for n, k in ((64, 64), (256, 64), (64, 256), (128, 128), (47, 101)))
+    assert f32_gradient_pays(8192, 256, 256) and not f32_gradient_pays(65536, 256, 256)
+    assert f32_gradient_pays(1024, 64, 1433) and not f32_gradient_pays(8192, 64, 1433)
+    assert not any(f32_gradient_pays(m, n, k) for m in (1024, 40009) for n, k in ((512, 512), (1024, 1024), (2048, 2048), (16384, 16384)))
+    assert f32_gradient_pays(1024, 1, 64) and not f32_gradient_pays(65536, 1, 64) and not f32_gradient_pays(65536, 64, 1)
