@@ -267,14 +267,14 @@ int bf_khop_fill_cpu(const int* out_rowptr, const int* out_col, int n, const int
 size_t bf_graph_transpose_scratch(int n, long long n_edges);
 int bf_graph_transpose(const int* rowptr, const int* col, int n, long long n_edges, int* t_rowptr /* [n+1] */,
                        int* t_row /* [E] */, int* t_eid /* [E] */, void* scratch, size_t scratch_bytes, cudaStream_t st);
-size_t bf_kv_task_scratch(int n);
-// by_length (optional, [n]): the keys by length of their row, longest first, split keys last
-int bf_kv_task_counts(const int* t_rowptr, int n, int chunk, int min_split, int* item_first /* [n+1] */,
-                      int* slot_first /* [n+1] */, int* split_first /* [n+1] */, int* by_length, void* scratch,
-                      size_t scratch_bytes, cudaStream_t st);
-// max_tasks / max_splits: rows of `tasks` and `splits`, which may be upper bounds of the totals; nothing is written behind them
-int bf_kv_task_fill(const int* t_rowptr, const int* slot_first, const int* split_first, const int* by_length, int n, int chunk,
-                    int max_tasks, int max_splits, int* tasks /* [T, 4] */, int* splits /* [S, 3] */, cudaStream_t st);
+// Work items of the CSR rows with more than min_split edges (chunk edges each) and the list of those rows.  singles: one item for
+// every other row behind them: 0 none, 1 in row order, 2 longest first.  max_tasks / max_splits: rows of `tasks` and `splits`, which
+// may be upper bounds; nothing is written behind them.  first[n] holds the totals (low half: items of cut rows, high half: cut
+// rows); a caller that reads them back last finds the list complete, whatever stream uses it next.
+size_t bf_row_tasks_scratch(int n, int singles);
+int bf_row_tasks(const int* rowptr, int n, int chunk, int min_split, int singles, int max_tasks, int max_splits,
+                 unsigned long long* first /* [n+1] */, int* tasks /* [T, 4] */, int* splits /* [S, 3] */, void* scratch,
+                 size_t scratch_bytes, cudaStream_t st);
 
 // ---- weight and bias gradient of an fp32 linear layer (linear_f32.cu) -------------------------------------
 // out = [dW (N*K) | db (N, with want_bias)]; partial: bf_f32_dw_slices(M, N, K) times as many floats as out

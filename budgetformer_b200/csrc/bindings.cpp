@@ -39,34 +39,36 @@ void check_qkv(const Tensor& t, const char* name) {
 const int* iptr(const Tensor& t) { return t.data_ptr<int>(); }
 
 // Work items of the CSR rows with more than min_split edges: items of `chunk` edges, split rows, and with `singles` one item
-// for every other row behind them, longest first.  The outputs are cut from buffers of the most items that n_edges edges can
-// make, so that the one host read (of the totals) comes last: what is returned is complete, whatever stream uses it next.
+// for every other row behind them.  The outputs are cut from buffers of the most items that n_edges edges can make, so that the one
+// host read (of the totals) comes last: what is returned is complete, whatever stream uses it next.
+// The singles are sorted by length from kSortedRows rows on: below, all lane groups of the dK/dV pass run side by side and the order
+// buys nothing (8 x 16, us in key order / by length: 5 k 23.7 / 23.3, 10 k 24.7 / 24.1, 20 k 28.4 / 26.7; 8 x 32: 30.3 / 29.6, 32.9 /
+// 31.9, 50.0 / 40.1), and the sort is six launches.
+constexpr int64_t kSortedRows = 8192;
 struct RowTasks {
-  Tensor tasks, splits, sizes;       // [T, 4], [S, 3], int64 [3] on the host = items, slots, split rows
+  Tensor tasks, splits;              // [T, 4], [S, 3]
+  int64_t n_slots = 0;               // items of split rows
 };
 RowTasks row_tasks(const Tensor& rowptr, int64_t n, int64_t n_edges, int64_t chunk, int64_t min_split, bool singles,
                    cudaStream_t st) {
   auto iopt = rowptr.options();
-  Tensor firsts = torch::empty({3, n + 1}, iopt);
-  Tensor by_length = singles ? torch::empty({n}, iopt) : Tensor();
-  int* by = singles ? by_length.data_ptr<int>() : nullptr;
-  {
-    const size_t bytes = bf_kv_task_scratch((int)n);
-    Tensor scratch = torch::empty({(int64_t)bytes}, iopt.dtype(torch::kUInt8));
-    check_cuda(bf_kv_task_counts(rowptr.data_ptr<int>(), (int)n, (int)chunk, (int)min_split, firsts[0].data_ptr<int>(),
-                                 firsts[1].data_ptr<int>(), firsts[2].data_ptr<int>(), by, scratch.data_ptr(), bytes, st),
-               "kv_task_counts");
-  }
   const int64_t max_splits = std::min(n, n_edges / (min_split + 1)), max_slots = max_splits > 0 ? n_edges / chunk + max_splits : 0;
   const int64_t max_items = singles ? n + max_slots : max_slots;
   TORCH_CHECK(max_items < (int64_t)INT32_MAX, "too many work items: ", max_items);
   RowTasks r;
   r.tasks = torch::empty({max_items, 4}, iopt);
   r.splits = torch::empty({max_splits, 3}, iopt);
-  check_cuda(bf_kv_task_fill(rowptr.data_ptr<int>(), firsts[1].data_ptr<int>(), firsts[2].data_ptr<int>(), by, (int)n, (int)chunk,
-                             (int)max_items, (int)max_splits, r.tasks.data_ptr<int>(), r.splits.data_ptr<int>(), st), "kv_task_fill");
-  r.sizes = firsts.select(1, n).to(torch::kCPU).to(torch::kLong);
-  const int64_t n_items = r.sizes[singles ? 0 : 1].item<int64_t>(), n_splits = r.sizes[2].item<int64_t>();
+  if (n == 0) return r;
+  Tensor first = torch::empty({n + 1}, iopt.dtype(torch::kLong));
+  const int order = singles ? (n > kSortedRows ? 2 : 1) : 0;
+  const size_t bytes = bf_row_tasks_scratch((int)n, order);
+  Tensor scratch = torch::empty({(int64_t)bytes}, iopt.dtype(torch::kUInt8));
+  check_cuda(bf_row_tasks(rowptr.data_ptr<int>(), (int)n, (int)chunk, (int)min_split, order, (int)max_items, (int)max_splits,
+                          reinterpret_cast<unsigned long long*>(first.data_ptr<int64_t>()), r.tasks.data_ptr<int>(),
+                          r.splits.data_ptr<int>(), scratch.data_ptr(), bytes, st), "row_tasks");
+  const int64_t total = first[n].item<int64_t>(), n_splits = total >> 32;
+  r.n_slots = total & 0xFFFFFFFF;
+  const int64_t n_items = r.n_slots + (singles ? n - n_splits : 0);
   TORCH_CHECK(n_items <= max_items && n_splits <= max_splits, "the row pointer names more than the ", n_edges, " edges of the list");
   r.tasks = r.tasks.narrow(0, 0, n_items);
   r.splits = r.splits.narrow(0, 0, n_splits);
@@ -202,7 +204,7 @@ int64_t edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor
     // a by-key view without its work list
     RowTasks r = row_tasks(t_rowptr, p.n, t_row.numel(), BF_LONG_CHUNK, BF_LONG_CHUNK, true, at::cuda::getCurrentCUDAStream());
     kv_task = r.tasks; kv_split = r.splits;
-    kv_slots = r.sizes[1].item<int64_t>();
+    kv_slots = r.n_slots;
   }
   TORCH_CHECK(kv_task.has_value() && kv_task->scalar_type() == torch::kInt && kv_task->is_contiguous() && kv_task->size(1) == 4 &&
               ((uintptr_t)kv_task->data_ptr()) % 16 == 0, "kv_task must be contiguous int32 [T, 4]");
@@ -435,7 +437,8 @@ std::vector<Tensor> graph_transpose(Tensor rowptr, Tensor col, int64_t n, int64_
                "graph_transpose");
   }
   RowTasks r = row_tasks(t_rowptr, n, n_edges, chunk, chunk, true, st);
-  return {t_rowptr, t_row, t_eid, r.tasks, r.splits, r.sizes};
+  const int64_t sizes[3] = {r.tasks.size(0), r.n_slots, r.splits.size(0)};
+  return {t_rowptr, t_row, t_eid, r.tasks, r.splits, torch::tensor(c10::ArrayRef<int64_t>(sizes, 3), torch::kLong)};
 }
 
 // C = A * W^T with fused epilogue.  `dst_ptrs` holds one device pointer per destination (1 = plain output).
@@ -836,6 +839,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("long_row_tasks", &long_row_tasks, unlocked());
   m.attr("LONG_ROW") = (int64_t)BF_LONG_ROW;
   m.attr("LONG_CHUNK") = (int64_t)BF_LONG_CHUNK;
+  m.attr("SORTED_ROWS") = kSortedRows;
   m.attr("BUILD_HUB_DEGREE") = (int64_t)BF_BUILD_HUB_DEGREE;
   m.def("build_attn_graph", &build_attn_graph, unlocked());
   m.def("budget_select_rows", &budget_select_rows);

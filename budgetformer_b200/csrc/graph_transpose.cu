@@ -58,59 +58,65 @@ __global__ void gather_rows_kernel(const int* __restrict__ erow, const int* __re
   if (i < n_edges) t_row[i] = erow[t_eid[i]];
 }
 
-// items per key (at least one, so that keys without edges still get their zero gradient written) and partial slots; only
-// rows with more than `min_split` edges are cut
-__global__ void task_counts_kernel(const int* __restrict__ t_rowptr, int n, int chunk, int min_split, int* __restrict__ n_items,
-                                   int* __restrict__ n_slots, int* __restrict__ is_split, int* __restrict__ length_key,
-                                   int* __restrict__ ids) {
+// Partial slots of every key's items (0: not cut, one item) in the low half and 1 per cut key in the high half, so that one prefix
+// sum serves both; rows with more than `min_split` edges are cut.  first[0] = 0 is the start of that sum.
+__global__ void task_counts_kernel(const int* __restrict__ t_rowptr, int n, int chunk, int min_split,
+                                   unsigned long long* __restrict__ counts, unsigned long long* __restrict__ first,
+                                   int* __restrict__ length_key, int* __restrict__ ids) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k == 0) first[0] = 0;
   if (k >= n) return;
   const int deg = t_rowptr[k + 1] - t_rowptr[k];
-  const int c = deg <= min_split ? 1 : (deg + chunk - 1) / chunk;
-  n_items[k] = c;
-  n_slots[k] = c > 1 ? c : 0;
-  is_split[k] = c > 1 ? 1 : 0;
+  const bool cut = deg > min_split;
+  counts[k] = cut ? (1ull << 32) | (unsigned)((deg + chunk - 1) / chunk) : 0ull;
   if (length_key != nullptr) {
-    length_key[k] = c > 1 ? min_split + 1 : min_split - deg;
+    length_key[k] = cut ? min_split + 1 : min_split - deg;
     ids[k] = k;
   }
 }
 
 // The list starts with the items of all split keys in key order (full-length items: the long work is scheduled first and runs
 // side by side in a warp); an item of a split key sits at its partial-slot index.  A lane looks at one key, and the warp writes the
-// items of those that are split one key after the other, 32 items at a time (hub keys own thousands).
-__global__ void task_fill_kernel(const int* __restrict__ t_rowptr, const int* __restrict__ slot_first,
-                                 const int* __restrict__ split_first, int n, int chunk, int max_tasks, int max_splits,
-                                 int4* __restrict__ tasks, int* __restrict__ splits) {
+// items of those that are split one key after the other, 32 items at a time (hub keys own thousands).  With `singles` the one item
+// of every other key (an empty one too: its zero gradient has to be written) follows behind them in key order.
+__global__ void task_fill_kernel(const int* __restrict__ t_rowptr, const unsigned long long* __restrict__ first, int n, int chunk,
+                                 int max_tasks, int max_splits, bool singles, int4* __restrict__ tasks, int* __restrict__ splits) {
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
-  int s0 = 0, cnt = 0;
-  if (gt < n) { s0 = slot_first[gt]; cnt = slot_first[gt + 1] - s0; }
+  int s0 = 0, cnt = 0, split = 0;
+  if (gt < n) {
+    const unsigned long long f = first[gt];
+    s0 = (int)(unsigned)f;
+    split = (int)(f >> 32);
+    cnt = (int)(unsigned)first[gt + 1] - s0;
+    if (singles && cnt == 0) {
+      const int at = (int)(unsigned)first[n] + (int)gt - split;
+      if (at < max_tasks) tasks[at] = make_int4((int)gt, t_rowptr[gt], t_rowptr[gt + 1], -1);
+    }
+  }
   unsigned left = __ballot_sync(0xffffffffu, cnt > 0);
   while (left != 0) {
     const int src = __ffs(left) - 1;
     left &= left - 1;
-    const int first = __shfl_sync(0xffffffffu, s0, src), m = __shfl_sync(0xffffffffu, cnt, src);
+    const int at = __shfl_sync(0xffffffffu, s0, src), m = __shfl_sync(0xffffffffu, cnt, src), s = __shfl_sync(0xffffffffu, split, src);
     const int k = (int)(gt - lane) + src;
     const int beg = t_rowptr[k], end = t_rowptr[k + 1];
-    for (int c = lane; c < m && first + c < max_tasks; c += 32) {
+    for (int c = lane; c < m && at + c < max_tasks; c += 32) {
       const int b = beg + c * chunk;
-      tasks[first + c] = make_int4(k, b, min(b + chunk, end), first + c);
+      tasks[at + c] = make_int4(k, b, min(b + chunk, end), at + c);
     }
-    const int s = split_first[k];
-    if (lane == 0 && s < max_splits) { splits[3 * s] = k; splits[3 * s + 1] = first; splits[3 * s + 2] = m; }
+    if (lane == 0 && s < max_splits) { splits[3 * s] = k; splits[3 * s + 1] = at; splits[3 * s + 2] = m; }
   }
 }
 
-// Behind them the single item of every other key, longest first (key order among equals): the lane groups of a warp that work
-// on neighbouring items finish together.  Sorting 2.9 M keys by their 7-bit length is one radix pass; a thread per key instead
-// of a warp writes the list in a tenth of the time.
-__global__ void task_singles_kernel(const int* __restrict__ t_rowptr, const int* __restrict__ slot_first,
-                                    const int* __restrict__ split_first, const int* __restrict__ keys, int n, int max_tasks,
-                                    int4* __restrict__ tasks) {
+// The single items, longest first instead (key order among equals): the lane groups of a warp that work on neighbouring items finish
+// together.  Sorting 2.9 M keys by their 7-bit length is one radix pass.
+__global__ void task_singles_kernel(const int* __restrict__ t_rowptr, const unsigned long long* __restrict__ first,
+                                    const int* __restrict__ keys, int n, int max_tasks, int4* __restrict__ tasks) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n - split_first[n]) return;
-  const int k = keys[i], at = slot_first[n] + i;
+  const unsigned long long total = first[n];
+  if (i >= n - (int)(total >> 32)) return;
+  const int k = keys[i], at = (int)(unsigned)total + i;
   if (at < max_tasks) tasks[at] = make_int4(k, t_rowptr[k], t_rowptr[k + 1], -1);
 }
 
@@ -150,59 +156,41 @@ extern "C" int bf_graph_transpose(const int* rowptr, const int* col, int n, long
   return (int)cudaGetLastError();
 }
 
-// Phase 1 of the work list: per-key counts and their exclusive prefix sums ([n+1] each, last element = total), and with
-// `by_length` the keys sorted by the length of their row, longest first, split keys behind all others ([n]).
-extern "C" int bf_kv_task_counts(const int* t_rowptr, int n, int chunk, int min_split, int* item_first, int* slot_first,
-                                 int* split_first, int* by_length, void* scratch, size_t scratch_bytes, cudaStream_t st) {
-  // scratch: six int[n] arrays (three counts; length keys, their sorted copy, ids) followed by the temporary storage of CUB
-  int* n_items = static_cast<int*>(scratch);
-  int* n_slots = n_items + n;
-  int* is_split = n_slots + n;
-  int* key_in = is_split + n;
-  int* key_out = key_in + n;
-  int* ids = key_out + n;
-  const size_t head = (6 * (size_t)n * sizeof(int) + 255) & ~(size_t)255;
-  void* tmp = static_cast<uint8_t*>(scratch) + head;
-  size_t tmp_bytes = scratch_bytes - head;
-  if (chunk < 1 || min_split < chunk) return (int)cudaErrorInvalidValue;
-  task_counts_kernel<<<(n + 255) / 256, 256, 0, st>>>(t_rowptr, n, chunk, min_split, n_items, n_slots, is_split,
-                                                      by_length != nullptr ? key_in : nullptr, ids);
-  cudaError_t e;
-  // exclusive prefix sums with the total appended: out[0] = 0, out[1..n] = inclusive sums
-  for (int which = 0; which < 3; ++which) {
-    const int* in = which == 0 ? n_items : which == 1 ? n_slots : is_split;
-    int* out = which == 0 ? item_first : which == 1 ? slot_first : split_first;
-    e = cudaMemsetAsync(out, 0, sizeof(int), st);
-    if (e != cudaSuccess) return (int)e;
-    size_t bytes = tmp_bytes;
-    e = cub::DeviceScan::InclusiveSum(tmp, bytes, in, out + 1, n, st);
-    if (e != cudaSuccess) return (int)e;
+extern "C" size_t bf_row_tasks_scratch(int n, int singles) {
+  size_t tmp = 0;
+  cub::DeviceScan::InclusiveSum(nullptr, tmp, (const unsigned long long*)nullptr, (unsigned long long*)nullptr, n);
+  size_t arrays = (size_t)n * sizeof(unsigned long long);
+  if (singles == 2) {
+    size_t sort_bytes = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (const int*)nullptr, (int*)nullptr, (const int*)nullptr, (int*)nullptr, n);
+    if (sort_bytes > tmp) tmp = sort_bytes;
+    arrays += 4 * (size_t)n * sizeof(int);
   }
-  if (by_length != nullptr) {
-    size_t bytes = tmp_bytes;
+  return ((arrays + 255) & ~(size_t)255) + ((tmp + 255) & ~(size_t)255) + 256;
+}
+
+extern "C" int bf_row_tasks(const int* rowptr, int n, int chunk, int min_split, int singles, int max_tasks, int max_splits,
+                            unsigned long long* first, int* tasks, int* splits, void* scratch, size_t scratch_bytes, cudaStream_t st) {
+  if (n <= 0 || chunk < 1 || min_split < chunk) return (int)cudaErrorInvalidValue;
+  // scratch: counts [n]; sorted singles: length keys, their sorted copy, ids and sorted ids [n] each; temporary storage of CUB
+  unsigned long long* counts = static_cast<unsigned long long*>(scratch);
+  int* key_in = reinterpret_cast<int*>(counts + n);
+  int *key_out = key_in + n, *ids = key_out + n, *by_length = ids + n;
+  const size_t arrays = (size_t)n * sizeof(unsigned long long) + (singles == 2 ? 4 * (size_t)n * sizeof(int) : 0);
+  const size_t head = (arrays + 255) & ~(size_t)255;
+  void* tmp = static_cast<uint8_t*>(scratch) + head;
+  const unsigned blocks = (unsigned)(((long long)n + 255) / 256);
+  task_counts_kernel<<<blocks, 256, 0, st>>>(rowptr, n, chunk, min_split, counts, first, singles == 2 ? key_in : nullptr, ids);
+  size_t bytes = scratch_bytes - head;
+  cudaError_t e = cub::DeviceScan::InclusiveSum(tmp, bytes, counts, first + 1, n, st);
+  if (e != cudaSuccess) return (int)e;
+  int4* out = reinterpret_cast<int4*>(tasks);
+  task_fill_kernel<<<blocks, 256, 0, st>>>(rowptr, first, n, chunk, max_tasks, max_splits, singles == 1, out, splits);
+  if (singles == 2) {
+    bytes = scratch_bytes - head;
     e = cub::DeviceRadixSort::SortPairs(tmp, bytes, key_in, key_out, ids, by_length, n, 0, bits_for(min_split + 2), st);
     if (e != cudaSuccess) return (int)e;
+    task_singles_kernel<<<blocks, 256, 0, st>>>(rowptr, first, by_length, n, max_tasks, out);
   }
-  return (int)cudaGetLastError();
-}
-
-extern "C" size_t bf_kv_task_scratch(int n) {
-  size_t scan_bytes = 0, sort_bytes = 0;
-  cub::DeviceScan::InclusiveSum(nullptr, scan_bytes, (const int*)nullptr, (int*)nullptr, n);
-  cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (const int*)nullptr, (int*)nullptr, (const int*)nullptr, (int*)nullptr, n);
-  const size_t tmp = scan_bytes > sort_bytes ? scan_bytes : sort_bytes;
-  return ((6 * (size_t)n * sizeof(int) + 255) & ~(size_t)255) + ((tmp + 255) & ~(size_t)255) + 256;
-}
-
-// Phase 2: write the items and the split list.  The totals are read on the device, so the caller can read them back last: then
-// the list is complete when the host knows its length, whatever stream uses it.  With `by_length` (of phase 1) the keys that are
-// not split get their single items; without it they get none.
-extern "C" int bf_kv_task_fill(const int* t_rowptr, const int* slot_first, const int* split_first, const int* by_length, int n,
-                               int chunk, int max_tasks, int max_splits, int* tasks, int* splits, cudaStream_t st) {
-  if (n <= 0) return 0;
-  int4* out = reinterpret_cast<int4*>(tasks);
-  const unsigned blocks = (unsigned)(((long long)n + 255) / 256);
-  if (max_splits > 0) task_fill_kernel<<<blocks, 256, 0, st>>>(t_rowptr, slot_first, split_first, n, chunk, max_tasks, max_splits, out, splits);
-  if (by_length != nullptr) task_singles_kernel<<<blocks, 256, 0, st>>>(t_rowptr, slot_first, split_first, by_length, n, max_tasks, out);
   return (int)cudaGetLastError();
 }

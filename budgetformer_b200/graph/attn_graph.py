@@ -24,6 +24,7 @@ import torch
 LONG_ROW = 128     # query rows with more edges are cut into work items of LONG_CHUNK edges (csrc/bf_kernels.h: BF_LONG_ROW,
 LONG_CHUNK = 64    # BF_LONG_CHUNK)
 _LIST_LOCKS = tuple(threading.Lock() for _ in range(64))   # one thread makes a graph's lists, the others wait for it
+SORTED_ROWS = 8192  # keys from which their work items are sorted by length (csrc/bindings.cpp: kSortedRows)
 CAPTURE_ROW = 1024  # longest rows that a forward recorded into a CUDA graph walks whole when their list was not made before
 KV_TASK_EDGES = 64  # edges per work item of the dK/dV pass (32 and 128 both measured slower on the 2.9 M-node graph)
 
@@ -215,7 +216,7 @@ class AttnGraph:
             from ..ops import _ext
             t_rowptr, t_row, t_eid, tasks, splits, sizes = _ext.load().graph_transpose(
                 self.rowptr.contiguous(), self.col.contiguous(), int(self.num_rows), int(KV_TASK_EDGES))
-            _ext.count_launches(6)                         # rows, key offsets, gather, counts, two fills (and the library's sorts)
+            _ext.count_launches(5)                         # rows, key offsets, gather, counts, fill (and the library's sorts)
             self.t_row, self.t_eid = t_row, t_eid
             self.t_task, self.t_split, self.kv_slots = tasks, splits, int(sizes[1])
             self.t_rowptr = t_rowptr                       # last: whoever finds it finds the others
@@ -252,10 +253,11 @@ class AttnGraph:
         slot = torch.cumsum(is_split.to(torch.int64), 0) - 1
         slot = torch.where(is_split, slot, torch.full_like(slot, -1))
         tasks = torch.stack([rows, beg, end, slot], 1)
-        # items of split keys first (long work is scheduled first), in key order; then one item per remaining key, longest first
-        # (the lane groups of a warp finish together), in key order among equals
+        # items of split keys first (long work is scheduled first), in key order; then one item per remaining key, above SORTED_ROWS
+        # keys longest first (the lane groups of a warp finish together), in key order among equals
         single = tasks[~is_split]
-        single = single[torch.sort(single[:, 2] - single[:, 1], descending=True, stable=True).indices]
+        if self.num_rows > SORTED_ROWS:
+            single = single[torch.sort(single[:, 2] - single[:, 1], descending=True, stable=True).indices]
         tasks = torch.cat([tasks[is_split], single], 0)
         self.t_task = tasks.to(torch.int32).contiguous()
         srows = torch.nonzero(split_row).flatten()

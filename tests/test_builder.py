@@ -206,4 +206,4 @@ def test_work_list_constants_match_the_kernels():
     from budgetformer_b200.ops import _ext
     ext = _ext.load()
     assert (attn_graph.LONG_ROW, attn_graph.LONG_CHUNK) == (ext.LONG_ROW, ext.LONG_CHUNK)
-    assert attn_graph.KV_TASK_EDGES == ext.LONG_CHUNK
+    assert attn_graph.KV_TASK_EDGES == ext.LONG_CHUNK and attn_graph.SORTED_ROWS == ext.SORTED_ROWS

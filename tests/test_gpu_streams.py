@@ -172,6 +172,31 @@ def test_forward_with_long_rows_is_captured(listed_before):
     assert float((out - ref).norm()) <= 2e-5 * float(ref.norm())
 
 
+@pytest.mark.parametrize("n", [1, 33, 8192, 8193, 20011])
+def test_work_lists_on_both_sides_of_the_sort(n):
+    """The device's by-key view and work list against the CPU construction: keys of no, one, 64 and 65 edges and popular ones, below
+    and above the number of keys from which single items are sorted by length; and the list of long query rows."""
+    from budgetformer_b200.graph.attn_graph import LONG_CHUNK, LONG_ROW, AttnGraph
+    gen = torch.Generator().manual_seed(n)
+    src = (torch.rand(6 * n, generator=gen) ** 4 * n).long().clamp_(max=n - 1)
+    src = torch.cat([src, torch.full((64,), n - 1), torch.full((65,), n // 2), torch.full((200,), n // 3)])
+    dst = torch.cat([torch.randint(0, n, (6 * n,), generator=gen), torch.full((329,), n // 5)])
+    ref = AttnGraph.from_edge_index(torch.stack([src, dst]), n).ensure_transpose()
+    dev = AttnGraph(n, ref.rowptr.cuda(), ref.col.cuda()).ensure_transpose()
+    for name in ("t_rowptr", "t_row", "t_eid", "t_task", "t_split"):
+        assert torch.equal(getattr(ref, name), getattr(dev, name).cpu()), name
+    assert ref.kv_slots == dev.kv_slots
+    deg = (ref.rowptr[1:] - ref.rowptr[:-1]).tolist()
+    tasks, splits = [], []
+    for row, d in enumerate(deg):
+        if d > LONG_ROW:
+            items = [(row, int(ref.rowptr[row]) + c, int(ref.rowptr[row]) + min(c + LONG_CHUNK, d)) for c in range(0, d, LONG_CHUNK)]
+            splits.append([row, len(tasks), len(items)])
+            tasks += [[*it, len(tasks) + i] for i, it in enumerate(items)]
+    task, split, least = dev.long_rows()
+    assert task.tolist() == tasks and split.tolist() == splits and least == LONG_ROW
+
+
 def test_by_key_view_without_its_work_list():
     """A graph that was given t_rowptr, t_row and t_eid alone: the backward pass makes the work list, and the gradients are those
     of the graph's own."""
