@@ -78,8 +78,8 @@ typedef struct {
   void *dq, *dk, *dv;               // [n, hl, hn], common row stride ldg (elements; 0 = hl*hn)
   long long ldg;
   float* zd;                        // [n, hl, 2] fp32 workspace: 1 / (Z + eps) and <dout, out> of every row
-  float* ds;                        // [E, hl] fp32 workspace: score gradients, from the dK/dV pass to the dQ pass (not used where
-                                    // bf_attn_bwd_keeps_scores is 0)
+  float* ds;                        // [E, hl] fp32 workspace: score gradients, from the dK/dV pass to the dQ pass.  Not used where
+                                    // bf_attn_bwd_keeps_scores is 0; NULL (untyped edges only): they are computed twice
   const int *t_row, *t_eid;         // edges grouped by key: query, and position in the query-grouped list
   float* detab;                     // zero-filled [2, hl, hn] fp32 or NULL
   bf_long_rows long_rows;           // scratch row: hl*hn floats

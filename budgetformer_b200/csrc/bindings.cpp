@@ -189,11 +189,16 @@ int64_t edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor
   LongRows lr = take_long_rows(rowptr, col.numel(), known_max_degree, long_task, long_split, long_min, (size_t)w);
   b.long_rows = lr.c;
   Tensor partial, qg;
-  const bool keeps = bf_attn_bwd_keeps_scores(p.dtype, p.n, p.hl, p.hn, p.variant) != 0;
   Tensor ds;
-  if (keeps) {
-    ds = torch::empty({std::max<int64_t>(col.numel(), 1), (int64_t)p.hl}, q.options().dtype(torch::kFloat));
-    b.ds = ds.data_ptr<float>();
+  if (bf_attn_bwd_keeps_scores(p.dtype, p.n, p.hl, p.hn, p.variant)) {
+    // 4 bytes per edge and head (0.49 GB at 15.3 M edges of 8 heads), the largest thing a backward pass allocates: where it does not
+    // fit, the scores are computed twice.  Typed edges have no such form.
+    try {
+      ds = torch::empty({std::max<int64_t>(col.numel(), 1), (int64_t)p.hl}, q.options().dtype(torch::kFloat));
+    } catch (const c10::OutOfMemoryError&) {
+      if (p.variant == 2) throw;
+    }
+    b.ds = ds.defined() ? ds.data_ptr<float>() : nullptr;
   }
   if (w * q.element_size() <= 64) {
     // narrow rows: one packed record per (query, head) for the dK/dV pass (see bf_attn_bwd_params)
@@ -221,7 +226,7 @@ int64_t edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor
     b.route_cq = (int)route[3]; b.route_ck = (int)route[4]; b.route_cv = (int)route[5];
   }
   check_cuda(bf_edge_attn_bwd(&p, &b, at::cuda::getCurrentCUDAStream()), "edge_attn_bwd");
-  return (keeps ? 3 : 2) + (b.n_kv_split > 0 ? 2 : 0) + (lr.c.n_task > 0 ? 3 : 0);
+  return (ds.defined() ? 3 : 2) + (b.n_kv_split > 0 ? 2 : 0) + (lr.c.n_task > 0 ? 3 : 0);
 }
 
 // Returns (rowptr int32 [n+1], col int32 [E], etype uint8 [E] or empty, totals int64 [2]).

@@ -1721,7 +1721,7 @@ extern "C" int bf_edge_attn_bwd(const bf_attn_params* p, const bf_attn_bwd_param
   b.f = to_args(*p);
   if (b.f.n_hub > 0 || !take_long_rows(&q->long_rows, &b.f) || q->kv_task == nullptr) return (int)cudaErrorInvalidValue;
   const bool keeps = bf_attn_bwd_keeps_scores(p->dtype, p->n, p->hl, p->hn, p->variant) != 0;
-  if (keeps && q->ds == nullptr) return (int)cudaErrorInvalidValue;
+  if (p->variant == 2 && q->ds == nullptr) return (int)cudaErrorInvalidValue;
   b.dout = q->dout; b.dq = q->dq; b.dk = q->dk; b.dv = q->dv;
   b.ldg = q->ldg > 0 ? q->ldg : (long long)p->hl * p->hn;
   b.zd = reinterpret_cast<float2*>(q->zd);

@@ -197,6 +197,36 @@ def test_work_lists_on_both_sides_of_the_sort(n):
     assert task.tolist() == tasks and split.tolist() == splits and least == LONG_ROW
 
 
+def test_backward_without_room_for_the_score_gradients():
+    """The buffer of kept score gradients is the largest thing a backward pass allocates.  Where the allocator cannot give it, the
+    scores are computed twice: the same gradients up to the order of fp32 sums."""
+    from budgetformer_b200.graph.attn_graph import AttnGraph
+    from budgetformer_b200.ops.edge_attention import edge_attention
+    n, deg = 4000, 2000
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    dst = torch.arange(n, device="cuda").repeat_interleave(deg)
+    graph = AttnGraph.from_edge_index(torch.stack([torch.randint(0, n, (n * deg,), generator=gen, device="cuda"), dst]), n).ensure_transpose()
+    graph.long_rows()
+    del dst
+    q, k, v, dout = (torch.randn(n, 8, 8, generator=gen, device="cuda") for _ in range(4))
+    args = [t.requires_grad_() for t in (q, k, v)]
+    want = torch.autograd.grad(edge_attention(*args, graph), args, dout)
+    out = edge_attention(*args, graph)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (200 << 20)) / total)   # the buffer takes 256 MB
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        got = torch.autograd.grad(out, args, dout)
+        assert torch.cuda.max_memory_allocated() - before < n * deg * 8 * 4
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for a, b in zip(got, want):
+        assert float((a - b).norm()) <= 2e-5 * (float(b.norm()) + float(dout.norm()))
+
+
 def test_by_key_view_without_its_work_list():
     """A graph that was given t_rowptr, t_row and t_eid alone: the backward pass makes the work list, and the gradients are those
     of the graph's own."""
