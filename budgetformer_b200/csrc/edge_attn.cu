@@ -695,8 +695,8 @@ struct BwdArgs {
   float* kv_partial;           // [n_kv_slots, 2*Hl*HN] fp32
   // Packed query records for narrow rows (optional): the first kernel writes q and dout of every (row, head) next to each other
   // and the dK/dV pass gathers one contiguous record per edge instead of two short rows, which matters when a row of q is only 32
-  // or 64 bytes.  dout goes in as it is: dout / (Z + eps) rounded to 16 bits would enter <dout, v> but not D, and the score
-  // gradient is a difference of the two (1.5 times the error in dQ).
+  // or 64 bytes.  Where dQ takes its score gradients from that pass, dout goes in as it is: dout / (Z + eps) rounded to 16 bits would
+  // enter <dout, v> but not D, and the score gradient is a difference of the two (1.5 times the error in dQ).
   void* qg;                    // [n, Hl, 2, HN] in the operand dtype, or null
   // Routed gradients (route.n_dest > 0): dq / dk / dv rows go to the owner of the row instead of the local buffers, at
   // column offsets cq / ck / cv of the destination's packed row
@@ -757,7 +757,7 @@ template <int NP> __device__ __forceinline__ void typed_sum(const float* et, int
 // dK/dV over the balanced work list, first of the two passes over the edges.  It gathers q, dout and (1/Z, D) of each query and
 // leaves the score gradient of every (edge, head) in `ds` (fp32, at the edge's own position), so that the dQ pass gathers k alone.
 // The list holds the items of split keys (64 edges each), then the rest sorted by length.
-template <typename T, int HN, int VAR>
+template <typename T, int HN, int VAR, bool PACKED>
 __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bwd_kv_kernel(BwdArgs b, StreamGeo sg) {
   constexpr bool EXPH = VAR == 2;
   constexpr int VN = EXPH ? Vec<T>::N : wide_elems<T, HN>(), NP = VN / 2, LPH = HN / VN;
@@ -784,16 +784,19 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
     return it;
   };
   const int hsafe = on ? head : 0, off = hsafe * HN + (lt % LPH) * VN, w_row = a.hl * HN;
-  const char* qb = reinterpret_cast<const char*>(static_cast<const T*>(a.q) + off);
-  const char* gb = reinterpret_cast<const char*>(static_cast<const T*>(b.dout) + off);
-  const char* zb = reinterpret_cast<const char*>(b.zd + hsafe);
-  unsigned long long sq = (unsigned long long)a.ldq * sizeof(T), sgr = (unsigned long long)w_row * sizeof(T);
-  const unsigned long long szd = (unsigned long long)a.hl * sizeof(float2);
-  if (b.qg != nullptr) {
+  // (the record form as a template argument: chosen at run time it cost the other one 5 % in registers)
+  const char *qb, *gb;
+  unsigned long long sq, sgr;
+  if (PACKED) {
     qb = reinterpret_cast<const char*>(static_cast<const T*>(b.qg) + (long long)hsafe * 2 * HN + (lt % LPH) * VN);
     gb = qb + HN * sizeof(T);
     sq = sgr = (unsigned long long)w_row * 2 * sizeof(T);
+  } else {
+    qb = reinterpret_cast<const char*>(static_cast<const T*>(a.q) + off); sq = (unsigned long long)a.ldq * sizeof(T);
+    gb = reinterpret_cast<const char*>(static_cast<const T*>(b.dout) + off); sgr = (unsigned long long)w_row * sizeof(T);
   }
+  const char* zb = reinterpret_cast<const char*>(b.zd + hsafe);
+  const unsigned long long szd = (unsigned long long)a.hl * sizeof(float2);
   // fetching side: items two segments ahead, the first query of a segment one segment ahead (see RowFetch)
   int fr = 0, fi = 0, fbeg, flen, beg1, len1, beg2, len2;
   auto bounds = [&](int r, int& beg, int& len) { const int4 it = item(r); beg = it.y; len = it.z; };
@@ -1169,7 +1172,7 @@ template <typename T, int HN> struct QueryTerms {
   }
 };
 
-// two edges of one query
+// two edges of one query; an absent second one repeats the first with weight 0 (no branch between them: their sums overlap)
 template <typename T, int HN>
 __device__ __forceinline__ void dq_pair(const BwdArgs& b, int e, int end, int head, int off, const QueryTerms<T, HN>& t, float* dq,
                                         unsigned hm) {
@@ -1183,13 +1186,12 @@ __device__ __forceinline__ void dq_pair(const BwdArgs& b, int e, int end, int he
   vr[1].load(static_cast<const T*>(a.v) + (long long)j1 * a.ldv + off);
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
-    if (u == 1 && e + 1 >= end) break;
     float d = 0.f, dv = 0.f;
 #pragma unroll
     for (int i = 0; i < VN; ++i) { d += t.qs[i] * kr[u].get(i); dv += t.dof[i] * vr[u].get(i); }
     d = head_sum<LPH>(d, hm);
     dv = head_sum<LPH>(dv, hm);
-    const bool inr = (d > -kClamp) && (d < kClamp);
+    const bool inr = (d > -kClamp) && (d < kClamp) && (u == 0 || e + 1 < end);
     const float w = __expf(fminf(fmaxf(d, -kClamp), kClamp));
     float mf = 1.f;
     if (a.variant == 1) mf = (a.thresh && !keep_edge(a.seed, (uint32_t)(e + u), (uint32_t)head, a.thresh)) ? 0.f : a.inv_keep;
@@ -1219,11 +1221,19 @@ __global__ void __launch_bounds__(256, 4) edge_attn_bwd_q_rows_kernel(BwdArgs b)
   const unsigned hm = head_mask<LPH>();
   QueryTerms<T, HN> t;
   t.load(b, row, head, off, hm);
-  if ((lt % LPH) == 0) b.zd[(long long)row * a.hl + head] = make_float2(t.invz, t.dterm);
+  const long long hz = (long long)row * a.hl + head;
   if (b.qg != nullptr) {
-    T* rec = static_cast<T*>(b.qg) + ((long long)row * a.hl + head) * 2 * HN + (lt % LPH) * VN;
+    // narrow rows: [q | dout / (Z + eps)] and D / (Z + eps), which only dK and dV see here (4 bytes of row terms instead of 8: 7 % of
+    // the dK/dV pass at 1 x 16 and 2.9 M rows)
+    T* rec = static_cast<T*>(b.qg) + hz * 2 * HN + (lt % LPH) * VN;
+    float gz[VN];
+#pragma unroll
+    for (int i = 0; i < VN; ++i) gz[i] = t.dof[i] * t.invz;
     *reinterpret_cast<uint4*>(rec) = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(a.q) + (long long)row * a.ldq + off));
-    store_vec<T>(rec + HN, t.dof);
+    store_vec<T>(rec + HN, gz);
+    if ((lt % LPH) == 0) reinterpret_cast<float*>(b.zd)[hz] = t.dterm * t.invz;
+  } else if ((lt % LPH) == 0) {
+    b.zd[hz] = make_float2(t.invz, t.dterm);
   }
   float dq[VN];
 #pragma unroll
@@ -1266,7 +1276,7 @@ __global__ void __launch_bounds__(256, 3) edge_attn_bwd_q_items_kernel(BwdArgs b
 }
 
 // one lane group per (work item, head chunk), two edges at a time: four 16-byte gathers in flight
-template <typename T, int HN>
+template <typename T, int HN, bool PACKED>
 __global__ void __launch_bounds__(256, 4) edge_attn_bwd_kv_rows_kernel(BwdArgs b) {
   constexpr int VN = Vec<T>::N, LPH = HN / VN;
   const AttnArgs& a = b.f;
@@ -1281,13 +1291,9 @@ __global__ void __launch_bounds__(256, 4) edge_attn_bwd_kv_rows_kernel(BwdArgs b
   if (!live || head >= a.hl) return;            // whole heads leave together; shuffles use head masks
   const int off = head * HN + (lt % LPH) * VN;
   const int4 it = __ldg(b.kv_task + item);
-  const T *qb = static_cast<const T*>(a.q) + off, *gb = static_cast<const T*>(b.dout) + off;
-  long long sq = a.ldq, sg = w_row;
-  if (b.qg != nullptr) {
-    qb = static_cast<const T*>(b.qg) + (long long)head * 2 * HN + (lt % LPH) * VN;
-    gb = qb + HN;
-    sq = sg = 2 * (long long)w_row;
-  }
+  const T* qb = PACKED ? static_cast<const T*>(b.qg) + (long long)head * 2 * HN + (lt % LPH) * VN : static_cast<const T*>(a.q) + off;
+  const T* gb = PACKED ? qb + HN : static_cast<const T*>(b.dout) + off;
+  const long long sq = PACKED ? 2 * (long long)w_row : a.ldq, sg = PACKED ? sq : w_row;
   Raw<T> kf, vf;                                // this key's k | v slice stays packed for the whole item
   kf.load(static_cast<const T*>(a.k) + (long long)it.x * a.ldk + off);
   vf.load(static_cast<const T*>(a.v) + (long long)it.x * a.ldv + off);
@@ -1310,21 +1316,22 @@ __global__ void __launch_bounds__(256, 4) edge_attn_bwd_kv_rows_kernel(BwdArgs b
     for (int u = 0; u < 2; ++u) {
       qr[u].load(qb + row[u] * sq);
       gr[u].load(gb + row[u] * sg);
-      zd[u] = __ldg(b.zd + (long long)row[u] * a.hl + head);
+      const long long hz = (long long)row[u] * a.hl + head;
+      zd[u] = PACKED ? make_float2(1.f, __ldg(reinterpret_cast<const float*>(b.zd) + hz)) : __ldg(b.zd + hz);
     }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      if (u == 1 && e + 1 >= it.z) break;
       float d = 0.f, dotv = 0.f;
 #pragma unroll
       for (int i = 0; i < VN; ++i) { d += qr[u].get(i) * kf.get(i); dotv += gr[u].get(i) * vf.get(i); }
       d = head_sum<LPH>(d, hm) * scale;
       dotv = head_sum<LPH>(dotv, hm);
-      const bool inr = (d > -kClamp) && (d < kClamp);
+      const bool ok = u == 0 || e + 1 < it.z;   // an absent second edge repeats the first with weight 0
+      const bool inr = (d > -kClamp) && (d < kClamp) && ok;
       const float w = __expf(fminf(fmaxf(d, -kClamp), kClamp)) * zd[u].x;
       float mf = 1.f;
       if (a.variant == 1) mf = (a.thresh && !keep_edge(a.seed, (uint32_t)eid[u], (uint32_t)head, a.thresh)) ? 0.f : a.inv_keep;
-      const float dss = inr ? (dotv * mf - zd[u].y) * w * scale : 0.f, wn = w * mf;
+      const float dss = inr ? (dotv * mf - zd[u].y) * w * scale : 0.f, wn = ok ? w * mf : 0.f;
 #pragma unroll
       for (int i = 0; i < VN; ++i) { dk[i] += dss * qr[u].get(i); dv[i] += wn * gr[u].get(i); }
     }
@@ -1490,7 +1497,8 @@ void launch_kv(const BwdArgs& b, cudaStream_t st) {
   constexpr int VN = VAR == 2 ? Vec<T>::N : wide_elems<T, HN>();
   const StreamGeo s = stream_geo<HN, VN>(b.f.hl, b.n_kv_task, VAR == 2 ? 4 : 3, 8);
   const dim3 grid = stream_grid<HN, VN>(b.f.hl, stream_warps(b.n_kv_task, s, s.per), s);
-  edge_attn_bwd_kv_kernel<T, HN, VAR><<<grid, kStreamThreads, 0, st>>>(b, s);
+  if (b.qg) edge_attn_bwd_kv_kernel<T, HN, VAR, true><<<grid, kStreamThreads, 0, st>>>(b, s);
+  else edge_attn_bwd_kv_kernel<T, HN, VAR, false><<<grid, kStreamThreads, 0, st>>>(b, s);
 }
 
 // Whether the forward pass takes edge_attn_fwd_rows_kernel.  Streams hide the latency of DRAM; where the gathered rows stay in L2
@@ -1570,7 +1578,10 @@ cudaError_t launch_recomputed_bwd_t(const BwdArgs& b, cudaStream_t st) {
     edge_attn_bwd_q_items_kernel<T, HN><<<(unsigned)(((long long)a.n_long_task * g.n_hc + 7) / 8), 256, 0, st>>>(b);
     launch_split<T, SPLIT_DQ>(b, a.long_task, a.n_long_task, a.long_split, a.n_long_split, a.long_partial, w_row, w_row, w_row, HN, st);
   }
-  if (b.n_kv_task > 0) edge_attn_bwd_kv_rows_kernel<T, HN><<<blocks(b.n_kv_task), 256, 0, st>>>(b);
+  if (b.n_kv_task > 0) {
+    if (b.qg) edge_attn_bwd_kv_rows_kernel<T, HN, true><<<blocks(b.n_kv_task), 256, 0, st>>>(b);
+    else edge_attn_bwd_kv_rows_kernel<T, HN, false><<<blocks(b.n_kv_task), 256, 0, st>>>(b);
+  }
   if (b.n_kv_split > 0)
     launch_split<T, SPLIT_KV>(b, b.kv_task, b.n_kv_slots, b.kv_split, b.n_kv_split, b.kv_partial, 2 * w_row, 2 * w_row, w_row, HN, st);
   return cudaGetLastError();
