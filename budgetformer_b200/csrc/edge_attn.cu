@@ -1511,12 +1511,16 @@ void launch_kv(const BwdArgs& b, cudaStream_t st) {
 // - 16 bits otherwise, 16 edges a row: 4 x 16 170 k (44 MB) 95 / 105, 8 x 32 50 k (51 MB) with dropout 153 / 178, 8 x 16 170 k (87 MB)
 //   198 / 186; 5 to 8 edges a row: 4 x 16 110 k 57 / 49, 8 x 16 50 k 36 / 31, 8 x 32 50 k 63 / 58 (longer rows pay the streams' cost
 //   per edge, short ones the other kernel's cost per row)
+// - with dropout on the stored output (a hash per element, for which the streams have no issue slots left): 8 x 16, 5 edges a row, 2 k
+//   5.2 / 6.2, 50 k 35 / 41, 170 k (87 MB) 128 / 144, 300 k (154 MB) 231 / 221; 8 x 32, 110 k (113 MB) 148 / 153, 170 k (174 MB) 233 / 235, 300 k 420 /
+//   399; 8 x 8, 700 k (179 MB) 279 / 302
 // - typed edges (two scaled queries, a select per element): 8 x 32, 25 edges, 50 k 167 / 201, 390 k (400 MB) 1879 / 1893
-inline bool rows_forward(int dtype, long long n, int hl, int hn, int variant, long long n_edges) {
+inline bool rows_forward(int dtype, long long n, int hl, int hn, int variant, bool out_dropout, long long n_edges) {
   const long long row = (long long)hl * hn * (dtype == BF_FP32 ? 4 : 2), gathered = 2 * n * row;
   if (variant == 2) return true;
-  if (dtype == BF_FP32 || row <= 64) return gathered <= 200'000'000;
+  if (dtype == BF_FP32 || row <= 64 || (hn == 8 && out_dropout)) return gathered <= 200'000'000;
   if (hn == 8) return gathered <= 100'000'000;
+  if (out_dropout) return gathered <= 120'000'000;
   return n_edges >= 12 * n && gathered <= 64'000'000;
 }
 
@@ -1706,7 +1710,7 @@ extern "C" int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_ro
   if (!take_long_rows(long_rows, &a)) return (int)cudaErrorInvalidValue;
   if (!to_route(route, p->n, (long long)p->hl * p->hn, &a.route_out)) return (int)cudaErrorInvalidValue;
   const int chunks = p->max_hub_degree > 0 ? (p->max_hub_degree + BF_HUB_CHUNK - 1) / BF_HUB_CHUNK : 1;
-  const bool rows = rows_forward(p->dtype, p->n, p->hl, p->hn, p->variant, n_edges);
+  const bool rows = rows_forward(p->dtype, p->n, p->hl, p->hn, p->variant, p->out_dropout_p > 0.f, n_edges);
 #define CALL_FWD(T, H) (int)launch_fwd_t<T, H>(a, rows, chunks, st)
   BF_DISPATCH(p->dtype, p->hn, CALL_FWD);
 #undef CALL_FWD
@@ -1716,7 +1720,7 @@ extern "C" int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_ro
 extern "C" int bf_edge_attn_fwd(const bf_attn_params* p, cudaStream_t st) {
   AttnArgs a = to_args(*p);
   const int chunks = p->max_hub_degree > 0 ? (p->max_hub_degree + BF_HUB_CHUNK - 1) / BF_HUB_CHUNK : 1;
-  const bool rows = rows_forward(p->dtype, p->n, p->hl, p->hn, p->variant, -1);       // the number of edges is not known here
+  const bool rows = rows_forward(p->dtype, p->n, p->hl, p->hn, p->variant, p->out_dropout_p > 0.f, -1);       // the number of edges is not known here
 #define CALL_FWD(T, H) (int)launch_fwd_t<T, H>(a, rows, chunks, st)
   BF_DISPATCH(p->dtype, p->hn, CALL_FWD);
 #undef CALL_FWD

@@ -227,6 +227,26 @@ def test_backward_without_room_for_the_score_gradients():
         assert float((a - b).norm()) <= 2e-5 * (float(b.norm()) + float(dout.norm()))
 
 
+@pytest.mark.parametrize("n,heads,hn,dtype", [(257, 8, 16, torch.bfloat16), (240007, 8, 16, torch.bfloat16), (101021, 4, 64, torch.float32)])
+def test_output_dropout_in_both_forward_kernels(n, heads, hn, dtype):
+    """Dropout fused into the stored output, on the sizes of either kernel: the plain output where the hash keeps, scaled, else 0."""
+    from budgetformer_b200.ops import _ext
+    from budgetformer_b200.ops.gemm import hash_keep_mask
+    graph = _graph(n, 3, 12, False)
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    q, k, v = (torch.randn(n, heads, hn, generator=gen, device="cuda").to(dtype) for _ in range(3))
+    res = []
+    for drop in ([], [0.25, 9.0, float(n), 0.0]):
+        out, z = torch.empty_like(q), torch.empty(n, heads, device="cuda")
+        _ext.load().edge_attn_fwd(q, k, v, out, z, graph.rowptr, graph.col, None, None, 0, 0.0, 0, 3, drop, [])
+        res.append((out.float().flatten(1), z))
+    keep = hash_keep_mask(9, n, heads * hn, 0.25, "cuda")
+    want = torch.where(keep, res[0][0] / 0.75, torch.zeros((), device="cuda"))
+    unit = {torch.float32: 2.0 ** -20, torch.bfloat16: 2.0 ** -7}[dtype]        # both are rounded; fp32: another order of sums
+    assert bool(((res[1][0] - want).abs() <= unit * want.abs() + 1e-6).all())
+    assert float((res[0][1] - res[1][1]).norm()) <= 1e-6 * float(res[0][1].norm())
+
+
 def test_by_key_view_without_its_work_list():
     """A graph that was given t_rowptr, t_row and t_eid alone: the backward pass makes the work list, and the gradients are those
     of the graph's own."""
