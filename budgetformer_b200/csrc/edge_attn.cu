@@ -20,6 +20,7 @@
 #include <string.h>
 
 #include "bf_kernels.h"
+#include "f32x2.cuh"
 
 namespace {
 
@@ -88,30 +89,6 @@ template <> struct Raw<float> {
   __device__ __forceinline__ void load(const float* p) { f = *reinterpret_cast<const float4*>(p); }
   __device__ __forceinline__ float get(int i) const { return i == 0 ? f.x : i == 1 ? f.y : i == 2 ? f.z : f.w; }
 };
-
-// Pairs of fp32 values in one 64-bit register: sm_100a multiplies and adds them two at a time (fma.rn.f32x2), each half rounded
-// like a plain fp32 fma.
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 pack2(float lo, float hi) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(f2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 
 // One 16-byte slice of a row widened to fp32 pairs.
 template <typename T> __device__ __forceinline__ void widen(const uint4& u, f2* p);

@@ -13,25 +13,10 @@
 #include <stdint.h>
 
 #include "bf_kernels.h"
+#include "f32x2.cuh"
 
 namespace {
 
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 pack2(float lo, float hi) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(f2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 // BYTES from src, or zeros
 template <int BYTES> __device__ __forceinline__ void copy_or_zero(void* dst, const void* src, bool ok) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);

@@ -23,7 +23,7 @@ setup(
     version="0.1.0",
     description="Blackwell-native (sm_100a) distributed full-graph Graph-Transformer training",
     packages=find_packages(include=["budgetformer_b200", "budgetformer_b200.*"]),
-    package_data={"budgetformer_b200": ["csrc/*.cu", "csrc/*.cpp", "csrc/*.h", "csrc/cpu/*.cpp"]},
+    package_data={"budgetformer_b200": ["csrc/*.cu", "csrc/*.cpp", "csrc/*.h", "csrc/*.cuh", "csrc/cpu/*.cpp"]},
     py_modules=["main_node_fullgraph_sp", "main_node_sp"],
     python_requires=">=3.10",
     install_requires=["torch>=2.6", "numpy", "scipy"],
