@@ -1338,48 +1338,38 @@ __global__ void __launch_bounds__(256, 4) edge_attn_bwd_kv_rows_kernel(BwdArgs b
 // ---------------------------------------------------------------------------------------------
 constexpr int SPLIT_WINDOW = 64;
 constexpr int SPLIT_THREADS = 256;
-constexpr int SPLIT_COLS = 4096;            // columns and normalisers of the forward pass that a block holds at a time
 constexpr int SPLIT_FWD = 0, SPLIT_DQ = 1, SPLIT_KV = 2;
 
-// Writes row `row` from the finished column sums sum(c), c < Hl*HN (forward: the numerators, and Hl normalisers behind them) or
-// 2*Hl*HN (dK | dV).  The whole block takes part.  The forward pass needs a head's normaliser beside its columns: heads go through
-// shared memory as many at a time as fit, so rows may be of any width.
-template <typename T, int MODE, typename F>
-__device__ __forceinline__ void split_finish(const BwdArgs& b, int row, int w, int hn, F sum) {
+// s[0 .. ncol) holds the finished sums of row `row`
+template <typename T, int MODE>
+__device__ __forceinline__ void split_finish(const BwdArgs& b, int row, int w, int hn, const float* s) {
   const AttnArgs& a = b.f;
   if (MODE == SPLIT_FWD) {
-    __shared__ float s_sum[SPLIT_COLS];
-    const int fit = SPLIT_COLS / (hn + 1);
-    for (int h0 = 0; h0 < a.hl; h0 += fit) {
-      const int heads = min(fit, a.hl - h0), nc = heads * hn;
-      for (int c = threadIdx.x; c < nc + heads; c += blockDim.x) s_sum[c] = sum(c < nc ? h0 * hn + c : w + h0 + (c - nc));
-      __syncthreads();
-      for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-        const int head = h0 + c / hn, col = h0 * hn + c;
-        const float zs = s_sum[nc + c / hn];
-        float inv = 1.f / (zs + kEps);
-        if (a.variant == 1) inv *= a.inv_keep;
-        float ov = s_sum[c] * inv;
-        if (a.out_thresh) ov = keep_out(a, row, col) ? ov * a.out_inv_keep : 0.f;
-        static_cast<T*>(a.out)[(long long)row * w + col] = from_float<T>(ov);
-        if (a.route_out.n_dest) *routed<T>(a.route_out, row, col) = from_float<T>(ov);
-        if (c % hn == 0) a.z[(long long)row * a.hl + head] = zs;
-      }
-      __syncthreads();
+    for (int c = threadIdx.x; c < w; c += blockDim.x) {
+      const int head = c / hn;
+      const float zs = s[w + head];
+      float inv = 1.f / (zs + kEps);
+      if (a.variant == 1) inv *= a.inv_keep;
+      float ov = s[c] * inv;
+      if (a.out_thresh) ov = keep_out(a, row, c) ? ov * a.out_inv_keep : 0.f;
+      static_cast<T*>(a.out)[(long long)row * w + c] = from_float<T>(ov);
+      if (a.route_out.n_dest) *routed<T>(a.route_out, row, c) = from_float<T>(ov);
+      if (c % hn == 0) a.z[(long long)row * a.hl + head] = zs;
     }
   } else if (MODE == SPLIT_DQ) {
     T* dst = grad_row<T>(b, b.dq, b.cq, row);
-    for (int c = threadIdx.x; c < w; c += blockDim.x) dst[c] = from_float<T>(sum(c));
+    for (int c = threadIdx.x; c < w; c += blockDim.x) dst[c] = from_float<T>(s[c]);
   } else {
     T* dk = grad_row<T>(b, b.dk, b.ck, row);
     T* dv = grad_row<T>(b, b.dv, b.cv, row);
-    for (int c = threadIdx.x; c < 2 * w; c += blockDim.x) (c < w ? dk + c : dv + (c - w))[0] = from_float<T>(sum(c));
+    for (int c = threadIdx.x; c < 2 * w; c += blockDim.x) (c < w ? dk + c : dv + (c - w))[0] = from_float<T>(s[c]);
   }
 }
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(SPLIT_THREADS) split_window_kernel(BwdArgs b, const int4* __restrict__ task, int n_slots,
                                                                      float* partial, int pitch, int ncol, int w, int hn) {
+  extern __shared__ float s_sum[];            // [ncol]
   __shared__ int s_key[SPLIT_WINDOW];
   const int s0 = blockIdx.x * SPLIT_WINDOW, s1 = min(s0 + SPLIT_WINDOW, n_slots);
   for (int i = threadIdx.x; i < s1 - s0; i += blockDim.x) s_key[i] = task[s0 + i].x;
@@ -1390,7 +1380,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_window_kernel(BwdArgs b, 
     int j = i + 1;
     while (j < s1 && s_key[j - s0] == key) ++j;
     const bool whole = !(i == s0 && before == key) && !(j == s1 && after == key);
-    auto sum = [&](int c) {
+    for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
       const float* pp = partial + (long long)i * pitch + c;
       float acc[8];
 #pragma unroll
@@ -1403,23 +1393,28 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_window_kernel(BwdArgs b, 
 #pragma unroll
       for (int u = 0; u < 7; ++u)
         if (u < n) acc[u] += pp[u * (long long)pitch];
-      return ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
-    };
-    if (whole) split_finish<T, MODE>(b, key, w, hn, sum);
-    else
-      for (int c = threadIdx.x; c < ncol; c += blockDim.x) partial[(long long)i * pitch + c] = sum(c);
+      const float sum = ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
+      if (whole) s_sum[c] = sum;
+      else partial[(long long)i * pitch + c] = sum;
+    }
+    if (whole) {
+      __syncthreads();
+      split_finish<T, MODE>(b, key, w, hn, s_sum);
+      __syncthreads();
+    }
     i = j;
   }
 }
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(SPLIT_THREADS) split_cross_kernel(BwdArgs b, const int* __restrict__ split, int n_split,
-                                                                    const float* partial, int pitch, int w, int hn) {
+                                                                    const float* partial, int pitch, int ncol, int w, int hn) {
+  extern __shared__ float s_sum[];            // [ncol]
   for (int s = blockIdx.x; s < n_split; s += gridDim.x) {
     const int first = split[3 * s + 1];
     const int w0 = first / SPLIT_WINDOW, w1 = (first + split[3 * s + 2] - 1) / SPLIT_WINDOW;
     if (w0 == w1) continue;                   // finished by its window
-    split_finish<T, MODE>(b, split[3 * s], w, hn, [&](int c) {
+    for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
       float acc[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) acc[u] = 0.f;
@@ -1430,16 +1425,27 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_cross_kernel(BwdArgs b, c
         for (int u = 0; u < 8; ++u) acc[u] += pp[(long long)(k + u) * SPLIT_WINDOW * pitch];
       }
       for (; k <= w1; ++k) acc[0] += pp[(long long)k * SPLIT_WINDOW * pitch];
-      return pp[(long long)first * pitch] + ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
-    });
+      s_sum[c] = pp[(long long)first * pitch] + ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
+    }
+    __syncthreads();
+    split_finish<T, MODE>(b, split[3 * s], w, hn, s_sum);
+    __syncthreads();
   }
 }
 
 template <typename T, int MODE>
 void launch_split(const BwdArgs& b, const int4* task, int n_slots, const int* split, int n_split, float* partial, int pitch,
                   int ncol, int w, int hn, cudaStream_t st) {
-  split_window_kernel<T, MODE><<<(n_slots + SPLIT_WINDOW - 1) / SPLIT_WINDOW, SPLIT_THREADS, 0, st>>>(b, task, n_slots, partial, pitch, ncol, w, hn);
-  split_cross_kernel<T, MODE><<<n_split < 148 * 8 ? n_split : 148 * 8, SPLIT_THREADS, 0, st>>>(b, split, n_split, partial, pitch, w, hn);
+  // Rows above some 6,100 elements (dK | dV; 12,000 otherwise) need more than a block's default 48 KB.  (Taking the columns in parts
+  // instead, by a loop or a grid dimension, made the reduction of popular keys 15 to 65 % slower: 86 to 142 us a layer at 612 k nodes,
+  // h = 256.)
+  const size_t smem = sizeof(float) * ncol;
+  if (smem + sizeof(int) * SPLIT_WINDOW > 48 * 1024) {
+    cudaFuncSetAttribute(split_window_kernel<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(split_cross_kernel<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  }
+  split_window_kernel<T, MODE><<<(n_slots + SPLIT_WINDOW - 1) / SPLIT_WINDOW, SPLIT_THREADS, smem, st>>>(b, task, n_slots, partial, pitch, ncol, w, hn);
+  split_cross_kernel<T, MODE><<<n_split < 148 * 8 ? n_split : 148 * 8, SPLIT_THREADS, smem, st>>>(b, split, n_split, partial, pitch, ncol, w, hn);
 }
 
 // Lanes of a group (VN elements each, whole heads, at most a warp), and how many segments each group takes: as many as leave two
