@@ -1,7 +1,7 @@
-// Budgeted sparse edge attention for sm_100a: forward, dQ pass (over queries) and dK/dV pass
-// (over the transposed graph).  Gather-only on regular rows: every query owns <= B sampled
-// in-edges, so one lane group streams them with 16-byte loads and keeps the running
-// numerator / normaliser in registers.  Rows longer than BF_LONG_ROW (the Graphormer virtual node,
+// Budgeted sparse edge attention for sm_100a: forward, dK/dV pass (over the transposed graph) and
+// dQ pass (over queries), each in two forms that a rule on size, type and shape chooses between.
+// Gather-only on regular rows: every query owns <= B sampled in-edges, so one lane group streams
+// them and keeps the running numerator / normaliser in registers.  Rows longer than BF_LONG_ROW (the Graphormer virtual node,
 // hubs of a graph without a budget, popular keys in the transposed graph) are cut into work items of
 // BF_LONG_CHUNK edges, one warp each, whose fp32 partial sums are added in a fixed order by two small
 // kernels: no atomics, bit-reproducible.  (The gradient of the edge-type table, a sum over all edges, does meet in atomics, one
@@ -343,11 +343,13 @@ __global__ void __launch_bounds__(256) edge_attn_fwd_rows_kernel(AttnArgs a) {
 // into a shared-memory ring kRing - 1 steps ahead of the arithmetic, across segment ends: a short segment costs no latency of
 // its own, and the gathers in flight take no registers.  A lane holds 32 bytes of a row where the head is wide enough, which
 // halves the scalar work per edge (score, exponential, cursor) against 16 bytes; the arithmetic runs in fp32 pairs.
-// Without this (two 16-byte gathers a step in registers, one row per lane group) issue slots and latency, not memory, bounded
-// the kernels: DRAM stood at 35-42 %, now 46 % (forward) and 56 % (dK/dV).  2.9 M nodes, 15.3 M edges, 8 heads x 16 bf16, us, before
-// and now: forward 2060 / 1460, dK/dV 3470 / 2680, dQ 2200 / 860 and 250 for the row terms; 612 k nodes, 8.8 M edges, 8 x 32 with
-// dropout: 1370 / 1220, 2610 / 2230, 1500 / 690; typed (392 k nodes, 9.1 M edges): 1370 / 1360, 4560 / 3130, 5440 / 1560.
-// Six blocks an SM in the forward pass instead of four: 17 % slower; two in the dK/dV pass instead of three: 15 %.
+// Without this (two 16-byte gathers a step in registers, one row per lane group) issue slots and latency, not memory, bound the
+// kernels where the rows come from DRAM: it stood at 36 (forward), 40 (dK/dV) and 42 % (dQ), now 46 and 56 %, and 37 % in a dQ that gathers
+// half the rows and is bound by issue.  2.9 M nodes, 15.3 M edges, 8 heads x 16 bf16, us, without and with streams: forward 2060 / 1460,
+// dK/dV 3470 / 2680, dQ 2200 / 860 and 250 for the row terms; 612 k nodes, 8.8 M edges, 8 x 32 with dropout: 1370 / 1220, 2610 / 2230,
+// 1500 / 690; typed (392 k nodes, 9.1 M edges): dK/dV 4560 / 3190, dQ 5440 / 1490.  Where the rows stay in L2 the picture turns: see
+// rows_forward and recomputed_backward.  Six blocks an SM in the forward pass instead of four: 17 % slower; two in the dK/dV pass instead
+// of three: 15 %.
 // ---------------------------------------------------------------------------------------------
 constexpr int kRing = 4;
 constexpr int kStreamThreads = 128;
