@@ -126,7 +126,7 @@ typedef struct {
   // sequence-parallel ranks split between them.  row_count == 0 builds all n queries.
   int row_begin, row_count;
   // Optional list of the queries whose in-edge row is longer than BF_BUILD_HUB_DEGREE (ascending ids, n_hub of them) and
-  // scratch of 32 * n_hub 64-bit words: those rows are ranked by one thread block each before the row-per-lane-group
+  // scratch of 32 * n_hub 64-bit words: those rows are ranked by a cluster of thread blocks each before the row-per-thread
   // kernel runs, which then reads the ranked list instead of streaming the row.  Same rows out either way; queries
   // missing from the list are streamed as before.
   const int* hub_rows;

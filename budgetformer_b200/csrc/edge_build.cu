@@ -1,13 +1,21 @@
-// Per-epoch attention-graph construction on the GPU: one warp per query node.
-//   1. real edges: stream the query's in-edge row, keep the b_real smallest (hash, src) in a
-//      lane-distributed sorted list (ballot + shuffle insertion; no global sort);
-//   2. random walks: lane w runs walk w (Philox counter RNG, dead ends stay), the W*L candidates are
-//      ranked into a second lane-distributed list of size b_rw;
-//   3. merge: sorted unique union by key id (Exphormer: typed concatenation + self loop) written to a
-//      fixed-width row [cap] plus a count; ell_to_csr compacts rows after a prefix sum.
+// Per-epoch attention-graph construction on the GPU: one thread per query node.
+//   1. real edges: the thread streams the query's in-edge row and keeps the smallest (hash, src) in a sorted register list;
+//      rows of more than kWideRow edges are ranked by the whole warp, rows of more than BF_BUILD_HUB_DEGREE by a cluster of
+//      blocks ahead of this kernel (no global sort);
+//   2. random walks: the same thread runs the query's walks two at a time (Philox counter RNG, dead ends stay) and ranks the
+//      W*L candidates into a second list;
+//   3. merge: sorted unique union by key id (Exphormer: typed concatenation + self loop), staged in shared memory and
+//      written as a fixed-width row [cap] plus a count; ell_to_csr compacts rows after a prefix sum.
 // Replaces the reference's argsort / scatter_reduce rounds / coalesce pipeline
 // (utils/fullgraph_sp_support.py:975-1192, gt_sp/utils.py:1198-1248, :877-887) and is bit-identical
 // to cpu/edge_builder.cpp and graph/builder_spec.py.
+//
+// What bounds it: instructions.  A row holds some 5 real candidates and W*L walk candidates, each a hash, a 10-round Philox and an
+// insertion of a few dozen instructions on one query's own data; with a group of lanes per query most lanes of those steps idle.
+// Selection, us, before (eight lanes, above budgets of 8 a warp per query) and now: 2.9 M nodes, 4 + 4, walks 2 x 4: 1471 / 224; 612 k nodes
+// of some 50 in-edges, 8 + 8, 4 x 6: 1135 / 338; 392 k nodes of 170, 16 + 16: 1452 / 287; 1 M nodes, 3 + 11, 6 x 8: 4122 / 659; 5 k nodes 9.0 / 8.7
+// (the walks' chain of reads).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -16,75 +24,66 @@
 
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr uint64_t kInf = ~0ull;
+constexpr uint32_t kNone = ~0u;               // no node: ids are below 2^31
+constexpr unsigned kAll = 0xffffffffu;
 
-// Lane groups: WIDTH lanes (8 or 32) cooperate on one query.  Every *_sync primitive names only the group's lanes,
-// so groups of one warp may diverge from each other (different degrees, different insertion counts).
-template <int WIDTH> __device__ __forceinline__ unsigned group_mask(int lane) {
-  return WIDTH == 32 ? 0xffffffffu : (((1u << WIDTH) - 1u) << (lane & ~(WIDTH - 1)));
-}
-template <int WIDTH> __device__ __forceinline__ unsigned group_ballot(unsigned gm, int lane, bool pred) {
-  const unsigned b = __ballot_sync(gm, pred);
-  return WIDTH == 32 ? b : ((b >> (lane & ~(WIDTH - 1))) & ((1u << WIDTH) - 1u));
-}
-
-// Insert every candidate (valid, comp) held by the group's lanes into the sorted lane-distributed list
-// (lane i of the group holds the i-th smallest composite; K <= WIDTH).
-template <int WIDTH>
-__device__ __forceinline__ void group_insert(uint64_t& list, int K, bool valid, uint64_t comp, int gl, unsigned gm, int lane) {
-  const unsigned kmask = K >= 32 ? 0xffffffffu : ((1u << K) - 1u);
-  for (int guard = 0; guard <= WIDTH; ++guard) {
-    const uint64_t kth = __shfl_sync(gm, list, K - 1, WIDTH);
-    const unsigned ball = group_ballot<WIDTH>(gm, lane, valid && comp < kth);
+// Insert the warp's candidates (valid, comp) into the sorted list that lane i holds the i-th smallest composite of (k <= 32).
+__device__ __forceinline__ void warp_insert(uint64_t& list, int k, bool valid, uint64_t comp, int lane) {
+  const unsigned kmask = k >= 32 ? kAll : ((1u << k) - 1u);
+  for (int guard = 0; guard <= 32; ++guard) {
+    const uint64_t kth = __shfl_sync(kAll, list, k - 1);
+    const unsigned ball = __ballot_sync(kAll, valid && comp < kth);
     if (ball == 0) break;
     const int src_lane = __ffs(ball) - 1;
-    const uint64_t c = __shfl_sync(gm, comp, src_lane, WIDTH);
-    const unsigned le = group_ballot<WIDTH>(gm, lane, list <= c) & kmask;
-    const int p = __popc(le);
-    const uint64_t up = __shfl_up_sync(gm, list, 1, WIDTH);
-    if (gl == p) list = c;
-    else if (gl > p && gl < K) list = up;
-    if (gl == src_lane) valid = false;
+    const uint64_t c = __shfl_sync(kAll, comp, src_lane);
+    const int p = __popc(__ballot_sync(kAll, list <= c) & kmask);
+    const uint64_t up = __shfl_up_sync(kAll, list, 1);
+    if (lane == p) list = c;
+    else if (lane > p && lane < k) list = up;
+    if (lane == src_lane) valid = false;
   }
 }
 
-// Keep the WIDTH smallest of the sorted list and one candidate per lane (kInf: none).  A bitonic sort of the candidates and one
-// bitonic merge: the same instructions for every group of the warp, where insertion takes a round per candidate and the groups'
-// rounds follow one another.  With eight lanes that is 10 exchanges; a full warp would need 21, and rows that long mostly carry
-// few candidates that still matter, so the 32-lane kernels insert (group_take).
-template <int WIDTH>
-__device__ __forceinline__ uint64_t exchange(uint64_t v, int j, bool want_min, unsigned gm) {
-  const uint64_t o = __shfl_xor_sync(gm, v, j);
-  return ((o < v) == want_min) ? o : v;
+// Composites below this hold the `want` smallest of `deg` candidates with room to spare, as far as their hashes are spread evenly:
+// whoever filters by it counts what is left and starts over without it where that is too little.
+__device__ __forceinline__ uint64_t rank_bound(int want, int deg) {
+  const uint64_t room = (uint64_t)(want + 4 * (int)ceilf(sqrtf((float)want)) + 4);
+  const uint64_t h = (room << 31) / (uint64_t)deg;
+  return h >= (1ull << 31) ? kInf : h << 32;
 }
-template <int WIDTH>
-__device__ __forceinline__ void group_merge(uint64_t& list, uint64_t comp, int gl, unsigned gm) {
+
+// one thread's sorted list of the K smallest composites
+template <int K> __device__ __forceinline__ void list_take(uint64_t (&list)[K], uint64_t c) {
+  if (c >= list[K - 1]) return;
+  bool below[K];
 #pragma unroll
-  for (int k = 2; k <= WIDTH; k <<= 1)
+  for (int i = 0; i < K; ++i) below[i] = c < list[i];
 #pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) comp = exchange<WIDTH>(comp, j, ((gl & j) == 0) == ((gl & k) != 0 && k < WIDTH ? false : true), gm);
-  const uint64_t rev = __shfl_sync(gm, comp, WIDTH - 1 - gl, WIDTH);
-  uint64_t v = rev < list ? rev : list;         // the WIDTH smallest of both, bitonic
-#pragma unroll
-  for (int j = WIDTH >> 1; j > 0; j >>= 1) v = exchange<WIDTH>(v, j, (gl & j) == 0, gm);
-  list = v;
+  for (int i = K - 1; i > 0; --i) list[i] = below[i - 1] ? list[i - 1] : (below[i] ? c : list[i]);
+  list[0] = below[0] ? c : list[0];
 }
-// candidates (valid, comp) of the group's lanes into the list
-template <int WIDTH>
-__device__ __forceinline__ void group_take(uint64_t& list, int K, bool valid, uint64_t comp, int gl, unsigned gm, int lane) {
-  if (WIDTH == 8) {
-    const uint64_t kth = __shfl_sync(gm, list, K - 1, WIDTH);
-    if (group_ballot<WIDTH>(gm, lane, valid && comp < kth) != 0) group_merge<WIDTH>(list, valid ? comp : kInf, gl, gm);
-  } else {
-    group_insert<WIDTH>(list, K, valid, comp, gl, gm, lane);
-  }
+
+// ascending sort of N values in registers: Batcher's odd-even merge sort (Knuth, The Art of Computer Programming 3, 5.2.2)
+template <int N, int P, int D> __device__ __forceinline__ void sort_pass(uint32_t (&x)[N]) {
+#pragma unroll
+  for (int i = 0; i + D < N; ++i)
+    if (i >= D % P && (i - D % P) / D % 2 == 0 && i / (2 * P) == (i + D) / (2 * P)) {
+      const uint32_t lo = min(x[i], x[i + D]), hi = max(x[i], x[i + D]);
+      x[i] = lo; x[i + D] = hi;
+    }
+  if constexpr (D > 1) sort_pass<N, P, D / 2>(x);
+  else if constexpr (2 * P < N) sort_pass<N, 2 * P, 2 * P>(x);
 }
+template <int N> __device__ __forceinline__ void sort_values(uint32_t (&x)[N]) { sort_pass<N, 1, 1>(x); }
 
 struct BuildArgs {
   const int *in_rowptr, *in_src, *out_rowptr, *out_col;
   int n;
   int row_begin;       // first query of this launch; rows are stored at index (query - row_begin)
-  int b_real, b_rw, walks, walk_len, exphormer;
+  int b_real, b_rw, walks, walk_len;
   long long seed;
   int cap;
   int* ell_col;        // [n, cap]
@@ -96,163 +95,266 @@ struct BuildArgs {
   unsigned long long* hub_top; // [n_hub, 32] ranked real candidates of those queries
 };
 
-// Real-edge ranking of the long rows: one block per listed query.  Each warp keeps the b_real smallest composites of
-// its share of the row (chunks of 32 edges, strided by the block), warp 0 merges the eight lists.  The b_real smallest
-// of a multiset do not depend on the order of insertion, so the result equals the single stream of the main kernel.
-__global__ void __launch_bounds__(256) budget_hub_topk_kernel(BuildArgs a) {
-  __shared__ uint64_t s_list[8][32];
-  const int row = a.hub_rows[blockIdx.x];
+// Real-edge ranking of the longest rows: a cluster of eight blocks per listed query.  Each of its 64 warps keeps the b_real smallest
+// composites of its share of the row that are below the row's rank_bound (about none of them), the blocks' first warps merge those
+// lists, and the first block's the eight results.  Where the bound left too few the pass is repeated without it.  The b_real smallest
+// of a multiset do not depend on the order of insertion, so the result equals the stream of one thread.
+// A row's time is the latency of its share: at 612 k nodes the longest has 10^5 edges, and one block
+// took 422 us for what a cluster does in 49 (392 k nodes, 66 M edges: 782 / 55).
+constexpr int kHubBlocks = 8, kHubWarps = 8, kHubLoads = 4;
+__global__ void __cluster_dims__(kHubBlocks, 1, 1) __launch_bounds__(kHubWarps * 32) budget_hub_topk_kernel(BuildArgs a) {
+  __shared__ uint64_t s_list[kHubWarps][32];
+  __shared__ uint64_t s_block[32];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int part = (int)cluster.block_rank();
+  const int hub = blockIdx.x / kHubBlocks;
+  const int row = a.hub_rows[hub];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool mine = row >= a.row_begin && (long long)row < (long long)a.row_begin + a.n;   // uniform over the block
-  uint64_t list = kInf;
+  const bool mine = row >= a.row_begin && (long long)row < (long long)a.row_begin + a.n;   // uniform over the cluster
   if (mine) {
     const int beg = a.in_rowptr[row], end = a.in_rowptr[row + 1];
     const int64_t rs = a.seed + BF_REAL_SEED_OFFSET;
-    for (long long base = (long long)beg + warp * 32; base < end; base += 256) {
-      const long long e = base + lane;
-      const bool valid = e < end;
-      const uint32_t s = valid ? (uint32_t)__ldg(a.in_src + e) : 0u;
-      group_insert<32>(list, a.b_real, valid, valid ? bf_edge_composite(s, (uint32_t)row, rs) : kInf, lane, 0xffffffffu, lane);
+    uint64_t bound = rank_bound(a.b_real, end - beg);
+    while (true) {
+      uint64_t list = kInf;
+      const long long step = (long long)kHubBlocks * kHubWarps * 32 * kHubLoads;
+      for (long long base = (long long)beg + (long long)(part * kHubWarps + warp) * 32 * kHubLoads; base < end; base += step) {
+        uint64_t c[kHubLoads];
+        bool any = false;
+#pragma unroll
+        for (int j = 0; j < kHubLoads; ++j) {
+          const long long e = base + j * 32 + lane;
+          c[j] = e < end ? bf_edge_composite((uint32_t)__ldg(a.in_src + e), (uint32_t)row, rs) : kInf;
+        }
+#pragma unroll
+        for (int j = 0; j < kHubLoads; ++j) any |= c[j] < bound;
+        if (__any_sync(kAll, any)) {
+#pragma unroll
+          for (int j = 0; j < kHubLoads; ++j) warp_insert(list, a.b_real, c[j] < bound, c[j], lane);
+        }
+      }
+      s_list[warp][lane] = lane < a.b_real ? list : kInf;
+      __syncthreads();
+      if (warp == 0) {
+        for (int w = 1; w < kHubWarps; ++w) {
+          const uint64_t c = s_list[w][lane];
+          warp_insert(list, a.b_real, c != kInf, c, lane);
+        }
+        s_block[lane] = lane < a.b_real ? list : kInf;
+      }
+      cluster.sync();
+      uint64_t got[kHubBlocks];                   // every block merges all eight, so that all of them see whether the pass sufficed
+      if (warp == 0) {
+#pragma unroll
+        for (int b = 0; b < kHubBlocks; ++b) got[b] = cluster.map_shared_rank(s_block, b)[lane];
+        list = kInf;
+#pragma unroll
+        for (int b = 0; b < kHubBlocks; ++b) warp_insert(list, a.b_real, got[b] != kInf, got[b], lane);
+        s_list[0][lane] = list;
+      }
+      cluster.sync();                             // also: no block leaves or starts over while another reads its list
+      if (bound == kInf || s_list[0][a.b_real - 1] != kInf) {
+        if (part == 0 && warp == 0) a.hub_top[(long long)hub * 32 + lane] = lane < a.b_real ? list : kInf;
+        break;
+      }
+      bound = kInf;
+      __syncthreads();
     }
-  }
-  s_list[warp][lane] = list;
-  __syncthreads();
-  if (warp == 0 && mine) {
-    for (int w = 1; w < 8; ++w) {
-      const uint64_t c = s_list[w][lane];
-      group_insert<32>(list, a.b_real, c != kInf, c, lane, 0xffffffffu, lane);
-    }
-    a.hub_top[(long long)blockIdx.x * 32 + lane] = list;
   }
 }
 
-template <int WIDTH>
-__global__ void __launch_bounds__(256) budget_select_kernel(BuildArgs a) {
+// Rows of more edges are ranked by the whole warp instead of their thread.  A lane that is alone with its long row holds the warp up
+// for some 50 instructions an edge; the warp takes about 20 for 32 edges and 200 for a row.
+constexpr int kWideRow = 32;
+constexpr int kPassed = 64;                       // candidates below rank_bound that the warp sorts (59 expected at most)
+constexpr int kSelectThreads = 128, kSelectWarps = kSelectThreads / 32;
+
+// The b_real smallest composites of one row, by all lanes: what passes rank_bound is collected in shared memory and ranked by
+// counting; s_top[0 .. b_real) holds them in order afterwards.
+__device__ __forceinline__ void warp_rank_row(const BuildArgs& a, uint32_t q, int beg, int end, uint64_t* s_pass, uint64_t* s_top, int lane) {
+  const int64_t rs = a.seed + BF_REAL_SEED_OFFSET;
+  const uint64_t bound = rank_bound(a.b_real, end - beg);
+  int passed = 0;
+  for (int base = beg; base < end; base += 128) {
+    uint64_t c[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int e = base + j * 32 + lane;
+      c[j] = e < end ? bf_edge_composite((uint32_t)__ldg(a.in_src + e), q, rs) : kInf;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool take = c[j] < bound;
+      const unsigned ball = __ballot_sync(kAll, take);
+      const int at = passed + __popc(ball & ((1u << lane) - 1u));
+      if (take && at < kPassed) s_pass[at] = c[j];
+      passed += __popc(ball);
+    }
+  }
+  __syncwarp();
+  if (passed >= a.b_real && passed <= kPassed) {
+    const uint64_t x0 = lane < passed ? s_pass[lane] : kInf, x1 = lane + 32 < passed ? s_pass[lane + 32] : kInf;
+    int r0 = 0, r1 = 0;
+    for (int t = 0; t < passed; ++t) {
+      const uint64_t y = s_pass[t];
+      r0 += (y < x0 || (y == x0 && t < lane)) ? 1 : 0;
+      r1 += (y < x1 || (y == x1 && t < lane + 32)) ? 1 : 0;
+    }
+    if (lane < passed && r0 < a.b_real) s_top[r0] = x0;
+    if (lane + 32 < passed && r1 < a.b_real) s_top[r1] = x1;
+  } else {                                        // hashes in lumps (repeated sources): rank all of them
+    uint64_t list = kInf;
+    for (int base = beg; base < end; base += 32) {
+      const int e = base + lane;
+      warp_insert(list, a.b_real, e < end, e < end ? bf_edge_composite((uint32_t)__ldg(a.in_src + e), q, rs) : kInf, lane);
+    }
+    if (lane < a.b_real) s_top[lane] = list;
+  }
+  __syncwarp();
+}
+
+// K: list length, the larger budget rounded up to 4, 8, 16 or 32
+template <int K, bool TYPED>
+__global__ void __launch_bounds__(kSelectThreads) budget_select_kernel(BuildArgs a) {
+  extern __shared__ int s_rows[];                 // [kSelectThreads][cap | 1]: odd pitch, lanes of a column in different banks
+  __shared__ uint64_t s_pass[kSelectWarps][kPassed], s_top[kSelectWarps][32];
   __shared__ unsigned s_tot[2];
+  __shared__ unsigned short s_cnt[kSelectThreads];
+  __shared__ uint8_t s_typed[TYPED ? kSelectThreads : 1][2];   // real and walk edges of a row
   if (threadIdx.x < 2) s_tot[threadIdx.x] = 0;
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int gl = lane & (WIDTH - 1);                       // lane inside the group
-  const unsigned gm = group_mask<WIDTH>(lane);
-  const long long slot = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / WIDTH;   // row of the output
-  const long long v = slot + a.row_begin;                                              // query node
-  if (slot < a.n) {
-    const uint32_t q = (uint32_t)v;
-    // ---- real edges ----
-    uint64_t rlist = kInf;
-    int r_cnt = 0;
-    if (a.b_real > 0) {
-      const int beg = a.in_rowptr[v], end = a.in_rowptr[v + 1];
-      const int64_t rs = a.seed + BF_REAL_SEED_OFFSET;
-      int hub = -1;
-      if (a.n_hub > 0 && end - beg > BF_BUILD_HUB_DEGREE) {   // ranked by budget_hub_topk_kernel if the caller listed it
-        int lo = 0, hi = a.n_hub - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (a.hub_rows[mid] < (int)v) lo = mid + 1; else hi = mid;
-        }
-        if (a.hub_rows[lo] == (int)v) hub = lo;
-      }
-      if (hub >= 0) {
-        rlist = gl < a.b_real ? (uint64_t)a.hub_top[(long long)hub * 32 + gl] : kInf;
-      } else {
-        for (int base = beg; base < end; base += WIDTH) {
-          const int e = base + gl;
-          const bool valid = e < end;
-          const uint32_t s = valid ? (uint32_t)__ldg(a.in_src + e) : 0u;
-          group_take<WIDTH>(rlist, a.b_real, valid, valid ? bf_edge_composite(s, q, rs) : kInf, gl, gm, lane);
-        }
-      }
-      r_cnt = min(end - beg, a.b_real);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long slot = (long long)blockIdx.x * kSelectThreads + threadIdx.x;         // row of the output
+  const bool live = slot < a.n;
+  const int v = live ? (int)(slot + a.row_begin) : 0;                                  // query node
+  const uint32_t q = (uint32_t)v;
+  uint64_t list[K];
+#pragma unroll
+  for (int i = 0; i < K; ++i) list[i] = kInf;
+  // ---- real edges ----
+  int beg = 0, deg = 0, hub = -1;
+  if (live && a.b_real > 0) { beg = a.in_rowptr[v]; deg = a.in_rowptr[v + 1] - beg; }
+  const int r_cnt = min(deg, a.b_real);
+  if (a.n_hub > 0 && deg > BF_BUILD_HUB_DEGREE) {         // ranked by budget_hub_topk_kernel if the caller listed it
+    int lo = 0, hi = a.n_hub - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (a.hub_rows[mid] < v) lo = mid + 1; else hi = mid;
     }
-    // ---- random walks ----
-    uint64_t wlist = kInf;
-    int w_cnt = 0;
-    if (a.b_rw > 0 && a.walks > 0 && a.walk_len > 0) {
-      const int64_t ws = a.seed + BF_RW_SEED_OFFSET;
-      int n_cand = 0;
-      // with fewer walks than half the lanes, the candidates of several steps are collected before they are ranked: lane
-      // t * walks + w takes walk w's candidate of step t
-      const int batch = WIDTH == 8 ? max(1, min(a.walk_len, WIDTH / a.walks)) : 1;
-      for (int wbase = 0; wbase < a.walks; wbase += WIDTH) {
-        const int w = wbase + gl;
-        const bool active = w < a.walks;
-        const uint64_t walk_id = (uint64_t)v * (uint64_t)a.walks + (uint64_t)w;
-        const int slot_step = batch > 1 ? gl / a.walks : 0, slot_lane = batch > 1 ? gl - slot_step * a.walks : gl;
-        uint64_t held = kInf;
-        int cur = (int)v, prev = (int)v, in_batch = 0;
-        for (int d = 1; d <= a.walk_len; ++d) {
-          bool emit = false;
-          if (active) {
-            const int ob = a.out_rowptr[cur], oe = a.out_rowptr[cur + 1];
-            const uint32_t deg = (uint32_t)(oe - ob);
-            prev = cur;
-            if (deg > 0) {
-              const uint32_t r = bf_walk_uniform32(walk_id, (uint32_t)d, (uint64_t)a.seed);
-              cur = __ldg(a.out_col + ob + (int)bf_mulhi32(r, deg));
-            }
-            emit = (d == 1) || (cur != prev);
+    if (a.hub_rows[lo] == v) hub = lo;
+  }
+  if (hub >= 0) {
+#pragma unroll
+    for (int i = 0; i < K; ++i)
+      if (i < a.b_real) list[i] = (uint64_t)a.hub_top[(long long)hub * 32 + i];
+  }
+  const bool wide = deg > kWideRow && hub < 0;
+  if (!wide && hub < 0) {
+    const int64_t rs = a.seed + BF_REAL_SEED_OFFSET;
+    for (int e = 0; e < deg; e += 4) {
+      uint32_t src[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) src[j] = e + j < deg ? (uint32_t)__ldg(a.in_src + beg + e + j) : kNone;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (src[j] != kNone) list_take<K>(list, bf_edge_composite(src[j], q, rs));
+    }
+  }
+  __syncwarp();
+  unsigned left = __ballot_sync(kAll, wide);
+  while (left != 0) {
+    const int owner = __ffs(left) - 1;
+    left &= left - 1;
+    const int b = __shfl_sync(kAll, beg, owner), d = __shfl_sync(kAll, deg, owner), row = __shfl_sync(kAll, v, owner);
+    warp_rank_row(a, (uint32_t)row, b, b + d, s_pass[warp], s_top[warp], lane);
+    if (lane == owner) {
+#pragma unroll
+      for (int i = 0; i < K; ++i)
+        if (i < a.b_real) list[i] = s_top[warp][i];
+    }
+    __syncwarp();
+  }
+  uint32_t id[2 * K];
+#pragma unroll
+  for (int i = 0; i < K; ++i) { id[i] = i < r_cnt ? (uint32_t)list[i] : kNone; list[i] = kInf; }
+  // ---- random walks, two at a time so that their dependent reads overlap ----
+  int w_cnt = 0;
+  if (live && a.b_rw > 0 && a.walks > 0 && a.walk_len > 0) {
+    const int64_t ws = a.seed + BF_RW_SEED_OFFSET;
+    for (int w = 0; w < a.walks; w += 2) {
+      const uint64_t walk_id = (uint64_t)v * (uint64_t)a.walks + (uint64_t)w;
+      int cur[2] = {v, v};
+      const bool second = w + 1 < a.walks;
+      for (int d = 1; d <= a.walk_len; ++d) {
+        int ob[2], oe[2], next[2];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) { ob[t] = a.out_rowptr[cur[t]]; oe[t] = a.out_rowptr[cur[t] + 1]; }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const uint32_t n_out = (uint32_t)(oe[t] - ob[t]);
+          next[t] = cur[t];
+          if (n_out > 0)
+            next[t] = __ldg(a.out_col + ob[t] + (int)bf_mulhi32(bf_walk_uniform32(walk_id + t, (uint32_t)d, (uint64_t)a.seed), n_out));
+        }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if ((t == 0 || second) && (d == 1 || next[t] != cur[t])) {
+            ++w_cnt;
+            list_take<K>(list, bf_edge_composite((uint32_t)next[t], q, ws));
           }
-          n_cand += __popc(group_ballot<WIDTH>(gm, lane, emit));
-          uint64_t comp = emit ? bf_edge_composite((uint32_t)cur, q, ws) : kInf;
-          if (batch > 1) {
-            comp = __shfl_sync(gm, comp, slot_lane, WIDTH);
-            if (slot_step == in_batch) held = comp;
-            if (++in_batch == batch || d == a.walk_len) {
-              group_take<WIDTH>(wlist, a.b_rw, held != kInf, held, gl, gm, lane);
-              held = kInf;
-              in_batch = 0;
-            }
-          } else {
-            group_take<WIDTH>(wlist, a.b_rw, emit, comp, gl, gm, lane);
-          }
+          cur[t] = next[t];
         }
       }
-      w_cnt = min(n_cand, a.b_rw);
     }
-    // ---- merge ----
-    const bool has_r = gl < r_cnt, has_w = gl < w_cnt;
-    const uint32_t sr = (uint32_t)rlist, sw = (uint32_t)wlist;
-    int* row = a.ell_col + slot * a.cap;
-    if (a.exphormer) {
-      int rank_r = 0, rank_w = 0;
-      for (int t = 0; t < WIDTH; ++t) {
-        const uint32_t yr = __shfl_sync(gm, sr, t, WIDTH);
-        const uint32_t yw = __shfl_sync(gm, sw, t, WIDTH);
-        if (t < r_cnt && (yr < sr || (yr == sr && t < gl))) ++rank_r;
-        if (t < w_cnt && (yw < sw || (yw == sw && t < gl))) ++rank_w;
-      }
-      uint8_t* trow = a.ell_type + slot * a.cap;
-      if (has_r) { row[rank_r] = (int)sr; trow[rank_r] = 0; }
-      if (has_w) { row[r_cnt + rank_w] = (int)sw; trow[r_cnt + rank_w] = 1; }
-      if (gl == 0) { row[r_cnt + w_cnt] = (int)v; trow[r_cnt + w_cnt] = 0; a.ell_cnt[slot] = r_cnt + w_cnt + 1; }
-    } else {
-      bool dup_r = false, dup_w = false;
-      for (int t = 0; t < WIDTH; ++t) {
-        const uint32_t yr = __shfl_sync(gm, sr, t, WIDTH);
-        const uint32_t yw = __shfl_sync(gm, sw, t, WIDTH);
-        if (t < r_cnt && t < gl && yr == sr) dup_r = true;
-        if (t < r_cnt && yr == sw) dup_w = true;
-        if (t < w_cnt && t < gl && yw == sw) dup_w = true;
-      }
-      const bool keep_r = has_r && !dup_r, keep_w = has_w && !dup_w;
-      int rank_r = 0, rank_w = 0;
-      for (int t = 0; t < WIDTH; ++t) {
-        const uint32_t yr = __shfl_sync(gm, sr, t, WIDTH);
-        const uint32_t yw = __shfl_sync(gm, sw, t, WIDTH);
-        const bool kr = __shfl_sync(gm, (int)keep_r, t, WIDTH) != 0;
-        const bool kw = __shfl_sync(gm, (int)keep_w, t, WIDTH) != 0;
-        if (kr && yr < sr) ++rank_r;
-        if (kw && yw < sr) ++rank_r;
-        if (kr && yr < sw) ++rank_w;
-        if (kw && yw < sw) ++rank_w;
-      }
-      if (keep_r) row[rank_r] = (int)sr;
-      if (keep_w) row[rank_w] = (int)sw;
-      const int total = __popc(group_ballot<WIDTH>(gm, lane, keep_r)) + __popc(group_ballot<WIDTH>(gm, lane, keep_w));
-      if (gl == 0) a.ell_cnt[slot] = total;
+    w_cnt = min(w_cnt, a.b_rw);
+  }
+#pragma unroll
+  for (int i = 0; i < K; ++i) id[K + i] = i < w_cnt ? (uint32_t)list[i] : kNone;
+  // ---- merge ----
+  const int pitch = a.cap | 1;
+  int* row = s_rows + threadIdx.x * pitch;
+  int total = 0;
+  if (TYPED) {
+    uint32_t side[K];
+#pragma unroll
+    for (int i = 0; i < K; ++i) side[i] = id[i];
+    sort_values<K>(side);
+#pragma unroll
+    for (int i = 0; i < K; ++i)
+      if (i < r_cnt) row[i] = (int)side[i];
+#pragma unroll
+    for (int i = 0; i < K; ++i) side[i] = id[K + i];
+    sort_values<K>(side);
+#pragma unroll
+    for (int i = 0; i < K; ++i)
+      if (i < w_cnt) row[r_cnt + i] = (int)side[i];
+    row[r_cnt + w_cnt] = v;
+    total = r_cnt + w_cnt + 1;
+    s_typed[threadIdx.x][0] = (uint8_t)r_cnt;
+    s_typed[threadIdx.x][1] = (uint8_t)w_cnt;
+  } else {
+    sort_values<2 * K>(id);
+    uint32_t prev = kNone;
+#pragma unroll
+    for (int i = 0; i < 2 * K; ++i) {
+      if (id[i] != kNone && id[i] != prev) row[total++] = (int)id[i];
+      prev = id[i];
     }
-    if (gl == 0) { atomicAdd(&s_tot[0], (unsigned)r_cnt); atomicAdd(&s_tot[1], (unsigned)w_cnt); }
+  }
+  if (live) a.ell_cnt[slot] = total;
+  s_cnt[threadIdx.x] = (unsigned short)(live ? total : 0);
+  const unsigned sum_r = __reduce_add_sync(kAll, live ? (unsigned)r_cnt : 0u), sum_w = __reduce_add_sync(kAll, (unsigned)w_cnt);
+  if (lane == 0) { atomicAdd(&s_tot[0], sum_r); atomicAdd(&s_tot[1], sum_w); }
+  __syncwarp();
+  // ---- the warp's 32 rows are one contiguous piece of the output ----
+  const long long out0 = (slot - lane) * (long long)a.cap;
+  const unsigned inv = (1u << 20) / (unsigned)a.cap + 1u;      // i / cap for i < 32 * cap <= 2080: i * (inv * cap - 2^20) < 2^20
+  for (int i = lane; i < 32 * a.cap; i += 32) {
+    const int r = (int)(((unsigned)i * inv) >> 20), c = i - r * a.cap, at = warp * 32 + r;
+    if (c < s_cnt[at]) {
+      a.ell_col[out0 + i] = s_rows[at * pitch + c];
+      if (TYPED) a.ell_type[out0 + i] = (uint8_t)(c >= s_typed[at][0] && c < s_typed[at][0] + s_typed[at][1] ? 1 : 0);
+    }
   }
   __syncthreads();
   if (threadIdx.x < 2 && s_tot[threadIdx.x]) atomicAdd(a.totals + threadIdx.x, (unsigned long long)s_tot[threadIdx.x]);
@@ -280,20 +382,22 @@ extern "C" int bf_budget_select(const bf_build_params* p, cudaStream_t st) {
   a.n = p->row_count > 0 ? p->row_count : p->n; a.row_begin = p->row_count > 0 ? p->row_begin : 0;
   if (a.row_begin < 0 || (long long)a.row_begin + a.n > p->n) return (int)cudaErrorInvalidValue;
   a.b_real = p->b_real; a.b_rw = p->b_rw; a.walks = p->walks; a.walk_len = p->walk_len;
-  a.exphormer = p->exphormer; a.seed = p->seed; a.cap = p->cap;
+  a.seed = p->seed; a.cap = p->cap;
   a.ell_col = p->ell_col; a.ell_type = p->ell_type; a.ell_cnt = p->ell_cnt;
   a.totals = reinterpret_cast<unsigned long long*>(p->totals);
-  // eight lanes per query when both budgets and the walk count fit in eight slots, else a full warp
-  const bool narrow = p->b_real <= 8 && p->b_rw <= 8 && p->walks <= 8;
-  const int width = narrow ? 8 : 32;
-  const long long blocks = ((long long)a.n * width + 255) / 256;
+  const long long blocks = ((long long)a.n + kSelectThreads - 1) / kSelectThreads;
   const bool hubs = p->hub_rows != nullptr && p->hub_top != nullptr && p->n_hub > 0 && p->b_real > 0;
   a.hub_rows = hubs ? p->hub_rows : nullptr; a.n_hub = hubs ? p->n_hub : 0; a.hub_top = hubs ? p->hub_top : nullptr;
-  if (blocks > 0 && hubs) budget_hub_topk_kernel<<<(unsigned)p->n_hub, 256, 0, st>>>(a);
-  if (blocks > 0) {
-    if (narrow) budget_select_kernel<8><<<(unsigned)blocks, 256, 0, st>>>(a);
-    else budget_select_kernel<32><<<(unsigned)blocks, 256, 0, st>>>(a);
-  }
+  if (blocks == 0) return (int)cudaSuccess;
+  if (hubs) budget_hub_topk_kernel<<<(unsigned)p->n_hub * kHubBlocks, kHubWarps * 32, 0, st>>>(a);
+  const int most = p->b_real > p->b_rw ? p->b_real : p->b_rw;
+  const bool typed = p->exphormer != 0;
+  const size_t smem = (size_t)kSelectThreads * (size_t)(a.cap | 1) * sizeof(int);
+  auto kern = most <= 4    ? (typed ? budget_select_kernel<4, true> : budget_select_kernel<4, false>)
+              : most <= 8  ? (typed ? budget_select_kernel<8, true> : budget_select_kernel<8, false>)
+              : most <= 16 ? (typed ? budget_select_kernel<16, true> : budget_select_kernel<16, false>)
+                           : (typed ? budget_select_kernel<32, true> : budget_select_kernel<32, false>);
+  kern<<<(unsigned)blocks, kSelectThreads, smem, st>>>(a);
   return (int)cudaGetLastError();
 }
 

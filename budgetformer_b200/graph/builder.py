@@ -70,7 +70,7 @@ def build_attn_graph(
 
 
 def _long_rows(topo: Topology, ext) -> Optional[torch.Tensor]:
-    """Queries whose in-edge row the device builder ranks with a whole thread block instead of one lane group (power-law
+    """Queries whose in-edge row the device builder ranks with a cluster of thread blocks instead of one warp (power-law
     graphs have rows of 10^5 - 10^6 in-edges that would otherwise be the tail of the selection kernel).
     ``BF_BUILD_HUB_BLOCKS=0`` switches the pre-pass off (measurements)."""
     import os

@@ -230,6 +230,29 @@ def test_gpu_builder_ranks_long_rows_with_a_block_per_row(cfg, exph, monkeypatch
     assert torch.equal(plain.col, gpu.col) and torch.equal(plain.rowptr, gpu.rowptr)
 
 
+@pytest.mark.parametrize("exph", [False, True])
+@pytest.mark.parametrize("cfg", [(0, 4, 1, 1), (4, 0, 2, 4), (3, 5, 3, 5), (8, 9, 5, 7), (16, 16, 2, 16), (17, 32, 7, 6)])
+def test_gpu_builder_at_the_edges_of_its_lists(cfg, exph):
+    """List lengths 4, 8, 16 and 32, odd walk counts, a last block of one thread, and rows around the lengths at which a thread, the
+    warp and a cluster of blocks rank them; rows whose sources repeat (their hashes come in lumps, so the estimated bound lets far too
+    few or too many pass) and rows without edges."""
+    br, bw, w, l = cfg
+    g = torch.Generator().manual_seed(7)
+    n = 128 * 9 + 1
+    degs = [0, 1, 2, 31, 32, 33, 34, 63, 64, 65, 127, 128, 129, 130, 4095, 4096, 4097, 9000]
+    rows = [torch.stack([torch.randint(0, n, (d,), generator=g), torch.full((d,), 3 + 7 * i)]) for i, d in enumerate(degs)]
+    rows += [torch.stack([torch.randint(0, few, (d,), generator=g), torch.full((d,), 600 + 5 * i)])
+             for i, (few, d) in enumerate([(1, 40), (2, 100), (5, 200), (3, 4090), (1, 5000), (4, 8200), (40, 300)])]
+    rows.append(torch.randint(0, n, (2, 4000), generator=g))
+    topo = Topology.from_edge_index(torch.cat(rows, 1), n)
+    cpu = build_attn_graph(topo, br, bw, w, l, 13, exphormer=exph)
+    gpu = build_attn_graph(topo.to("cuda"), br, bw, w, l, 13, exphormer=exph)
+    assert torch.equal(cpu.rowptr, gpu.rowptr.cpu()) and torch.equal(cpu.col, gpu.col.cpu())
+    if exph:
+        assert torch.equal(cpu.etype, gpu.etype.cpu())
+    assert cpu._totals.tolist() == gpu._totals.cpu().tolist()
+
+
 def test_gpu_builder_seed_changes_graph_and_is_reproducible():
     topo, _ = random_topology(500, 5000, seed=2)
     t = topo.to("cuda")
