@@ -139,6 +139,8 @@ typedef struct {
 int bf_budget_select(const bf_build_params* p, cudaStream_t st);
 int bf_ell_to_csr(const int* ell_col, const uint8_t* ell_type, const int* rowptr, int n, int cap, int* col,
                   uint8_t* etype, cudaStream_t st);
+size_t bf_count_offsets_scratch(int n);
+int bf_count_offsets(const int* counts, int n, int* rowptr, void* scratch, size_t scratch_bytes, cudaStream_t st);
 
 // ---- feed-forward block with the hidden tile kept on chip (ffn_fused_tcgen05.cu) ----------------
 typedef struct {

@@ -244,6 +244,16 @@ Tensor attach_hub_rows(bf_build_params& p, const OptTensor& hub_rows, const Tens
   return top;
 }
 
+// rowptr [n + 1] of the first n counts on the current stream
+Tensor count_offsets(const Tensor& counts, int64_t n) {
+  Tensor rowptr = torch::empty({n + 1}, counts.options());
+  const size_t bytes = bf_count_offsets_scratch((int)n);
+  Tensor scratch = torch::empty({(int64_t)bytes}, counts.options().dtype(torch::kUInt8));
+  check_cuda(bf_count_offsets(counts.data_ptr<int>(), (int)n, rowptr.data_ptr<int>(), scratch.data_ptr(), bytes,
+                              at::cuda::getCurrentCUDAStream()), "count_offsets");
+  return rowptr;
+}
+
 std::vector<Tensor> build_attn_graph(Tensor in_rowptr, Tensor in_src, Tensor out_rowptr, Tensor out_col, int64_t n,
                                      int64_t b_real, int64_t b_rw, int64_t walks, int64_t walk_len, bool exphormer,
                                      int64_t seed, int64_t num_threads, OptTensor hub_rows) {
@@ -255,9 +265,9 @@ std::vector<Tensor> build_attn_graph(Tensor in_rowptr, Tensor in_src, Tensor out
   auto iopt = in_src.options();
   Tensor ell_col = torch::empty({n, std::max(cap, 1)}, iopt);
   Tensor ell_type = exphormer ? torch::empty({n, std::max(cap, 1)}, iopt.dtype(torch::kUInt8)) : Tensor();
-  Tensor ell_cnt = torch::zeros({n}, iopt);
-  Tensor totals = torch::zeros({2}, iopt.dtype(torch::kLong));
   const bool cuda = in_src.is_cuda();
+  Tensor ell_cnt = cuda ? torch::empty({n}, iopt) : torch::zeros({n}, iopt);
+  Tensor totals = torch::zeros({2}, iopt.dtype(torch::kLong));
   if (cuda) {
     c10::cuda::CUDAGuard guard(in_src.device());
     bf_build_params p{};
@@ -276,8 +286,8 @@ std::vector<Tensor> build_attn_graph(Tensor in_rowptr, Tensor in_src, Tensor out
                          ell_cnt.data_ptr<int>(), reinterpret_cast<unsigned long long*>(totals.data_ptr<int64_t>()),
                          (int)num_threads);
   }
-  Tensor rowptr = torch::zeros({n + 1}, iopt);
-  rowptr.slice(0, 1).copy_(torch::cumsum(ell_cnt, 0, torch::kInt));
+  Tensor rowptr = cuda ? count_offsets(ell_cnt, n) : torch::zeros({n + 1}, iopt);
+  if (!cuda) rowptr.slice(0, 1).copy_(torch::cumsum(ell_cnt, 0, torch::kInt));
   // The edge count sizes the output; this is the one host read of the build.
   const int64_t n_edges = n > 0 ? rowptr[n].item<int64_t>() : 0;
   Tensor col = torch::empty({n_edges}, iopt);
@@ -333,8 +343,7 @@ std::vector<Tensor> ell_rows_to_csr(Tensor ell_col, Tensor ell_cnt, OptTensor el
   c10::cuda::CUDAGuard guard(ell_col.device());
   auto iopt = ell_col.options();
   const bool typed = ell_type.has_value();
-  Tensor rowptr = torch::zeros({n + 1}, iopt);
-  rowptr.slice(0, 1).copy_(torch::cumsum(ell_cnt.slice(0, 0, n), 0, torch::kInt));
+  Tensor rowptr = count_offsets(ell_cnt, n);
   const int64_t n_edges = n > 0 ? rowptr[n].item<int64_t>() : 0;
   Tensor col = torch::empty({n_edges}, iopt);
   Tensor etype = typed ? torch::empty({n_edges}, iopt.dtype(torch::kUInt8)) : torch::empty({0}, iopt.dtype(torch::kUInt8));
