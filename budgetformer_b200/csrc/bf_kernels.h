@@ -210,7 +210,14 @@ typedef struct {
   long long src_ld;
   void* a_copy;                     // optional local [M, K] matrix (row stride ld_copy) that receives the gathered operand
   long long ld_copy;
+  // Second output of a GELU product: the pre-activation, rounded to the operands' type ([M, ldz]); the activation is taken of the
+  // rounded value.  One local 16-bit destination, act 2.
+  void* z_out;
+  long long ldz;
 } bf_gemm_params;
+
+// the products of gemm_rows_tcgen05.cu (cudaErrorNotSupported: not one of them); bf_gemm_tn asks here first
+int bf_gemm_rows(const bf_gemm_params* p, cudaStream_t st);
 
 int bf_gemm_supported(int M, int N, int K);
 int bf_gemm_tn(const bf_gemm_params* p, cudaStream_t st);

@@ -458,7 +458,7 @@ std::vector<Tensor> graph_transpose(Tensor rowptr, Tensor col, int64_t n, int64_
 // C = A * W^T with fused epilogue.  `dst_ptrs` holds one device pointer per destination (1 = plain output).
 void gemm_tn(Tensor A, Tensor W, OptTensor bias, int64_t act, double dropout_p, int64_t seed, OptTensor residual,
              OptTensor relu_mask, double out_scale, bool out_fp32, std::vector<int64_t> dst_ptrs, int64_t dst_row_offset,
-             int64_t ldc, Tensor status, OptTensor relu_bits_out, OptTensor relu_bits_in, int64_t mask_mode) {
+             int64_t ldc, Tensor status, OptTensor relu_bits_out, OptTensor relu_bits_in, int64_t mask_mode, OptTensor z_out = {}) {
   TORCH_CHECK(A.is_cuda() && W.is_cuda() && A.dim() == 2 && W.dim() == 2, "gemm_tn: A [M,K], W [N,K] on CUDA");
   TORCH_CHECK(A.scalar_type() == W.scalar_type() && (A.scalar_type() == torch::kBFloat16 || A.scalar_type() == torch::kHalf),
               "gemm_tn: bf16/fp16 operands");
@@ -498,6 +498,12 @@ void gemm_tn(Tensor A, Tensor W, OptTensor bias, int64_t act, double dropout_p, 
     p.relu_mask = relu_mask->data_ptr(); p.ldm = relu_mask->stride(0);
     TORCH_CHECK(mask_mode == 0 || mask_mode == 1, "gemm_tn: mask_mode 0 (ReLU gradient) or 1 (GELU gradient)");
     p.mask_mode = (int)mask_mode;
+  }
+  if (z_out.has_value()) {
+    TORCH_CHECK(act == 2 && bias.has_value() && z_out->is_cuda() && z_out->scalar_type() == A.scalar_type() && z_out->dim() == 2 &&
+                z_out->stride(1) == 1 && z_out->size(0) == p.M && z_out->size(1) == p.N && (z_out->stride(0) * 2) % 16 == 0 &&
+                ((uintptr_t)z_out->data_ptr()) % 16 == 0, "gemm_tn: z_out [M, N] in the operands' type, of a GELU product with a bias");
+    p.z_out = z_out->data_ptr(); p.ldz = z_out->stride(0);
   }
   p.out_scale = (float)out_scale; p.out_fp32 = out_fp32 ? 1 : 0;
   p.n_dest = (int)dst_ptrs.size(); p.dst_row_offset = dst_row_offset; p.ldc = ldc;
@@ -864,6 +870,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("build_attn_graph_rows_cpu", &build_attn_graph_rows_cpu);
   m.def("graph_transpose", &graph_transpose, unlocked());
   m.def("gemm_tn", &gemm_tn);
+  m.def("gemm_tn", [](Tensor A, Tensor W, OptTensor bias, int64_t act, double dropout_p, int64_t seed, OptTensor residual,
+                      OptTensor relu_mask, double out_scale, bool out_fp32, std::vector<int64_t> dst_ptrs, int64_t dst_row_offset,
+                      int64_t ldc, Tensor status, OptTensor relu_bits_out, OptTensor relu_bits_in, int64_t mask_mode) {
+    gemm_tn(A, W, bias, act, dropout_p, seed, residual, relu_mask, out_scale, out_fp32, dst_ptrs, dst_row_offset, ldc, status,
+            relu_bits_out, relu_bits_in, mask_mode);
+  });
   m.def("gemm_tn_pull", &gemm_tn_pull);
   m.def("gemm_dw", &gemm_dw);
   m.def("ffn_fused_fwd", &ffn_fused_fwd);

@@ -2,6 +2,9 @@
 //
 //   C[M, N] = A[M, K] * B[N, K]^T      bf16 / fp16 operands, fp32 accumulation in tensor memory
 //
+// It takes the products that gemm_rows_tcgen05.cu does not: several destinations, a gathered operand, fp32 output, a 16-bit ReLU mask
+// and rare combinations of epilogue features.
+//
 // * operands are staged by TMA (cp.async.bulk.tensor, 128-byte swizzle, one 64-element K panel per
 //   stage; a ragged last panel is zero-filled) into a 3- or 4-deep shared-memory ring; one elected thread
 //   issues tcgen05.mma (M = 128, N = BLOCK_N <= 256, K = 16 per instruction) and releases ring stages with
@@ -15,8 +18,8 @@
 //   all-to-all (3 projections + 3 all-to-alls + 6 copies in the reference: gt_sp/layer.py:35-41,264-266)
 //   executed by the GEMM itself, tile by tile, over NVLink - one bulk store per destination slice of a row
 //   tile (plain 32-byte st.global only when a slice is not a multiple of 16 columns);
-// * the epilogue feature set is a template parameter for the combinations the layers use (bf16), a generic
-//   instance covers everything else;
+// * the epilogue feature set is a template parameter for the pushes and the gathered projection, a generic instance covers everything
+//   else;
 // * with `n_src > 1` the A operand itself is gathered over NVLink: columns [s*K/n_src, (s+1)*K/n_src) of a row
 //   tile are this rank's rows of source s's buffer (the heads->nodes all-to-all of gt_sp/layer.py:280 and its
 //   backward twin).  One loader warp per ring stage fetches them with 16-byte asynchronous copies (cp.async from the
@@ -648,6 +651,9 @@ extern "C" int bf_gemm_tn(const bf_gemm_params* p, cudaStream_t st) {
   if (p->n_dest > 1 && cols_per_dest % 16 != 0) return (int)cudaErrorInvalidValue;
   if ((p->ldb * 2) % 16 != 0 || ((uintptr_t)p->B) % 16 != 0) return (int)cudaErrorInvalidValue;
   if (!gathered && ((p->lda * 2) % 16 != 0 || ((uintptr_t)p->A) % 16 != 0)) return (int)cudaErrorInvalidValue;
+  if ((p->relu_bits_out || p->relu_bits_in) && p->N % 16 != 0) return (int)cudaErrorInvalidValue;
+  const int rows = bf_gemm_rows(p, st);
+  if (rows != (int)cudaErrorNotSupported || p->z_out) return rows;
   GemmArgs g;
   g.M = p->M; g.N = p->N; g.K = p->K;
   // a residual / mask tile is staged in the output buffers: 128-wide tiles leave room for three of them
@@ -735,9 +741,9 @@ extern "C" int bf_gemm_tn(const bf_gemm_params* p, cudaStream_t st) {
   }
   const size_t smem = 1024 + g.stages * stage_bytes + (size_t)g.out_bufs * out_bytes + sizeof(Control) + 64 + bias_bytes;
   g.n_groups = (g.block_n % 64 == 0) ? 4 : (g.block_n % 32 == 0) ? 2 : 1;
-  // epilogue specialisation: the combinations the model layers use on bf16; everything else takes the generic kernel
+  // The pushes of a bf16 layer without dropout, and the gathered output projection; everything else reads its features at run time.
   int epi = -1;
-  if (!g.is_fp16 && !p->out_fp32) {
+  if (!g.is_fp16 && !p->out_fp32 && g.mask_mode == 0) {
     int f = 0;
     if (p->bias) f |= EPI_BIAS;
     if (p->act == 1) f |= EPI_RELU;
@@ -748,37 +754,24 @@ extern "C" int bf_gemm_tn(const bf_gemm_params* p, cudaStream_t st) {
     if (g.out_scale != 1.f) f |= EPI_SCALE;
     if (f == 0 || f == EPI_BIAS) epi = f;
     else if ((f | EPI_DROP) == (EPI_BIAS | EPI_DROP | EPI_RES)) epi = EPI_BIAS | EPI_DROP | EPI_RES;
-    else if ((f | EPI_DROP) == (EPI_BIAS | EPI_RELU | EPI_DROP)) epi = EPI_BIAS | EPI_RELU | EPI_DROP;
-    else if ((f | EPI_SCALE) == (EPI_MASK | EPI_SCALE)) epi = EPI_MASK | EPI_SCALE;
-    else if (f == EPI_SCALE) epi = EPI_SCALE;
-    if (g.mask_mode == 1) epi = -1;                 // the GELU-gradient mask lives in the generic kernel only
   }
   using Kern = void (*)(const CUtensorMap, const CUtensorMap, const OutMaps, const CUtensorMap, const GemmArgs);
   Kern kern = gemm_tn_tcgen05_kernel<-1, false>;
   if (gathered) {
-    // gathered operand: the output projection's epilogue is specialised, the input-gradient GEMM takes the generic one
     if (epi != (EPI_BIAS | EPI_DROP | EPI_RES)) epi = -1;
     kern = epi < 0 ? (Kern)gemm_tn_tcgen05_kernel<-1, true> : (Kern)gemm_tn_tcgen05_kernel<EPI_BIAS | EPI_DROP | EPI_RES, true>;
-  } else {
-    switch (epi) {
-      case 0: kern = gemm_tn_tcgen05_kernel<0, false>; break;
-      case EPI_BIAS: kern = gemm_tn_tcgen05_kernel<EPI_BIAS, false>; break;
-      case EPI_BIAS | EPI_DROP | EPI_RES: kern = gemm_tn_tcgen05_kernel<EPI_BIAS | EPI_DROP | EPI_RES, false>; break;
-      case EPI_BIAS | EPI_RELU | EPI_DROP: kern = gemm_tn_tcgen05_kernel<EPI_BIAS | EPI_RELU | EPI_DROP, false>; break;
-      case EPI_MASK | EPI_SCALE: kern = gemm_tn_tcgen05_kernel<EPI_MASK | EPI_SCALE, false>; break;
-      case EPI_SCALE: kern = gemm_tn_tcgen05_kernel<EPI_SCALE, false>; break;
-      default: break;
-    }
+  } else if (epi == 0) {
+    kern = gemm_tn_tcgen05_kernel<0, false>;
+  } else if (epi == EPI_BIAS) {
+    kern = gemm_tn_tcgen05_kernel<EPI_BIAS, false>;
   }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   {
     // the attribute belongs to (function, device): remember it per device, not per process
     constexpr int MAX_DEV = 64;
-    static bool attr_set[MAX_DEV][10] = {};
-    const int slot = gathered ? (epi < 0 ? 8 : 9)
-                     : epi < 0 ? 0 : epi == 0 ? 1 : epi == EPI_BIAS ? 2 : epi == (EPI_BIAS | EPI_DROP | EPI_RES) ? 3
-                     : epi == (EPI_BIAS | EPI_RELU | EPI_DROP) ? 4 : epi == EPI_SCALE ? 6 : 5;
+    static bool attr_set[MAX_DEV][5] = {};
+    const int slot = gathered ? (epi < 0 ? 3 : 4) : epi == 0 ? 1 : epi == EPI_BIAS ? 2 : 0;
     if (dev < 0 || dev >= MAX_DEV || !attr_set[dev][slot]) {
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
       if (e != cudaSuccess) return (int)e;

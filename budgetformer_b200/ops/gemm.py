@@ -78,11 +78,13 @@ def gemm_tn(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = Non
             dropout_p: float = 0.0, dropout_seed: int = 0, residual: Optional[torch.Tensor] = None,
             relu_mask: Optional[torch.Tensor] = None, out_scale: float = 1.0, out: Optional[torch.Tensor] = None,
             out_dtype: Optional[torch.dtype] = None, relu_bits_out: Optional[torch.Tensor] = None,
-            relu_bits_in: Optional[torch.Tensor] = None, gelu_grad_of: Optional[torch.Tensor] = None) -> torch.Tensor:
+            relu_bits_in: Optional[torch.Tensor] = None, gelu_grad_of: Optional[torch.Tensor] = None,
+            z_out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``act(dropout(a @ w.T * out_scale + bias)) [masked] + residual`` in one kernel.  ``relu_bits_out`` (int16
     ``[N / 16, M]``) receives one bit per element (result > 0); ``relu_bits_in`` zeroes the result where its bit is clear;
     ``gelu_grad_of`` (``[M, N]`` pre-activations) multiplies the result by ``gelu'(z)`` after the dropout mask - the
-    hidden gradient of a GELU feed-forward block straight out of the GEMM."""
+    hidden gradient of a GELU feed-forward block straight out of the GEMM; ``z_out`` (``[M, N]``, with ``act="gelu"`` and a bias) receives the
+    pre-activation in its dtype, and the activation is taken of those rounded values."""
     if gelu_grad_of is not None:
         assert relu_mask is None, "one mask operand per call"
         relu_mask = gelu_grad_of
@@ -99,7 +101,7 @@ def gemm_tn(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = Non
             bias = bias.clone()
     ext.gemm_tn(a, w, bias, ACT[act], float(dropout_p), int(dropout_seed),
                 residual, relu_mask, float(out_scale), bool(fp32_out), [out.data_ptr()], 0, out.stride(0),
-                status_tensor(a.device), relu_bits_out, relu_bits_in, 1 if gelu_grad_of is not None else 0)
+                status_tensor(a.device), relu_bits_out, relu_bits_in, 1 if gelu_grad_of is not None else 0, z_out)
     _ext.count_launches(1)
     return out
 

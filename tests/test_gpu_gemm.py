@@ -73,6 +73,88 @@ def test_gemm_epilogues(act):
     gemm.check_status("cuda")
 
 
+# One panel and several, groups of panels in one and in several chunks, column groups on different blocks, weights that stay in shared
+# memory and weights that stream; ragged rows (a warp without any, one row), panels cut by N, K with a zero-filled tail.
+_ROW_SHAPES = [(1, 64, 64), (31, 16, 16), (33, 48, 72), (128, 128, 128), (129, 384, 128), (8191, 192, 64), (4097, 80, 272),
+               (2500, 320, 128), (2049, 448, 64), (40001, 128, 384), (30011, 768, 256), (20003, 256, 512), (19001, 256, 768),
+               (1500, 512, 1024), (60000, 1024, 256)]
+_ROW_EPILOGUES = ["none", "bias", "drop", "res", "bias drop", "bias res", "bias drop res", "bias relu", "bias gelu", "bias relu bits",
+                  "bias relu drop bits", "mask", "mask scale", "gelugrad", "gelugrad drop", "bias gelu z", "bias gelu drop z"]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m,n,k", _ROW_SHAPES)
+def test_gemm_row_streaming_epilogues(m, n, k, dtype):
+    """Every epilogue against fp32 products, into a view of a larger matrix whose other elements stay as they are.  One rounding to 16
+    bits (half a unit in the last of 8 or 11 places: 2^-8, 2^-11 of the value), the operands' products added up in fp32, and 2^-20 for the activations."""
+    torch.manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda").to(dtype)
+    w = (torch.randn(n, k, device="cuda") / k ** 0.5).to(dtype)
+    bias = torch.randn(n, device="cuda")
+    side = torch.randn(m, n, device="cuda").to(dtype)
+    base = a.double() @ w.double().t()
+    slack = (a.double().abs() @ w.double().abs().t() + 4) * k ** 0.5 * 2.0 ** -22 + 2.0 ** -20
+    p, seed = 0.3125, 77                                 # a float: the kernel takes its threshold from one
+    keep = gemm.hash_keep_mask(seed, m, n, p, "cuda")
+    half_ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    bits = torch.randint(-2 ** 15, 2 ** 15, (n // 16, m), device="cuda").to(torch.int16)
+    unpack = lambda b: torch.stack([(b.int() >> i) & 1 for i in range(16)], 1).reshape(n, m).t().bool()
+    for epi in _ROW_EPILOGUES:
+        f = epi.split()
+        kw, want = {}, base.clone()
+        big = torch.full((m + 2, n + 8), 7.0, device="cuda", dtype=dtype)
+        out = big[1:m + 1, :n]
+        if "scale" in f:
+            kw["out_scale"] = 1.25
+            want = want * 1.25
+        if "bias" in f:
+            want = want + bias.double()
+        z = None
+        if "z" in f:
+            z = kw["z_out"] = torch.empty(m, n, device="cuda", dtype=dtype)
+        if "relu" in f:
+            kw["act"] = "relu"
+            want = want.clamp(min=0)
+        if "gelu" in f:
+            kw["act"] = "gelu"
+        if "mask" in f:
+            kw["relu_bits_in"] = bits
+        if "bits" in f:
+            kw["relu_bits_out"] = torch.zeros_like(bits)
+        if "res" in f:
+            kw["residual"] = side
+        if "gelugrad" in f:
+            kw["gelu_grad_of"] = side
+        if "drop" in f:
+            kw.update(dropout_p=p, dropout_seed=seed)
+        gemm.gemm_tn(a, w, bias if "bias" in f else None, out=out, **kw)
+        gemm.check_status("cuda")
+        if z is not None:
+            assert ((z.double() - want).abs() <= slack + half_ulp * want.abs()).all(), epi
+            want = z.double()
+        if "gelu" in f:
+            want = torch.nn.functional.gelu(want)
+        if "drop" in f:
+            want = torch.where(keep, want / (1 - p), 0.0)
+        if "mask" in f:
+            want = torch.where(unpack(bits), want, 0.0)
+        if "gelugrad" in f:
+            x = side.double()
+            want = want * (0.5 * (1 + torch.erf(x / 2 ** 0.5)) + x * torch.exp(-x * x / 2) / (2 * torch.pi) ** 0.5)
+        if "res" in f:
+            want = want + side.double()
+        err = (out.double() - want).abs() - (2 * slack + half_ulp * want.abs() * (1 + 2.0 ** -7))
+        if dtype == torch.float16:
+            err -= 2.0 ** -25                            # half a unit of the subnormals
+        assert float(err.max()) <= 0, (epi, float(err.max()))
+        if "bits" in f:
+            got = unpack(kw["relu_bits_out"])
+            assert torch.equal(got | (want.abs() < 4 * slack), (want > 0) | (want.abs() < 4 * slack)), epi
+        edge = big.clone()
+        edge[1:m + 1, :n] = 7.0
+        assert bool((edge == 7.0).all()), epi
+
+
 def test_gemm_strided_input_rows():
     big = torch.randn(700, 3 * 128, device="cuda").bfloat16()
     a = big[:, 128:256]
