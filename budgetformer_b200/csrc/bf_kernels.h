@@ -152,7 +152,7 @@ typedef struct {
   const float* b1;                  // [ffn] fp32 or NULL
   const float* b2;                  // [hidden] fp32 or NULL
   long long M;
-  int hidden, ffn;                  // supported: 128 / 256 (bf_ffn_fused_supported)
+  int hidden, ffn;                  // supported: 128 / 256, 64 / 128 (bf_ffn_fused_supported)
   int dtype;                        // BF_BF16 or BF_FP16
   int act;                          // 1 ReLU, 2 GELU (erf)
   float dropout1, dropout2;         // on the hidden tile / on the output before the residual; masks = hash(seed, row, col)
@@ -165,6 +165,11 @@ typedef struct {
   long long ldh;
   void* relu_bits_out;              // uint16 [ffn / 16, ldmb >= M] or NULL
   long long ldmb;
+  // ... and for GELU the pre-activation, rounded to the operands' type; the activation is taken of the rounded value
+  void* z_out;                      // [M, ffn] 16-bit, row stride ldz, or NULL
+  long long ldz;
+  const void* R;                    // residual other than X (residual = 0): [M, hidden] 16-bit, row stride ldr, or NULL
+  long long ldr;
 } bf_ffn_params;
 
 int bf_ffn_fused_supported(long long M, int hidden, int ffn);

@@ -46,7 +46,7 @@ struct RowsArgs {
   int M, N, m_tiles, k_panels;
   int panels, groups, group_panels, chunk_panels;   // a group is processed in chunks (one accumulator each) of chunk_panels panels
   int n_acc, stages, resident, n_buf;
-  int is_fp16;
+  uint32_t one;                                     // 1
   const float* bias;
   uint32_t thresh, seed;
   float keep_scale, out_scale;
@@ -292,27 +292,26 @@ gemm_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         }
         if (EPI & F_GELU) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float2 x = unpack2(v[i]);
-            v[i] = pack2(gelu_erf_f32(x.x), gelu_erf_f32(x.y));
-          }
+          for (int i = 0; i < 16; ++i) v[i] = gelu2(v[i]);
         }
+        uint32_t positive = 0;                                     // one bit a result (bits_out goes with ReLU)
         if (EPI & F_DROP) {
           const f2 s = pack2(g.keep_scale, g.keep_scale);
           const uint32_t hash = hash0 + (uint32_t)(32 * h) * kHashCol;
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             float2 x = unpack2(mul2(v[i], s));
-            const bool k0 = hash_keep(hash + (uint32_t)(2 * i) * kHashCol, g.thresh, thresh_hi);
-            const bool k1 = hash_keep(hash + (uint32_t)(2 * i + 1) * kHashCol, g.thresh, thresh_hi);
-            if (EPI & F_RELU) { x.x = k0 && x.x > 0.f ? x.x : 0.f; x.y = k1 && x.y > 0.f ? x.y : 0.f; }
-            else { x.x = k0 ? x.x : 0.f; x.y = k1 ? x.y : 0.f; }
-            v[i] = pack2(x.x, x.y);
+            bool k0 = hash_keep(hash + (uint32_t)(2 * i) * kHashCol, g.thresh, thresh_hi);
+            bool k1 = hash_keep(hash + (uint32_t)(2 * i + 1) * kHashCol, g.thresh, thresh_hi);
+            if (EPI & F_RELU) { k0 = k0 && x.x > 0.f; k1 = k1 && x.y > 0.f; }
+            if (EPI & F_BITS_OUT) { set_bit(positive, k0, 1u << (2 * i), g.one); set_bit(positive, k1, 2u << (2 * i), g.one); }
+            v[i] = pack2(k0 ? x.x : 0.f, k1 ? x.y : 0.f);
           }
         } else if (EPI & F_RELU) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const float2 x = unpack2(v[i]);
+            if (EPI & F_BITS_OUT) { set_bit(positive, x.x > 0.f, 1u << (2 * i), g.one); set_bit(positive, x.y > 0.f, 2u << (2 * i), g.one); }
             v[i] = pack2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f));
           }
         }
@@ -327,16 +326,10 @@ gemm_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           }
         }
         if (EPI & F_BITS_OUT) {
-          uint32_t m = 0;
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float2 x = unpack2(v[i]);
-            m |= (x.x > 0.f ? 1u << (2 * i) : 0u) | (x.y > 0.f ? 2u << (2 * i) : 0u);
-          }
           if (row_ok) {
             unsigned short* bo = g.bits_out + (long long)((col0 >> 4) + 2 * h) * g.ldmb + row;
-            if (col0 + 32 * h < g.N) bo[0] = (unsigned short)m;
-            if (col0 + 32 * h + 16 < g.N) bo[g.ldmb] = (unsigned short)(m >> 16);
+            if (col0 + 32 * h < g.N) bo[0] = (unsigned short)positive;
+            if (col0 + 32 * h + 16 < g.N) bo[g.ldmb] = (unsigned short)(positive >> 16);
           }
         }
         if (STAGED) {
@@ -346,10 +339,7 @@ gemm_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               if (EPI & F_RES) v[4 * q + i] = add2(v[4 * q + i], widen16<FP16>(w[i]));
-              else {
-                const float2 z = unpack2(widen16<FP16>(w[i]));
-                v[4 * q + i] = mul2(v[4 * q + i], pack2(gelu_erf_grad_f32(z.x), gelu_erf_grad_f32(z.y)));
-              }
+              else v[4 * q + i] = mul2(v[4 * q + i], gelu_grad2(widen16<FP16>(w[i])));
             }
           }
         }
@@ -508,7 +498,7 @@ extern "C" int bf_gemm_rows(const bf_gemm_params* p, cudaStream_t st) {
   if (p->z_out) f |= F_KEEP_Z;
   RowsKernel kern = rows_kernel(f, fp16);
   if (kern == nullptr) return (int)cudaErrorNotSupported;
-  g.M = p->M; g.N = p->N; g.is_fp16 = fp16;
+  g.M = p->M; g.N = p->N; g.one = 1u;
   g.m_tiles = (p->M + kTileM - 1) / kTileM;
   g.k_panels = (p->K + kPanel - 1) / kPanel;
   g.panels = (p->N + kPanel - 1) / kPanel;

@@ -117,9 +117,9 @@ EncodeTiledFn get_encode_fn() {
 }
 
 // 2-D row-major 16-bit tensor [rows, cols] with row stride ld (elements); box = [box_rows, box_cols]; 64-column boxes
-// use the 128-byte swizzle, other widths are unswizzled.
+// use the 128-byte swizzle, other widths are unswizzled, or on request 32-column boxes with the 64-byte swizzle.
 int make_map(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_rows,
-             int is_fp16, int box_cols = 64) {
+             int is_fp16, int box_cols = 64, bool swizzle64 = false) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return -1;
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
@@ -128,7 +128,7 @@ int make_map(CUtensorMap* map, const void* base, long long rows, long long cols,
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, is_fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                  box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : swizzle64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -2;
 }

@@ -1,8 +1,7 @@
 """Feed-forward block on the tcgen05 GEMM: ``y = residual + drop2(W2 drop1(act(W1 x + b1)) + b2)``.
 
-Forward is two kernels (activation + dropout in the first epilogue, bias + dropout + residual in the
-second); forward passes without a backward (evaluation) run as one kernel with the hidden tile kept on chip
-(``ffn_onchip``).  Backward for ReLU uses the mask epilogue: ``dh = (g W2) * [h > 0] / (1 - p1)`` comes out of
+Forward is one kernel with the hidden tile kept on chip (``ffn_onchip``) where the weights fit beside it, else two
+(activation + dropout in the first epilogue, bias + dropout + residual in the second).  Backward for ReLU uses the mask epilogue: ``dh = (g W2) * [h > 0] / (1 - p1)`` comes out of
 the GEMM directly, so the hidden gradient is never touched by a separate elementwise pass.  GELU keeps
 the pre-activation and the same GEMM's epilogue multiplies by ``gelu'(z)`` (``_FusedFFNGelu``).  Replaces Linear -> act -> Dropout -> Linear ->
 Dropout -> add of the reference layers (e.g. models/gt_dist_node_level.py:655-660)."""
@@ -21,21 +20,23 @@ from .norm import hash_dropout, new_seed
 # the ReLU mask travels from forward to backward as one bit per hidden element (off: the backward re-reads h)
 USE_RELU_BITS = True
 # Forward passes that no backward will follow run the whole block in one kernel with the hidden tile kept on chip
-# (csrc/ffn_fused_tcgen05.cu; model width 128, hidden width 256).  "all" (default): evaluation passes and the first
+# (csrc/ffn_fused_tcgen05.cu; model / hidden width 128 / 256 and 64 / 128).  "all" (default): evaluation passes and the first
 # forward of recomputed layers (recompute / keep_mha tiers; its hash dropout masks are reproduced by the recomputation,
 # which runs the two-GEMM form because the backward needs the hidden matrix); "1": evaluation passes only; "0": off.
 ONCHIP_FFN = os.environ.get("BF_FFN_ONCHIP", "all")
-# training forward of the ReLU block on the same kernel with the hidden matrix and the ReLU bits as side outputs
-# (1.05 against 1.42 ms per layer at 2.9 M rows); "0": two GEMMs
+# training forward on the same kernel with the hidden matrix and the ReLU bits, or the GELU's pre-activation, as side outputs
+# (at 800 k rows of 128 / 256 255 and 299 us for ReLU and GELU, against 305 and 316 us of two GEMMs; at 50 k rows 31 and 33 against 38 and 42); "0": two GEMMs
 ONCHIP_FFN_TRAIN = os.environ.get("BF_FFN_ONCHIP_TRAIN", "1") == "1"
 
 
 def ffn_onchip(x: torch.Tensor, w1, b1, w2, b2, *, act: str, residual: bool, p1: float = 0.0, seed1: int = 0,
                p2: float = 0.0, seed2: int = 0, h_out: Optional[torch.Tensor] = None,
-               relu_bits_out: Optional[torch.Tensor] = None) -> torch.Tensor:
+               relu_bits_out: Optional[torch.Tensor] = None, z_out: Optional[torch.Tensor] = None,
+               other: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``[x +] drop2(act(x W1^T + b1) W2^T + b2)`` in one kernel; the ``[rows, ffn]`` hidden matrix never reaches HBM
     unless ``h_out`` asks for it as a side output (then it is written once and not read back; ``relu_bits_out`` receives
-    one bit per hidden element, value > 0).  No autograd.  Shapes: see ``onchip_supported``."""
+    one bit per hidden element, value > 0; ``z_out`` the pre-activation of a GELU).  ``other`` is a residual that is not ``x``.  No
+    autograd.  Shapes: see ``onchip_supported``."""
     from . import _ext
     ext = _ext.load()
 
@@ -46,15 +47,20 @@ def ffn_onchip(x: torch.Tensor, w1, b1, w2, b2, *, act: str, residual: bool, p1:
         return b.clone() if b.data_ptr() % 16 else b
     y = ext.ffn_fused_fwd(x, gemm.operand_copy(w1, x.dtype), f32(b1), gemm.operand_copy(w2, x.dtype), f32(b2),
                           gemm.ACT[act], bool(residual), float(p1), int(seed1), float(p2), int(seed2),
-                          gemm.status_tensor(x.device), h_out, relu_bits_out)
+                          gemm.status_tensor(x.device), h_out, relu_bits_out, z_out, other)
     _ext.count_launches(1)
     return y
 
 
-def onchip_supported(x: torch.Tensor, w1, w2) -> bool:
-    # bf16 only: the fp16 instantiation of the kernel exists but is not covered by the GPU tests
-    if not (x.is_cuda and x.dim() == 2 and x.dtype == torch.bfloat16 and x.stride(1) == 1
-            and (x.stride(0) * 2) % 16 == 0 and x.data_ptr() % 16 == 0 and x.size(0) > 0):
+def _rows_ok(x: torch.Tensor) -> bool:
+    return (x.is_cuda and x.dim() == 2 and x.dtype in (torch.bfloat16, torch.float16) and x.stride(1) == 1
+            and (x.stride(0) * 2) % 16 == 0 and x.data_ptr() % 16 == 0 and x.size(0) > 0)
+
+
+def onchip_supported(x: torch.Tensor, w1, w2, residual: Optional[torch.Tensor] = None) -> bool:
+    if not _rows_ok(x):
+        return False
+    if residual is not None and not (_rows_ok(residual) and residual.shape == x.shape and residual.dtype == x.dtype):
         return False
     from . import _ext
     return bool(_ext.load().ffn_fused_supported(x.size(0), x.size(1), w1.size(0))) and tuple(w2.shape) == (x.size(1), w1.size(0))
@@ -70,11 +76,11 @@ class _FusedFFNRelu(torch.autograd.Function):
         # the input-gradient GEMM instead of leaving a separate full-size addition to autograd
         res_is_x = residual is not None and residual.data_ptr() == x.data_ptr() and residual.shape == x.shape \
             and residual.stride() == x.stride()
-        if ONCHIP_FFN_TRAIN and bits is not None and (residual is None or res_is_x) and onchip_supported(x, w1, w2):
+        if ONCHIP_FFN_TRAIN and bits is not None and onchip_supported(x, w1, w2, residual):
             # one kernel: the hidden matrix is written once as a side output and never read back by the forward pass
             h = torch.empty((x.size(0), w1.size(0)), dtype=x.dtype, device=x.device)
             y = ffn_onchip(x, w1, b1, w2, b2, act="relu", residual=res_is_x, p1=p1, seed1=seed1, p2=p2, seed2=seed2,
-                           h_out=h, relu_bits_out=bits)
+                           h_out=h, relu_bits_out=bits, other=None if res_is_x else residual)
         else:
             h = gemm.gemm_tn(x, w1h, b1, "relu", dropout_p=p1, dropout_seed=seed1, relu_bits_out=bits)
             y = gemm.gemm_tn(h, w2h, b2, None, dropout_p=p2, dropout_seed=seed2, residual=residual)
@@ -114,22 +120,31 @@ class _FusedFFNRelu(torch.autograd.Function):
 
 
 class _FusedFFNGelu(torch.autograd.Function):
-    """GELU form (Graphormer).  Forward: GEMM (bias) -> z, one pass ``h = dropout(gelu(z))``, GEMM (bias, dropout,
-    residual).  Backward: the hidden gradient ``dz = (g W2) * keep / (1 - p1) * gelu'(z)`` comes out of the GEMM's
+    """GELU form (Graphormer).  Forward: one kernel with z and h as side outputs, or a GEMM that leaves z and
+    ``h = dropout(gelu(z))`` and a second one (bias, dropout, residual).  Backward: the hidden gradient ``dz = (g W2) * keep / (1 - p1) * gelu'(z)`` comes out of the GEMM's
     epilogue (dropout mask regenerated from its seed, derivative evaluated on the saved pre-activation), so neither the
     GELU derivative nor the dropout mask is a separate pass over the ``[rows, ffn]`` gradient."""
 
     @staticmethod
     def forward(ctx, x, w1, b1, w2, b2, residual, p1, p2, seed1, seed2, slot=None):
-        from .norm import gelu_dropout
         w1h, w2h = gemm.operand_copy(w1, x.dtype), gemm.operand_copy(w2, x.dtype)
-        z = gemm.gemm_tn(x, w1h, b1)
-        h = gelu_dropout(z, seed1, p1)
-        y = gemm.gemm_tn(h, w2h, b2, None, dropout_p=p2, dropout_seed=seed2, residual=residual)
-        ctx.weights = (w1, w2)
-        ctx.save_for_backward(x, z, h)
         res_is_x = residual is not None and residual.data_ptr() == x.data_ptr() and residual.shape == x.shape \
             and residual.stride() == x.stride()
+        z = torch.empty((x.size(0), w1.size(0)), dtype=x.dtype, device=x.device)
+        if ONCHIP_FFN_TRAIN and onchip_supported(x, w1, w2, residual):
+            h = torch.empty_like(z)
+            y = ffn_onchip(x, w1, b1, w2, b2, act="gelu", residual=res_is_x, p1=p1, seed1=seed1, p2=p2, seed2=seed2, h_out=h,
+                           z_out=z, other=None if res_is_x else residual)
+        else:
+            if b1 is None:
+                from .norm import gelu_dropout
+                z = gemm.gemm_tn(x, w1h, out=z)
+                h = gelu_dropout(z, seed1, p1)
+            else:
+                h = gemm.gemm_tn(x, w1h, b1, "gelu", dropout_p=p1, dropout_seed=seed1, z_out=z)
+            y = gemm.gemm_tn(h, w2h, b2, None, dropout_p=p2, dropout_seed=seed2, residual=residual)
+        ctx.weights = (w1, w2)
+        ctx.save_for_backward(x, z, h)
         ctx.cfg = (float(p1), float(p2), int(seed1), int(seed2), residual is not None, w1.dtype,
                    b1 is not None, b2 is not None, res_is_x)
         ctx.slot = slot
@@ -169,12 +184,12 @@ def fused_ffn(x: torch.Tensor, w1, b1, w2, b2, *, act: str = "relu", residual: O
     res_is_x = residual is not None and residual.data_ptr() == x.data_ptr() and residual.shape == x.shape \
         and residual.stride() == x.stride()
     forward_only = not torch.is_grad_enabled() and (not training or ONCHIP_FFN == "all")
-    if ok and forward_only and ONCHIP_FFN != "0" and act in ("relu", "gelu") and (residual is None or res_is_x) \
-            and onchip_supported(x, w1, w2):
+    if ok and forward_only and ONCHIP_FFN != "0" and act in ("relu", "gelu") and onchip_supported(x, w1, w2, residual):
         # same order of seed draws as the two-GEMM forms below, so that a recomputation reproduces the masks
         s1 = new_seed() if p1 > 0 else 0
         s2 = new_seed() if p2 > 0 else 0
-        return ffn_onchip(x, w1, b1, w2, b2, act=act, residual=res_is_x, p1=p1, seed1=s1, p2=p2, seed2=s2)
+        return ffn_onchip(x, w1, b1, w2, b2, act=act, residual=res_is_x, p1=p1, seed1=s1, p2=p2, seed2=s2,
+                          other=None if res_is_x else residual)
     if ok and act == "relu":
         return _FusedFFNRelu.apply(x, w1, b1, w2, b2, residual, p1, p2, new_seed() if p1 > 0 else 0,
                                    new_seed() if p2 > 0 else 0, out_grad_colsum)

@@ -313,6 +313,62 @@ def test_ffn_with_the_hidden_tile_on_chip_matches_reference(act, residual, p1, p
     gemm.check_status("cuda")
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("h", [64, 128])
+@pytest.mark.parametrize("m", [1, 127, 128 * 3 + 33, 128 * 148 * 3 + 5])
+def test_ffn_on_chip_widths_types_and_residuals(m, h, dtype):
+    """Both widths and types, ReLU and GELU, each residual, with and without dropout and side outputs; fewer tiles than blocks, several a
+    block, a ragged last one.  Hidden values against fp64 (one rounding to 8 or 11 bits, products added in fp32), the output against fp64
+    products of the kernel's own hidden matrix."""
+    from budgetformer_b200.ops.ffn import ffn_onchip, onchip_supported
+    torch.manual_seed(m + h)
+    f = 2 * h
+    big = torch.randn(m, h + 8, device="cuda").to(dtype)
+    x, other = big[:, :h], torch.randn(m, h, device="cuda").to(dtype)
+    l1, l2 = torch.nn.Linear(h, f).cuda(), torch.nn.Linear(f, h).cuda()
+    assert onchip_supported(x, l1.weight, l2.weight, other)
+    w1, w2 = l1.weight.detach().to(dtype).double(), l2.weight.detach().to(dtype).double()
+    b1, b2 = l1.bias.detach().double(), l2.bias.detach().double()
+    half_ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    tiny = 0.0 if dtype == torch.bfloat16 else 2.0 ** -25
+    near = lambda got, want, slack: ((got.double() - want).abs() <= half_ulp * (1 + 2.0 ** -7) * want.abs() + slack + tiny).all()
+    zref = x.double() @ w1.t() + b1
+    zslack = (x.double().abs() @ w1.abs().t() + 4) * h ** 0.5 * 2.0 ** -22 + 2.0 ** -20
+    k1, k2 = gemm.hash_keep_mask(41, m, f, 0.25, "cuda"), gemm.hash_keep_mask(43, m, h, 0.125, "cuda")
+    for act in ("relu", "gelu"):
+        for p1, p2, res in ((0.0, 0.0, None), (0.25, 0.0, "x"), (0.25, 0.125, "other"), (0.0, 0.125, "other")):
+            kw = dict(act=act, residual=res == "x", p1=p1, seed1=41, p2=p2, seed2=43, other=other if res == "other" else None)
+            hid = torch.empty(m, f, device="cuda", dtype=dtype)
+            side = dict(h_out=hid)
+            if act == "gelu":
+                side["z_out"] = torch.empty_like(hid)
+            else:
+                side["relu_bits_out"] = torch.empty(f // 16, m, device="cuda", dtype=torch.int16)
+            y = ffn_onchip(x, l1.weight, l1.bias, l2.weight, l2.bias, **kw, **side)
+            plain = ffn_onchip(x, l1.weight, l1.bias, l2.weight, l2.bias, **kw)
+            gemm.check_status("cuda")
+            if act == "gelu":
+                assert near(side["z_out"], zref, zslack)
+                want = torch.nn.functional.gelu(side["z_out"].double())
+            else:
+                want = zref.clamp(min=0)
+            if p1 > 0:
+                want = torch.where(k1, want / (1 - p1), 0.0)
+            assert near(hid, want, 2 * zslack)
+            if act == "relu":
+                bits = torch.stack([(side["relu_bits_out"].int() >> i) & 1 for i in range(16)], 1).reshape(f, m).t().bool()
+                sure = want.abs() > 4 * zslack
+                assert torch.equal(bits & sure, (want > 0) & sure)
+                assert torch.equal(y, plain)
+            out = hid.double() @ w2.t() + b2
+            if p2 > 0:
+                out = torch.where(k2, out / (1 - p2), 0.0)
+            if res is not None:
+                out = out + (x if res == "x" else other).double()
+            assert near(y, out, (hid.double().abs() @ w2.abs().t() + 8) * f ** 0.5 * 2.0 ** -22)
+            _close(plain, out, dtype)
+
+
 def test_ffn_on_chip_side_outputs_equal_the_two_gemm_form():
     """Training variant of the one-kernel block: the hidden matrix written from the on-chip operand and the ReLU bit mask
     equal what the first GEMM of the two-GEMM form writes (same masks, same rounding), over a ragged row count."""
