@@ -227,6 +227,21 @@ int bf_gemm_rows(const bf_gemm_params* p, cudaStream_t st);
 int bf_gemm_supported(int M, int N, int K);
 int bf_gemm_tn(const bf_gemm_params* p, cudaStream_t st);
 
+// ---- per-step work on parameters and gradients (param_kernels.cu) -------------------------------------
+// dst[r * ld_dst + c] (transpose: dst[c * ld_dst + r]) = src[r * ld_src + c], in the type `dtype` (BF_BF16, BF_FP16 or BF_FP32)
+typedef struct {
+  const float* src;
+  void* dst;
+  int rows, cols, ld_src, ld_dst, transpose, dtype;
+} bf_copy_item;
+int bf_weight_copies(const bf_copy_item* items, int n, cudaStream_t st);
+// dst[offset .. offset + count) = src, or zeros where src is NULL
+typedef struct {
+  const float* src;
+  long long offset, count;
+} bf_gather_item;
+int bf_gather_f32(const bf_gather_item* items, int n, float* dst, cudaStream_t st);
+
 // ---- tcgen05 weight-gradient GEMM (gemm_dw_tcgen05.cu) ----------------------------------------------
 // dW[N, K] (= or +=) scale * dY[M, N]^T X[M, K]; dbias[N] (= or +=) scale * column sums of dY (optional).
 typedef struct {

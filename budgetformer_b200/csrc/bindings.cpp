@@ -1,6 +1,7 @@
 // PyTorch bindings: tensor checks, allocation of workspaces and stream plumbing around the C
 // launchers declared in bf_kernels.h.  No kernel code lives here.
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -628,8 +629,9 @@ std::vector<Tensor> gemm_dw(Tensor dY, Tensor X, bool want_bias, Tensor status) 
   TORCH_CHECK(bf_gemm_dw_supported(p.M, p.N, p.K), "gemm_dw: unsupported shape");
   TORCH_CHECK(!want_bias || bf_gemm_dw_bias_supported(p.K), "gemm_dw: bias gradient not available for K = ", p.K);
   auto f32 = torch::TensorOptions().dtype(torch::kFloat).device(dY.device());
-  Tensor dW = torch::empty({p.N, p.K}, f32);
-  Tensor db = want_bias ? torch::empty({p.N}, f32) : Tensor();
+  Tensor out = torch::empty({(int64_t)p.N * p.K + (want_bias ? p.N : 0)}, f32);
+  Tensor dW = out.as_strided({p.N, p.K}, {p.K, 1}, 0);
+  Tensor db = want_bias ? out.as_strided({p.N}, {1}, (int64_t)p.N * p.K) : Tensor();
   Tensor scratch = torch::empty({(int64_t)(bf_gemm_dw_scratch_bytes(p.M, p.N, p.K) / 4)}, f32);
   p.dW = dW.data_ptr<float>();
   p.dbias = want_bias ? db.data_ptr<float>() : nullptr;
@@ -708,14 +710,14 @@ std::vector<Tensor> layernorm_bwd(Tensor dy, Tensor x, Tensor stats, Tensor gamm
   TORCH_CHECK(dy.is_cuda() && dy.dim() == 2 && dy.stride(1) == 1 && x.stride(1) == 1 && dy.scalar_type() == x.scalar_type());
   c10::cuda::CUDAGuard guard(x.device());
   Tensor dx = torch::empty({x.size(0), x.size(1)}, x.options());
-  Tensor dgamma = torch::zeros({x.size(1)}, x.options().dtype(torch::kFloat));
-  Tensor dbeta = torch::zeros({x.size(1)}, x.options().dtype(torch::kFloat));
   const int64_t h = x.size(1);
+  Tensor sums = torch::zeros({want_dxsum ? 3 : 2, h}, x.options().dtype(torch::kFloat));
+  Tensor dgamma = sums.select(0, 0), dbeta = sums.select(0, 1);
   const bool wide = x.scalar_type() != torch::kFloat && (h == 64 || h == 128 || h == 256) &&
                     (dy.stride(0) * 2) % 16 == 0 && (x.stride(0) * 2) % 16 == 0 &&
                     ((uintptr_t)dy.data_ptr()) % 16 == 0 && ((uintptr_t)x.data_ptr()) % 16 == 0;
   Tensor dxsum;
-  if (want_dxsum && wide) dxsum = torch::zeros({h}, x.options().dtype(torch::kFloat));
+  if (want_dxsum && wide) dxsum = sums.select(0, 2);
   check_cuda(bf_layernorm_bwd(dy.data_ptr(), dy.stride(0), x.data_ptr(), x.stride(0), stats.data_ptr<float>(),
                               gamma.data_ptr<float>(), dx.data_ptr(), dx.stride(0), dgamma.data_ptr<float>(),
                               dbeta.data_ptr<float>(), dxsum.defined() ? dxsum.data_ptr<float>() : nullptr,
@@ -739,6 +741,101 @@ Tensor f32_weight_grad(Tensor dy, Tensor x, bool want_bias) {
   return out;
 }
 
+// Copies of fp32 matrices in the layouts that the GEMMs take, made by one launch.  `outs` holds (type, rows, cols) of every result (rows 0: a vector); `items`
+// eight integers a block to copy: source, its first row, rows, columns, result, offset in the result (elements), its row pitch,
+// transposed.  The results of one type share a buffer.
+std::vector<Tensor> weight_copies(std::vector<Tensor> srcs, std::vector<int64_t> items, std::vector<int64_t> outs) {
+  TORCH_CHECK(!srcs.empty() && items.size() % 8 == 0 && outs.size() % 3 == 0, "weight_copies: bad tables");
+  c10::cuda::CUDAGuard guard(srcs[0].device());
+  for (const Tensor& t : srcs)
+    TORCH_CHECK(t.is_cuda() && t.device() == srcs[0].device() && t.scalar_type() == torch::kFloat && t.is_contiguous() &&
+                (t.dim() == 1 || t.dim() == 2), "weight_copies: contiguous fp32 on one device");
+  const size_t n_out = outs.size() / 3, n = items.size() / 8;
+  const torch::ScalarType types[3] = {torch::kBFloat16, torch::kHalf, torch::kFloat};
+  int64_t total[3] = {0, 0, 0};
+  std::vector<int64_t> at(n_out);
+  for (size_t i = 0; i < n_out; ++i) {
+    const int64_t t = outs[3 * i];
+    TORCH_CHECK(t >= 0 && t < 3 && outs[3 * i + 1] >= 0 && outs[3 * i + 2] > 0);
+    at[i] = total[t];
+    total[t] += (std::max<int64_t>(outs[3 * i + 1], 1) * outs[3 * i + 2] + 63) / 64 * 64;
+  }
+  Tensor flat[3];
+  for (int t = 0; t < 3; ++t)
+    if (total[t] > 0) flat[t] = torch::empty({total[t]}, srcs[0].options().dtype(types[t]));
+  std::vector<bf_copy_item> table(n);
+  for (size_t i = 0; i < n; ++i) {
+    const int64_t* v = items.data() + 8 * i;
+    TORCH_CHECK(v[0] >= 0 && v[0] < (int64_t)srcs.size() && v[4] >= 0 && v[4] < (int64_t)n_out);
+    const Tensor& src = srcs[v[0]];
+    const int64_t src_cols = src.dim() == 2 ? src.size(1) : 1, src_rows = src.size(0);     // a vector is a column
+    const int64_t* o = outs.data() + 3 * v[4];
+    const int64_t last = v[7] ? (v[3] - 1) * v[6] + v[2] : (v[2] - 1) * v[6] + v[3];
+    TORCH_CHECK(v[1] >= 0 && v[2] > 0 && v[1] + v[2] <= src_rows && v[3] > 0 && v[3] <= src_cols && v[5] >= 0 && v[6] > 0 &&
+                v[5] + last <= std::max<int64_t>(o[1], 1) * o[2], "weight_copies: a block outside its matrices");
+    table[i] = {src.data_ptr<float>() + v[1] * src_cols, static_cast<char*>(flat[o[0]].data_ptr()) + (at[v[4]] + v[5]) * flat[o[0]].element_size(),
+                (int)v[2], (int)v[3], (int)src_cols, (int)v[6], (int)v[7], (int)o[0]};
+  }
+  check_cuda(bf_weight_copies(table.data(), (int)n, at::cuda::getCurrentCUDAStream()), "weight_copies");
+  std::vector<Tensor> r;
+  for (size_t i = 0; i < n_out; ++i) {
+    const int64_t* o = outs.data() + 3 * i;
+    r.push_back(o[1] == 0 ? flat[o[0]].as_strided({o[2]}, {1}, at[i]) : flat[o[0]].as_strided({o[1], o[2]}, {o[2], 1}, at[i]));
+  }
+  return r;
+}
+
+// The gradients of a bucket's parameters: let go of before a backward pass, so that autograd keeps what the nodes produced instead of
+// adding it to zeros, and gathered into the flat bucket behind it, of which `.grad` is a view again.
+struct GradBucket {
+  std::vector<Tensor> params, views;
+  std::vector<int64_t> offsets;
+  Tensor flat;
+  GradBucket(std::vector<Tensor> p, std::vector<int64_t> o, Tensor f) : params(std::move(p)), offsets(std::move(o)), flat(std::move(f)) {
+    TORCH_CHECK(params.size() == offsets.size() && flat.is_cuda() && flat.dim() == 1 && flat.is_contiguous() && flat.scalar_type() == torch::kFloat);
+    for (size_t i = 0; i < params.size(); ++i) {
+      TORCH_CHECK(params[i].scalar_type() == torch::kFloat && params[i].device() == flat.device() && offsets[i] >= 0 &&
+                  offsets[i] + params[i].numel() <= flat.numel());
+      views.push_back(flat.narrow(0, offsets[i], params[i].numel()).view(params[i].sizes()));
+    }
+  }
+  void bind() {
+    for (size_t i = 0; i < params.size(); ++i) params[i].mutable_grad() = views[i];
+  }
+  void release() {
+    for (Tensor& p : params) p.mutable_grad() = Tensor();
+  }
+  void gather() {
+    c10::cuda::CUDAGuard guard(flat.device());
+    auto st = at::cuda::getCurrentCUDAStream();
+    at::NoGradGuard no_grad;
+    std::vector<bf_gather_item> items;
+    std::vector<size_t> copied;
+    for (size_t i = 0; i < params.size(); ++i) {
+      const Tensor g = params[i].grad();
+      bf_gather_item it{nullptr, offsets[i], params[i].numel()};
+      if (g.defined()) {
+        if (g.layout() == torch::kStrided && g.is_cuda() && g.device() == flat.device() && g.scalar_type() == torch::kFloat &&
+            g.is_contiguous() && g.numel() == it.count) {
+          it.src = g.data_ptr<float>();
+          if (it.src == views[i].data_ptr<float>()) continue;          // someone put it there
+          c10::cuda::CUDACachingAllocator::recordStream(g.storage().data_ptr(), st);
+        } else {
+          copied.push_back(i);
+          continue;
+        }
+      }
+      if (it.count > 0) items.push_back(it);
+    }
+    if (!items.empty()) check_cuda(bf_gather_f32(items.data(), (int)items.size(), flat.data_ptr<float>(), st), "gather_f32");
+    for (size_t i : copied) {
+      const Tensor g = params[i].grad();
+      views[i].copy_(g.layout() == torch::kStrided ? g : g.to_dense());
+    }
+    bind();
+  }
+};
+
 Tensor colsum(Tensor x) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.stride(1) == 1);
   c10::cuda::CUDAGuard guard(x.device());
@@ -753,7 +850,7 @@ std::vector<Tensor> bn_stats(Tensor x, OptTensor shift) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.stride(1) == 1);
   c10::cuda::CUDAGuard guard(x.device());
   auto fopt = x.options().dtype(torch::kFloat);
-  Tensor s1 = torch::zeros({x.size(1)}, fopt), s2 = torch::zeros({x.size(1)}, fopt);
+  Tensor sums = torch::zeros({2, x.size(1)}, fopt), s1 = sums.select(0, 0), s2 = sums.select(0, 1);
   check_cuda(bf_bn_stats(x.data_ptr(), x.stride(0), shift.has_value() ? shift->data_ptr<float>() : nullptr, x.size(0),
                          (int)x.size(1), s1.data_ptr<float>(), s2.data_ptr<float>(), dtype_code(x),
                          at::cuda::getCurrentCUDAStream()), "bn_stats");
@@ -765,7 +862,7 @@ std::vector<Tensor> bn_bwd_reduce(Tensor dy, Tensor x, Tensor mean, Tensor rstd)
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.stride(1) == 1 && dy.stride(1) == 1 && dy.scalar_type() == x.scalar_type());
   c10::cuda::CUDAGuard guard(x.device());
   auto fopt = x.options().dtype(torch::kFloat);
-  Tensor dbeta = torch::zeros({x.size(1)}, fopt), dgamma = torch::zeros({x.size(1)}, fopt);
+  Tensor sums = torch::zeros({2, x.size(1)}, fopt), dbeta = sums.select(0, 0), dgamma = sums.select(0, 1);
   check_cuda(bf_bn_bwd_reduce(dy.data_ptr(), dy.stride(0), x.data_ptr(), x.stride(0), mean.data_ptr<float>(),
                               rstd.data_ptr<float>(), x.size(0), (int)x.size(1), dbeta.data_ptr<float>(),
                               dgamma.data_ptr<float>(), dtype_code(x), at::cuda::getCurrentCUDAStream()), "bn_bwd_reduce");
@@ -899,6 +996,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_supported", &gemm_supported);
   m.def("layernorm_fwd", &layernorm_fwd);
   m.def("layernorm_bwd", &layernorm_bwd);
+  m.def("weight_copies", &weight_copies);
+  py::class_<GradBucket>(m, "GradBucket")
+      .def(py::init<std::vector<Tensor>, std::vector<int64_t>, Tensor>())
+      .def("bind", &GradBucket::bind)
+      .def("release", &GradBucket::release)
+      .def("gather", &GradBucket::gather);
   m.def("hash_dropout", &hash_dropout);
   m.def("gelu_dropout", &gelu_dropout);
   m.def("bn_stats", &bn_stats);

@@ -232,15 +232,36 @@ gemm_dw_tcgen05_kernel(const __grid_constant__ CUtensorMap map_y, const __grid_c
   }
 }
 
-// out[i] (= or +=) sum over slices of partial[s][i], slices added in order.
-__global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ partial, long long n_elem, int splits,
-                                                        float* __restrict__ out, int accumulate, float scale) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_elem) return;
+// out[i] (= or +=) sum over slices of partial[s][i], and likewise the bias gradient behind it, in one launch.  A block has 64 elements
+// and four threads for each, which take every fourth slice eight loads at a time; the four sums meet in a fixed order.  Bound by the
+// latency of up to 148 slices: one thread an element with its loads one behind the other, and a launch of its own for the bias, took
+// 11.0 us a layer (Graphormer's layers, width 128, 169 k rows), this takes 6.2.
+__global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ partial, long long n_elem,
+                                                        const float* __restrict__ bias_partial, int n_bias, int splits,
+                                                        float* __restrict__ out, float* __restrict__ out_bias, int accumulate, float scale) {
+  __shared__ float s_sum[4][64];
+  const int lane = threadIdx.x & 63, part = threadIdx.x >> 6;
+  const long long i = (long long)blockIdx.x * 64 + lane;
+  const bool weight = i < n_elem, bias = !weight && i < n_elem + n_bias;
+  const float* p = weight ? partial + i : bias_partial + (i - n_elem);
+  const long long step = weight ? n_elem : n_bias;
   float acc = 0.f;
-  for (int s = 0; s < splits; ++s) acc += partial[(long long)s * n_elem + i];
-  acc *= scale;
-  out[i] = accumulate ? out[i] + acc : acc;
+  if (weight || bias) {
+    for (int s = part; s < splits; s += 32) {
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = s + 4 * j < splits ? __ldg(p + (long long)(s + 4 * j) * step) : 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc += v[j];
+    }
+  }
+  s_sum[part][lane] = acc;
+  __syncthreads();
+  if (part == 0 && (weight || bias)) {
+    acc = ((s_sum[0][lane] + s_sum[1][lane]) + (s_sum[2][lane] + s_sum[3][lane])) * scale;
+    float* o = weight ? out + i : out_bias + (i - n_elem);
+    *o = accumulate ? *o + acc : acc;
+  }
 }
 
 }  // namespace
@@ -319,10 +340,8 @@ extern "C" int bf_gemm_dw(const bf_gemm_dw_params* p, cudaStream_t st) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   const long long n_elem = (long long)p->N * p->K;
-  dw_reduce_kernel<<<(unsigned)((n_elem + 255) / 256), 256, 0, st>>>(g.partial, n_elem, g.splits, p->dW, p->accumulate,
-                                                                    p->scale == 0.f ? 1.f : p->scale);
-  if (g.bias_chunk >= 0)
-    dw_reduce_kernel<<<(unsigned)((p->N + 255) / 256), 256, 0, st>>>(g.bias_partial, p->N, g.splits, p->dbias, p->accumulate,
-                                                                    p->scale == 0.f ? 1.f : p->scale);
+  const int n_bias = g.bias_chunk >= 0 ? p->N : 0;
+  dw_reduce_kernel<<<(unsigned)((n_elem + n_bias + 63) / 64), 256, 0, st>>>(g.partial, n_elem, g.bias_partial, n_bias, g.splits, p->dW,
+                                                                           p->dbias, p->accumulate, p->scale == 0.f ? 1.f : p->scale);
   return (int)cudaGetLastError();
 }

@@ -23,8 +23,9 @@ namespace {
 
 // erow[e] = row of edge e, iota[e] = e.  A block takes 256 rows; where they hold at most kStaged edges (an attention graph has 5 to 30
 // a row) its threads mark their rows' edges in shared memory and the block writes them out along memory.  Otherwise eight lanes
-// take a row, and rows above 64 edges (the virtual node's holds every node) are left to the whole warp, one after the other.  Bound by the
-// bytes written: 15 M edges 83 us with eight lanes a row everywhere, 31 now.
+// take a row, and rows above 64 edges (the virtual node's holds every node) are left to the whole block, one after the other.  Bound by the
+// bytes written: 15 M edges 83 us with eight lanes a row everywhere, 31 now; 169 k nodes and a row of all of them 44 us with that row on one
+// warp, @HUBROW@ now.
 constexpr int kStaged = 8192;
 __global__ void __launch_bounds__(256) edge_rows_kernel(const int* __restrict__ rowptr, int n, int* __restrict__ erow, int* __restrict__ iota) {
   __shared__ uint8_t s_row[kStaged];
@@ -40,22 +41,22 @@ __global__ void __launch_bounds__(256) edge_rows_kernel(const int* __restrict__ 
     for (int e = threadIdx.x; e < b1 - b0; e += 256) { erow[b0 + e] = r0 + s_row[e]; iota[b0 + e] = b0 + e; }
     return;
   }
-  for (int p = 0; p < 8; ++p) {
-    const int first = r0 + p * 32 + (threadIdx.x >> 5) * 4;          // four rows a warp
-    const int row = first + (lane >> 3);
-    int beg = 0, end = 0;
-    if (row < n) { beg = rowptr[row]; end = rowptr[row + 1]; }
-    const bool wide = end - beg > 64;
-    if (!wide)
-      for (int e = beg + (lane & 7); e < end; e += 8) { erow[e] = row; iota[e] = e; }
-    unsigned left = __ballot_sync(0xffffffffu, wide && (lane & 7) == 0);
-    while (left != 0) {
-      const int src = __ffs(left) - 1;
-      left &= left - 1;
-      const int b = __shfl_sync(0xffffffffu, beg, src), e1 = __shfl_sync(0xffffffffu, end, src);
-      const int r = first + (src >> 3);
-      for (int e = b + lane; e < e1; e += 32) { erow[e] = r; iota[e] = e; }
+  __shared__ int s_wide[256], s_n;
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  for (int r = threadIdx.x >> 3; r < rows; r += 32) {
+    const int beg = rowptr[r0 + r], end = rowptr[r0 + r + 1];
+    if (end - beg > 64) {
+      if ((lane & 7) == 0) s_wide[atomicAdd(&s_n, 1)] = r0 + r;
+    } else {
+      for (int e = beg + (lane & 7); e < end; e += 8) { erow[e] = r0 + r; iota[e] = e; }
     }
+  }
+  __syncthreads();
+  for (int w = 0; w < s_n; ++w) {
+    const int r = s_wide[w], end = rowptr[r + 1];
+#pragma unroll 4
+    for (int e = rowptr[r] + (int)threadIdx.x; e < end; e += 256) { erow[e] = r; iota[e] = e; }
   }
 }
 

@@ -119,8 +119,26 @@ class SPContext:
     def packed_projection(self, layer: int, wq, wk, wv, bq, bk, bv, dtype):
         """``[Wq; Wk; Wv]`` with its rows in the order of ``perm`` (and the bias likewise), in the activation dtype.  The
         pack is rebuilt only when one of the six tensors changed since it was made."""
+        ws, bs = (wq, wk, wv), (bq, bk, bv)
+        h = self.h
+        if (dtype in gemm._KIND and all(tuple(t.shape) == (h, h) and t.is_leaf for t in ws) and gemm._plain_sources(ws)
+                and (bq is None or all(t.shape == (h,) and t.is_leaf for t in bs) and gemm._plain_sources(bs))):
+            def rows(transposed):
+                # destination-rank major, then k | v | q, then head columns: the runs of ``perm``
+                return tuple((part, r * self.hl, self.hl, h, (3 * r + i) * self.hl * (1 if transposed else h),
+                              3 * h if transposed else h, int(transposed)) for r in range(self.P) for i, part in enumerate((1, 2, 0)))
+            key = (id(self), layer, dtype)
+            w = gemm.recipe_copy(key + ("w",), ws, lambda: rows(False), (gemm._KIND[dtype], 3 * h, h))
+            b = None
+            if bq is not None:                            # vectors are matrices of one column
+                b = gemm.recipe_copy(key + ("b",), bs, lambda: tuple(
+                    (part, r * self.hl, self.hl, 1, (3 * r + i) * self.hl, 1, 0)
+                    for r in range(self.P) for i, part in enumerate((1, 2, 0))), (gemm._KIND[torch.float32], 0, 3 * h))
+            self._packs[layer] = (None, w, b, lambda: gemm.recipe_copy(key + ("t",), ws, lambda: rows(True),
+                                                                       (gemm._KIND[dtype], h, 3 * h)), gemm._stamp(ws), ws)
+            return w, b
         parts = [t for t in (wq, wk, wv, bq, bk, bv) if t is not None]
-        stamp = (gemm._WEIGHT_GEN, dtype) + tuple((t._version, t.data_ptr()) for t in parts)
+        stamp = (dtype,) + gemm._stamp(parts)
         hit = self._packs.get(layer)
         if hit is None or hit[0] != stamp:
             w = torch.cat([wq, wk, wv], 0).detach().to(dtype)[self.perm].contiguous()
@@ -130,7 +148,19 @@ class SPContext:
 
     def transposed_projection(self, layer: int, w: torch.Tensor) -> torch.Tensor:
         hit = self._packs.get(layer)
-        return hit[3] if (hit is not None and hit[1] is w) else w.t().contiguous()
+        if hit is None or hit[1] is not w:
+            return w.t().contiguous()
+        if hit[0] is None:                                # made from the parameters, unless they changed since the pack was
+            return hit[3]() if gemm._stamp(hit[5]) == hit[4] else w.t().contiguous()
+        return hit[3]
+
+    def unpack_rows(self, t: torch.Tensor):
+        """The q, k and v rows of a matrix (or vector) whose rows are in the order of ``perm``."""
+        if self.P == 1:                                   # k | v | q: three runs
+            k, v, q = t.split(self.h, 0)
+        else:
+            q, k, v = t[self.inv_perm].split(self.h, 0)
+        return q, k, v
 
     def split_packed(self, t: torch.Tensor):
         """(q, k, v) views ``[rows, heads, hn]`` of a packed ``[rows, qkv_ld]`` buffer (column order k | v | q)."""
@@ -238,13 +268,11 @@ class _QKVPush(torch.autograd.Function):
         if dx is None:
             dx = gemm.gemm_tn(dloc, wt, residual=dres)
         dw, db_src = gemm.weight_grad(dloc, x, ctx.has_bias)
-        dw = dw[sp.inv_perm]
         if debug.enabled():
             debug.poison(buf.tensor)                  # consumed: whoever reads it before the next producer sees NaN
-        dwq, dwk, dwv = (t.to(ctx.wdtype) for t in dw.split(sp.h, 0))
+        dwq, dwk, dwv = (t.to(ctx.wdtype) for t in sp.unpack_rows(dw))
         if ctx.has_bias:
-            db = db_src[sp.inv_perm]
-            dbq, dbk, dbv = (t.to(ctx.wdtype) for t in db.split(sp.h, 0))
+            dbq, dbk, dbv = (t.to(ctx.wdtype) for t in sp.unpack_rows(db_src))
         else:
             dbq = dbk = dbv = None
         return dx, dwq, dwk, dwv, dbq, dbk, dbv, None, None, None

@@ -6,6 +6,9 @@ function used by the models on B200: forward, input gradient and weight gradient
 Shapes the kernels do not cover (features not a multiple of 8 / 16, fp32 operands) fall back to PyTorch."""
 from __future__ import annotations
 
+import itertools
+import threading
+import weakref
 from typing import Optional
 
 import torch
@@ -16,28 +19,145 @@ ACT = {None: 0, "none": 0, "relu": 1, "gelu": 2}
 _STATUS = {}
 
 # ---- operand copies of the weights ------------------------------------------------------------------------
-# The kernels take weights in the activation dtype (and the input-gradient GEMM takes them transposed).  Those copies
-# only change when the weights do: they are kept per parameter and rebuilt when the parameter's version counter moves
-# (in-place updates by PyTorch optimizers, ``load_state_dict``) or when an optimizer that writes the storage directly
-# announces a step through ``weights_changed()`` (``ops.optim.FlatAdamW``).
+# The kernels take weights in the activation dtype (and the input-gradient GEMM takes them transposed, the packed projection several
+# in one).  Those copies only change when the weights do: they are kept per parameter and rebuilt when the parameter's version counter moves
+# (in-place updates by PyTorch optimizers, ``load_state_dict``) or when an optimizer that writes the storage of its parameters directly
+# announces a step (``ops.optim.FlatAdamW``: ``watch_weights``, ``weights_changed``).  Whoever finds a copy stale has all stale copies rebuilt that
+# were used on the same stream since they were last made: one launch (``csrc/param_kernels.cu``) in the place of one to three a copy.
 _WEIGHT_GEN = 0
 _WEIGHT_COPIES = {}
+_RECIPES = {}
+_GROUPS = {}                                          # recipes whose weights have the same optimizer (None: no watched one)
+_RECIPE_LOCK = threading.Lock()
+_KIND = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 
-def weights_changed() -> None:
+_OWNERS = {}                                          # id of a parameter -> (weak reference, its optimizer's counter of steps)
+_STEPS = itertools.count(1)                           # never the same value twice, whichever optimizer it belongs to
+
+
+def watch_weights(params, counter: list) -> None:
+    """``counter[0]`` changes whenever the storage of ``params`` is written past their version counters."""
+    for k in [k for k, (ref, _) in _OWNERS.items() if ref() is None]:
+        del _OWNERS[k]
+    for p in params:
+        _OWNERS[id(p)] = (weakref.ref(p), counter)
+
+
+def weights_changed(counter: Optional[list] = None) -> None:
+    """The weights watched with ``counter`` have changed; without it, any weight may have."""
     global _WEIGHT_GEN
-    _WEIGHT_GEN += 1
+    if counter is not None:
+        counter[0] = next(_STEPS)
+    else:
+        _WEIGHT_GEN += 1
+
+
+def _generation(t: torch.Tensor) -> int:
+    owner = _OWNERS.get(id(t))
+    return owner[1][0] if owner is not None and owner[0]() is t else 0
+
+
+class _Recipe:
+    """A matrix made of blocks of fp32 matrices: ``blocks`` holds (source, first row, rows, columns, offset, row pitch, transposed)."""
+
+    __slots__ = ("srcs", "blocks", "out_spec", "stamp", "out", "used", "stream", "device", "group")
+
+    def __init__(self, srcs, blocks, out_spec):
+        owner = _OWNERS.get(id(srcs[0]))
+        self.group = id(owner[1]) if owner is not None and owner[0]() is srcs[0] else None
+        self.srcs = tuple(weakref.ref(t) for t in srcs)
+        self.blocks, self.out_spec = blocks, out_spec
+        self.stamp, self.out, self.used, self.stream = None, None, True, None
+        self.device = srcs[0].device
+
+    def sources(self):
+        ts = [r() for r in self.srcs]
+        return None if any(t is None for t in ts) else ts
+
+
+def _stamp(srcs):
+    return (_WEIGHT_GEN,) + tuple((t._version, t.data_ptr(), _generation(t)) for t in srcs)
+
+
+def _rebuild(wanted: _Recipe, srcs) -> torch.Tensor:
+    """Make ``wanted`` anew, and with it the stale copies that this stream used since they were made."""
+    with _RECIPE_LOCK:
+        stream = torch._C._cuda_getCurrentRawStream(wanted.device.index)
+        todo, sources = [wanted], [srcs]
+        if not torch.cuda.is_current_stream_capturing():
+            group, dead = _GROUPS[wanted.group], []
+            for key, r in group.items():
+                if r is wanted or not r.used or r.stream != stream or r.device != wanted.device:
+                    continue
+                ts = r.sources()
+                if ts is None:
+                    dead.append(key)
+                elif r.stamp != _stamp(ts) and _plain_sources(ts):
+                    todo.append(r)
+                    sources.append(ts)
+            for key in dead:
+                del group[key]
+                _RECIPES.pop(key, None)
+        at, flat, items, outs = {}, [], [], []
+        for i, (r, ts) in enumerate(zip(todo, sources)):
+            for t in ts:
+                if id(t) not in at:
+                    at[id(t)] = len(flat)
+                    flat.append(t.detach())
+            for blk in r.blocks:
+                items.extend((at[id(ts[blk[0]])], blk[1], blk[2], blk[3], i, blk[4], blk[5], blk[6]))
+            outs.extend(r.out_spec)
+        made = _ext.load().weight_copies(flat, items, outs)
+        _ext.count_launches((len(items) // 8 + 63) // 64)
+        for r, ts, out in zip(todo, sources, made):
+            r.out, r.stream, r.used = out, stream, r is wanted
+            r.stamp = _stamp(ts)
+        return wanted.out
+
+
+def _plain_sources(srcs) -> bool:
+    """fp32, contiguous and plain: what the copy kernel reads."""
+    return all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.numel() > 0 and t.device == srcs[0].device
+               and not torch._C._functorch.is_functorch_wrapped_tensor(t) for t in srcs)
+
+
+def recipe_copy(key, srcs, blocks, out_spec) -> torch.Tensor:
+    """The matrix that ``blocks`` (a function that lists them) put together, kept under ``key`` until one of ``srcs`` changes."""
+    r = _RECIPES.get(key)
+    if r is None or any(ref() is not t for ref, t in zip(r.srcs, srcs)) or r.device != srcs[0].device:
+        old, r = r, _Recipe(srcs, blocks(), out_spec)
+        with _RECIPE_LOCK:
+            if old is not None:
+                _GROUPS[old.group].pop(key, None)
+            _RECIPES[key] = r
+            _GROUPS.setdefault(r.group, {})[key] = r
+            if len(_RECIPES) > 4096:                   # parameters of discarded models: drop what is dead
+                for k in [k for k, v in _RECIPES.items() if v.sources() is None]:
+                    _GROUPS[_RECIPES.pop(k).group].pop(k, None)
+                for g in [g for g, v in _GROUPS.items() if not v]:
+                    del _GROUPS[g]
+    out = r.out
+    if out is None or r.stamp != _stamp(srcs):
+        out = _rebuild(r, srcs)
+    elif not r.used:
+        r.stream, r.used = torch._C._cuda_getCurrentRawStream(r.device.index), True
+    return out
 
 
 def operand_copy(weight: torch.Tensor, dtype, transpose: bool = False, index: Optional[torch.Tensor] = None,
                  tag: str = "") -> torch.Tensor:
     """``weight[index].to(dtype)`` (``.t()`` when ``transpose``), contiguous, cached until the weight changes."""
+    if index is None and weight.dim() == 2 and weight.is_leaf and dtype in _KIND and _plain_sources((weight,)):
+        n, k = weight.shape
+        return recipe_copy((id(weight), dtype, bool(transpose), tag), (weight,),
+                           lambda: ((0, 0, n, k, 0, n if transpose else k, int(transpose)),),
+                           (_KIND[dtype], k, n) if transpose else (_KIND[dtype], n, k))
     key = (id(weight), dtype, bool(transpose), tag)
-    stamp = (_WEIGHT_GEN, weight._version, weight.data_ptr())
+    stamp = _stamp((weight,))
     hit = _WEIGHT_COPIES.get(key)
     if hit is not None and hit[0] == stamp and hit[2]() is weight:
         return hit[1]
-    import weakref
     w = weight.detach()
     if index is not None:
         w = w[index]

@@ -22,6 +22,9 @@ class FlatAdamW(torch.optim.Optimizer):
         self.buckets = buckets
         self.max_grad_norm = float(max_grad_norm)
         self._step = 0
+        self._written = [0]
+        from .gemm import watch_weights
+        watch_weights(params, self._written)
         self._flat_p: List[torch.Tensor] = []
         self._m: List[torch.Tensor] = []
         self._v: List[torch.Tensor] = []
@@ -47,8 +50,10 @@ class FlatAdamW(torch.optim.Optimizer):
     def step(self, closure=None):
         ext = _ext.load()
         self._step += 1
+        for b in self.buckets:
+            b.flat                                     # the gradients are in the bucket (not only once the launches are recorded)
         from .gemm import weights_changed
-        weights_changed()                              # the kernels below rewrite the parameters' storage directly
+        weights_changed(self._written)                 # the kernels below rewrite the parameters' storage directly
         g0 = self.param_groups[0]
         lr, (b1, b2), eps, wd = g0["lr"], g0["betas"], g0["eps"], g0["weight_decay"]
         clip = self.max_grad_norm > 0

@@ -6,8 +6,9 @@ mean over its local training nodes, and gradients are averaged over ranks.  Diff
 
 * the initial sync packs the whole ``state_dict`` into one flat buffer per dtype (one broadcast
   instead of one per tensor);
-* gradients live permanently inside flat fp32 buckets (``param.grad`` is a view), so there is no
-  copy-in / copy-out around the collective;
+* gradients live inside flat fp32 buckets (``param.grad`` is a view).  On the GPU the parameters let go of their views
+  before a backward pass, autograd keeps the tensors that its nodes produced, and one kernel gathers them into the bucket
+  (``csrc/param_kernels.cu``): accumulating into zeroed views took a launch a parameter;
 * on GPUs with symmetric memory the bucket is reduced by a one-shot kernel that reads every peer's
   bucket over NVLink, applies the 1/P scale and writes the result (``parallel/symm.py``); otherwise a
   single ``all_reduce`` is issued.
@@ -56,17 +57,44 @@ class _Bucket:
             off += (p.numel() + self.ALIGN - 1) // self.ALIGN * self.ALIGN
         self.n_valid = off                         # padded slots stay zero and are harmless to reduce / update
         n_pad = (off + 1023) // 1024 * 1024
-        self.flat = torch.zeros(n_pad, dtype=dtype, device=device)
+        self._flat = torch.zeros(n_pad, dtype=dtype, device=device)
+        self._native = None                        # release / gather of the gradients (fp32 on a GPU)
+        self._away = False                         # the gradients are with the parameters, not in the bucket
         self.symm = None                           # filled by parallel.symm when available
         self._bind()
 
+    @property
+    def flat(self) -> torch.Tensor:
+        """The bucket, with the gradients of the last backward pass in it."""
+        if self._away:
+            self.collect()
+        return self._flat
+
     def _bind(self):
+        self._native = None
+        if self._flat.is_cuda and self._flat.dtype == torch.float32:
+            from ..ops import _ext
+            self._native = _ext.load().GradBucket(list(self.params), list(self.offsets), self._flat)
+            self._native.bind()
+            return
         for p, off in zip(self.params, self.offsets):
-            p.grad = self.flat[off:off + p.numel()].view_as(p)
+            p.grad = self._flat[off:off + p.numel()].view_as(p)
+
+    def let_go(self) -> None:
+        """Before a backward pass: gradients start from nothing."""
+        self._native.release()
+        self._away = True
+
+    def collect(self) -> None:
+        """Behind a backward pass: every gradient, or zeros, into the bucket; ``param.grad`` is a view of it again."""
+        self._away = False
+        self._native.gather()
+        from ..ops import _ext
+        _ext.count_launches(1)
 
     def rebind_to(self, flat: torch.Tensor):
         flat[: self.flat.numel()].copy_(self.flat)
-        self.flat = flat
+        self._flat = flat
         self._bind()
 
 
@@ -105,8 +133,13 @@ class GradientReducer:
             self._symm_ok = False
 
     def prepare_backward(self) -> None:
-        """Grads accumulate into the bucket views; they must start from zero every step."""
+        """Gradients must start from zero every step."""
         for b in self.buckets:
+            if b._native is not None:
+                b.let_go()
+                if getattr(b, "norm", None) is not None:
+                    b.norm["ready"] = False
+                continue
             for p in b.params:
                 if p.grad is None or p.grad.data_ptr() < b.flat.data_ptr() or \
                         p.grad.data_ptr() >= b.flat.data_ptr() + b.flat.numel() * b.flat.element_size():
@@ -117,6 +150,8 @@ class GradientReducer:
                 b.norm["ready"] = False
 
     def finalize_backward(self) -> None:
+        for b in self.buckets:
+            b.flat                                 # gathers what the backward pass left with the parameters
         if self.world_size <= 1:
             return
         for b in self.buckets:
@@ -132,7 +167,7 @@ class GradientReducer:
                 profile_call("grad_all_reduce", _run, device=b.flat.device, payload_bytes=nbytes)
 
     def grad_views_ok(self) -> bool:
-        return all(p.grad is not None for b in self.buckets for p in b.params)
+        return all(b.flat is not None for b in self.buckets) and all(p.grad is not None for b in self.buckets for p in b.params)
 
 
 def build_gradient_reducer(model, process_group=None, bucket_cap_mb: float = 25.0, world_size: Optional[int] = None,
