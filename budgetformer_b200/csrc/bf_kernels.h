@@ -78,8 +78,8 @@ typedef struct {
   void *dq, *dk, *dv;               // [n, hl, hn], common row stride ldg (elements; 0 = hl*hn)
   long long ldg;
   float* zd;                        // [n, hl, 2] fp32 workspace: 1 / (Z + eps) and <dout, out> of every row
-  float* ds;                        // [E, hl] fp32 workspace: score gradients, from the dK/dV pass to the dQ pass.  Not used where
-                                    // bf_attn_bwd_keeps_scores is 0; NULL (untyped edges only): they are computed twice
+  float* ds;                        // [E, hl] fp32 workspace: score gradients, from the dK/dV pass to the dQ pass.  Worth its memory where
+                                    // bf_attn_bwd_keeps_scores is 1; NULL (untyped edges only): they are computed twice
   const int *t_row, *t_eid;         // edges grouped by key: query, and position in the query-grouped list
   float* detab;                     // zero-filled [2, hl, hn] fp32 or NULL
   bf_long_rows long_rows;           // scratch row: hl*hn floats
@@ -100,11 +100,12 @@ typedef struct {
 
 int bf_edge_attn_fwd(const bf_attn_params* p, cudaStream_t st);
 // as above; additionally every output row is stored into its owner's buffer (route may be NULL), and long rows come as
-// work items (long_rows may be NULL; its scratch has bf_attn_fwd_long_pitch floats per item); n_edges chooses between two kernels
+// work items (long_rows may be NULL; its scratch has bf_attn_fwd_long_pitch floats per item); n_edges and irregular (no bound on the
+// row length is known, rows differ) choose between two kernels
 int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_route* route, const bf_long_rows* long_rows, long long n_edges,
-                            cudaStream_t st);
+                            int irregular, cudaStream_t st);
 size_t bf_attn_fwd_long_pitch(int hl, int hn);
-int bf_attn_bwd_keeps_scores(int dtype, long long n, int hl, int hn, int variant);
+int bf_attn_bwd_keeps_scores(int dtype, long long n, int hl, int hn, int variant, long long n_edges, int irregular);
 int bf_edge_attn_bwd(const bf_attn_params* p, const bf_attn_bwd_params* q, cudaStream_t st);
 
 // ---- attention-graph construction (edge_build.cu) -------------------------------------------

@@ -115,6 +115,10 @@ LongRows take_long_rows(const Tensor& rowptr, int64_t n_edges, int64_t known_max
   return r;
 }
 
+// Whether the query rows may differ in length: no bound is known and the list holds whatever row is long.  (A list from a higher
+// length on belongs to a graph of bounded rows with a few virtual nodes.)
+int rows_irregular(int64_t known_max, int64_t list_min) { return known_max < 0 && list_min <= BF_LONG_ROW; }
+
 // out_drop = {p, seed, rows per owning rank, column offset} or empty: dropout fused into the attention output
 void fill_common(bf_attn_params& p, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out,
                  const Tensor& z, const Tensor& rowptr, const Tensor& col, const OptTensor& etype,
@@ -162,7 +166,7 @@ int64_t edge_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor
   fill_common(p, q, k, v, out, z, rowptr, col, etype, etab, variant, dropout_p, seed, out_drop);
   LongRows lr = take_long_rows(rowptr, col.numel(), known_max_degree, long_task, long_split, long_min, bf_attn_fwd_long_pitch(p.hl, p.hn));
   const bf_attn_route r = parse_route(route, 3);
-  check_cuda(bf_edge_attn_fwd_routed(&p, &r, &lr.c, col.numel(), at::cuda::getCurrentCUDAStream()), "edge_attn_fwd");
+  check_cuda(bf_edge_attn_fwd_routed(&p, &r, &lr.c, col.numel(), rows_irregular(known_max_degree, long_min), at::cuda::getCurrentCUDAStream()), "edge_attn_fwd");
   return 1 + (lr.c.n_task > 0 ? 3 : 0);
 }
 
@@ -191,7 +195,7 @@ int64_t edge_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor out, Tensor z, Tensor
   b.long_rows = lr.c;
   Tensor partial, qg;
   Tensor ds;
-  if (bf_attn_bwd_keeps_scores(p.dtype, p.n, p.hl, p.hn, p.variant)) {
+  if (bf_attn_bwd_keeps_scores(p.dtype, p.n, p.hl, p.hn, p.variant, col.numel(), rows_irregular(known_max_degree, long_min))) {
     // 4 bytes per edge and head (0.49 GB at 15.3 M edges of 8 heads), the largest thing a backward pass allocates: where it does not
     // fit, the scores are computed twice.  Typed edges have no such form.
     try {

@@ -399,53 +399,80 @@ struct Rows {
   long long base;
   int stride, n;
   bool on;
-  __device__ __forceinline__ bool bounds(const AttnArgs& a, int r, int& beg, int& len) const {
+  // of the group, whether or not this lane's head exists
+  __device__ __forceinline__ bool extent(const AttnArgs& a, int r, int& beg, int& len) const {
     beg = len = 0;
     const long long row = base + (long long)r * stride;
-    if (!on || row >= n) return false;
+    if (row >= n) return false;
     beg = __ldg(a.rowptr + row);
     len = __ldg(a.rowptr + row + 1) - beg;
     if (a.long_row > 0 && len > a.long_row) { len = 0; return false; }
     return true;
+  }
+  // of the lane
+  __device__ __forceinline__ bool bounds(const AttnArgs& a, int r, int& beg, int& len) const {
+    if (on && extent(a, r, beg, len)) return true;
+    beg = len = 0;
+    return false;
   }
 };
 
 // every segment takes at least one step, so that the ring never runs more than kRing segments ahead
 __device__ __forceinline__ int steps_of(int len) { return max(1, (int)__reduce_max_sync(kFull, (unsigned)len)); }
 
+// What a lane group reads of its edges ahead of them, one edge a lane: the chunk that the stream is in, the chunk behind it, and the first
+// chunk of the next segment.  A step takes its edge by a shuffle.  (With a load for every edge, one step ahead, each trip to memory for
+// a new sector of the list held all groups of the warp up: dK/dV and dQ of eight heads of 16, bf16, 300 k
+// nodes of ten edges 1070 us then and 902 now; 700 k packed nodes of eight 7431 and 6949 with the forward pass, twice over.)
+struct Chunk {
+  int now, next, other;
+  __device__ __forceinline__ int at(int gbase, int i, int mask) const { return __shfl_sync(kFull, now, gbase + (i & mask)); }
+};
+
 // The fetching side of a stream over rows, one warp-uniform step at a time: edge i of segment r, its key (and type).  The bounds
-// are read two segments ahead and the first key of a segment one segment ahead (the keys behind it mostly share its sector):
-// a chain of row pointer, key, row would otherwise stall every segment for two trips to memory.
+// are read two segments ahead and the first keys of a segment one segment ahead: a chain of row pointer, key, row would
+// otherwise stall every segment for two trips to memory.
 template <bool TYPED> struct RowFetch {
   int r, i, m, beg, len, beg1, len1, beg2, len2;
-  int key, key1, type, type1;
-  __device__ __forceinline__ void start(const AttnArgs& a, const Rows& rows, int n_seg) {
+  int lt, mask, gbase;           // lane in its group, group size - 1, first lane of the group
+  Chunk key_, type_;
+  __device__ __forceinline__ void read(const AttnArgs& a, int b, int n, int from, int& key, int& type) const {
+    if (from + lt < n) { key = __ldg(a.col + b + from + lt); if (TYPED) type = a.etype[b + from + lt]; }
+  }
+  __device__ __forceinline__ void start(const AttnArgs& a, const Rows& rows, int n_seg, int lane, int ltl) {
+    mask = (1 << ltl) - 1;
+    lt = lane & mask;
+    gbase = lane & ~mask;
     r = i = 0;
-    rows.bounds(a, 0, beg, len);
+    rows.extent(a, 0, beg, len);
     beg1 = len1 = beg2 = len2 = 0;
-    if (1 < n_seg) rows.bounds(a, 1, beg1, len1);
-    if (2 < n_seg) rows.bounds(a, 2, beg2, len2);
+    if (1 < n_seg) rows.extent(a, 1, beg1, len1);
+    if (2 < n_seg) rows.extent(a, 2, beg2, len2);
     m = steps_of(len);
-    key = key1 = type = type1 = 0;
-    if (len > 0) { key = __ldg(a.col + beg); if (TYPED) type = a.etype[beg]; }
-    if (len1 > 0) { key1 = __ldg(a.col + beg1); if (TYPED) type1 = a.etype[beg1]; }
+    key_.now = key_.next = key_.other = type_.now = type_.next = type_.other = 0;
+    read(a, beg, len, 0, key_.now, type_.now);
+    read(a, beg, len, mask + 1, key_.next, type_.next);
+    read(a, beg1, len1, 0, key_.other, type_.other);
   }
   __device__ __forceinline__ bool has() const { return i < len; }
   __device__ __forceinline__ int edge() const { return beg + i; }
+  __device__ __forceinline__ int key() const { return key_.at(gbase, i, mask); }        // by all lanes of the warp
+  __device__ __forceinline__ int type() const { return TYPED ? type_.at(gbase, i, mask) : 0; }
   __device__ __forceinline__ void advance(const AttnArgs& a, const Rows& rows, int n_seg) {
     if (r >= n_seg) return;
     if (++i == m) {
       i = 0;
       ++r;
-      beg = beg1; len = len1; key = key1; type = type1;      // empty past the last segment
+      beg = beg1; len = len1; key_.now = key_.other; type_.now = type_.other;      // empty past the last segment
       beg1 = beg2; len1 = len2;
       beg2 = len2 = 0;
-      if (len1 > 0) { key1 = __ldg(a.col + beg1); if (TYPED) type1 = a.etype[beg1]; }
-      if (r + 2 < n_seg) rows.bounds(a, r + 2, beg2, len2);
+      read(a, beg, len, mask + 1, key_.next, type_.next);
+      read(a, beg1, len1, 0, key_.other, type_.other);
+      if (r + 2 < n_seg) rows.extent(a, r + 2, beg2, len2);
       if (r < n_seg) m = steps_of(len);
-    } else if (i < len) {
-      key = __ldg(a.col + beg + i);
-      if (TYPED) type = a.etype[beg + i];
+    } else if ((i & mask) == 0) {
+      key_.now = key_.next; type_.now = type_.next;
+      read(a, beg, len, i + mask + 1, key_.next, type_.next);
     }
   }
 };
@@ -468,11 +495,12 @@ __global__ void __launch_bounds__(kStreamThreads, 4) edge_attn_fwd_kernel(AttnAr
   const unsigned long long skb = (unsigned long long)a.ldk * sizeof(T), svb = (unsigned long long)a.ldv * sizeof(T);
 
   RowFetch<false> f;
-  f.start(a, rows, n_seg);
+  f.start(a, rows, n_seg, lane, sg.ltl);
   auto issue = [&](int slot) {
-    if (f.has()) {
-      S::copy(ring[slot][0], tid, kb + (unsigned)f.key * skb);
-      S::copy(ring[slot][1], tid, vb + (unsigned)f.key * svb);
+    const unsigned key = (unsigned)f.key();
+    if (rows.on && f.has()) {
+      S::copy(ring[slot][0], tid, kb + key * skb);
+      S::copy(ring[slot][1], tid, vb + key * svb);
     }
     copy_commit();
     f.advance(a, rows, n_seg);
@@ -737,14 +765,15 @@ template <int NP> __device__ __forceinline__ void typed_sum(const float* et, int
 // leaves the score gradient of every (edge, head) in `ds` (fp32, at the edge's own position), so that the dQ pass gathers k alone.
 // The list holds the items of split keys (64 edges each), then the rest sorted by length.
 template <typename T, int HN, int VAR, bool PACKED>
-__global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bwd_kv_kernel(BwdArgs b, StreamGeo sg) {
+__global__ void __launch_bounds__(kStreamThreads, 3) edge_attn_bwd_kv_kernel(BwdArgs b, StreamGeo sg) {
   constexpr bool EXPH = VAR == 2;
-  constexpr int VN = EXPH ? Vec<T>::N : wide_elems<T, HN>(), NP = VN / 2, LPH = HN / VN;
+  constexpr int VN = wide_elems<T, HN>(), NP = VN / 2, LPH = HN / VN;
   using S = Slices<T, VN>;
   const AttnArgs& a = b.f;
   __shared__ uint4 ring[kRing][2][S::N][kStreamThreads];
   __shared__ float2 ring_zd[kRing][kStreamThreads];
   __shared__ int ring_eid[kRing][kStreamThreads];
+  __shared__ uint4 s_et[EXPH ? 2 : 1][EXPH ? VN / 4 : 1][32];       // the type table's part of this block's heads: slices of four, by lane
   const int tid = threadIdx.x, lane = tid & 31, lt = lane & ((1 << sg.ltl) - 1), groups = 32 >> sg.ltl;
   const int head = blockIdx.y * ((1 << sg.ltl) / LPH) + lt / LPH;
   const bool on = head < a.hl;
@@ -753,6 +782,14 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
   const long long warp = (long long)blockIdx.x * (kStreamThreads / 32) + (tid >> 5);
   const long long stride = (long long)gridDim.x * (kStreamThreads / 32) * groups;
   const long long warp0 = warp * groups, item0 = warp0 + (lane >> sg.ltl);
+  if (EXPH) {
+    for (int i = tid; i < 2 * (VN / 4) << sg.ltl; i += kStreamThreads) {
+      const int l = i & ((1 << sg.ltl) - 1), sl = (i >> sg.ltl) % (VN / 4), t = (i >> sg.ltl) / (VN / 4);
+      const int h = blockIdx.y * ((1 << sg.ltl) / LPH) + l / LPH;
+      if (h < a.hl) s_et[t][sl][l] = __ldg(reinterpret_cast<const uint4*>(a.etab + (long long)t * a.hl * HN + h * HN + (l % LPH) * VN) + sl);
+    }
+    __syncthreads();
+  }
   if (warp0 >= b.n_kv_task) return;             // the whole warp
   const int n_seg = (int)((b.n_kv_task - warp0 + stride - 1) / stride);
   auto item = [&](int r) {                      // key row, first edge, length, partial slot (-2: none)
@@ -776,43 +813,73 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
   }
   const char* zb = reinterpret_cast<const char*>(b.zd + hsafe);
   const unsigned long long szd = (unsigned long long)a.hl * sizeof(float2);
-  // fetching side: items two segments ahead, the first query of a segment one segment ahead (see RowFetch)
-  int fr = 0, fi = 0, fbeg, flen, beg1, len1, beg2, len2;
-  auto bounds = [&](int r, int& beg, int& len) { const int4 it = item(r); beg = it.y; len = it.z; };
-  bounds(0, fbeg, flen);
-  bounds(1, beg1, len1);
-  bounds(2, beg2, len2);
-  int fm = steps_of(flen);
-  int i_row = 0, eid_n = 0, i_row1 = 0, eid1 = 0;
-  if (flen > 0) { i_row = __ldg(b.t_row + fbeg); eid_n = __ldg(b.t_eid + fbeg); }
-  if (len1 > 0) { i_row1 = __ldg(b.t_row + beg1); eid1 = __ldg(b.t_eid + beg1); }
-  unsigned types = 0;                           // edge type of every ring slot; the newest is still on its way in `ty`
-  int ty = 0;
+  // fetching side: items two segments ahead, the first queries of a segment one segment ahead (see RowFetch); with edge types, whose
+  // place in memory comes from the list, a segment more
+  constexpr int AHEAD = EXPH ? 3 : 2;
+  const int mask = (1 << sg.ltl) - 1, gbase = lane & ~mask;
+  int fr = 0, fi = 0, fbeg[AHEAD + 1], flen[AHEAD + 1];
+  auto extent = [&](int r, int& beg, int& len) {
+    const long long t = item0 + r * stride;
+    beg = len = 0;
+    if (t < b.n_kv_task) { const int4 x = __ldg(b.kv_task + t); beg = x.y; len = x.z - x.y; }
+  };
+#pragma unroll
+  for (int s = 0; s <= AHEAD; ++s) extent(s, fbeg[s], flen[s]);
+  int fm = steps_of(flen[0]);
+  Chunk rowc{0, 0, 0}, eidc{0, 0, 0}, typec{0, 0, 0};
+  int row2 = 0, eid2 = 0;                       // typed: first chunk of the segment after the next
+  auto read = [&](int beg, int len, int from, int& row, int& eid) {
+    if (from + lt < len) { row = __ldg(b.t_row + beg + from + lt); eid = __ldg(b.t_eid + beg + from + lt); }
+  };
+  auto read_type = [&](int len, int from, int eid, int& type) {
+    if (EXPH && from + lt < len) type = __ldg(a.etype + eid);
+  };
+  read(fbeg[0], flen[0], 0, rowc.now, eidc.now);
+  read(fbeg[0], flen[0], mask + 1, rowc.next, eidc.next);
+  read(fbeg[1], flen[1], 0, rowc.other, eidc.other);
+  read_type(flen[0], 0, eidc.now, typec.now);
+  if (EXPH) {
+    if (mask == 0) read_type(flen[0], 1, eidc.next, typec.next);
+    read(fbeg[2], flen[2], 0, row2, eid2);
+    read_type(flen[1], 0, eidc.other, typec.other);
+  }
+  unsigned types = 0;                           // edge type of every ring slot
   auto issue = [&](int slot) {
-    if (EXPH) {
-      const int prev = (slot + kRing - 1) & (kRing - 1);
-      types = (types & ~(1u << prev)) | ((ty ? 1u : 0u) << prev);
-    }
-    if (fi < flen) {
-      S::copy(ring[slot][0], tid, qb + (unsigned)i_row * sq);
-      S::copy(ring[slot][1], tid, gb + (unsigned)i_row * sgr);
-      copy_async<8>(&ring_zd[slot][tid], zb + (unsigned)i_row * szd);
-      ring_eid[slot][tid] = eid_n;
-      if (EXPH) ty = a.etype[eid_n];
+    const unsigned i_row = (unsigned)rowc.at(gbase, fi, mask);
+    const int eid = eidc.at(gbase, fi, mask);
+    const int ty = EXPH ? typec.at(gbase, fi, mask) : 0;
+    if (on && fi < flen[0]) {
+      S::copy(ring[slot][0], tid, qb + i_row * sq);
+      S::copy(ring[slot][1], tid, gb + i_row * sgr);
+      copy_async<8>(&ring_zd[slot][tid], zb + i_row * szd);
+      ring_eid[slot][tid] = eid;
+      if (EXPH) types = (types & ~(1u << slot)) | ((ty ? 1u : 0u) << slot);
     }
     copy_commit();
     if (fr >= n_seg) return;
     if (++fi == fm) {
       fi = 0;
       ++fr;
-      fbeg = beg1; flen = len1; i_row = i_row1; eid_n = eid1;
-      beg1 = beg2; len1 = len2;
-      if (len1 > 0) { i_row1 = __ldg(b.t_row + beg1); eid1 = __ldg(b.t_eid + beg1); }
-      bounds(fr + 2, beg2, len2);
-      if (fr < n_seg) fm = steps_of(flen);
-    } else if (fi < flen) {
-      i_row = __ldg(b.t_row + fbeg + fi);
-      eid_n = __ldg(b.t_eid + fbeg + fi);
+      rowc.now = rowc.other; eidc.now = eidc.other; typec.now = typec.other;
+#pragma unroll
+      for (int s = 0; s < AHEAD; ++s) { fbeg[s] = fbeg[s + 1]; flen[s] = flen[s + 1]; }
+      read(fbeg[0], flen[0], mask + 1, rowc.next, eidc.next);
+      if (EXPH) {
+        if (mask == 0) read_type(flen[0], 1, eidc.next, typec.next);
+        rowc.other = row2; eidc.other = eid2;
+        read_type(flen[1], 0, eidc.other, typec.other);
+        read(fbeg[2], flen[2], 0, row2, eid2);
+      } else {
+        read(fbeg[1], flen[1], 0, rowc.other, eidc.other);
+      }
+      extent(fr + AHEAD, fbeg[AHEAD], flen[AHEAD]);
+      if (fr < n_seg) fm = steps_of(flen[0]);
+    } else if ((fi & mask) == 0) {
+      rowc.now = rowc.next; eidc.now = eidc.next; typec.now = typec.next;
+      read(fbeg[0], flen[0], fi + mask + 1, rowc.next, eidc.next);
+      if (EXPH && mask == 0) read_type(flen[0], fi + 1, eidc.next, typec.next);
+    } else if (EXPH && (fi & mask) == ((mask + 1) >> 1)) {
+      read_type(flen[0], (fi & ~mask) + mask + 1, eidc.next, typec.next);      // the next chunk's, half a chunk ahead
     }
   };
 #pragma unroll
@@ -827,27 +894,17 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
   if (it.w != -2) { S::load(kb + (long long)it.x * a.ldk, kn); S::load(vb + (long long)it.x * a.ldv, vn); }
   int slot = 0;
   for (int r = 0; r < n_seg; ++r) {
-    f2 k0[NP], k1[NP], vf[NP], dk0[NP], dk1[NP], dv[NP];
+    f2 kf[NP], vf[NP], dk[NP], dv[NP];
     const float scale = inv_sqrt_hn<HN>();
-    S::spread(kn, k0);
+    S::spread(kn, kf);
     S::spread(vn, vf);
 #pragma unroll
-    for (int i = 0; i < NP; ++i) dk0[i] = dv[i] = pack2(0.f, 0.f);
-    if (EXPH) {
-      const float* et = a.etab + off;
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        dk1[i] = pack2(0.f, 0.f);
-        k1[i] = mul2(k0[i], pack2(__ldg(et + w_row + 2 * i), __ldg(et + w_row + 2 * i + 1)));
-        k0[i] = mul2(k0[i], pack2(__ldg(et + 2 * i), __ldg(et + 2 * i + 1)));
-      }
-    }
+    for (int i = 0; i < NP; ++i) dk[i] = dv[i] = pack2(0.f, 0.f);
     const int4 cur = it;
     it = itn;
     itn = item(r + 2);
     if (it.w != -2) { S::load(kb + (long long)it.x * a.ldk, kn); S::load(vb + (long long)it.x * a.ldv, vn); }
     const int m = steps_of(cur.z);
-    unsigned seen = 0;                          // edge types of the item: only their products count (0 * inf is not 0)
     for (int i = 0; i < m; ++i) {
       issue((slot + kRing - 1) & (kRing - 1));
       copy_wait<kRing - 1>();
@@ -856,17 +913,16 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
       S::read(ring[slot][1], tid, gf);
       const int eid = ring_eid[slot][tid];
       const float2 zd = ring_zd[slot][tid];
-      const bool t1 = EXPH && ((types >> slot) & 1u);
-      float d;
-      if (EXPH) {
-        f2 kk[NP];
+      if (EXPH) {                               // q * E of the edge's type enters the score and dK alike
+        const uint4 (*et)[32] = s_et[(types >> slot) & 1u];
 #pragma unroll
-        for (int u = 0; u < NP; ++u) kk[u] = t1 ? k1[u] : k0[u];
-        d = dot2<NP>(qf, kk);
-      } else {
-        d = dot2<NP>(qf, k0);
+        for (int u = 0; u < NP; u += 2) {
+          const uint4 e = et[u / 2][lt];
+          qf[u] = mul2(qf[u], pack2(__uint_as_float(e.x), __uint_as_float(e.y)));
+          qf[u + 1] = mul2(qf[u + 1], pack2(__uint_as_float(e.z), __uint_as_float(e.w)));
+        }
       }
-      d = head_sum<LPH>(d, kFull) * scale;
+      const float d = head_sum<LPH>(dot2<NP>(qf, kf), kFull) * scale;
       const float dotv = head_sum<LPH>(dot2<NP>(gf, vf), kFull);
       if (i < cur.z) {                          // a group whose item is over holds a stale slot: nothing of it is used
         const bool inr = (d > -kClamp) && (d < kClamp);
@@ -877,34 +933,20 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
         const float wn = w * mf;
         if ((lt % LPH) == 0) b.ds[(long long)eid * a.hl + head] = dss;
         const f2 s2 = pack2(dss, dss), w2 = pack2(wn, wn);
-        if (EXPH) {
-          seen |= t1 ? 2u : 1u;
-          if (t1) {
 #pragma unroll
-            for (int u = 0; u < NP; ++u) dk1[u] = fma2(s2, qf[u], dk1[u]);
-          } else {
-#pragma unroll
-            for (int u = 0; u < NP; ++u) dk0[u] = fma2(s2, qf[u], dk0[u]);
-          }
-        } else {
-#pragma unroll
-          for (int u = 0; u < NP; ++u) dk0[u] = fma2(s2, qf[u], dk0[u]);
-        }
+        for (int u = 0; u < NP; ++u) dk[u] = fma2(s2, qf[u], dk[u]);
 #pragma unroll
         for (int u = 0; u < NP; ++u) dv[u] = fma2(w2, gf[u], dv[u]);
       }
       slot = (slot + 1) & (kRing - 1);
     }
-    if (EXPH) {
-      typed_sum<NP>(a.etab + off, w_row, seen, dk0, dk1);
-    }
     if (cur.w == -1) {
-      S::store(grad_row<T>(b, b.dk, b.ck, cur.x) + off, dk0);
+      S::store(grad_row<T>(b, b.dk, b.ck, cur.x) + off, dk);
       S::store(grad_row<T>(b, b.dv, b.cv, cur.x) + off, dv);
     } else if (cur.w >= 0) {
       float* pp = b.kv_partial + (long long)cur.w * 2 * w_row + off;
 #pragma unroll
-      for (int i = 0; i < NP; i += 2) { store_pairs<float, 2>(pp + 2 * i, dk0 + i); store_pairs<float, 2>(pp + w_row + 2 * i, dv + i); }
+      for (int i = 0; i < NP; i += 2) { store_pairs<float, 2>(pp + 2 * i, dk + i); store_pairs<float, 2>(pp + w_row + 2 * i, dv + i); }
     }
   }
   copy_wait<0>();
@@ -913,8 +955,8 @@ __global__ void __launch_bounds__(kStreamThreads, VAR == 2 ? 4 : 3) edge_attn_bw
 // dQ, the second pass: dq_i = sum over the row's edges of ds * k_j [* E_type].  With the typed sums S_t = sum of ds * k_j over the
 // edges of type t, dq = S_0 * E_0 + S_1 * E_1 and dE_t += q_i * S_t: one product per edge and a few per row.
 template <typename T, int HN, bool EXPH>
-__global__ void __launch_bounds__(kStreamThreads, EXPH ? 4 : 7) edge_attn_bwd_q_kernel(BwdArgs b, StreamGeo sg) {
-  constexpr int VN = EXPH ? Vec<T>::N : wide_elems<T, HN>(), NP = VN / 2, LPH = HN / VN;
+__global__ void __launch_bounds__(kStreamThreads, EXPH ? 3 : 7) edge_attn_bwd_q_kernel(BwdArgs b, StreamGeo sg) {
+  constexpr int VN = wide_elems<T, HN>(), NP = VN / 2, LPH = HN / VN;
   using S = Slices<T, VN>;
   const AttnArgs& a = b.f;
   __shared__ uint4 ring[kRing][S::N][kStreamThreads];
@@ -937,13 +979,15 @@ __global__ void __launch_bounds__(kStreamThreads, EXPH ? 4 : 7) edge_attn_bwd_q_
   const float* dsb = b.ds + hsafe;
   if (n_seg > 0) {
     RowFetch<EXPH> f;
-    f.start(a, rows, n_seg);
+    f.start(a, rows, n_seg, lane, sg.ltl);
     unsigned types = 0;
     auto issue = [&](int slot) {
-      if (f.has()) {
-        S::copy(ring[slot], tid, kb + (unsigned)f.key * skb);
+      const unsigned key = (unsigned)f.key();
+      const int type = f.type();
+      if (rows.on && f.has()) {
+        S::copy(ring[slot], tid, kb + key * skb);
         copy_async<4>(&ring_ds[slot][tid], dsb + (long long)f.edge() * a.hl);
-        if (EXPH) types = (types & ~(1u << slot)) | ((f.type ? 1u : 0u) << slot);
+        if (EXPH) types = (types & ~(1u << slot)) | ((type ? 1u : 0u) << slot);
       }
       copy_commit();
       f.advance(a, rows, n_seg);
@@ -1479,8 +1523,8 @@ inline long long stream_warps(long long n, const StreamGeo& s, int per) {
 
 template <typename T, int HN, int VAR>
 void launch_kv(const BwdArgs& b, cudaStream_t st) {
-  constexpr int VN = VAR == 2 ? Vec<T>::N : wide_elems<T, HN>();
-  const StreamGeo s = stream_geo<HN, VN>(b.f.hl, b.n_kv_task, VAR == 2 ? 4 : 3, 8);
+  constexpr int VN = wide_elems<T, HN>();
+  const StreamGeo s = stream_geo<HN, VN>(b.f.hl, b.n_kv_task, 3, 8);
   const dim3 grid = stream_grid<HN, VN>(b.f.hl, stream_warps(b.n_kv_task, s, s.per), s);
   if (b.qg) edge_attn_bwd_kv_kernel<T, HN, VAR, true><<<grid, kStreamThreads, 0, st>>>(b, s);
   else edge_attn_bwd_kv_kernel<T, HN, VAR, false><<<grid, kStreamThreads, 0, st>>>(b, s);
@@ -1500,9 +1544,25 @@ void launch_kv(const BwdArgs& b, cudaStream_t st) {
 //   5.2 / 6.2, 50 k 35 / 41, 170 k (87 MB) 128 / 144, 300 k (154 MB) 231 / 221; 8 x 32, 110 k (113 MB) 148 / 153, 170 k (174 MB) 233 / 235, 300 k 420 /
 //   399; 8 x 8, 700 k (179 MB) 279 / 302
 // - typed edges (two scaled queries, a select per element): 8 x 32, 25 edges, 50 k 167 / 201, 390 k (400 MB) 1879 / 1893
-inline bool rows_forward(int dtype, long long n, int hl, int hn, int variant, bool out_dropout, long long n_edges) {
+//
+// The figures above, and the rule for them, are for query rows of much the same length (a budgeted graph: the builder's bound on the
+// row length is known, or only a few virtual nodes' rows exceed it).  A lane group of a stream walks several rows one after another and a warp
+// waits for its longest group, so rows that differ (an edge list with Poisson degrees, say: no bound is known) cost the streams 10 to
+// 30 % that a warp of one row does not lose.  Measured there with a cold L2, us, rows against streams; 4 / 10 / 20 edges a row:
+// - fp32, 4 x 64: 60 k (123 MB) 92 / 108, 143 / 225, 294 / 456; 150 k (307 MB) 223 / 192, 360 / 379, 652 / 767; 400 k (819 MB) 604 / 496, 1012 / 994,
+//   1783 / 1914; 8 x 8: 150 k (77 MB) 68 / 91, 102 / 199, 210 / 349; 400 k (205 MB) 174 / 143, 276 / 311, 495 / 540
+// - 16 bits, 8 x 8: 150 k (38 MB) 50 / 78, 76 / 164, 159 / 284; 400 k (102 MB) 123 / 120, 197 / 234, 353 / 386; 4 x 64: 60 k (61 MB) 66 / 79,
+//   103 / 154, 228 / 314; 150 k (154 MB) 155 / 119, 252 / 256, 480 / 470
+inline bool rows_forward(int dtype, long long n, int hl, int hn, int variant, bool out_dropout, long long n_edges, bool irregular) {
   const long long row = (long long)hl * hn * (dtype == BF_FP32 ? 4 : 2), gathered = 2 * n * row;
   if (variant == 2) return true;
+  if (irregular) {
+    const bool deep = n_edges >= 8 * n;
+    if (dtype == BF_FP32) return n_edges >= 16 * n || gathered <= (deep ? 320'000'000 : 200'000'000);
+    if (row <= 64) return gathered <= 200'000'000;
+    if (hn == 8) return gathered <= (deep ? 250'000'000 : out_dropout ? 200'000'000 : 120'000'000);
+    return gathered <= (out_dropout ? 120'000'000 : deep ? 100'000'000 : 64'000'000);
+  }
   if (dtype == BF_FP32 || row <= 64 || (hn == 8 && out_dropout)) return gathered <= 200'000'000;
   if (hn == 8) return gathered <= 100'000'000;
   if (out_dropout) return gathered <= 120'000'000;
@@ -1548,9 +1608,29 @@ inline size_t type_table_bytes(int w_row) { return sizeof(float) * 2 * (size_t)w
 // - fp32, rows of 512 bytes and more that stay in L2 (the dK/dV stream holds 12 warps an SM, this form 32): 8 x 16, 2 k 26 / 32, 10 k
 //   41 / 43, 50 k (51 MB) with 16 edges a row 219 / 253 and with five 121 / 111, 110 k (113 MB) 356 / 311; 4 x 64, 10 k (20 MB) 61 / 66,
 //   50 k (102 MB) 248 / 190; 8 x 8, 10 k 37 / 32, 50 k 136 / 117
-inline bool recomputed_backward(int dtype, long long n, int hl, int hn, int variant) {
+//
+// As in rows_forward, those are rows of much the same length.  Where no bound is known, with a cold L2, 4 / 10 / 20 edges a row:
+// - fp32, 8 x 8 (256 bytes): 60 k (31 MB) 103 / 97, 144 / 141, 257 / 254; 150 k (77 MB) 201 / 202, 305 / 322, 519 / 558; 4 x 64: 20 k (41 MB)
+//   136 / 142, 202 / 229, 309 / 375; 60 k (123 MB) 314 / 316, 457 / 513, 739 / 854 (416 / 400 where degrees are even); 150 k (307 MB) 687 / 604,
+//   1097 / 1027, 1798 / 1746
+// - 16 bits, 3 x 16 (96 bytes): 20 k 87 / 97, 97 / 111, 143 / 157; 400 k (77 MB) 336 / 408, 546 / 817, 921 / 1503; 8 x 8: 150 k (38 MB) 142 / 169,
+//   215 / 288, 368 / 472; 400 k (102 MB) 315 / 360, 514 / 603, 874 / 993; 4 x 64: 20 k (20 MB) 114 / 110, 136 / 134, 292 / 280; 60 k (61 MB)
+//   217 / 197, 317 / 301, 604 / 630; 400 k (410 MB) 1099 / 811, 1862 / 1411, 3301 / 2666
+// Heads that leave lanes of the streams' groups idle (12 x 16 in groups of 8 heads) are counted by what the groups hold.
+inline bool recomputed_backward(int dtype, long long n, int hl, int hn, int variant, long long n_edges, bool irregular) {
   const long long row = (long long)hl * hn * (dtype == BF_FP32 ? 4 : 2), gathered = 2 * n * row;
   if (variant == 2) return false;
+  if (irregular) {
+    const bool deep = n_edges >= 8 * n;
+    if (row <= 96) return true;
+    if (dtype == BF_FP32) return row <= 128 || gathered <= (deep ? 110'000'000 : 60'000'000);
+    if (hn == 8) return gathered <= 160'000'000;
+    const int lanes = hn / 16;                                                  // of a head: 32 bytes each
+    int heads = 1;                                                              // of a group
+    while (2 * heads * lanes <= 32 && 2 * heads <= hl) heads *= 2;
+    if (5 * ((hl + heads - 1) / heads * heads) > 6 * hl) return gathered <= (deep ? 110'000'000 : 30'000'000);
+    return gathered <= 10'000'000;
+  }
   if (row <= 32) return true;
   if (row <= 64) return gathered > 64'000'000;
   return dtype == BF_FP32 && row >= 512 && gathered <= 64'000'000;
@@ -1598,10 +1678,11 @@ cudaError_t launch_bwd_t(const BwdArgs& b, cudaStream_t st) {
   if (a.n > 0) {
     if (a.variant == 2) {
       // every block ends in 2 * Hl * HN atomics: longer streams where the rows allow it
-      constexpr int VN = Vec<T>::N;
-      const StreamGeo s = stream_geo<HN, VN>(a.hl, a.n, 4, 32);
-      if (type_table_bytes(w_row) + kRing * kStreamThreads * (sizeof(uint4) + sizeof(float)) > 48 * 1024 && type_table_bytes(w_row) <= 48 * 1024) {
-        // beside the ring (10 KB) the type table's gradient of rows above 4,864 elements goes over the default 48 KB of a block
+      constexpr int VN = wide_elems<T, HN>();
+      const StreamGeo s = stream_geo<HN, VN>(a.hl, a.n, 3, 32);
+      constexpr size_t ring = kRing * kStreamThreads * (VN * sizeof(T) + sizeof(float));
+      if (type_table_bytes(w_row) + ring > 48 * 1024 && type_table_bytes(w_row) <= 48 * 1024) {
+        // beside the ring (10 or 18 KB) the type table's gradient of wide rows goes over the default 48 KB of a block
         const cudaError_t e = cudaFuncSetAttribute(edge_attn_bwd_q_kernel<T, HN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
         if (e != cudaSuccess) return e;
       }
@@ -1690,12 +1771,12 @@ bool to_route(const bf_attn_route* r, int n, long long width, Route* out) {
 extern "C" size_t bf_attn_fwd_long_pitch(int hl, int hn) { return (size_t)fwd_pitch(hl * hn, hl); }
 
 extern "C" int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_route* route, const bf_long_rows* long_rows,
-                                       long long n_edges, cudaStream_t st) {
+                                       long long n_edges, int irregular, cudaStream_t st) {
   AttnArgs a = to_args(*p);
   if (!take_long_rows(long_rows, &a)) return (int)cudaErrorInvalidValue;
   if (!to_route(route, p->n, (long long)p->hl * p->hn, &a.route_out)) return (int)cudaErrorInvalidValue;
   const int chunks = p->max_hub_degree > 0 ? (p->max_hub_degree + BF_HUB_CHUNK - 1) / BF_HUB_CHUNK : 1;
-  const bool rows = rows_forward(p->dtype, p->n, p->hl, p->hn, p->variant, p->out_dropout_p > 0.f, n_edges);
+  const bool rows = rows_forward(p->dtype, p->n, p->hl, p->hn, p->variant, p->out_dropout_p > 0.f, n_edges, irregular != 0);
 #define CALL_FWD(T, H) (int)launch_fwd_t<T, H>(a, rows, chunks, st)
   BF_DISPATCH(p->dtype, p->hn, CALL_FWD);
 #undef CALL_FWD
@@ -1705,27 +1786,26 @@ extern "C" int bf_edge_attn_fwd_routed(const bf_attn_params* p, const bf_attn_ro
 extern "C" int bf_edge_attn_fwd(const bf_attn_params* p, cudaStream_t st) {
   AttnArgs a = to_args(*p);
   const int chunks = p->max_hub_degree > 0 ? (p->max_hub_degree + BF_HUB_CHUNK - 1) / BF_HUB_CHUNK : 1;
-  const bool rows = rows_forward(p->dtype, p->n, p->hl, p->hn, p->variant, p->out_dropout_p > 0.f, -1);       // the number of edges is not known here
+  const bool rows = rows_forward(p->dtype, p->n, p->hl, p->hn, p->variant, p->out_dropout_p > 0.f, -1, false);       // the number of edges is not known here
 #define CALL_FWD(T, H) (int)launch_fwd_t<T, H>(a, rows, chunks, st)
   BF_DISPATCH(p->dtype, p->hn, CALL_FWD);
 #undef CALL_FWD
   return (int)cudaErrorInvalidValue;
 }
 
-extern "C" int bf_attn_bwd_keeps_scores(int dtype, long long n, int hl, int hn, int variant) {
-  return recomputed_backward(dtype, n, hl, hn, variant) ? 0 : 1;
+extern "C" int bf_attn_bwd_keeps_scores(int dtype, long long n, int hl, int hn, int variant, long long n_edges, int irregular) {
+  return recomputed_backward(dtype, n, hl, hn, variant, n_edges, irregular != 0) ? 0 : 1;
 }
 
 extern "C" int bf_edge_attn_bwd(const bf_attn_params* p, const bf_attn_bwd_params* q, cudaStream_t st) {
   BwdArgs b;
   b.f = to_args(*p);
   if (b.f.n_hub > 0 || !take_long_rows(&q->long_rows, &b.f) || q->kv_task == nullptr) return (int)cudaErrorInvalidValue;
-  const bool keeps = bf_attn_bwd_keeps_scores(p->dtype, p->n, p->hl, p->hn, p->variant) != 0;
   if (p->variant == 2 && q->ds == nullptr) return (int)cudaErrorInvalidValue;
   b.dout = q->dout; b.dq = q->dq; b.dk = q->dk; b.dv = q->dv;
   b.ldg = q->ldg > 0 ? q->ldg : (long long)p->hl * p->hn;
   b.zd = reinterpret_cast<float2*>(q->zd);
-  b.ds = keeps ? q->ds : nullptr;
+  b.ds = q->ds;
   b.t_row = q->t_row; b.t_eid = q->t_eid; b.detab = q->detab;
   b.kv_task = reinterpret_cast<const int4*>(q->kv_task); b.n_kv_task = q->n_kv_task;
   b.kv_split = q->kv_split; b.n_kv_split = q->n_kv_split; b.n_kv_slots = q->n_kv_split > 0 ? q->n_kv_slots : 0; b.kv_partial = q->kv_partial;

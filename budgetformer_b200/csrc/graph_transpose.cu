@@ -25,7 +25,7 @@ namespace {
 // a row) its threads mark their rows' edges in shared memory and the block writes them out along memory.  Otherwise eight lanes
 // take a row, and rows above 64 edges (the virtual node's holds every node) are left to the whole block, one after the other.  Bound by the
 // bytes written: 15 M edges 83 us with eight lanes a row everywhere, 31 now; 169 k nodes and a row of all of them 44 us with that row on one
-// warp, @HUBROW@ now.
+// warp, 34 now.
 constexpr int kStaged = 8192;
 __global__ void __launch_bounds__(256) edge_rows_kernel(const int* __restrict__ rowptr, int n, int* __restrict__ erow, int* __restrict__ iota) {
   __shared__ uint8_t s_row[kStaged];

@@ -65,6 +65,45 @@ def test_attention_streams(n, heads, hn, max_deg, dtype, variant):
         assert float((a.double() - b.double()).norm()) <= tol * (float(b.double().norm()) + float(dout.double().norm())) + 1e-6
 
 
+@pytest.mark.parametrize("bounded", [True, False])
+@pytest.mark.parametrize("variant", ["plain", "gps", "exphormer"])
+@pytest.mark.parametrize("heads,hn,dtype", [(8, 16, torch.bfloat16), (3, 32, torch.float16), (5, 64, torch.bfloat16), (1, 128, torch.bfloat16),
+                                            (32, 8, torch.float16), (4, 16, torch.float32), (12, 16, torch.bfloat16), (2, 128, torch.float32)])
+def test_attention_chunks_of_edges(heads, hn, dtype, variant, bounded):
+    """Query rows and keys of 0 to 70 edges: one edge less than a lane group's chunk of the list, the chunk and one more, for groups of
+    every width, between empty ones.  With a known bound on the rows (streams) and without (a warp of one row)."""
+    from budgetformer_b200.graph.attn_graph import AttnGraph
+    from budgetformer_b200.ops.edge_attention import edge_attention
+    n = 1130
+    gen = torch.Generator().manual_seed(heads + hn)
+    deg = torch.where(torch.arange(n) % 8 == 1, torch.arange(n) % 71, torch.zeros((), dtype=torch.long))
+    a = torch.repeat_interleave(torch.arange(n), deg)
+    b = torch.randint(0, n, (a.numel(),), generator=gen)
+    edges = torch.cat([torch.stack([a, b]), torch.stack([b, a])], 1)
+    if variant == "exphormer":
+        edges = torch.cat([edges, torch.randint(0, 2, (1, edges.size(1)), generator=gen)])
+    graph = AttnGraph.from_edge_index(edges, n).to("cuda")
+    if bounded:
+        graph.max_degree = int((graph.rowptr[1:] - graph.rowptr[:-1]).max())
+        assert graph.max_degree <= 128 and graph.num_edges < 12 * n          # what keeps 16-bit rows on the streams
+    gen = torch.Generator(device="cuda").manual_seed(hn)
+    q, k, v, dout = (torch.randn(n, heads, hn, generator=gen, device="cuda").to(dtype) for _ in range(4))
+    tab = torch.randn(2, heads, hn, generator=gen, device="cuda") if variant == "exphormer" else None
+    p = 0.3 if variant == "gps" else 0.0
+    want = _reference(q, k, v, dout, graph, tab, variant, p, 5)
+    args = [x.requires_grad_() for x in (q, k, v)] + ([tab.requires_grad_()] if tab is not None else [])
+    out = edge_attention(q, k, v, graph, variant=variant, etable=tab, dropout_p=p, dropout_seed=5)
+    got = [out] + list(torch.autograd.grad(out, args, dout))
+    # bounds as in test_attention_streams
+    tol = {torch.float32: 2e-5, torch.float16: 4e-3, torch.bfloat16: 2.5e-2}[dtype]
+    rows = lambda t: t.double().flatten(1).norm(dim=1)
+    per_key = torch.bincount(graph.col.long(), minlength=n).double().clamp(min=1).sqrt() * heads ** 0.5 * hn ** 0.5
+    for i, (x, y) in enumerate(zip(got[:4], want[:4])):
+        assert bool((rows(x.double() - y.double()) <= tol * (rows(y) + (rows(dout) if i < 2 else per_key)) + 1e-6).all()), i
+    for x, y in zip(got[4:], want[4:]):
+        assert float((x.double() - y.double()).norm()) <= tol * (float(y.double().norm()) + float(dout.double().norm())) + 1e-6
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("heads,hn", [(1, 8), (1, 16), (1, 32), (2, 16), (4, 8)])
 def test_narrow_rows_keep_the_precision_of_dq(heads, hn, dtype):
