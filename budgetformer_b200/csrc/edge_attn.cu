@@ -1374,16 +1374,16 @@ __global__ void __launch_bounds__(256, 4) edge_attn_bwd_kv_rows_kernel(BwdArgs b
 
 // ---------------------------------------------------------------------------------------------
 // Rows cut into work items: their partial sums lie side by side in slot order.  Pass 1 gives every window of SPLIT_WINDOW
-// slots to a block, which adds the slots of each row inside its window (threads run along the columns, so every slot is one
-// coalesced read) and finishes the rows that lie in the window whole; of a row that goes on, the window's sum replaces its
-// first slot there.  Pass 2 adds those window sums for the rows that cross a window's end.  The association depends on the
+// slots to a block.  A warp takes 128 columns of one row's slots inside the window, four columns a lane, or every eighth slot of them
+// where there are more than eight, adds them and finishes the row if it lies in the window whole; of a row that goes on, the window's sum replaces its first slot there.  Pass 2 adds those window sums for the rows that cross a window's end.  The association depends on the
 // slot numbers alone: bit-reproducible.  A row of 10^6 edges (16 k slots) is thus 244 blocks and one short tail instead of
 // one block's walk, and 10^4 rows of two or three slots are a few hundred blocks instead of 10^4 (each of 1,024 threads):
-// both passes over the dK/dV slots take 84 us on a 612 k-node power-law graph at h = 256 (632 us with a block per row),
-// 42 us at 700 k nodes / h = 128 (78 us).
+// both passes over the dK/dV slots take 98 us on a 612 k-node power-law graph at h = 256 (632 us with a block per row),
+// 22 us at 700 k nodes / h = 128 (78 us).
 // ---------------------------------------------------------------------------------------------
 constexpr int SPLIT_WINDOW = 64;
-constexpr int SPLIT_THREADS = 256;
+constexpr int SPLIT_WARPS = 16;
+constexpr int SPLIT_THREADS = 256;               // of the second pass
 constexpr int SPLIT_FWD = 0, SPLIT_DQ = 1, SPLIT_KV = 2;
 
 // s[0 .. ncol) holds the finished sums of row `row`
@@ -1412,43 +1412,134 @@ __device__ __forceinline__ void split_finish(const BwdArgs& b, int row, int w, i
   }
 }
 
+// four columns from c on (all of one head) of the finished sums of row `row`; z: the head's sum of weights (forward)
+template <typename T> __device__ __forceinline__ void store4(T* p, const float* f) {
+  if constexpr (sizeof(T) == 4) {
+    *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
+  } else {
+    uint2 u;
+    T* t = reinterpret_cast<T*>(&u);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t[i] = from_float<T>(f[i]);
+    *reinterpret_cast<uint2*>(p) = u;
+  }
+}
 template <typename T, int MODE>
-__global__ void __launch_bounds__(SPLIT_THREADS) split_window_kernel(BwdArgs b, const int4* __restrict__ task, int n_slots,
-                                                                     float* partial, int pitch, int ncol, int w, int hn) {
-  extern __shared__ float s_sum[];            // [ncol]
-  __shared__ int s_key[SPLIT_WINDOW];
-  const int s0 = blockIdx.x * SPLIT_WINDOW, s1 = min(s0 + SPLIT_WINDOW, n_slots);
-  for (int i = threadIdx.x; i < s1 - s0; i += blockDim.x) s_key[i] = task[s0 + i].x;
-  const int before = s0 > 0 ? task[s0 - 1].x : -1, after = s1 < n_slots ? task[s1].x : -1;
+__device__ __forceinline__ void split_finish4(const BwdArgs& b, int row, int w, int hn, int c, float* f, float z) {
+  const AttnArgs& a = b.f;
+  if (MODE == SPLIT_FWD) {
+    float inv = 1.f / (z + kEps);
+    if (a.variant == 1) inv *= a.inv_keep;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      f[i] *= inv;
+      if (a.out_thresh) f[i] = keep_out(a, row, c + i) ? f[i] * a.out_inv_keep : 0.f;
+    }
+    store4<T>(static_cast<T*>(a.out) + (long long)row * w + c, f);
+    if (a.route_out.n_dest) store4<T>(routed<T>(a.route_out, row, c), f);
+    if (c % hn == 0) a.z[(long long)row * a.hl + c / hn] = z;
+  } else if (MODE == SPLIT_DQ) {
+    store4<T>(grad_row<T>(b, b.dq, b.cq, row) + c, f);
+  } else if (c < w) {
+    store4<T>(grad_row<T>(b, b.dk, b.ck, row) + c, f);
+  } else {
+    store4<T>(grad_row<T>(b, b.dv, b.cv, row) + c - w, f);
+  }
+}
+
+// Bound by the latency of a row's reads where there are few windows: with the block walking its rows one after the other, two barriers
+// each, a call took 20 to 35 us however few slots it had: 60 k nodes, 4 x 64 fp32, the three of a pass 99 us then and 31 now; 700 k nodes, 8 x 16
+// bf16, four dK/dV calls 141 and 64; one row of 41 windows 9 and 4.4.  (A long row's window by the warps of its columns alone: 31.)  Heads are of 128 columns at most, so that a warp's columns hold them whole.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(SPLIT_WARPS * 32) split_window_kernel(BwdArgs b, const int4* __restrict__ task, int n_slots,
+                                                                        float* partial, int pitch, int w, int hn) {
+  __shared__ int s_key[SPLIT_WINDOW], s_run[SPLIT_WINDOW + 1], s_first[2];
+  static_assert(SPLIT_WINDOW == 64 && SPLIT_WARPS % 8 == 0, "two warps look for the rows' first slots, eight share a long one");
+  const int s0 = blockIdx.x * SPLIT_WINDOW, n = min(SPLIT_WINDOW, n_slots - s0);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = threadIdx.x;
+  const int before = s0 > 0 ? task[s0 - 1].x : -1, after = s0 + n < n_slots ? task[s0 + n].x : -1;
+  unsigned firsts = 0;
+  if (warp < 2) {
+    const int key = t < n ? task[s0 + t].x : 0;
+    s_key[t] = key;
+    const bool first = t < n && (t == 0 || task[s0 + t - 1].x != key);
+    firsts = __ballot_sync(kFull, first);
+    if (lane == 0) s_first[warp] = __popc(firsts);
+  }
   __syncthreads();
-  for (int i = s0; i < s1;) {
-    const int key = s_key[i - s0];
-    int j = i + 1;
-    while (j < s1 && s_key[j - s0] == key) ++j;
-    const bool whole = !(i == s0 && before == key) && !(j == s1 && after == key);
-    for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
-      const float* pp = partial + (long long)i * pitch + c;
-      float acc[8];
+  const int runs = s_first[0] + s_first[1];
+  if (warp < 2 && (firsts >> lane & 1u)) s_run[(warp ? s_first[0] : 0) + __popc(firsts & ((1u << lane) - 1u))] = t;
+  if (t == 0) s_run[runs] = n;
+  __syncthreads();
+  const int width = MODE == SPLIT_KV ? 2 * w : w, chunks = (width + 127) / 128;
+  auto total = [](float x0, float x1, float x2, float x3, float x4, float x5, float x6, float x7) {
+    return ((x0 + x4) + (x2 + x6)) + ((x1 + x5) + (x3 + x7));
+  };
+  // the sums over the eight residues of the slot number in its run, in x, to the row or to the run's first slot
+  auto finish = [&](int i, int j, int c, const float4 (&x)[8], const float (&xz)[8]) {
+    const int key = s_key[i];
+    float f[4] = {total(x[0].x, x[1].x, x[2].x, x[3].x, x[4].x, x[5].x, x[6].x, x[7].x),
+                  total(x[0].y, x[1].y, x[2].y, x[3].y, x[4].y, x[5].y, x[6].y, x[7].y),
+                  total(x[0].z, x[1].z, x[2].z, x[3].z, x[4].z, x[5].z, x[6].z, x[7].z),
+                  total(x[0].w, x[1].w, x[2].w, x[3].w, x[4].w, x[5].w, x[6].w, x[7].w)};
+    const float z = MODE == SPLIT_FWD ? total(xz[0], xz[1], xz[2], xz[3], xz[4], xz[5], xz[6], xz[7]) : 0.f;
+    if (!(i == 0 && before == key) && !(j == n && after == key)) {
+      split_finish4<T, MODE>(b, key, w, hn, c, f, z);
+    } else {
+      float* first = partial + (long long)(s0 + i) * pitch;
+      *reinterpret_cast<float4*>(first + c) = make_float4(f[0], f[1], f[2], f[3]);
+      if (MODE == SPLIT_FWD && c % hn == 0) first[w + c / hn] = z;
+    }
+  };
+  for (int unit = warp; unit < runs * chunks; unit += SPLIT_WARPS) {
+    const int run = unit / chunks, c = (unit - run * chunks) * 128 + 4 * lane;
+    const int i = s_run[run], j = s_run[run + 1];
+    if (j - i > 8) continue;
+    float4 x[8];
+    float xz[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) acc[u] = 0.f;
-      int n = j - i;
-      for (; n >= 8; n -= 8, pp += 8 * (long long)pitch) {
+    for (int u = 0; u < 8; ++u) {
+      const float* pp = partial + (long long)(s0 + i + u) * pitch;
+      const bool on = c < width && u < j - i;
+      x[u] = on ? *reinterpret_cast<const float4*>(pp + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      xz[u] = MODE == SPLIT_FWD && on ? pp[w + c / hn] : 0.f;
+    }
+    __syncwarp();                               // all lanes of a head have read its sum of weights
+    if (c < width) finish(i, j, c, x, xz);
+  }
+  __shared__ float4 s_x[SPLIT_WARPS][32];
+  __shared__ float s_z[MODE == SPLIT_FWD ? SPLIT_WARPS : 1][32];
+  for (int run = 0; run < runs; ++run) {
+    const int i = s_run[run], j = s_run[run + 1];
+    if (j - i <= 8) continue;
+    for (int part = 0; part < chunks; part += SPLIT_WARPS / 8) {
+      const int c = (part + (warp >> 3)) * 128 + 4 * lane;
+      float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+      float sz = 0.f;
+      if (c < width) {
+        const float* pp = partial + (long long)(s0 + i) * pitch;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) acc[u] += pp[u * (long long)pitch];
+        for (int k = 0; k < SPLIT_WINDOW / 8; ++k) {
+          const int slot = 8 * k + (warp & 7);
+          if (slot < j - i) {
+            const float4 x = *reinterpret_cast<const float4*>(pp + (long long)slot * pitch + c);
+            sum.x += x.x; sum.y += x.y; sum.z += x.z; sum.w += x.w;
+            if (MODE == SPLIT_FWD) sz += pp[(long long)slot * pitch + w + c / hn];
+          }
+        }
       }
+      s_x[warp][lane] = sum;
+      if (MODE == SPLIT_FWD) s_z[warp][lane] = sz;
+      __syncthreads();
+      if ((warp & 7) == 0 && c < width) {
+        float4 x[8];
+        float xz[8];
 #pragma unroll
-      for (int u = 0; u < 7; ++u)
-        if (u < n) acc[u] += pp[u * (long long)pitch];
-      const float sum = ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
-      if (whole) s_sum[c] = sum;
-      else partial[(long long)i * pitch + c] = sum;
-    }
-    if (whole) {
-      __syncthreads();
-      split_finish<T, MODE>(b, key, w, hn, s_sum);
+        for (int u = 0; u < 8; ++u) { x[u] = s_x[warp + u][lane]; xz[u] = MODE == SPLIT_FWD ? s_z[warp + u][lane] : 0.f; }
+        finish(i, j, c, x, xz);
+      }
       __syncthreads();
     }
-    i = j;
   }
 }
 
@@ -1486,11 +1577,8 @@ void launch_split(const BwdArgs& b, const int4* task, int n_slots, const int* sp
   // instead, by a loop or a grid dimension, made the reduction of popular keys 15 to 65 % slower: 86 to 142 us a layer at 612 k nodes,
   // h = 256.)
   const size_t smem = sizeof(float) * ncol;
-  if (smem + sizeof(int) * SPLIT_WINDOW > 48 * 1024) {
-    cudaFuncSetAttribute(split_window_kernel<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(split_cross_kernel<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
-  split_window_kernel<T, MODE><<<(n_slots + SPLIT_WINDOW - 1) / SPLIT_WINDOW, SPLIT_THREADS, smem, st>>>(b, task, n_slots, partial, pitch, ncol, w, hn);
+  if (smem > 48 * 1024) cudaFuncSetAttribute(split_cross_kernel<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  split_window_kernel<T, MODE><<<(n_slots + SPLIT_WINDOW - 1) / SPLIT_WINDOW, SPLIT_WARPS * 32, 0, st>>>(b, task, n_slots, partial, pitch, w, hn);
   split_cross_kernel<T, MODE><<<n_split < 148 * 8 ? n_split : 148 * 8, SPLIT_THREADS, smem, st>>>(b, split, n_split, partial, pitch, ncol, w, hn);
 }
 

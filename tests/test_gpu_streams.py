@@ -104,6 +104,31 @@ def test_attention_chunks_of_edges(heads, hn, dtype, variant, bounded):
         assert float((x.double() - y.double()).norm()) <= tol * (float(y.double().norm()) + float(dout.double().norm())) + 1e-6
 
 
+@pytest.mark.parametrize("heads,hn,dtype", [(3, 8, torch.float16), (5, 64, torch.bfloat16), (2, 128, torch.float32), (9, 16, torch.float32)])
+def test_sums_of_cut_rows(heads, hn, dtype):
+    """Query rows and keys of two slots (of 64 edges) to several windows (of 64 slots), with eight slots and nine among them, side by side so
+    that windows start and end inside them; widths below, at and off a warp's 128 columns."""
+    from budgetformer_b200.graph.attn_graph import AttnGraph
+    from budgetformer_b200.ops.edge_attention import edge_attention
+    degs = torch.tensor([129, 512, 513, 576, 577, 0, 5, 1000, 4096, 4160, 130, 200, 8200, 640, 150, 3, 129, 600] + [140] * 30)
+    n, gen = 1200, torch.Generator().manual_seed(heads)
+    a = torch.repeat_interleave(torch.arange(len(degs)), degs)
+    b = torch.randint(100, n, (a.numel(),), generator=gen)
+    graph = AttnGraph.from_edge_index(torch.cat([torch.stack([a, b]), torch.stack([b, a])], 1), n).to("cuda")
+    gen = torch.Generator(device="cuda").manual_seed(hn)
+    q, k, v, dout = (torch.randn(n, heads, hn, generator=gen, device="cuda").to(dtype) for _ in range(4))
+    want = _reference(q, k, v, dout, graph, None, "plain", 0.0, 0)
+    args = [x.requires_grad_() for x in (q, k, v)]
+    out = edge_attention(*args, graph)
+    got = [out] + list(torch.autograd.grad(out, args, dout))
+    # bounds as in test_attention_streams, with the fp32 sums' share for rows of 8 k terms
+    tol = {torch.float32: 4e-5, torch.float16: 4e-3, torch.bfloat16: 2.5e-2}[dtype]
+    rows = lambda t: t.double().flatten(1).norm(dim=1)
+    per_key = torch.bincount(graph.col.long(), minlength=n).double().clamp(min=1).sqrt() * heads ** 0.5 * hn ** 0.5
+    for i, (x, y) in enumerate(zip(got, want)):
+        assert bool((rows(x.double() - y.double()) <= tol * (rows(y) + (rows(dout) if i < 2 else per_key)) + 1e-6).all()), i
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("heads,hn", [(1, 8), (1, 16), (1, 32), (2, 16), (4, 8)])
 def test_narrow_rows_keep_the_precision_of_dq(heads, hn, dtype):
