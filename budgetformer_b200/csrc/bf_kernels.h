@@ -333,6 +333,13 @@ int bf_bn_stats(const void* x, long long ldx, const float* shift /* [cols] or NU
                 float* s1 /* += sum (x - shift) */, float* s2 /* += sum (x - shift)^2 */, int dtype, cudaStream_t st);
 int bf_bn_bwd_reduce(const void* dy, long long lddy, const void* x, long long ldx, const float* mean, const float* rstd,
                      long long rows, int cols, float* dbeta /* += */, float* dgamma /* += */, int dtype, cudaStream_t st);
+// the sums' coefficients: out [5, cols] = mean, biased variance, 1 / std, a, b of y = x*a + b, with the running statistics (both or
+// neither) and their int64 count (or NULL) moved along; out [3, cols] = a, b, c0 of dx = dy*a + x*b + c0.  Rows: *count_dev, or count if NULL
+int bf_bn_finish(const float* s1, const float* s2, const float* count_dev, float count, const float* shift, const float* weight,
+                 const float* bias, float eps, int cols, float* out, float* run_mean, float* run_var, float momentum,
+                 long long* tracked, cudaStream_t st);
+int bf_bn_bwd_finish(const float* sb, const float* sg, const float* count_dev, float count, const float* mean, const float* rstd,
+                     const float* weight, float* out, int cols, cudaStream_t st);
 int bf_col_affine(const void* x, long long ldx, const void* in2, long long ld2, const float* a, const float* b,
                   const float* c0, void* y, long long ldy, long long rows, int cols, int dtype, cudaStream_t st);
 

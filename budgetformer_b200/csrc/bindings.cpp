@@ -873,6 +873,40 @@ std::vector<Tensor> bn_bwd_reduce(Tensor dy, Tensor x, Tensor mean, Tensor rstd)
   return {dbeta, dgamma};
 }
 
+// a vector of `cols` fp32 values on x's device, or NULL
+float* column_values(const OptTensor& t, const Tensor& like, const char* what) {
+  if (!t.has_value()) return nullptr;
+  TORCH_CHECK(t->device() == like.device() && t->scalar_type() == torch::kFloat && t->is_contiguous() && t->numel() == like.numel(),
+              what, ": contiguous fp32, one value a column");
+  return t->data_ptr<float>();
+}
+
+// [5, cols]: mean, biased variance, 1 / std and the coefficients a, b of y = x*a + b; moves the running statistics and their count
+Tensor bn_finish(Tensor s1, Tensor s2, OptTensor count_dev, double count, OptTensor shift, OptTensor weight, OptTensor bias, double eps,
+                 OptTensor run_mean, OptTensor run_var, double momentum, OptTensor tracked) {
+  TORCH_CHECK(s1.is_cuda() && (!count_dev.has_value() || (count_dev->is_cuda() && count_dev->scalar_type() == torch::kFloat && count_dev->numel() == 1)));
+  TORCH_CHECK(!tracked.has_value() || (tracked->device() == s1.device() && tracked->scalar_type() == torch::kLong && tracked->numel() == 1));
+  c10::cuda::CUDAGuard guard(s1.device());
+  Tensor out = torch::empty({5, s1.numel()}, s1.options());
+  check_cuda(bf_bn_finish(column_values(s1, s1, "s1"), column_values(s2, s1, "s2"), count_dev.has_value() ? count_dev->data_ptr<float>() : nullptr,
+                          (float)count, column_values(shift, s1, "shift"), column_values(weight, s1, "weight"), column_values(bias, s1, "bias"),
+                          (float)eps, (int)s1.numel(), out.data_ptr<float>(), column_values(run_mean, s1, "running mean"),
+                          column_values(run_var, s1, "running variance"), (float)momentum,
+                          tracked.has_value() ? (long long*)tracked->data_ptr<int64_t>() : nullptr, at::cuda::getCurrentCUDAStream()), "bn_finish");
+  return out;
+}
+
+// [3, cols]: the coefficients a, b, c0 of dx = dy*a + x*b + c0
+Tensor bn_bwd_finish(Tensor sb, Tensor sg, OptTensor count_dev, double count, Tensor mean, Tensor rstd, OptTensor weight) {
+  TORCH_CHECK(sb.is_cuda() && (!count_dev.has_value() || (count_dev->is_cuda() && count_dev->scalar_type() == torch::kFloat && count_dev->numel() == 1)));
+  c10::cuda::CUDAGuard guard(sb.device());
+  Tensor out = torch::empty({3, sb.numel()}, sb.options());
+  check_cuda(bf_bn_bwd_finish(column_values(sb, sb, "sb"), column_values(sg, sb, "sg"), count_dev.has_value() ? count_dev->data_ptr<float>() : nullptr,
+                              (float)count, column_values(mean, sb, "mean"), column_values(rstd, sb, "rstd"), column_values(weight, sb, "weight"),
+                              out.data_ptr<float>(), (int)sb.numel(), at::cuda::getCurrentCUDAStream()), "bn_bwd_finish");
+  return out;
+}
+
 // y = x*a + b, or y = in2*a + x*b + c0 when in2 is given (per-column fp32 coefficients)
 Tensor col_affine(Tensor x, OptTensor in2, Tensor a, Tensor b, OptTensor c0) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.stride(1) == 1);
@@ -1010,6 +1044,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gelu_dropout", &gelu_dropout);
   m.def("bn_stats", &bn_stats);
   m.def("bn_bwd_reduce", &bn_bwd_reduce);
+  m.def("bn_finish", &bn_finish);
+  m.def("bn_bwd_finish", &bn_bwd_finish);
   m.def("col_affine", &col_affine);
   m.def("f32_weight_grad", &f32_weight_grad);
   m.def("colsum", &colsum);

@@ -559,6 +559,52 @@ __global__ void __launch_bounds__(256) colstats_kernel(const T* __restrict__ x, 
   }
 }
 
+// From the column sums to the coefficients of col_affine, a thread a column.  Forward: `out` holds five rows of `cols` floats, mean,
+// variance (biased), 1 / std, a and b; the running statistics and their count move along when given (run_mean may be `shift`: a thread
+// reads its column before it writes it).  Backward: three rows, a, b and c0.  The number of rows is `count`, or *count_dev where the
+// sums come from several ranks.  Bound by the launch: 14 and 8 elementwise launches of 1.5 us each before, and one of 2 us now.
+struct BnFinish {
+  const float *s1, *s2, *count_dev, *shift, *weight, *bias;
+  float count, eps, momentum;
+  float *run_mean, *run_var, *out;
+  long long* tracked;
+  int cols;
+};
+__global__ void __launch_bounds__(128) bn_finish_kernel(BnFinish f) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c == 0 && f.tracked) ++*f.tracked;
+  if (c >= f.cols) return;
+  const float n = f.count_dev ? *f.count_dev : f.count;
+  const float m1 = f.s1[c] / n;
+  float var = f.s2[c] / n - m1 * m1;
+  if (var < 0.f) var = 0.f;                     // and NaN stays NaN
+  const float mean = m1 + (f.shift ? f.shift[c] : 0.f);
+  const float rstd = rsqrtf(var + f.eps);
+  const float a = (f.weight ? f.weight[c] : 1.f) * rstd;
+  f.out[c] = mean;
+  f.out[f.cols + c] = var;
+  f.out[2 * f.cols + c] = rstd;
+  f.out[3 * f.cols + c] = a;
+  f.out[4 * f.cols + c] = (f.bias ? f.bias[c] : 0.f) - mean * a;
+  if (f.run_mean) {
+    const float unbias = n / fmaxf(n - 1.f, 1.f);
+    f.run_mean[c] = f.run_mean[c] * (1.f - f.momentum) + f.momentum * mean;
+    f.run_var[c] = f.run_var[c] * (1.f - f.momentum) + f.momentum * (var * unbias);
+  }
+}
+// dx = g * rstd * (dy - mean(dy) - xhat * mean(dy * xhat)),  xhat = (x - mean) * rstd
+__global__ void __launch_bounds__(128) bn_bwd_finish_kernel(const float* __restrict__ sb, const float* __restrict__ sg,
+                                                            const float* __restrict__ count_dev, float count,
+                                                            const float* __restrict__ mean, const float* __restrict__ rstd,
+                                                            const float* __restrict__ weight, float* __restrict__ out, int cols) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  const float n = count_dev ? *count_dev : count, r = rstd[c], a = (weight ? weight[c] : 1.f) * r, g = sg[c] / n;
+  out[c] = a;
+  out[cols + c] = -a * r * g;
+  out[2 * cols + c] = a * (mean[c] * r * g - sb[c] / n);
+}
+
 // TWO = false: y = x*a + b;  TWO = true: y = in2*a + x*b + c0
 // A thread keeps one chunk of 8 columns, with its coefficients in registers, and walks the rows U at a time: U (or 2 U)
 // independent 16-byte loads in flight and no index division.  612 k x 256 bf16: 117 us (y = x*a + b) and 223 us (three matrices),
@@ -782,6 +828,22 @@ extern "C" int bf_bn_bwd_reduce(const void* dy, long long lddy, const void* x, l
 #define CALL(T) colstats_kernel<T, 2><<<(unsigned)blocks, 256, smem, st>>>((const T*)x, ldx, (const T*)dy, lddy, mean, rstd, rows, cols, dbeta, dgamma)
   BF_DT_SWITCH(dtype, CALL)
 #undef CALL
+  return (int)cudaGetLastError();
+}
+
+extern "C" int bf_bn_finish(const float* s1, const float* s2, const float* count_dev, float count, const float* shift, const float* weight,
+                            const float* bias, float eps, int cols, float* out, float* run_mean, float* run_var, float momentum,
+                            long long* tracked, cudaStream_t st) {
+  if (cols < 0 || (run_mean == nullptr) != (run_var == nullptr)) return (int)cudaErrorInvalidValue;
+  const BnFinish f{s1, s2, count_dev, shift, weight, bias, count, eps, momentum, run_mean, run_var, out, tracked, cols};
+  bn_finish_kernel<<<cols / 128 + 1, 128, 0, st>>>(f);
+  return (int)cudaGetLastError();
+}
+
+extern "C" int bf_bn_bwd_finish(const float* sb, const float* sg, const float* count_dev, float count, const float* mean,
+                                const float* rstd, const float* weight, float* out, int cols, cudaStream_t st) {
+  if (cols < 0) return (int)cudaErrorInvalidValue;
+  bn_bwd_finish_kernel<<<cols / 128 + 1, 128, 0, st>>>(sb, sg, count_dev, count, mean, rstd, weight, out, cols);
   return (int)cudaGetLastError();
 }
 

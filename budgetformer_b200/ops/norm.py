@@ -168,32 +168,44 @@ class _BatchNormTrain(torch.autograd.Function):
     ``E[(x-s)^2] - E[x-s]^2`` well conditioned), then one fused multiply-add per element.  With ``group`` the
     statistics and the backward reductions are summed over the ranks of the group, i.e. SyncBatchNorm over the
     sequence-parallel node shards; without it every rank normalises with its own rows like the reference.  CUDA
-    tensors run on the row kernels of ``csrc/norm_fused.cu``, anything else on the same arithmetic in PyTorch."""
+    tensors run on the row kernels of ``csrc/norm_fused.cu``, anything else on the same arithmetic in PyTorch.
+    ``running`` = (mean, variance, momentum, count or None) of fp32 buffers that the kernel between the two passes moves along."""
 
     @staticmethod
-    def forward(ctx, x, weight, bias, shift, eps, group):
+    def forward(ctx, x, weight, bias, shift, eps, group, running):
         s1, s2 = _bn_stats(x, shift)
-        count = torch.tensor([float(x.size(0))], device=x.device)
+        count, on_device = float(x.size(0)), None                   # rows: here, or summed over the ranks
         if group is not None:
             import torch.distributed as dist
-            packed = torch.cat([s1, s2, count])
+            packed = torch.cat([s1, s2, torch.tensor([count], device=x.device)])
             dist.all_reduce(packed, group=group)
             h = x.size(1)
-            s1, s2, count = packed[:h], packed[h:2 * h], packed[2 * h:]
-        m1 = s1 / count
-        var = (s2 / count - m1 * m1).clamp_min_(0.0)                # biased variance
-        mean = m1 + (shift if shift is not None else 0.0)
-        rstd = torch.rsqrt(var + eps)
-        g32 = weight.float() if weight is not None else torch.ones_like(mean)
-        b32 = bias.float() if bias is not None else torch.zeros_like(mean)
-        a = g32 * rstd
-        y = _col_affine(x, None, a, b32 - mean * a, None)
+            s1, s2, on_device = packed[:h], packed[h:2 * h], packed[2 * h:]
+        g32 = weight.float().contiguous() if weight is not None else None
+        b32 = bias.float().contiguous() if bias is not None else None
+        if x.is_cuda:
+            _ext.count_launches(1)
+            mean, var, rstd, a, b = _ext.load().bn_finish(s1, s2, on_device, count, shift, g32, b32, eps,
+                                                          *(running if running is not None else (None, None, 0.0, None))).unbind(0)
+            if running is not None:
+                torch.autograd.graph.increment_version([t for t in running if isinstance(t, torch.Tensor)])
+        else:
+            n = count if on_device is None else on_device
+            m1 = s1 / n
+            var = (s2 / n - m1 * m1).clamp_min_(0.0)                # biased variance
+            mean = m1 + (shift if shift is not None else 0.0)
+            rstd = torch.rsqrt(var + eps)
+            a = g32 * rstd if g32 is not None else rstd
+            b = (b32 if b32 is not None else 0.0) - mean * a
+        y = _col_affine(x, None, a, b, None)
         ctx.save_for_backward(x, mean, rstd, g32)
-        ctx.group, ctx.count = group, count
+        ctx.group, ctx.count = group, (count, on_device)
         ctx.pdtype = weight.dtype if weight is not None else torch.float32
         ctx.has_affine = (weight is not None, bias is not None)
-        ctx.mark_non_differentiable(mean, var, count)
-        return y, mean, var, count
+        ctx.mark_non_differentiable(mean, var)
+        if on_device is not None:
+            ctx.mark_non_differentiable(mean, var, on_device)
+        return y, mean, var, count if on_device is None else on_device
 
     @staticmethod
     def backward(ctx, dy, _dmean, _dvar, _dcount):
@@ -207,14 +219,19 @@ class _BatchNormTrain(torch.autograd.Function):
             packed = torch.cat([dbeta, dgamma])
             dist.all_reduce(packed, group=ctx.group)
             sb, sg = packed[:dbeta.numel()], packed[dbeta.numel():]
-        n = ctx.count
-        # dx = g*rstd * (dy - mean(dy) - xhat * mean(dy*xhat)),  xhat = (x - mean) * rstd
-        a = g32 * rstd
-        b = -a * rstd * (sg / n)
-        c0 = a * (-(sb / n) + mean * rstd * (sg / n))
+        count, on_device = ctx.count
+        if x.is_cuda:
+            _ext.count_launches(1)
+            a, b, c0 = _ext.load().bn_bwd_finish(sb, sg, on_device, count, mean, rstd, g32).unbind(0)
+        else:
+            # dx = g*rstd * (dy - mean(dy) - xhat * mean(dy*xhat)),  xhat = (x - mean) * rstd
+            n = count if on_device is None else on_device
+            a = g32 * rstd if g32 is not None else rstd
+            b = -a * rstd * (sg / n)
+            c0 = a * (-(sb / n) + mean * rstd * (sg / n))
         dx = _col_affine(x, dy, a, b, c0)
         has_w, has_b = ctx.has_affine
-        return dx, (dgamma.to(ctx.pdtype) if has_w else None), (dbeta.to(ctx.pdtype) if has_b else None), None, None, None
+        return dx, (dgamma.to(ctx.pdtype) if has_w else None), (dbeta.to(ctx.pdtype) if has_b else None), None, None, None, None
 
 
 def batch_norm(x: torch.Tensor, bn: torch.nn.BatchNorm1d, group=None) -> torch.Tensor:
@@ -224,13 +241,20 @@ def batch_norm(x: torch.Tensor, bn: torch.nn.BatchNorm1d, group=None) -> torch.T
     training = bn.training or not bn.track_running_stats
     synced = group is not None and torch.distributed.is_initialized() and torch.distributed.get_world_size(group) > 1
     if training and (_bn_kernel_ok(x) or synced):
+        tracked = bn.track_running_stats and bn.running_mean is not None
         shift = bn.running_mean.float().contiguous() if bn.running_mean is not None else None
-        y, mean, var, count = _BatchNormTrain.apply(x, bn.weight, bn.bias, shift, float(bn.eps), group if synced else None)
-        if bn.track_running_stats and bn.running_mean is not None:
+        running = None
+        # the statistics kernel moves plain fp32 buffers along; with a cumulative average the factor is known on the device only
+        if tracked and x.is_cuda and bn.momentum is not None and bn.num_batches_tracked.dtype == torch.int64 and all(
+                t.device == x.device and t.is_contiguous() for t in (bn.running_mean, bn.running_var, bn.num_batches_tracked)) and all(
+                t.dtype == torch.float32 for t in (bn.running_mean, bn.running_var)):
+            running = (bn.running_mean, bn.running_var, float(bn.momentum), bn.num_batches_tracked)
+        y, mean, var, count = _BatchNormTrain.apply(x, bn.weight, bn.bias, shift, float(bn.eps), group if synced else None, running)
+        if tracked and running is None:
             with torch.no_grad():
                 bn.num_batches_tracked += 1
                 mom = bn.momentum if bn.momentum is not None else 1.0 / float(bn.num_batches_tracked)
-                unbias = count / torch.clamp(count - 1.0, min=1.0)
+                unbias = count / (torch.clamp(count - 1.0, min=1.0) if isinstance(count, torch.Tensor) else max(count - 1.0, 1.0))
                 bn.running_mean.mul_(1 - mom).add_(mean.to(bn.running_mean.dtype), alpha=mom)
                 bn.running_var.mul_(1 - mom).add_((var * unbias).to(bn.running_var.dtype), alpha=mom)
         return y

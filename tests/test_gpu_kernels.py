@@ -321,6 +321,53 @@ def test_batch_norm_kernels_match_pytorch(dtype):
     assert (batch_norm(x, bn).float() - ref(x.float())).abs().max() < tol
 
 
+@pytest.mark.parametrize("h,affine,momentum,track,stats", [
+    (8, True, 0.1, True, torch.float32), (128, True, 0.3, True, torch.float32), (136, False, 0.1, True, torch.float32),
+    (64, True, None, True, torch.float32), (64, True, 0.1, False, torch.float32), (64, True, 0.1, True, torch.float64)])
+def test_batch_norm_coefficients_by_one_launch(h, affine, momentum, track, stats):
+    """Every form of the module: columns up to and past a block of the coefficient kernel, no affine part, a cumulative average, no
+    running statistics, running statistics of another type (these three move outside the kernel)."""
+    from budgetformer_b200.ops.norm import batch_norm
+    make = lambda: torch.nn.BatchNorm1d(h, affine=affine, momentum=momentum, track_running_stats=track)
+    gen = torch.Generator(device="cuda").manual_seed(h)
+    bn, ref = make().cuda(), make().cuda().double()
+    if track:
+        bn.running_mean, bn.running_var = bn.running_mean.to(stats), bn.running_var.to(stats)
+    for step in range(3):
+        x = torch.randn(1009, h, generator=gen, device="cuda") * 2 + 1 + step
+        xa, xb = x.clone().requires_grad_(), x.double().requires_grad_()
+        g = torch.randn(1009, h, generator=gen, device="cuda")
+        version = bn.running_mean._version if track else 0
+        ya, yb = batch_norm(xa, bn), ref(xb)
+        ya.backward(g); yb.backward(g.double())
+        # fp32 sums of 10^3 terms of size 1 to 10: 1e-5 of the result's scale
+        assert (ya - yb).abs().max() <= 1e-5 * yb.abs().max()
+        assert (xa.grad - xb.grad).abs().max() <= 1e-5 * xb.grad.abs().max()
+        if track:
+            assert int(bn.num_batches_tracked) == step + 1 and bn.running_mean._version > version
+            assert (bn.running_mean - ref.running_mean).abs().max() <= 1e-5 and (bn.running_var - ref.running_var).abs().max() <= 1e-4
+
+
+def test_batch_norm_coefficients_with_the_count_on_the_device():
+    """What a statistics group gives: sums and a number of rows that only the device knows."""
+    from budgetformer_b200.ops import _ext
+    ext, h = _ext.load(), 72
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    x, dy = (torch.randn(500, h, generator=gen, device="cuda") for _ in range(2))
+    count = torch.tensor([500.0], device="cuda")
+    for dev, host in ((count, 0.0), (None, 500.0)):
+        mean, var, rstd, a, b = ext.bn_finish(x.sum(0), (x * x).sum(0), dev, host, None, None, None, 1e-5, None, None, 0.0, None).unbind(0)
+        ref = x.double()
+        want = torch.nn.functional.batch_norm(ref, None, None, training=True, eps=1e-5)
+        assert (mean - ref.mean(0)).abs().max() < 1e-6 and (var - ref.var(0, unbiased=False)).abs().max() < 1e-5
+        assert (x * a + b - want).abs().max() < 1e-5
+        sb, sg = dy.sum(0), (dy * (x - mean) * rstd).sum(0)
+        a, b, c0 = ext.bn_bwd_finish(sb, sg, dev, host, mean, rstd, None).unbind(0)
+        xr = ref.requires_grad_()
+        torch.nn.functional.batch_norm(xr, None, None, training=True, eps=1e-5).backward(dy.double())
+        assert (dy * a + x * b + c0 - xr.grad).abs().max() < 1e-5
+
+
 @pytest.mark.parametrize("variant", ["plain", "gps", "exphormer"])
 def test_edge_attention_kernels_against_coo_oracle(variant):
     """Forward and backward of the CUDA kernels against the float32 oracle written on the reference's COO layout
