@@ -30,6 +30,7 @@ from __future__ import annotations
 
 import os
 import types
+import weakref
 from typing import List, Optional
 
 import torch
@@ -60,7 +61,7 @@ class SPContext:
         # seed shared by all ranks for masks that one rank generates and another regenerates (set by the trainer every
         # step from the run seed and the epoch; None = not set)
         self.step_seed: Optional[int] = None
-        self._packs = {}                                  # layer -> (stamp, packed W, packed bias, packed W transposed)
+        self._packs = {}                                  # layer -> (stamp, packed W, packed bias, packed W transposed or what makes it, Ws, references, recipe)
         self.P, self.rank = self.sw.world, self.sw.rank
         assert self.P == world
         self.rows_local, self.total_rows = int(rows_local), int(rows_local) * self.P
@@ -121,6 +122,13 @@ class SPContext:
         pack is rebuilt only when one of the six tensors changed since it was made."""
         ws, bs = (wq, wk, wv), (bq, bk, bv)
         h = self.h
+        parts = [t for t in (wq, wk, wv, bq, bk, bv) if t is not None]
+        stamp = [dtype] + gemm._stamp(parts)
+        hit = self._packs.get(layer)
+        if (hit is not None and hit[0] == stamp and len(hit[5]) == len(parts) and all(ref() is t for ref, t in zip(hit[5], parts))
+                and (hit[6] is None or hit[6].used)):
+            return hit[1], hit[2]
+        refs = tuple(weakref.ref(t) for t in parts)
         if (dtype in gemm._KIND and all(tuple(t.shape) == (h, h) and t.is_leaf for t in ws) and gemm._plain_sources(ws)
                 and (bq is None or all(t.shape == (h,) and t.is_leaf for t in bs) and gemm._plain_sources(bs))):
             def rows(transposed):
@@ -134,24 +142,21 @@ class SPContext:
                 b = gemm.recipe_copy(key + ("b",), bs, lambda: tuple(
                     (part, r * self.hl, self.hl, 1, (3 * r + i) * self.hl, 1, 0)
                     for r in range(self.P) for i, part in enumerate((1, 2, 0))), (gemm._KIND[torch.float32], 0, 3 * h))
-            self._packs[layer] = (None, w, b, lambda: gemm.recipe_copy(key + ("t",), ws, lambda: rows(True),
-                                                                       (gemm._KIND[dtype], h, 3 * h)), gemm._stamp(ws), ws)
+            self._packs[layer] = (stamp, w, b, lambda: gemm.recipe_copy(key + ("t",), ws, lambda: rows(True),
+                                                                        (gemm._KIND[dtype], h, 3 * h)), ws, refs, gemm._RECIPES.get(key + ("w",)))
             return w, b
-        parts = [t for t in (wq, wk, wv, bq, bk, bv) if t is not None]
-        stamp = (dtype,) + gemm._stamp(parts)
-        hit = self._packs.get(layer)
-        if hit is None or hit[0] != stamp:
-            w = torch.cat([wq, wk, wv], 0).detach().to(dtype)[self.perm].contiguous()
-            b = None if bq is None else torch.cat([bq, bk, bv], 0).detach().float()[self.perm].contiguous()
-            hit = self._packs[layer] = (stamp, w, b, w.t().contiguous())
-        return hit[1], hit[2]
+        w = torch.cat([wq, wk, wv], 0).detach().to(dtype)[self.perm].contiguous()
+        b = None if bq is None else torch.cat([bq, bk, bv], 0).detach().float()[self.perm].contiguous()
+        self._packs[layer] = (stamp, w, b, w.t().contiguous(), ws, refs, None)
+        return w, b
 
     def transposed_projection(self, layer: int, w: torch.Tensor) -> torch.Tensor:
         hit = self._packs.get(layer)
         if hit is None or hit[1] is not w:
             return w.t().contiguous()
-        if hit[0] is None:                                # made from the parameters, unless they changed since the pack was
-            return hit[3]() if gemm._stamp(hit[5]) == hit[4] else w.t().contiguous()
+        if callable(hit[3]):                              # made from the parameters, unless they changed since the pack was
+            now = gemm._stamp(hit[4])
+            return hit[3]() if now == hit[0][1:1 + len(now)] else w.t().contiguous()
         return hit[3]
 
     def unpack_rows(self, t: torch.Tensor):

@@ -53,11 +53,6 @@ def weights_changed(counter: Optional[list] = None) -> None:
         _WEIGHT_GEN += 1
 
 
-def _generation(t: torch.Tensor) -> int:
-    owner = _OWNERS.get(id(t))
-    return owner[1][0] if owner is not None and owner[0]() is t else 0
-
-
 class _Recipe:
     """A matrix made of blocks of fp32 matrices: ``blocks`` holds (source, first row, rows, columns, offset, row pitch, transposed)."""
 
@@ -77,7 +72,11 @@ class _Recipe:
 
 
 def _stamp(srcs):
-    return (_WEIGHT_GEN,) + tuple((t._version, t.data_ptr(), _generation(t)) for t in srcs)
+    out = [_WEIGHT_GEN]
+    for t in srcs:
+        owner = _OWNERS.get(id(t))
+        out += (t._version, t.data_ptr(), owner[1][0] if owner is not None and owner[0]() is t else 0)
+    return out
 
 
 def _rebuild(wanted: _Recipe, srcs) -> torch.Tensor:
@@ -148,13 +147,17 @@ def recipe_copy(key, srcs, blocks, out_spec) -> torch.Tensor:
 def operand_copy(weight: torch.Tensor, dtype, transpose: bool = False, index: Optional[torch.Tensor] = None,
                  tag: str = "") -> torch.Tensor:
     """``weight[index].to(dtype)`` (``.t()`` when ``transpose``), contiguous, cached until the weight changes."""
-    if index is None and weight.dim() == 2 and weight.is_leaf and dtype in _KIND and _plain_sources((weight,)):
-        n, k = weight.shape
-        return recipe_copy((id(weight), dtype, bool(transpose), tag), (weight,),
-                           lambda: ((0, 0, n, k, 0, n if transpose else k, int(transpose)),),
-                           (_KIND[dtype], k, n) if transpose else (_KIND[dtype], n, k))
     key = (id(weight), dtype, bool(transpose), tag)
     stamp = _stamp((weight,))
+    if index is None:
+        r = _RECIPES.get(key)
+        if r is not None and r.used and r.srcs[0]() is weight and r.stamp == stamp:
+            return r.out                               # a forward pass asks this a dozen times: before any other look at the tensor
+        # a tensor that is no parameter (a padded weight, made in every call) comes once: nothing to make beside it
+        if isinstance(weight, torch.nn.Parameter) and weight.dim() == 2 and weight.is_leaf and dtype in _KIND and _plain_sources((weight,)):
+            n, k = weight.shape
+            return recipe_copy(key, (weight,), lambda: ((0, 0, n, k, 0, n if transpose else k, int(transpose)),),
+                               (_KIND[dtype], k, n) if transpose else (_KIND[dtype], n, k))
     hit = _WEIGHT_COPIES.get(key)
     if hit is not None and hit[0] == stamp and hit[2]() is weight:
         return hit[1]
