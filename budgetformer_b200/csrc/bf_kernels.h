@@ -338,6 +338,9 @@ int bf_bn_bwd_reduce(const void* dy, long long lddy, const void* x, long long ld
 int bf_bn_finish(const float* s1, const float* s2, const float* count_dev, float count, const float* shift, const float* weight,
                  const float* bias, float eps, int cols, float* out, float* run_mean, float* run_var, float momentum,
                  long long* tracked, cudaStream_t st);
+// out [2, cols] = a, b of y = x*a + b from running statistics
+int bf_bn_running(const float* mean, const float* var, const float* weight, const float* bias, float eps, float* out, int cols,
+                  cudaStream_t st);
 int bf_bn_bwd_finish(const float* sb, const float* sg, const float* count_dev, float count, const float* mean, const float* rstd,
                      const float* weight, float* out, int cols, cudaStream_t st);
 int bf_col_affine(const void* x, long long ldx, const void* in2, long long ld2, const float* a, const float* b,

@@ -896,6 +896,18 @@ Tensor bn_finish(Tensor s1, Tensor s2, OptTensor count_dev, double count, OptTen
   return out;
 }
 
+// y = x*a + b with a and b from running statistics
+Tensor col_affine(Tensor x, OptTensor in2, Tensor a, Tensor b, OptTensor c0);
+Tensor bn_apply(Tensor x, Tensor mean, Tensor var, OptTensor weight, OptTensor bias, double eps) {
+  TORCH_CHECK(mean.device() == x.device() && mean.is_cuda() && x.dim() == 2 && mean.numel() == x.size(1));
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor out = torch::empty({2, mean.numel()}, mean.options());
+  check_cuda(bf_bn_running(column_values(mean, mean, "running mean"), column_values(var, mean, "running variance"),
+                           column_values(weight, mean, "weight"), column_values(bias, mean, "bias"), (float)eps, out.data_ptr<float>(),
+                           (int)mean.numel(), at::cuda::getCurrentCUDAStream()), "bn_running");
+  return col_affine(x, std::nullopt, out.select(0, 0), out.select(0, 1), std::nullopt);
+}
+
 // [3, cols]: the coefficients a, b, c0 of dx = dy*a + x*b + c0
 Tensor bn_bwd_finish(Tensor sb, Tensor sg, OptTensor count_dev, double count, Tensor mean, Tensor rstd, OptTensor weight) {
   TORCH_CHECK(sb.is_cuda() && (!count_dev.has_value() || (count_dev->is_cuda() && count_dev->scalar_type() == torch::kFloat && count_dev->numel() == 1)));
@@ -1046,6 +1058,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bn_bwd_reduce", &bn_bwd_reduce);
   m.def("bn_finish", &bn_finish);
   m.def("bn_bwd_finish", &bn_bwd_finish);
+  m.def("bn_apply", &bn_apply);
   m.def("col_affine", &col_affine);
   m.def("f32_weight_grad", &f32_weight_grad);
   m.def("colsum", &colsum);

@@ -346,6 +346,10 @@ def test_batch_norm_coefficients_by_one_launch(h, affine, momentum, track, stats
         if track:
             assert int(bn.num_batches_tracked) == step + 1 and bn.running_mean._version > version
             assert (bn.running_mean - ref.running_mean).abs().max() <= 1e-5 and (bn.running_var - ref.running_var).abs().max() <= 1e-4
+    bn.eval(), ref.eval()
+    with torch.no_grad():
+        ya, yb = batch_norm(x, bn), ref(x.double())
+    assert ya.dtype == x.dtype and (ya - yb).abs().max() <= 3e-5 * yb.abs().max()       # the running statistics' 1e-5 as well
 
 
 def test_batch_norm_coefficients_with_the_count_on_the_device():
