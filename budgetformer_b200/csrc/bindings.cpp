@@ -567,7 +567,7 @@ void gemm_tn_pull(std::vector<int64_t> src_ptrs, int64_t src_row_offset, int64_t
 // y = [x +] drop2(act(x W1^T + b1) W2^T + b2) with the hidden tile kept on chip (no autograd: forward-only uses)
 Tensor ffn_fused_fwd(Tensor x, Tensor w1, OptTensor b1, Tensor w2, OptTensor b2, int64_t act, bool residual, double p1,
                      int64_t seed1, double p2, int64_t seed2, Tensor status, OptTensor h_out, OptTensor relu_bits_out,
-                     OptTensor z_out = {}, OptTensor res = {}) {
+                     OptTensor z_out, OptTensor res, bool round_z) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.stride(1) == 1 &&
               (x.scalar_type() == torch::kBFloat16 || x.scalar_type() == torch::kHalf), "ffn_fused_fwd: x [M, h] 16-bit on CUDA");
   TORCH_CHECK(w1.is_cuda() && w2.is_cuda() && w1.is_contiguous() && w2.is_contiguous() && w1.scalar_type() == x.scalar_type() &&
@@ -610,6 +610,7 @@ Tensor ffn_fused_fwd(Tensor x, Tensor w1, OptTensor b1, Tensor w2, OptTensor b2,
                 z_out->size(1) == w1.size(0) && z_out->scalar_type() == x.scalar_type(), "ffn_fused_fwd: z_out [M, f] in the dtype of x");
     p.z_out = z_out->data_ptr(); p.ldz = z_out->stride(0);
   }
+  p.round_z = round_z ? 1 : 0;
   if (res.has_value()) {
     TORCH_CHECK(!residual && res->is_cuda() && res->dim() == 2 && res->stride(1) == 1 && res->size(0) == x.size(0) &&
                 res->size(1) == x.size(1) && res->scalar_type() == x.scalar_type(), "ffn_fused_fwd: res [M, h] in the dtype of x");
@@ -1037,10 +1038,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_tn_pull", &gemm_tn_pull);
   m.def("gemm_dw", &gemm_dw);
   m.def("ffn_fused_fwd", &ffn_fused_fwd);
-  m.def("ffn_fused_fwd", [](Tensor x, Tensor w1, OptTensor b1, Tensor w2, OptTensor b2, int64_t act, bool residual, double p1,
-                            int64_t seed1, double p2, int64_t seed2, Tensor status, OptTensor h_out, OptTensor relu_bits_out) {
-    return ffn_fused_fwd(x, w1, b1, w2, b2, act, residual, p1, seed1, p2, seed2, status, h_out, relu_bits_out);
-  });
   m.def("ffn_fused_supported", [](int64_t M, int64_t h, int64_t f) { return bf_ffn_fused_supported(M, (int)h, (int)f) != 0; });
   m.def("gemm_dw_supported", &gemm_dw_supported);
   m.def("gemm_supported", &gemm_supported);

@@ -17,7 +17,8 @@
 //
 // Without a backward pass the kernel moves X in and Y out.  A training forward asks for side outputs: the hidden matrix
 // (stored from registers, 64 bytes a lane, it took 95 us of 235 at 800 k rows); for ReLU one bit per element (value > 0); for GELU the pre-activation, rounded, of
-// which the activation is then taken.  Dropout masks are the hash masks of the GEMM epilogues, so a recomputation on the
+// which the activation is then taken (round_z: also without that output, so that evaluation and the first pass of a recomputed layer
+// give what a training pass gives).  Dropout masks are the hash masks of the GEMM epilogues, so a recomputation on the
 // two-GEMM path reproduces them.
 //
 // Bound by the ALU pipe of the epilogue: the dropout hash, selection and packing of a hidden element take a scheduler 18 cycles a warp,
@@ -62,6 +63,7 @@ struct FfnArgs {
   int* status;
   // side outputs of a training forward
   int keep_h, keep_z;
+  int round_z;                   // GELU of the pre-activation rounded to 16 bits
   unsigned short* bits_out;      // [F / 16, ldmb >= M] or null
   long long ldmb;
 };
@@ -273,7 +275,7 @@ ffn_fused_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         ff_load<32>(taddr, v);
         const int hcol = c * FF_HC + ucol;                   // hidden column of element 0
         ff_add_bias<32>(s_b1 + hcol, v);
-        if (SIDE && ACT == 2 && g.keep_z) {                  // what the backward pass differentiates at: the rounded value
+        if (ACT == 2 && g.round_z) {                         // what the backward pass differentiates at: the rounded value
           uint32_t w[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -281,7 +283,7 @@ ffn_fused_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
             w[i] = narrow16<FP16>(x.x, x.y);
             v[i] = widen16<FP16>(w[i]);
           }
-          put(w, map_z, hcol, tile_of(u / NU) * FF_M);
+          if (SIDE && g.keep_z) put(w, map_z, hcol, tile_of(u / NU) * FF_M);
         }
         if (ACT == 2) {
 #pragma unroll
@@ -456,6 +458,7 @@ extern "C" int bf_ffn_fused_fwd(const bf_ffn_params* p, cudaStream_t st) {
   g.status = p->status;
   g.keep_h = p->H_out != nullptr;
   g.keep_z = p->z_out != nullptr;
+  g.round_z = g.keep_z || p->round_z;
   g.bits_out = static_cast<unsigned short*>(p->relu_bits_out);
   g.ldmb = p->ldmb;
   if (g.keep_h && ((p->ldh * 2) % 16 != 0 || p->ldh < F)) return (int)cudaErrorInvalidValue;

@@ -32,11 +32,11 @@ ONCHIP_FFN_TRAIN = os.environ.get("BF_FFN_ONCHIP_TRAIN", "1") == "1"
 def ffn_onchip(x: torch.Tensor, w1, b1, w2, b2, *, act: str, residual: bool, p1: float = 0.0, seed1: int = 0,
                p2: float = 0.0, seed2: int = 0, h_out: Optional[torch.Tensor] = None,
                relu_bits_out: Optional[torch.Tensor] = None, z_out: Optional[torch.Tensor] = None,
-               other: Optional[torch.Tensor] = None) -> torch.Tensor:
+               other: Optional[torch.Tensor] = None, round_z: bool = False) -> torch.Tensor:
     """``[x +] drop2(act(x W1^T + b1) W2^T + b2)`` in one kernel; the ``[rows, ffn]`` hidden matrix never reaches HBM
     unless ``h_out`` asks for it as a side output (then it is written once and not read back; ``relu_bits_out`` receives
-    one bit per hidden element, value > 0; ``z_out`` the pre-activation of a GELU).  ``other`` is a residual that is not ``x``.  No
-    autograd.  Shapes: see ``onchip_supported``."""
+    one bit per hidden element, value > 0; ``z_out`` the pre-activation of a GELU, rounded, of which
+    the activation is then taken; ``round_z`` the same without that output).  ``other`` is a residual that is not ``x``.  No autograd.  Shapes: see ``onchip_supported``."""
     from . import _ext
     ext = _ext.load()
 
@@ -47,7 +47,7 @@ def ffn_onchip(x: torch.Tensor, w1, b1, w2, b2, *, act: str, residual: bool, p1:
         return b.clone() if b.data_ptr() % 16 else b
     y = ext.ffn_fused_fwd(x, gemm.operand_copy(w1, x.dtype), f32(b1), gemm.operand_copy(w2, x.dtype), f32(b2),
                           gemm.ACT[act], bool(residual), float(p1), int(seed1), float(p2), int(seed2),
-                          gemm.status_tensor(x.device), h_out, relu_bits_out, z_out, other)
+                          gemm.status_tensor(x.device), h_out, relu_bits_out, z_out, other, bool(round_z))
     _ext.count_launches(1)
     return y
 
@@ -188,8 +188,11 @@ def fused_ffn(x: torch.Tensor, w1, b1, w2, b2, *, act: str = "relu", residual: O
         # same order of seed draws as the two-GEMM forms below, so that a recomputation reproduces the masks
         s1 = new_seed() if p1 > 0 else 0
         s2 = new_seed() if p2 > 0 else 0
+        # GELU of the rounded pre-activation, as in training: evaluation and the first pass of a recomputed layer agree with it.  bf16 of
+        # width 128 without a residual of its own has always taken the unrounded one here.
+        round_z = act == "gelu" and not (x.dtype == torch.bfloat16 and x.size(1) == 128 and (residual is None or res_is_x))
         return ffn_onchip(x, w1, b1, w2, b2, act=act, residual=res_is_x, p1=p1, seed1=s1, p2=p2, seed2=s2,
-                          other=None if res_is_x else residual)
+                          other=None if res_is_x else residual, round_z=round_z)
     if ok and act == "relu":
         return _FusedFFNRelu.apply(x, w1, b1, w2, b2, residual, p1, p2, new_seed() if p1 > 0 else 0,
                                    new_seed() if p2 > 0 else 0, out_grad_colsum)

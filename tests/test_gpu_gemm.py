@@ -392,6 +392,26 @@ def test_ffn_on_chip_side_outputs_equal_the_two_gemm_form():
     _close(y_b, y_a.float(), torch.bfloat16)
 
 
+@pytest.mark.parametrize("h,dtype,other", [(128, torch.bfloat16, True), (64, torch.bfloat16, True), (64, torch.bfloat16, False),
+                                           (128, torch.float16, True), (64, torch.float16, False)])
+def test_gelu_block_evaluates_what_it_trains(h, dtype, other):
+    """Without gradients the block runs without side outputs; what it returns, with and without dropout, is what the training form
+    returns, bit for bit: both take the activation of the rounded pre-activation."""
+    from budgetformer_b200.ops.ffn import fused_ffn
+    torch.manual_seed(h)
+    x = torch.randn(1000, h, device="cuda").to(dtype)
+    res = torch.randn(1000, h, device="cuda").to(dtype) if other else x
+    l1, l2 = torch.nn.Linear(h, 2 * h).cuda(), torch.nn.Linear(2 * h, h).cuda()
+    for p in (0.0, 0.25):
+        got = []
+        for grad in (True, False):
+            torch.manual_seed(5)                              # the masks' seeds
+            with torch.set_grad_enabled(grad):
+                got.append(fused_ffn(x, l1.weight, l1.bias, l2.weight, l2.bias, act="gelu", residual=res, p1=p, p2=p))
+        assert got[0].grad_fn is not None and got[1].grad_fn is None
+        assert torch.equal(*got), p
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("h", [64, 128, 200, 512])
 def test_layernorm_kernel(dtype, h):
