@@ -57,6 +57,12 @@ __device__ __forceinline__ float ex2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+// min(|x|, 30), NaN of NaN (fminf would give 30, and GELU then 0)
+__device__ __forceinline__ float tail_arg(float x) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(fabsf(x)), "f"(30.f));
+  return r;
+}
 __device__ __forceinline__ float2 normal_tail2(float m0, float m1) {
   const f2 m = pack2(m0, m1);
   const float c[11] = {-1.f, -1.1511205434799194f, -0.4590774476528168f, -0.05285348370671272f, 0.007505788933485746f, -0.0004156184149906039f,
@@ -69,15 +75,15 @@ __device__ __forceinline__ float2 normal_tail2(float m0, float m1) {
 }
 __device__ __forceinline__ f2 gelu2(f2 v) {
   const float2 x = unpack2(v);
-  const float m0 = fminf(fabsf(x.x), 30.f), m1 = fminf(fabsf(x.y), 30.f);
+  const float m0 = tail_arg(x.x), m1 = tail_arg(x.y);
   const float2 e = normal_tail2(m0, m1);
-  // x >= 0: x - m e;  x < 0: x e (also where |x| is past the clamp)
+  // x >= 0: x - m e;  x < 0: x e (also where |x| is past the clamp);  NaN: e is
   return fma2(pack2(fminf(x.x, -m0), fminf(x.y, -m1)), pack2(e.x, e.y), pack2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
 }
 // d/dx of the above: Phi(x) + x * phi(x)
 __device__ __forceinline__ f2 gelu_grad2(f2 v) {
   const float2 x = unpack2(v);
-  const float2 e = normal_tail2(fminf(fabsf(x.x), 30.f), fminf(fabsf(x.y), 30.f));
+  const float2 e = normal_tail2(tail_arg(x.x), tail_arg(x.y));
   const float2 q = unpack2(mul2(mul2(v, v), pack2(-0.72134752f, -0.72134752f)));      // -x^2 / 2 in powers of two
   const f2 phi = mul2(pack2(0.3989422804f, 0.3989422804f), pack2(ex2_approx(q.x), ex2_approx(q.y)));
   return fma2(v, phi, pack2(x.x < 0.f ? e.x : 1.f - e.x, x.y < 0.f ? e.y : 1.f - e.y));
