@@ -142,6 +142,8 @@ void fill_common(bf_attn_params& p, const Tensor& q, const Tensor& k, const Tens
   p.dtype = dtype_code(q); p.variant = (int)variant;
   p.dropout_p = (float)dropout_p; p.dropout_seed = (uint32_t)seed;
   TORCH_CHECK(variant != 2 || (p.etype && p.etab), "exphormer variant needs edge types and a type table");
+  TORCH_CHECK(variant != 2 || (etab->is_contiguous() && etab->numel() >= 2 * q.size(1) * q.size(2) && ((uintptr_t)p.etab) % 16 == 0),
+              "the type table must be contiguous [2, heads, head_dim] on a 16-byte boundary");
 }
 
 // route = {} or {rows per destination, first row of this rank's slab, destination row stride (elements),

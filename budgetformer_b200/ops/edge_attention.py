@@ -130,6 +130,15 @@ class _EdgeAttentionCUDA(torch.autograd.Function):
         return dq, dk, dv, (detab.to(etable.dtype) if has_tab else None), None, None, None, None
 
 
+def type_table(etable: torch.Tensor) -> torch.Tensor:
+    """The edge-type table as the kernels read it: fp32, contiguous, two rows (a list of one type may come with one), and on a
+    16-byte boundary (a view into a larger tensor may start anywhere)."""
+    tab = etable.to(torch.float32).contiguous()
+    if tab.size(0) < 2:
+        tab = torch.cat([tab, tab.new_zeros((2 - tab.size(0),) + tab.shape[1:])])
+    return tab.clone() if tab.data_ptr() % 16 else tab
+
+
 _VARIANTS = {"plain": 0, "gps": 1, "exphormer": 2}
 
 
@@ -153,5 +162,5 @@ def edge_attention(
                                         dropout_p=dropout_p, dropout_seed=dropout_seed)
     if variant == "exphormer" and (etable is None or graph.etype is None):
         variant = "plain"
-    tab = etable.to(torch.float32).contiguous() if (variant == "exphormer") else None
+    tab = type_table(etable) if (variant == "exphormer") else None
     return _EdgeAttentionCUDA.apply(q, k, v, tab, graph, _VARIANTS[variant], float(dropout_p), int(dropout_seed))

@@ -40,7 +40,7 @@ from ..graph.attn_graph import AttnGraph, as_attn_graph
 from ..parallel import symm
 from . import _ext, gemm
 from ..utils import debug
-from .edge_attention import _VARIANTS
+from .edge_attention import _VARIANTS, type_table
 from .ffn import fused_ffn
 from .norm import ColsumSlot, batch_norm, hash_dropout, layer_norm, new_seed
 
@@ -458,7 +458,7 @@ def _attention(layer, x2d, graph: AttnGraph, sp: SPContext, idx: int, passthroug
     if variant == "exphormer" and (etab is None or graph.etype is None):
         variant, etab = "plain", None
     p_att = core.attention_dropout_rate if (variant == "gps" and layer.training) else 0.0
-    tab = etab.to(torch.float32).contiguous() if etab is not None else None
+    tab = type_table(etab) if etab is not None else None
     out = _PackedEdgeAttention.apply(qkv, tab, graph, sp, idx, _VARIANTS[variant], p_att, new_seed() if p_att > 0 else 0,
                                      float(out_p), int(out_seed))
     return (out, xr) if passthrough else out

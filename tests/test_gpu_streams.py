@@ -531,3 +531,30 @@ def test_row_element_kernels(rows, cols, dtype):
     assert bool(((hash_dropout(x, 5, 0.25).float() - want).abs() <= unit * want.abs() + 1e-7).all())
     want = torch.where(keep, torch.nn.functional.gelu(x.float()) * (1.0 / 0.75), torch.zeros((), device="cuda"))
     assert bool(((gelu_dropout(x, 5, 0.25).float() - want).abs() <= unit * want.abs() + 1e-6).all())
+
+
+def test_type_table_at_any_address():
+    """Tables that are views at odd offsets give what an aligned copy gives, forward and backward; so does one row for a list of one type."""
+    from budgetformer_b200.ops.edge_attention import edge_attention
+    from helpers import random_attn_graph
+    graph = random_attn_graph(typed=True).to("cuda")
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v, dout = (torch.randn(graph.rowptr.numel() - 1, 4, 16, generator=g, device="cuda").bfloat16() for _ in range(4))
+    flat = torch.randn(2 * 64 + 4, generator=g, device="cuda")
+
+    def grads(table):
+        args = [t.detach().requires_grad_() for t in (q, k, v, table)]
+        out = edge_attention(*args[:3], graph, variant="exphormer", etable=args[3])
+        return [out] + list(torch.autograd.grad(out, args, dout))
+
+    for off in (1, 2, 3):
+        view = flat[off:off + 128].view(2, 4, 16)
+        assert view.data_ptr() % 16
+        for x, y in zip(grads(view), grads(view.clone())):
+            assert torch.allclose(x.float(), y.float(), rtol=1e-5, atol=1e-5)     # the table's gradient meets in atomics
+    graph.etype.zero_()
+    table = flat[:128].view(2, 4, 16).clone()
+    one, two = grads(table[:1]), grads(table)
+    for x, y in zip(one[:4], two[:4]):
+        assert torch.equal(x, y)
+    assert torch.allclose(one[4], two[4][:1], rtol=1e-5, atol=1e-5)

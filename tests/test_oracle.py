@@ -149,3 +149,21 @@ def test_oracle_schedules_equal_the_schedulers():
     for step in (0, 1, 3, 5, 6, 50, 100, 130):
         assert abs(oracle.schedules.cosine_with_warmup(step, 5, 100, 1e-3) - cosine_with_warmup_value(step, 5, 100, 1e-3)) < 1e-12
         assert abs(oracle.schedules.polynomial_decay(step, 5, 100, 1e-3, 1e-9) - polynomial_decay_value(step, 5, 100, 1e-3, 1e-9, 1.0)) < 1e-12
+
+
+def test_type_table_is_laid_out_for_the_kernels():
+    """A table that starts off a 16-byte boundary, in another type, strided or of one row comes out aligned, fp32, contiguous and of two
+    rows, with its values and its gradient."""
+    from budgetformer_b200.ops.edge_attention import type_table
+    flat = torch.randn(4 * 2 * 3 * 8 + 8)
+    odd = flat[1:1 + 48].view(2, 3, 8)
+    assert odd.data_ptr() % 16 and odd.is_contiguous()
+    for t in (odd, odd.half(), flat[3:3 + 96].view(2, 3, 16)[..., ::2], odd[:1]):
+        t = t.detach().requires_grad_()
+        tab = type_table(t)
+        assert tab.dtype == torch.float32 and tab.is_contiguous() and tab.data_ptr() % 16 == 0 and tab.size(0) == 2
+        assert torch.equal(tab[:t.size(0)], t.float())
+        tab[:t.size(0)].sum().backward()
+        assert torch.equal(t.grad, torch.ones_like(t))
+    whole = torch.randn(2, 3, 8)
+    assert type_table(whole) is whole
