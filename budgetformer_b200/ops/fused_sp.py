@@ -61,7 +61,7 @@ class SPContext:
         # seed shared by all ranks for masks that one rank generates and another regenerates (set by the trainer every
         # step from the run seed and the epoch; None = not set)
         self.step_seed: Optional[int] = None
-        self._packs = {}                                  # layer -> (stamp, packed W, packed bias, packed W transposed or what makes it, Ws, references, recipe)
+        self._packs = {}                                  # layer -> (stamp, packed W, packed bias, packed W transposed or what makes it, Ws, references, recipes)
         self.P, self.rank = self.sw.world, self.sw.rank
         assert self.P == world
         self.rows_local, self.total_rows = int(rows_local), int(rows_local) * self.P
@@ -125,9 +125,12 @@ class SPContext:
         parts = [t for t in (wq, wk, wv, bq, bk, bv) if t is not None]
         stamp = [dtype] + gemm._stamp(parts)
         hit = self._packs.get(layer)
-        if (hit is not None and hit[0] == stamp and len(hit[5]) == len(parts) and all(ref() is t for ref, t in zip(hit[5], parts))
-                and (hit[6] is None or hit[6].used)):
-            return hit[1], hit[2]
+        if hit is not None and hit[0] == stamp and len(hit[5]) == len(parts) and all(ref() is t for ref, t in zip(hit[5], parts)):
+            made = [r.made for r in hit[6]]
+            if all(m is not None and m[1] is t for m, t in zip(made, hit[1:3])):
+                for r, m in zip(hit[6], made):
+                    r.take(m)
+                return hit[1], hit[2]
         refs = tuple(weakref.ref(t) for t in parts)
         if (dtype in gemm._KIND and all(tuple(t.shape) == (h, h) and t.is_leaf for t in ws) and gemm._plain_sources(ws)
                 and (bq is None or all(t.shape == (h,) and t.is_leaf for t in bs) and gemm._plain_sources(bs))):
@@ -135,19 +138,22 @@ class SPContext:
                 # destination-rank major, then k | v | q, then head columns: the runs of ``perm``
                 return tuple((part, r * self.hl, self.hl, h, (3 * r + i) * self.hl * (1 if transposed else h),
                               3 * h if transposed else h, int(transposed)) for r in range(self.P) for i, part in enumerate((1, 2, 0)))
-            key = (id(self), layer, dtype)
+            key = (id(self), layer, dtype, self.P, h)
             w = gemm.recipe_copy(key + ("w",), ws, lambda: rows(False), (gemm._KIND[dtype], 3 * h, h))
             b = None
             if bq is not None:                            # vectors are matrices of one column
                 b = gemm.recipe_copy(key + ("b",), bs, lambda: tuple(
                     (part, r * self.hl, self.hl, 1, (3 * r + i) * self.hl, 1, 0)
                     for r in range(self.P) for i, part in enumerate((1, 2, 0))), (gemm._KIND[torch.float32], 0, 3 * h))
-            self._packs[layer] = (stamp, w, b, lambda: gemm.recipe_copy(key + ("t",), ws, lambda: rows(True),
-                                                                        (gemm._KIND[dtype], h, 3 * h)), ws, refs, gemm._RECIPES.get(key + ("w",)))
+            recipes = tuple(gemm._RECIPES[key + (k,)] for k in ("w", "b")[:1 if b is None else 2])
+            if all(r.out is t for r, t in zip(recipes, (w, b))):          # not while a graph is recorded: nothing is in them yet
+                self._packs[layer] = (stamp, w, b, lambda: gemm.recipe_copy(key + ("t",), ws, lambda: rows(True),
+                                                                            (gemm._KIND[dtype], h, 3 * h)), ws, refs, recipes)
             return w, b
         w = torch.cat([wq, wk, wv], 0).detach().to(dtype)[self.perm].contiguous()
         b = None if bq is None else torch.cat([bq, bk, bv], 0).detach().float()[self.perm].contiguous()
-        self._packs[layer] = (stamp, w, b, w.t().contiguous(), ws, refs, None)
+        if not (w.is_cuda and torch.cuda.is_current_stream_capturing()):
+            self._packs[layer] = (stamp, w, b, w.t().contiguous(), ws, refs, ())
         return w, b
 
     def transposed_projection(self, layer: int, w: torch.Tensor) -> torch.Tensor:

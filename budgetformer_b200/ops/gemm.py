@@ -22,84 +22,165 @@ _STATUS = {}
 # The kernels take weights in the activation dtype (and the input-gradient GEMM takes them transposed, the packed projection several
 # in one).  Those copies only change when the weights do: they are kept per parameter and rebuilt when the parameter's version counter moves
 # (in-place updates by PyTorch optimizers, ``load_state_dict``) or when an optimizer that writes the storage of its parameters directly
-# announces a step (``ops.optim.FlatAdamW``: ``watch_weights``, ``weights_changed``).  Whoever finds a copy stale has all stale copies rebuilt that
-# were used on the same stream since they were last made: one launch (``csrc/param_kernels.cu``) in the place of one to three a copy.
+# announces a step (``ops.optim.FlatAdamW``: ``watch_weights``, ``weights_changed``).  A weight that belongs to no such optimizer may be
+# written through ``.data`` by whatever runs beside one (a moving average of a model): any of their steps makes its copies stale.
+#
+# A copy is made on the stream that asks for it.  With it go the copies that the last announced step of the same optimizer made stale, if the
+# step was announced on this stream, nothing wrote the weights after it, and no other stream has used the copies since they were last
+# made: one launch (``csrc/param_kernels.cu``) in the place of one to three a copy.  A copy that another stream asks for waits there for its launch.
 _WEIGHT_GEN = 0
 _WEIGHT_COPIES = {}
 _RECIPES = {}
-_GROUPS = {}                                          # recipes whose weights have the same optimizer (None: no watched one)
+_GROUPS = {}                                          # id of an optimizer's counter -> the recipes of its weights
 _RECIPE_LOCK = threading.Lock()
 _KIND = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 
-_OWNERS = {}                                          # id of a parameter -> (weak reference, its optimizer's counter of steps)
+_OWNERS = {}                                          # id of a parameter -> (weak reference, counters of the optimizers that write it)
 _STEPS = itertools.count(1)                           # never the same value twice, whichever optimizer it belongs to
+_LAST_STEP = 0
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def watch_weights(params, counter: list) -> None:
-    """``counter[0]`` changes whenever the storage of ``params`` is written past their version counters."""
+    """``counter[0]`` changes whenever an optimizer writes ``params``, past their version counters maybe.  ``counter[1:]`` is filled in
+    here: the stream of the last announced step, the device of the parameters, and their versions behind the step where it moves them."""
     for k in [k for k, (ref, _) in _OWNERS.items() if ref() is None]:
         del _OWNERS[k]
+    counter[1:] = [None, None, None]
     for p in params:
-        _OWNERS[id(p)] = (weakref.ref(p), counter)
+        owner = _OWNERS.get(id(p))
+        counters = owner[1] if owner is not None and owner[0]() is p else ()
+        if all(c is not counter for c in counters):
+            _OWNERS[id(p)] = (weakref.ref(p), counters + (counter,))
+        if counter[2] is None and p.is_cuda:
+            counter[2] = p.device.index
 
 
-def weights_changed(counter: Optional[list] = None) -> None:
-    """The weights watched with ``counter`` have changed; without it, any weight may have."""
-    global _WEIGHT_GEN
+def watch_optimizer(optimizer) -> None:
+    """``watch_weights`` for an optimizer of PyTorch, whose steps move the version counters: its steps announce themselves."""
+    params = [p for g in optimizer.param_groups for p in g["params"]]
+    counter = [0]
+    watch_weights(params, counter)
+    counter[3] = {}
+
+    def announce(*_):
+        weights_changed(counter, {id(p): p._version for p in params})
+
+    optimizer.register_step_post_hook(announce)
+
+
+def weights_changed(counter: Optional[list] = None, versions: Optional[dict] = None) -> None:
+    """The weights watched with ``counter`` are written by what the current stream runs next, or have been by what it ran last where
+    their ``versions`` are given; without a counter, any weight may have changed."""
+    global _WEIGHT_GEN, _LAST_STEP
     if counter is not None:
         counter[0] = next(_STEPS)
+        if versions is None:
+            _LAST_STEP = counter[0]
+        if len(counter) > 3 and counter[2] is not None:
+            counter[1], counter[3] = _raw_stream(counter[2]), versions
     else:
         _WEIGHT_GEN += 1
 
 
-class _Recipe:
-    """A matrix made of blocks of fp32 matrices: ``blocks`` holds (source, first row, rows, columns, offset, row pitch, transposed)."""
+def _counters(t: torch.Tensor) -> tuple:
+    owner = _OWNERS.get(id(t))
+    return owner[1] if owner is not None and owner[0]() is t else ()
 
-    __slots__ = ("srcs", "blocks", "out_spec", "stamp", "out", "used", "stream", "device", "group")
 
-    def __init__(self, srcs, blocks, out_spec):
-        owner = _OWNERS.get(id(srcs[0]))
-        self.group = id(owner[1]) if owner is not None and owner[0]() is srcs[0] else None
-        self.srcs = tuple(weakref.ref(t) for t in srcs)
-        self.blocks, self.out_spec = blocks, out_spec
-        self.stamp, self.out, self.used, self.stream = None, None, True, None
-        self.device = srcs[0].device
-
-    def sources(self):
-        ts = [r() for r in self.srcs]
-        return None if any(t is None for t in ts) else ts
+def _only_counter(t: torch.Tensor) -> Optional[list]:
+    counters = _counters(t)
+    return counters[0] if len(counters) == 1 else None
 
 
 def _stamp(srcs):
     out = [_WEIGHT_GEN]
     for t in srcs:
-        owner = _OWNERS.get(id(t))
-        out += (t._version, t.data_ptr(), owner[1][0] if owner is not None and owner[0]() is t else 0)
+        steps = 0
+        counters = _counters(t)
+        for c in counters:
+            steps = max(steps, c[0])
+        if not counters or counters[0][3] is not None:      # whose optimizer, if any, writes through the version counters
+            steps = max(steps, _LAST_STEP)
+        out += (t._version, t.data_ptr(), steps)
     return out
 
 
-def _rebuild(wanted: _Recipe, srcs) -> torch.Tensor:
-    """Make ``wanted`` anew, and with it the stale copies that this stream used since they were made."""
+class _Recipe:
+    """A matrix made of blocks of fp32 matrices: ``blocks`` holds (source, first row, rows, columns, offset, row pitch, transposed).
+    ``made`` is the copy: (stamp, tensor, stream, event behind its launch, list of the other streams that have waited for it)."""
+
+    __slots__ = ("srcs", "blocks", "out_spec", "made", "used", "device", "counter")
+
+    def __init__(self, srcs, blocks, out_spec):
+        self.srcs = tuple(weakref.ref(t) for t in srcs)
+        self.blocks, self.out_spec = blocks, out_spec
+        self.made, self.used, self.counter = None, True, None
+        self.device = srcs[0].device
+
+    @property
+    def out(self):
+        return None if self.made is None else self.made[1]
+
+    def sources(self):
+        ts = [r() for r in self.srcs]
+        return None if any(t is None for t in ts) else ts
+
+    def take(self, made) -> torch.Tensor:
+        """``made`` for the current stream."""
+        _, out, stream, event, others = made
+        now = _raw_stream(self.device.index)
+        # while a graph is recorded, what was made before lies behind the synchronisation that the recording began with
+        if now != stream and now not in others and not torch.cuda.is_current_stream_capturing():
+            here = torch.cuda.current_stream(self.device)
+            here.wait_event(event)
+            out.record_stream(here)
+            others.append(now)
+        self.used = True
+        return out
+
+
+def _by_the_step(old, new, srcs, counter) -> bool:
+    """Of two stamps of ``srcs``: nothing wrote them after the last step announced with ``counter``."""
+    versions = counter[3] or {}
+    return old[0] == new[0] and old[2::3] == new[2::3] and all(
+        v == was or v == versions.get(id(t)) for v, was, t in zip(new[1::3], old[1::3], srcs))
+
+
+def _rebuild(key, wanted: _Recipe, srcs, stamp) -> torch.Tensor:
+    """Make ``wanted`` anew, and with it what its optimizer's last step made stale on this stream."""
     with _RECIPE_LOCK:
-        stream = torch._C._cuda_getCurrentRawStream(wanted.device.index)
-        todo, sources = [wanted], [srcs]
-        if not torch.cuda.is_current_stream_capturing():
-            group, dead = _GROUPS[wanted.group], []
-            for key, r in group.items():
-                if r is wanted or not r.used or r.stream != stream or r.device != wanted.device:
-                    continue
-                ts = r.sources()
-                if ts is None:
-                    dead.append(key)
-                elif r.stamp != _stamp(ts) and _plain_sources(ts):
-                    todo.append(r)
-                    sources.append(ts)
-            for key in dead:
-                del group[key]
-                _RECIPES.pop(key, None)
+        stream = _raw_stream(wanted.device.index)
+        # recorded launches have not run: what they make belongs to the graph alone, and nobody else may find it
+        recording = torch.cuda.is_current_stream_capturing()
+        todo = [(wanted, srcs, stamp)]
+        if not recording:
+            counter = _only_counter(srcs[0])
+            if counter is not wanted.counter:
+                _leave_group(key, wanted)
+                if counter is not None:
+                    wanted.counter = counter
+                    _GROUPS.setdefault(id(counter), {})[key] = wanted
+            if counter is not None and wanted.made is not None and counter[1] == stream and counter[2] == wanted.device.index:
+                group, dead = _GROUPS[id(counter)], []
+                for k, r in group.items():
+                    made = r.made
+                    if r is wanted or not r.used or made is None or made[2] != stream or made[4] or r.device != wanted.device:
+                        continue
+                    ts = r.sources()
+                    if ts is None:
+                        dead.append((k, r))
+                        continue
+                    now = _stamp(ts)
+                    if (made[0] != now and _by_the_step(made[0], now, ts, counter) and all(_only_counter(t) is counter for t in ts)
+                            and _plain_sources(ts)):
+                        todo.append((r, ts, now))
+                for k, r in dead:
+                    _leave_group(k, r)
+                    _RECIPES.pop(k, None)
         at, flat, items, outs = {}, [], [], []
-        for i, (r, ts) in enumerate(zip(todo, sources)):
+        for i, (r, ts, _) in enumerate(todo):
             for t in ts:
                 if id(t) not in at:
                     at[id(t)] = len(flat)
@@ -109,10 +190,22 @@ def _rebuild(wanted: _Recipe, srcs) -> torch.Tensor:
             outs.extend(r.out_spec)
         made = _ext.load().weight_copies(flat, items, outs)
         _ext.count_launches((len(items) // 8 + 63) // 64)
-        for r, ts, out in zip(todo, sources, made):
-            r.out, r.stream, r.used = out, stream, r is wanted
-            r.stamp = _stamp(ts)
-        return wanted.out
+        if recording:
+            return made[0]
+        event = torch.cuda.Event()
+        event.record(torch.cuda.current_stream(wanted.device))
+        for (r, _, now), out in zip(todo, made):
+            r.made, r.used = (now, out, stream, event, []), r is wanted
+        return made[0]
+
+
+def _leave_group(key, r: _Recipe) -> None:
+    if r.counter is not None:
+        group = _GROUPS.get(id(r.counter), {})
+        group.pop(key, None)
+        if not group:
+            _GROUPS.pop(id(r.counter), None)
+        r.counter = None
 
 
 def _plain_sources(srcs) -> bool:
@@ -128,20 +221,15 @@ def recipe_copy(key, srcs, blocks, out_spec) -> torch.Tensor:
         old, r = r, _Recipe(srcs, blocks(), out_spec)
         with _RECIPE_LOCK:
             if old is not None:
-                _GROUPS[old.group].pop(key, None)
+                _leave_group(key, old)
             _RECIPES[key] = r
-            _GROUPS.setdefault(r.group, {})[key] = r
             if len(_RECIPES) > 4096:                   # parameters of discarded models: drop what is dead
-                for k in [k for k, v in _RECIPES.items() if v.sources() is None]:
-                    _GROUPS[_RECIPES.pop(k).group].pop(k, None)
-                for g in [g for g, v in _GROUPS.items() if not v]:
-                    del _GROUPS[g]
-    out = r.out
-    if out is None or r.stamp != _stamp(srcs):
-        out = _rebuild(r, srcs)
-    elif not r.used:
-        r.stream, r.used = torch._C._cuda_getCurrentRawStream(r.device.index), True
-    return out
+                for k, v in [(k, v) for k, v in _RECIPES.items() if v.sources() is None]:
+                    _leave_group(k, _RECIPES.pop(k))
+    stamp, made = _stamp(srcs), r.made
+    if made is None or made[0] != stamp:
+        return _rebuild(key, r, srcs, stamp)
+    return r.take(made)
 
 
 def operand_copy(weight: torch.Tensor, dtype, transpose: bool = False, index: Optional[torch.Tensor] = None,
@@ -151,8 +239,9 @@ def operand_copy(weight: torch.Tensor, dtype, transpose: bool = False, index: Op
     stamp = _stamp((weight,))
     if index is None:
         r = _RECIPES.get(key)
-        if r is not None and r.used and r.srcs[0]() is weight and r.stamp == stamp:
-            return r.out                               # a forward pass asks this a dozen times: before any other look at the tensor
+        made = r.made if r is not None else None
+        if made is not None and made[0] == stamp and r.srcs[0]() is weight:
+            return r.take(made)                        # a forward pass asks this a dozen times: before any other look at the tensor
         # a tensor that is no parameter (a padded weight, made in every call) comes once: nothing to make beside it
         if isinstance(weight, torch.nn.Parameter) and weight.dim() == 2 and weight.is_leaf and dtype in _KIND and _plain_sources((weight,)):
             n, k = weight.shape
@@ -166,6 +255,8 @@ def operand_copy(weight: torch.Tensor, dtype, transpose: bool = False, index: Op
         w = w[index]
     w = w.to(dtype)
     w = w.t().contiguous() if transpose else w.contiguous()
+    if weight.is_cuda and torch.cuda.is_current_stream_capturing():
+        return w                                       # not computed yet
     _WEIGHT_COPIES[key] = (stamp, w, weakref.ref(weight))
     if len(_WEIGHT_COPIES) > 4096:                     # parameters of discarded models: drop what is dead
         for k in [k for k, v in _WEIGHT_COPIES.items() if v[2]() is None]:

@@ -26,6 +26,7 @@ from ..control.multi_tier import parse_force_multi_tier_plan, TIER_FROM_ID, TIER
 from ..graph.attn_graph import AttnGraph
 from ..graph.engine import BudgetState, EdgeEngine, edge_seed_for_epoch, resolve_budget_state
 from ..models import MODEL_REGISTRY
+from ..ops import gemm
 from ..parallel import comm
 from ..parallel.initialize import (get_sequence_parallel_group, get_sequence_parallel_rank,
                                    get_sequence_parallel_src_rank, get_sequence_parallel_world_size,
@@ -181,6 +182,8 @@ class FullGraphTrainer:
             self.flat_optimizer = True
         else:
             self.optimizer = torch.optim.AdamW(self.model.parameters(), lr=args.peak_lr, weight_decay=args.weight_decay)
+            if self.device.type == "cuda":
+                gemm.watch_optimizer(self.optimizer)       # its steps announce themselves to the weights' 16-bit copies
         self.lr_scheduler = build_lr_scheduler(args, self.optimizer, self.n_train_global)
         self._apply_memory_limit()
         self._apply_forced_plan()

@@ -64,6 +64,75 @@ def test_operand_copies_follow_their_own_optimizer():
     assert copy(c) is before[2]
 
 
+def test_a_copy_made_on_one_stream_is_ready_on_another():
+    """A stream that finds a copy which another one made waits for its launch; from then on the maker's stream no longer renews it along
+    with others, since nothing would order the two."""
+    a, b = (torch.nn.Parameter(torch.randn(256, 256, device="cuda")) for _ in range(2))
+    counter = [0]
+    gemm.watch_weights([a, b], counter)
+    side = torch.cuda.Stream()
+    for p in (a, b):
+        gemm.operand_copy(p, torch.bfloat16)
+    recipe = gemm._RECIPES[(id(b), torch.bfloat16, False, "")]
+    for step in range(2):
+        before = recipe.out
+        torch.cuda._sleep(100_000_000)                       # some 50 ms: the copies' launch lies behind it
+        with torch.no_grad():
+            a.data.add_(1.0)
+            b.data.add_(1.0)
+        gemm.weights_changed(counter)
+        gemm.operand_copy(a, torch.bfloat16)
+        assert (recipe.out is before) == (step == 1)         # renewed by the main stream the first time only
+        with torch.cuda.stream(side):
+            got = gemm.operand_copy(b, torch.bfloat16).clone()
+        side.synchronize()
+        if step == 0:
+            assert torch.equal(got, b.detach().bfloat16())
+    torch.cuda.synchronize()
+
+
+def test_only_what_the_announced_step_made_stale_is_renewed_along():
+    """Copies of weights that no watched optimizer owns, or that were written again after its step, wait for their own request: the
+    stream that renews another copy does not know when they are written."""
+    a, b, c, d = (torch.nn.Parameter(torch.randn(32, 32, device="cuda")) for _ in range(4))
+    recipe = lambda p: gemm._RECIPES[(id(p), torch.bfloat16, False, "")]
+    copy = lambda p: gemm.operand_copy(p, torch.bfloat16)
+    opt = torch.optim.SGD([a, b, c], lr=0.5)
+    gemm.watch_optimizer(opt)
+    before = [copy(p) for p in (a, b, c, d)]
+    for p in (a, b, c):
+        p.grad = torch.ones_like(p)
+    opt.step()
+    with torch.no_grad():
+        c.add_(1.0)
+        d.add_(1.0)
+    assert torch.equal(copy(a), a.detach().bfloat16())
+    assert recipe(b).out is not before[1] and recipe(c).out is before[2] and recipe(d).out is before[3]
+    for p in (b, c, d):
+        assert torch.equal(copy(p), p.detach().bfloat16())
+
+
+def test_a_copy_of_a_recorded_launch_is_not_found_by_others():
+    """A forward pass that is recorded before any other makes its copies inside the graph: an eager pass before the first replay makes
+    its own."""
+    from budgetformer_b200.ops.gemm import fused_linear
+    lin = torch.nn.Linear(64, 32).cuda()
+    x = torch.randn(128, 64, device="cuda").bfloat16()
+    other = torch.nn.Linear(64, 32).cuda()
+    torch.cuda.synchronize()
+    with torch.no_grad():
+        fused_linear(x, other.weight, other.bias)            # the launch's own first use is no part of this
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = fused_linear(x, lin.weight, lin.bias)
+        eager = fused_linear(x, lin.weight, lin.bias)
+        want = torch.nn.functional.linear(x.float(), lin.weight.bfloat16().float(), lin.bias)
+        assert torch.allclose(eager.float(), want, rtol=2.0 ** -7, atol=2.0 ** -7)
+        graph.replay()
+        assert torch.equal(out, eager)
+
+
 def _net():
     torch.manual_seed(2)
     return torch.nn.Sequential(torch.nn.Linear(37, 65), torch.nn.ReLU(), torch.nn.Linear(65, 3, bias=False), torch.nn.Linear(3, 1)).cuda()

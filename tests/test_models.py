@@ -256,3 +256,24 @@ def test_widths_of_the_fp32_gradient_kernel():
     assert f32_gradient_pays(1024, 64, 1433) and not f32_gradient_pays(8192, 64, 1433)
     assert not any(f32_gradient_pays(m, n, k) for m in (1024, 40009) for n, k in ((512, 512), (1024, 1024), (2048, 2048), (16384, 16384)))
     assert f32_gradient_pays(1024, 1, 64) and not f32_gradient_pays(65536, 1, 64) and not f32_gradient_pays(65536, 64, 1)
+
+
+def test_weight_copies_follow_every_write():
+    """Copies are renewed by a step of any optimizer that owns the weight, and by any announced step where none does (a moving average
+    is written through ``.data``, past the version counter); another optimizer's step leaves owned ones alone."""
+    from budgetformer_b200.ops import gemm
+    own, ema = (torch.nn.Parameter(torch.randn(8, 16)) for _ in range(2))
+    first, second, foreign = [0], [0], [0]
+    gemm.watch_weights([own], first)
+    gemm.watch_weights([own], second)                      # a second optimizer over the same weights
+    copy = lambda p: gemm.operand_copy(p, torch.bfloat16)
+    for counter in (first, second, first):
+        held = copy(own)
+        own.data.mul_(3.0)
+        gemm.weights_changed(counter)
+        assert copy(own) is not held and torch.equal(copy(own), own.detach().bfloat16())
+    held = copy(own), copy(ema)
+    ema.data.mul_(3.0)
+    gemm.weights_changed(foreign)
+    assert copy(own) is held[0]
+    assert copy(ema) is not held[1] and torch.equal(copy(ema), ema.detach().bfloat16())
