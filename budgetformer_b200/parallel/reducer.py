@@ -60,14 +60,22 @@ class _Bucket:
         self._flat = torch.zeros(n_pad, dtype=dtype, device=device)
         self._native = None                        # release / gather of the gradients (fp32 on a GPU)
         self._away = False                         # the gradients are with the parameters, not in the bucket
+        self._home = None                          # stream of the last let_go
+        self._gathered = None                      # stream that gathered since, and the streams that waited for it
         self.symm = None                           # filled by parallel.symm when available
         self._bind()
 
     @property
     def flat(self) -> torch.Tensor:
-        """The bucket, with the gradients of the last backward pass in it."""
+        """The bucket, with the gradients of the last backward pass in it, for the current stream."""
         if self._away:
             self.collect()
+        if self._gathered is not None:
+            stream, ready = self._gathered
+            now = torch._C._cuda_getCurrentRawStream(self._flat.device.index)
+            if now not in ready and not torch.cuda.is_current_stream_capturing():
+                torch.cuda.current_stream(self._flat.device).wait_stream(stream)
+                ready.add(now)
         return self._flat
 
     def _bind(self):
@@ -84,11 +92,18 @@ class _Bucket:
         """Before a backward pass: gradients start from nothing."""
         self._native.release()
         self._away = True
+        self._home, self._gathered = torch.cuda.current_stream(self._flat.device), None
 
     def collect(self) -> None:
-        """Behind a backward pass: every gradient, or zeros, into the bucket; ``param.grad`` is a view of it again."""
-        self._away = False
+        """Behind a backward pass: every gradient, or zeros, into the bucket; ``param.grad`` is a view of it again.  The current stream
+        gathers, which may be that of a reader beside the training loop: the loop's stream waits for it."""
         self._native.gather()
+        self._away = False
+        here = torch.cuda.current_stream(self._flat.device)
+        self._gathered = here, {here.cuda_stream}
+        if here != self._home and not torch.cuda.is_current_stream_capturing():
+            self._home.wait_stream(here)
+            self._gathered[1].add(self._home.cuda_stream)
         from ..ops import _ext
         _ext.count_launches(1)
 

@@ -180,3 +180,36 @@ def test_gradient_bucket_takes_any_gradient():
     red.finalize_backward()
     for p, w in zip(m, want):
         assert torch.equal(p.grad, w) and p.grad.is_contiguous()
+
+
+def test_gradient_bucket_read_on_a_side_stream():
+    """Whoever reads the bucket first gathers the gradients, on its own stream: the training loop's stream, and a third one that reads it
+    afterwards, see them complete."""
+    from budgetformer_b200.parallel.reducer import GradientReducer
+    net, ref = _net(), _net()
+    red = GradientReducer(net, None, 25.0, 1)
+    x = torch.randn(50, 37, device="cuda")
+    main, side, third = torch.cuda.current_stream(), torch.cuda.Stream(), torch.cuda.Stream()
+    for _ in range(2):
+        ref.zero_grad()
+        ref(x).square().mean().backward()
+        red.prepare_backward()
+        net(x).square().mean().backward()
+        done = main.record_event()
+        side.wait_event(done)
+        third.wait_event(done)
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(50_000_000)                    # some 25 ms in front of the gather
+            on_side = [b.flat.clone() for b in red.buckets]
+        on_main = [p.grad.clone() for p in net.parameters()]
+        with torch.cuda.stream(third):
+            on_third = [b.flat.clone() for b in red.buckets]
+        torch.cuda.synchronize()
+        for got, q in zip(on_main, ref.parameters()):
+            assert torch.equal(got, q.grad)
+        for a, b in zip(on_side, on_third):
+            assert torch.equal(a, b)
+        with torch.no_grad():
+            for p, q in zip(net.parameters(), ref.parameters()):
+                p.mul_(1.25)
+                q.mul_(1.25)
