@@ -54,7 +54,7 @@ def ffn_onchip(x: torch.Tensor, w1, b1, w2, b2, *, act: str, residual: bool, p1:
 
 def _rows_ok(x: torch.Tensor) -> bool:
     return (x.is_cuda and x.dim() == 2 and x.dtype in (torch.bfloat16, torch.float16) and x.stride(1) == 1
-            and (x.stride(0) * 2) % 16 == 0 and x.data_ptr() % 16 == 0 and x.size(0) > 0)
+            and x.stride(0) >= x.size(1) and (x.stride(0) * 2) % 16 == 0 and x.data_ptr() % 16 == 0 and x.size(0) > 0)
 
 
 def onchip_supported(x: torch.Tensor, w1, w2, residual: Optional[torch.Tensor] = None) -> bool:

@@ -392,6 +392,27 @@ def test_ffn_on_chip_side_outputs_equal_the_two_gemm_form():
     _close(y_b, y_a.float(), torch.bfloat16)
 
 
+@pytest.mark.parametrize("act", ["relu", "gelu"])
+@pytest.mark.parametrize("h", [64, 128])
+def test_ffn_rows_that_overlap(h, act):
+    """One row broadcast as the residual, and inputs and residuals whose rows overlap in memory, give what contiguous ones give, in
+    evaluation and in training."""
+    from budgetformer_b200.ops.ffn import fused_ffn
+    torch.manual_seed(2)
+    m = 200
+    l1, l2 = torch.nn.Linear(h, 2 * h).cuda(), torch.nn.Linear(2 * h, h).cuda()
+    flat = torch.randn(m * h, device="cuda").bfloat16()
+    windows = flat.as_strided((m, h), (h // 2, 1))
+    x = torch.randn(m, h, device="cuda").bfloat16()
+    for inp, res in ((x, flat[:h].expand(m, h)), (x, windows), (windows, x), (windows, windows)):
+        for grad in (False, True):
+            with torch.set_grad_enabled(grad):
+                got = fused_ffn(inp, l1.weight, l1.bias, l2.weight, l2.bias, act=act, residual=res)
+                want = fused_ffn(inp.contiguous(), l1.weight, l1.bias, l2.weight, l2.bias, act=act, residual=res.contiguous())
+            gemm.check_status("cuda")
+            _close(got, want.float(), torch.bfloat16)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_gelu_carries_values_that_are_not_finite(dtype):
     """A NaN or an infinity in the bias reaches the activation as in PyTorch's GELU (NaN stays NaN, inf stays inf), in the product's
