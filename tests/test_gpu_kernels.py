@@ -288,6 +288,24 @@ def test_device_transpose_matches_torch_path(hub):
         assert dev.kv_slots > 0 and dev.t_split.size(0) >= 1
 
 
+@pytest.mark.parametrize("longest", [64, 65, 4000, 8100])
+def test_device_transpose_of_one_longer_row(longest):
+    """Blocks of 256 rows with at most 8,192 edges: rows up to 64 are marked by their threads, one longer sends its block another way.
+    The last block holds one row."""
+    from budgetformer_b200.graph.attn_graph import AttnGraph
+    g = torch.Generator().manual_seed(longest)
+    n = 256 * 3 + 1
+    deg = torch.randint(0, 20, (n,), generator=g)
+    deg[256:512] = 0
+    deg[300], deg[511], deg[n - 1] = longest, 60, longest
+    dst = torch.repeat_interleave(torch.arange(n), deg)
+    ref = AttnGraph.from_edge_index(torch.stack([torch.randint(0, n, (dst.numel(),), generator=g), dst]), n).ensure_transpose()
+    dev = AttnGraph(n, ref.rowptr.cuda(), ref.col.cuda(), None).ensure_transpose()
+    for name in ("t_rowptr", "t_row", "t_eid"):
+        a, b = getattr(ref, name), getattr(dev, name).cpu()
+        assert torch.equal(a.to(b.dtype), b), name
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_batch_norm_kernels_match_pytorch(dtype):
     """Forward, running statistics and all three gradients of the row BatchNorm against nn.BatchNorm1d in fp32."""
