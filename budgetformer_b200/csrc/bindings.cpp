@@ -269,14 +269,15 @@ std::vector<Tensor> build_attn_graph(Tensor in_rowptr, Tensor in_src, Tensor out
   for (const Tensor* t : {&in_rowptr, &in_src, &out_rowptr, &out_col})
     TORCH_CHECK(t->scalar_type() == torch::kInt && t->is_contiguous(), "topology must be contiguous int32");
   const int cap = (int)(b_real + b_rw + (exphormer ? 1 : 0));
+  const bool cuda = in_src.is_cuda();
+  c10::cuda::OptionalCUDAGuard guard;               // every launch below, on the topology's device and its current stream
+  if (cuda) guard.set_device(in_src.device());
   auto iopt = in_src.options();
   Tensor ell_col = torch::empty({n, std::max(cap, 1)}, iopt);
   Tensor ell_type = exphormer ? torch::empty({n, std::max(cap, 1)}, iopt.dtype(torch::kUInt8)) : Tensor();
-  const bool cuda = in_src.is_cuda();
   Tensor ell_cnt = cuda ? torch::empty({n}, iopt) : torch::zeros({n}, iopt);
   Tensor totals = torch::zeros({2}, iopt.dtype(torch::kLong));
   if (cuda) {
-    c10::cuda::CUDAGuard guard(in_src.device());
     bf_build_params p{};
     p.in_rowptr = iptr(in_rowptr); p.in_src = iptr(in_src); p.out_rowptr = iptr(out_rowptr); p.out_col = iptr(out_col);
     p.n = (int)n; p.b_real = (int)b_real; p.b_rw = (int)b_rw; p.walks = (int)walks; p.walk_len = (int)walk_len;
