@@ -133,6 +133,7 @@ typedef struct {
   const int* hub_rows;
   int n_hub;
   unsigned long long* hub_top;
+  long long in_edges;      // of all n queries (0: not known); long rows on average decide between two kernels
 } bf_build_params;
 
 #define BF_BUILD_HUB_DEGREE 4096

@@ -281,7 +281,7 @@ std::vector<Tensor> build_attn_graph(Tensor in_rowptr, Tensor in_src, Tensor out
     bf_build_params p{};
     p.in_rowptr = iptr(in_rowptr); p.in_src = iptr(in_src); p.out_rowptr = iptr(out_rowptr); p.out_col = iptr(out_col);
     p.n = (int)n; p.b_real = (int)b_real; p.b_rw = (int)b_rw; p.walks = (int)walks; p.walk_len = (int)walk_len;
-    p.exphormer = exphormer ? 1 : 0; p.seed = seed; p.cap = std::max(cap, 1);
+    p.exphormer = exphormer ? 1 : 0; p.seed = seed; p.cap = std::max(cap, 1); p.in_edges = in_src.numel();
     p.ell_col = ell_col.data_ptr<int>(); p.ell_type = exphormer ? ell_type.data_ptr<uint8_t>() : nullptr;
     p.ell_cnt = ell_cnt.data_ptr<int>();
     p.totals = reinterpret_cast<unsigned long long*>(totals.data_ptr<int64_t>());
@@ -334,7 +334,7 @@ void budget_select_rows(Tensor in_rowptr, Tensor in_src, Tensor out_rowptr, Tens
   bf_build_params p{};
   p.in_rowptr = iptr(in_rowptr); p.in_src = iptr(in_src); p.out_rowptr = iptr(out_rowptr); p.out_col = iptr(out_col);
   p.n = (int)n; p.b_real = (int)b_real; p.b_rw = (int)b_rw; p.walks = (int)walks; p.walk_len = (int)walk_len;
-  p.exphormer = exphormer ? 1 : 0; p.seed = seed; p.cap = cap;
+  p.exphormer = exphormer ? 1 : 0; p.seed = seed; p.cap = cap; p.in_edges = in_src.numel();
   p.ell_col = ell_col.data_ptr<int>(); p.ell_type = exphormer ? ell_type->data_ptr<uint8_t>() : nullptr;
   p.ell_cnt = ell_cnt.data_ptr<int>();
   p.totals = reinterpret_cast<unsigned long long*>(totals.data_ptr<int64_t>());

@@ -253,6 +253,31 @@ def test_gpu_builder_at_the_edges_of_its_lists(cfg, exph):
     assert cpu._totals.tolist() == gpu._totals.cpu().tolist()
 
 
+@pytest.mark.parametrize("exph", [False, True])
+@pytest.mark.parametrize("n", [1200, 30001, 66001])
+@pytest.mark.parametrize("cfg", [(4, 4, 2, 4), (8, 8, 8, 8), (7, 3, 3, 5), (2, 8, 1, 16), (8, 8, 11, 4), (3, 12, 5, 7), (16, 16, 33, 3), (25, 4, 2, 4), (32, 32, 3, 6), (32, 0, 0, 0)])
+def test_gpu_builder_forms(cfg, n, exph):
+    """Eight lanes or a warp per query (few queries for their walks), a thread with eight walks or two under way; long rows among short ones (the warp
+    ranks them), warps whose rows are all of medium length (their lanes do), and rows of up to 4,096 edges at the largest budgets, where
+    hashes fill the estimated bound's slots now and then."""
+    br, bw, w, l = cfg
+    g = torch.Generator().manual_seed(br + w)
+    at, rows = 0, []
+    for i in range(64):                                   # two warps of 33 to 110 edges, one of mixed lengths
+        rows.append((at + i, 33 + i * 5 % 78))
+    for i, d in enumerate([500, 3, 4096, 40, 0, 70, 31, 33, 1500, 700, 4000, 2, 900, 1000, 1100, 1200, 1300]):
+        rows.append((96 + i, d))
+    dst = torch.repeat_interleave(torch.tensor([r for r, _ in rows]), torch.tensor([d for _, d in rows]))
+    ei = torch.stack([torch.randint(0, n, (dst.numel(),), generator=g), dst])
+    topo = Topology.from_edge_index(torch.cat([ei, torch.randint(0, n, (2, 3000), generator=g)], 1), n)
+    cpu = build_attn_graph(topo, br, bw, w, l, 29, exphormer=exph)
+    gpu = build_attn_graph(topo.to("cuda"), br, bw, w, l, 29, exphormer=exph)
+    assert torch.equal(cpu.rowptr, gpu.rowptr.cpu()) and torch.equal(cpu.col, gpu.col.cpu())
+    if exph:
+        assert torch.equal(cpu.etype, gpu.etype.cpu())
+    assert cpu._totals.tolist() == gpu._totals.cpu().tolist()
+
+
 def test_gpu_builder_seed_changes_graph_and_is_reproducible():
     topo, _ = random_topology(500, 5000, seed=2)
     t = topo.to("cuda")
