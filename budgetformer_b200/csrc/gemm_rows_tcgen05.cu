@@ -14,7 +14,7 @@
 // * Epilogue features are template parameters.  Masks, biases and activations as in gemm_tcgen05.cu, in the same order.
 //
 // us at 800 k rows before (gemm_tcgen05.cu) and now, and the time of its bytes at the measured copy rate (outputs x features): 384 x 128
-// + bias 168 / 152 / 125; 128 x 128 + bias, dropout, residual 203 / 119 / 94; 128 x 128 + dropout 159 / 83 / 63 (without 77 / 87 / 63);
+// + bias 168 / 152 / 125; 128 x 128 + bias, dropout, residual 203 / 119 / 94; 128 x 128 + dropout 159 / 83 / 63 (without 72 / 72 / 63);
 // 128 x 384 + residual 174 / 170 / 157; 256 x 128 + bit mask 173 / 123 / 98; 128 x 256 + residual 168 / 138 / 125; 256 x 128 * gelu'
 // 601 / 354 / 157; 128 x 272 + dropout 161 / 124 / 98.  At 400 k rows: 768 x 256 229 / 202 / 125; 256 x 256 + residual 205 / 120 / 94; 512 x 256
 // + ReLU, dropout, bits 298 / 200 / 98; 256 x 512 + residual 209 / 152 / 125; 112 x 256 215 / 58 / 45.  At 2 k rows 6 us either way.
@@ -196,6 +196,7 @@ gemm_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const int units_per_tile = g.group_panels;
     const uint32_t thresh_hi = g.thresh >> 16;
     const bool ahead = STAGED && g.n_buf == 2;
+    const bool twin = !STAGED && !KEEP_Z && g.n_buf == 2;          // results alternate between two blocks
     bool ok = true;
     // unit (t, p): row tile t, panel p of the group; acc_seq counts the accumulators of this CTA up to the unit's
     int t = first_tile, p = team, seq0 = 0;
@@ -233,12 +234,15 @@ gemm_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         for (int q = 0; q < 4; ++q)
           if (col0 + 16 * q < g.N) bits[q] = __ldg(g.bits_in + (long long)((col0 >> 4) + q) * g.ldmb + row);
       }
-      uint8_t* block = block0 + (size_t)(STAGED ? buf : 0) * 4 * kBlockBytes;
+      uint8_t* block = block0 + (size_t)(KEEP_Z ? 0 : buf) * 4 * kBlockBytes;
       if (STAGED && any_row && !mbar_wait(&ctl->staged[ew][buf], buf_phase, abort_flag)) { ok = false; break; }
       if (!mbar_wait(&ctl->acc_full[acc], (uint32_t)(seq / g.n_acc) & 1u, abort_flag)) { ok = false; break; }
       tc_fence_after();
       if (!STAGED) {
-        if (lane == 0) tma_store_wait_read<0>();                   // this buffer's last store
+        if (lane == 0) {                                           // this buffer's last store
+          if (twin) tma_store_wait_read<1>();
+          else tma_store_wait_read<0>();
+        }
         __syncwarp();
       }
       const uint32_t taddr = tlane + (uint32_t)(acc * chunk_cols + in_chunk * kPanel);
@@ -371,6 +375,7 @@ gemm_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         if (ahead) { buf ^= 1; if (buf == 0) buf_phase ^= 1u; }
         else buf_phase ^= 1u;
       }
+      if (twin) buf ^= 1;
       t = tn; p = pn; seq0 = seqn;
     }
     if (lane == 0) tma_store_wait_all();
@@ -423,8 +428,9 @@ RowsKernel rows_kernel(int f, bool fp16) {
   }
 }
 
-// Shared-memory plan: panels of a group, chunk, ring depth, staging buffers.  False: no plan fits.
-bool plan_rows(RowsArgs& g, bool staged, bool keep_z, int sms, size_t budget) {
+// Shared-memory plan: panels of a group, chunk, ring depth, staging buffers (`twice`: two a team where they leave the ring four
+// stages).  False: no plan fits.
+bool plan_rows(RowsArgs& g, bool twice, bool keep_z, int sms, size_t budget) {
   const size_t panel_bytes = (size_t)g.k_panels * kPanel * 128;              // one panel's rows of B
   const size_t out_bytes = (size_t)kTeams * 4 * kBlockBytes;                 // one staging buffer a team
   auto chunk_of = [](int gp) { return gp % 2 == 0 ? 2 : gp == 3 ? 3 : 1; };
@@ -451,7 +457,7 @@ bool plan_rows(RowsArgs& g, bool staged, bool keep_z, int sms, size_t budget) {
     g.n_acc = g.chunk_panels == 3 ? 2 : 4;
     const size_t left = budget - best * panel_bytes;
     g.n_buf = keep_z ? 2 : 1;
-    if (staged && left >= 2 * out_bytes + (size_t)4 * kAStage) g.n_buf = 2;
+    if (twice && left >= 2 * out_bytes + (size_t)4 * kAStage) g.n_buf = 2;
     const int deep = (int)((left - g.n_buf * out_bytes) / kAStage);
     g.stages = deep < kMaxStages ? deep : kMaxStages;
     if (g.stages < (g.group_panels > g.chunk_panels ? g.k_panels : 1)) return false;
@@ -515,7 +521,16 @@ extern "C" int bf_gemm_rows(const bf_gemm_params* p, cudaStream_t st) {
   const size_t tail = ((sizeof(RowsControl) + 15) & ~size_t(15)) + (p->bias ? (size_t)group_cols * 4 : 0);
   const size_t budget = 227 * 1024 - 1024 - tail;
   const bool staged = (f & (F_RES | F_GELU_GRAD)) != 0;
-  if (!plan_rows(g, staged, (f & F_KEEP_Z) != 0, sms, budget)) return (int)cudaErrorNotSupported;
+  // A second staging buffer lets a warp write while its last store is read: 800 k rows of 128 x 128 plain 77 -> 72 us, with a bias 78 -> 72, with
+  // a bit mask 78 -> 74.  With dropout the ALU pipe is what is short, and the shallower ring costs: 76 -> 78, with ReLU and bits 90 -> 94.
+  const bool twice = staged || !(f & F_DROP);
+  if (!plan_rows(g, twice, (f & F_KEEP_Z) != 0, sms, budget)) return (int)cudaErrorNotSupported;
+  // With no epilogue to speak of, reading A twice, streaming B or a short ring shows: bf16 goes back to the other kernel there.  us at 800 k
+  // rows there / here: 256 x 256 plain 151 / 158, with a bias 154 / 162; 128 x 384 143 / 150, 144 / 150; 256 x 512 246 / 269, 246 / 280;
+  // 256 x 768 334 / 357, 339 / 351.  (More columns than features: 384 x 128 152 / 141, 512 x 256 276 / 257; fp16, which has no such instance there: 256 x 256
+  // 247 / 162; 50 k rows: within 1 us.)
+  if (!fp16 && (f == 0 || f == F_BIAS) && p->N <= p->K && g.m_tiles >= 4 * sms && (!g.resident || g.groups > 1 || g.stages < 5))
+    return (int)cudaErrorNotSupported;
   CUtensorMap map_a, map_b, map_out, map_z, map_in;
   memset(&map_z, 0, sizeof(map_z));
   memset(&map_in, 0, sizeof(map_in));

@@ -2,8 +2,8 @@
 //
 //   C[M, N] = A[M, K] * B[N, K]^T      bf16 / fp16 operands, fp32 accumulation in tensor memory
 //
-// It takes the products that gemm_rows_tcgen05.cu does not: several destinations, a gathered operand, fp32 output, a 16-bit ReLU mask
-// and rare combinations of epilogue features.
+// It takes the products that gemm_rows_tcgen05.cu does not: several destinations, a gathered operand, fp32 output, a 16-bit ReLU mask,
+// rare combinations of epilogue features, and bf16 products without an epilogue where it is faster (rule and figures there).
 //
 // * operands are staged by TMA (cp.async.bulk.tensor, 128-byte swizzle, one 64-element K panel per
 //   stage; a ragged last panel is zero-filled) into a 3- or 4-deep shared-memory ring; one elected thread
@@ -741,7 +741,7 @@ extern "C" int bf_gemm_tn(const bf_gemm_params* p, cudaStream_t st) {
   }
   const size_t smem = 1024 + g.stages * stage_bytes + (size_t)g.out_bufs * out_bytes + sizeof(Control) + 64 + bias_bytes;
   g.n_groups = (g.block_n % 64 == 0) ? 4 : (g.block_n % 32 == 0) ? 2 : 1;
-  // The pushes of a bf16 layer without dropout, and the gathered output projection; everything else reads its features at run time.
+  // Plain bf16 products and pushes, with a bias or without, and the gathered output projection; everything else reads its features at run time.
   int epi = -1;
   if (!g.is_fp16 && !p->out_fp32 && g.mask_mode == 0) {
     int f = 0;

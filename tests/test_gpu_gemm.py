@@ -155,6 +155,28 @@ def test_gemm_row_streaming_epilogues(m, n, k, dtype):
         assert bool((edge == 7.0).all()), epi
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n,k", [(256, 256), (128, 384), (256, 512), (128, 128), (112, 264)])
+def test_plain_products_of_many_rows(n, k, dtype):
+    """Products with no epilogue but a bias around the number of rows (592 tiles) from which bf16 goes to either kernel by its shape."""
+    torch.manual_seed(n + k)
+    w = (torch.randn(n, k, device="cuda") / k ** 0.5).to(dtype)
+    bias = torch.randn(n, device="cuda")
+    half_ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for m in (591 * 128, 591 * 128 + 1, 592 * 128 + 37):
+        a = torch.randn(m, k, device="cuda").to(dtype)
+        base = a.double() @ w.double().t()
+        for b in (None, bias):
+            want = base if b is None else base + b.double()
+            big = torch.full((m + 2, n + 8), 7.0, device="cuda", dtype=dtype)
+            gemm.gemm_tn(a, w, b, out=big[1:m + 1, :n])
+            gemm.check_status("cuda")
+            # one rounding, and the products added up in fp32 (|a| |w| summed: about 0.64 k^0.5, at most 15, and the bias)
+            err = (big[1:m + 1, :n].double() - want).abs() - half_ulp * want.abs() - 24 * k ** 0.5 * 2.0 ** -22
+            assert float(err.max()) <= (2.0 ** -25 if dtype == torch.float16 else 0.0)
+            assert bool((big[0] == 7.0).all()) and bool((big[m + 1] == 7.0).all()) and bool((big[:, n:] == 7.0).all())
+
+
 def test_gemm_strided_input_rows():
     big = torch.randn(700, 3 * 128, device="cuda").bfloat16()
     a = big[:, 128:256]
