@@ -423,10 +423,12 @@ __device__ __forceinline__ int steps_of(int len) { return max(1, (int)__reduce_m
 // What a lane group reads of its edges ahead of them, one edge a lane: the chunk that the stream is in, the chunk behind it, and the first
 // chunk of the next segment.  A step takes its edge by a shuffle.  (With a load for every edge, one step ahead, each trip to memory for
 // a new sector of the list held all groups of the warp up: dK/dV and dQ of eight heads of 16, bf16, 300 k
-// nodes of ten edges 1070 us then and 902 now; 700 k packed nodes of eight 7431 and 6949 with the forward pass, twice over.)
+// nodes of ten edges 1070 us then and 902 now; 700 k packed nodes of eight 7431 and 6949 with the forward pass, twice over.  dQ of 612 k
+// nodes of 16 edges 8 x 32 bf16, 793 and 734; on a power-law graph of that size, whose dQ pass is bound by what L2 holds, 695 and 702.)
+// The shuffle's own width folds the edge into its group: with the lane computed, that pass took 2 % longer.
 struct Chunk {
   int now, next, other;
-  __device__ __forceinline__ int at(int gbase, int i, int mask) const { return __shfl_sync(kFull, now, gbase + (i & mask)); }
+  __device__ __forceinline__ int at(int i, int lanes) const { return __shfl_sync(kFull, now, i, lanes); }      // i modulo the group's lanes
 };
 
 // The fetching side of a stream over rows, one warp-uniform step at a time: edge i of segment r, its key (and type).  The bounds
@@ -434,7 +436,7 @@ struct Chunk {
 // otherwise stall every segment for two trips to memory.
 template <bool TYPED> struct RowFetch {
   int r, i, m, beg, len, beg1, len1, beg2, len2;
-  int lt, mask, gbase;           // lane in its group, group size - 1, first lane of the group
+  int lt, mask;                  // lane in its group, group size - 1
   Chunk key_, type_;
   __device__ __forceinline__ void read(const AttnArgs& a, int b, int n, int from, int& key, int& type) const {
     if (from + lt < n) { key = __ldg(a.col + b + from + lt); if (TYPED) type = a.etype[b + from + lt]; }
@@ -442,7 +444,6 @@ template <bool TYPED> struct RowFetch {
   __device__ __forceinline__ void start(const AttnArgs& a, const Rows& rows, int n_seg, int lane, int ltl) {
     mask = (1 << ltl) - 1;
     lt = lane & mask;
-    gbase = lane & ~mask;
     r = i = 0;
     rows.extent(a, 0, beg, len);
     beg1 = len1 = beg2 = len2 = 0;
@@ -456,8 +457,8 @@ template <bool TYPED> struct RowFetch {
   }
   __device__ __forceinline__ bool has() const { return i < len; }
   __device__ __forceinline__ int edge() const { return beg + i; }
-  __device__ __forceinline__ int key() const { return key_.at(gbase, i, mask); }        // by all lanes of the warp
-  __device__ __forceinline__ int type() const { return TYPED ? type_.at(gbase, i, mask) : 0; }
+  __device__ __forceinline__ int key() const { return key_.at(i, mask + 1); }           // by all lanes of the warp
+  __device__ __forceinline__ int type() const { return TYPED ? type_.at(i, mask + 1) : 0; }
   __device__ __forceinline__ void advance(const AttnArgs& a, const Rows& rows, int n_seg) {
     if (r >= n_seg) return;
     if (++i == m) {
@@ -816,7 +817,7 @@ __global__ void __launch_bounds__(kStreamThreads, 3) edge_attn_bwd_kv_kernel(Bwd
   // fetching side: items two segments ahead, the first queries of a segment one segment ahead (see RowFetch); with edge types, whose
   // place in memory comes from the list, a segment more
   constexpr int AHEAD = EXPH ? 3 : 2;
-  const int mask = (1 << sg.ltl) - 1, gbase = lane & ~mask;
+  const int mask = (1 << sg.ltl) - 1;
   int fr = 0, fi = 0, fbeg[AHEAD + 1], flen[AHEAD + 1];
   auto extent = [&](int r, int& beg, int& len) {
     const long long t = item0 + r * stride;
@@ -845,9 +846,9 @@ __global__ void __launch_bounds__(kStreamThreads, 3) edge_attn_bwd_kv_kernel(Bwd
   }
   unsigned types = 0;                           // edge type of every ring slot
   auto issue = [&](int slot) {
-    const unsigned i_row = (unsigned)rowc.at(gbase, fi, mask);
-    const int eid = eidc.at(gbase, fi, mask);
-    const int ty = EXPH ? typec.at(gbase, fi, mask) : 0;
+    const unsigned i_row = (unsigned)rowc.at(fi, mask + 1);
+    const int eid = eidc.at(fi, mask + 1);
+    const int ty = EXPH ? typec.at(fi, mask + 1) : 0;
     if (on && fi < flen[0]) {
       S::copy(ring[slot][0], tid, qb + i_row * sq);
       S::copy(ring[slot][1], tid, gb + i_row * sgr);
@@ -1378,8 +1379,8 @@ __global__ void __launch_bounds__(256, 4) edge_attn_bwd_kv_rows_kernel(BwdArgs b
 // where there are more than eight, adds them and finishes the row if it lies in the window whole; of a row that goes on, the window's sum replaces its first slot there.  Pass 2 adds those window sums for the rows that cross a window's end.  The association depends on the
 // slot numbers alone: bit-reproducible.  A row of 10^6 edges (16 k slots) is thus 244 blocks and one short tail instead of
 // one block's walk, and 10^4 rows of two or three slots are a few hundred blocks instead of 10^4 (each of 1,024 threads):
-// both passes over the dK/dV slots take 98 us on a 612 k-node power-law graph at h = 256 (632 us with a block per row),
-// 22 us at 700 k nodes / h = 128 (78 us).
+// both passes over the dK/dV slots take 103 us a layer on a 612 k-node power-law graph at h = 256 (113 with a block that walks its
+// window's rows, 632 with a block per row), 22 us at 700 k nodes / h = 128 (41, 78).
 // ---------------------------------------------------------------------------------------------
 constexpr int SPLIT_WINDOW = 64;
 constexpr int SPLIT_WARPS = 16;
