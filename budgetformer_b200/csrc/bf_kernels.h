@@ -170,7 +170,7 @@ typedef struct {
   // ... and for GELU the pre-activation, rounded to the operands' type; the activation is taken of the rounded value
   void* z_out;                      // [M, ffn] 16-bit, row stride ldz, or NULL
   long long ldz;
-  int round_z;                      // GELU without z_out: of the rounded pre-activation all the same
+  int round_z;                      // GELU without z_out: of the rounded pre-activation all the same (without side outputs: fp16 and 64 / 128 always)
   const void* R;                    // residual other than X (residual = 0): [M, hidden] 16-bit, row stride ldr, or NULL
   long long ldr;
 } bf_ffn_params;
