@@ -97,12 +97,16 @@ def _only_counter(t: torch.Tensor) -> Optional[list]:
 def _stamp(srcs):
     out = [_WEIGHT_GEN]
     for t in srcs:
-        steps = 0
-        counters = _counters(t)
-        for c in counters:
-            steps = max(steps, c[0])
-        if not counters or counters[0][3] is not None:      # whose optimizer, if any, writes through the version counters
-            steps = max(steps, _LAST_STEP)
+        owner = _OWNERS.get(id(t))                    # once a lookup of a copy: _counters without the calls
+        if owner is None or owner[0]() is not t:
+            steps = _LAST_STEP
+        else:
+            counters = owner[1]
+            steps = counters[0][0]
+            if len(counters) > 1:
+                steps = max(c[0] for c in counters)
+            if counters[0][3] is not None and steps < _LAST_STEP:      # whose optimizer writes through the version counters
+                steps = _LAST_STEP
         out += (t._version, t.data_ptr(), steps)
     return out
 
