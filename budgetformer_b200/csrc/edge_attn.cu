@@ -71,6 +71,7 @@ template <typename T> struct Raw;
 template <> struct Raw<__nv_bfloat16> {
   uint4 u;
   __device__ __forceinline__ void load(const __nv_bfloat16* p) { u = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ void load_if(bool on, const __nv_bfloat16* p) { u = make_uint4(0u, 0u, 0u, 0u); if (on) u = *reinterpret_cast<const uint4*>(p); }
   __device__ __forceinline__ float get(int i) const {
     const uint32_t w = (i >> 1) == 0 ? u.x : (i >> 1) == 1 ? u.y : (i >> 1) == 2 ? u.z : u.w;
     return (i & 1) ? __uint_as_float(w & 0xFFFF0000u) : __uint_as_float(w << 16);
@@ -79,6 +80,7 @@ template <> struct Raw<__nv_bfloat16> {
 template <> struct Raw<__half> {
   uint4 u;
   __device__ __forceinline__ void load(const __half* p) { u = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ void load_if(bool on, const __half* p) { u = make_uint4(0u, 0u, 0u, 0u); if (on) u = *reinterpret_cast<const uint4*>(p); }
   __device__ __forceinline__ float get(int i) const {
     const uint32_t w = (i >> 1) == 0 ? u.x : (i >> 1) == 1 ? u.y : (i >> 1) == 2 ? u.z : u.w;
     return __half2float(__ushort_as_half((unsigned short)((i & 1) ? (w >> 16) : (w & 0xFFFFu))));
@@ -87,8 +89,16 @@ template <> struct Raw<__half> {
 template <> struct Raw<float> {
   float4 f;
   __device__ __forceinline__ void load(const float* p) { f = *reinterpret_cast<const float4*>(p); }
+  __device__ __forceinline__ void load_if(bool on, const float* p) { f = make_float4(0.f, 0.f, 0.f, 0.f); if (on) f = *reinterpret_cast<const float4*>(p); }
   __device__ __forceinline__ float get(int i) const { return i == 0 ? f.x : i == 1 ? f.y : i == 2 ? f.z : f.w; }
 };
+
+template <typename T> __device__ __forceinline__ void load_vec_if(bool on, const T* p, float* f) {
+  Raw<T> r;
+  r.load_if(on, p);
+#pragma unroll
+  for (int i = 0; i < 16 / (int)sizeof(T); ++i) f[i] = r.get(i);
+}
 
 // One 16-byte slice of a row widened to fp32 pairs.
 template <typename T> __device__ __forceinline__ void widen(const uint4& u, f2* p);
@@ -240,7 +250,7 @@ __device__ __forceinline__ bool keep_out(const AttnArgs& a, int row, int c) {
   return x >= a.out_thresh;
 }
 
-// Two edges of one query for one task lane (second one optional).
+// Two edges of one query for one task lane (second one optional: absent, it is zeros, since weight 0 times an infinity is NaN).
 template <typename T, int HN>
 __device__ __forceinline__ void fwd_pair(const AttnArgs& a, int head, int off, int e0, int e1, bool has1, unsigned hm,
                                          const float* qs0, const float* qs1, float* acc, float& zsum) {
@@ -252,9 +262,9 @@ __device__ __forceinline__ void fwd_pair(const AttnArgs& a, int head, int off, i
   const int j1 = has1 ? __ldg(a.col + e1) : j0;
   float k0[VN], v0[VN], k1[VN], v1[VN];
   load_vec<T>(kp + (long long)j0 * a.ldk + off, k0);
-  load_vec<T>(kp + (long long)j1 * a.ldk + off, k1);
+  load_vec_if<T>(has1, kp + (long long)j1 * a.ldk + off, k1);
   load_vec<T>(vp + (long long)j0 * a.ldv + off, v0);
-  load_vec<T>(vp + (long long)j1 * a.ldv + off, v1);
+  load_vec_if<T>(has1, vp + (long long)j1 * a.ldv + off, v1);
   int t0 = 0, t1 = 0;
   if (a.variant == 2) { t0 = a.etype[e0]; t1 = has1 ? a.etype[e1] : 0; }
   float d0 = 0.f, d1 = 0.f;
@@ -1196,7 +1206,7 @@ template <typename T, int HN> struct QueryTerms {
   }
 };
 
-// two edges of one query; an absent second one repeats the first with weight 0 (no branch between them: their sums overlap)
+// two edges of one query; an absent second one is zeros (no branch between them: their sums overlap)
 template <typename T, int HN>
 __device__ __forceinline__ void dq_pair(const BwdArgs& b, int e, int end, int head, int off, const QueryTerms<T, HN>& t, float* dq,
                                         unsigned hm) {
@@ -1206,8 +1216,8 @@ __device__ __forceinline__ void dq_pair(const BwdArgs& b, int e, int end, int he
   Raw<T> kr[2], vr[2];
   kr[0].load(static_cast<const T*>(a.k) + (long long)j0 * a.ldk + off);
   vr[0].load(static_cast<const T*>(a.v) + (long long)j0 * a.ldv + off);
-  kr[1].load(static_cast<const T*>(a.k) + (long long)j1 * a.ldk + off);
-  vr[1].load(static_cast<const T*>(a.v) + (long long)j1 * a.ldv + off);
+  kr[1].load_if(e + 1 < end, static_cast<const T*>(a.k) + (long long)j1 * a.ldk + off);
+  vr[1].load_if(e + 1 < end, static_cast<const T*>(a.v) + (long long)j1 * a.ldv + off);
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     float d = 0.f, dv = 0.f;
@@ -1338,8 +1348,8 @@ __global__ void __launch_bounds__(256, 4) edge_attn_bwd_kv_rows_kernel(BwdArgs b
     float2 zd[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      qr[u].load(qb + row[u] * sq);
-      gr[u].load(gb + row[u] * sg);
+      qr[u].load_if(e + u < it.z, qb + row[u] * sq);
+      gr[u].load_if(e + u < it.z, gb + row[u] * sg);
       const long long hz = (long long)row[u] * a.hl + head;
       zd[u] = PACKED ? make_float2(1.f, __ldg(reinterpret_cast<const float*>(b.zd) + hz)) : __ldg(b.zd + hz);
     }
@@ -1350,7 +1360,7 @@ __global__ void __launch_bounds__(256, 4) edge_attn_bwd_kv_rows_kernel(BwdArgs b
       for (int i = 0; i < VN; ++i) { d += qr[u].get(i) * kf.get(i); dotv += gr[u].get(i) * vf.get(i); }
       d = head_sum<LPH>(d, hm) * scale;
       dotv = head_sum<LPH>(dotv, hm);
-      const bool ok = u == 0 || e + 1 < it.z;   // an absent second edge repeats the first with weight 0
+      const bool ok = u == 0 || e + 1 < it.z;   // an absent second edge is zeros, with the first's row terms
       const bool inr = (d > -kClamp) && (d < kClamp) && ok;
       const float w = __expf(fminf(fmaxf(d, -kClamp), kClamp)) * zd[u].x;
       float mf = 1.f;

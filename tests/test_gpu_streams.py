@@ -16,6 +16,11 @@ def _graph(n, max_deg, seed, typed):
     return AttnGraph.from_edge_index(torch.stack(rows), n).to("cuda")
 
 
+def _graph_of(edges, n):
+    from budgetformer_b200.graph.attn_graph import AttnGraph
+    return AttnGraph.from_edge_index(edges, n).to("cuda")
+
+
 def _reference(q, k, v, dout, graph, tab, variant, p, seed):
     from budgetformer_b200.ops.edge_attention import edge_attention_reference
     t = [x.detach().double().requires_grad_() for x in (q, k, v)]
@@ -558,3 +563,29 @@ def test_type_table_at_any_address():
     for x, y in zip(one[:4], two[:4]):
         assert torch.equal(x, y)
     assert torch.allclose(one[4], two[4][:1], rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("heads,hn,dtype", [(9, 128, torch.bfloat16), (4, 64, torch.float32), (3, 8, torch.float16), (8, 16, torch.bfloat16)])
+@pytest.mark.parametrize("variant", ["plain", "gps"])
+def test_an_absent_edge_is_not_multiplied(heads, hn, dtype, variant):
+    """Rows and keys of odd length are padded to pairs by some of the kernels: an infinity in the last edge's value or output gradient
+    comes out as one, not as the NaN that weight 0 makes of it."""
+    from budgetformer_b200.ops.edge_attention import edge_attention
+    n, gen = 700, torch.Generator().manual_seed(hn)
+    deg = torch.arange(n) % 8
+    dst = torch.repeat_interleave(torch.arange(n), deg)
+    graph = _graph_of(torch.stack([torch.randint(0, n, (dst.numel(),), generator=gen), dst]), n)
+    gen = torch.Generator(device="cuda").manual_seed(heads)
+    q, k, v, dout = (torch.randn(n, heads, hn, generator=gen, device="cuda").to(dtype) for _ in range(4))
+    bad = torch.zeros(n, heads, hn, dtype=torch.bool, device="cuda")
+    bad.view(-1)[torch.randint(0, bad.numel(), (40,), generator=gen, device="cuda")] = True
+    neg = v.masked_fill(bad, float("-inf"))
+    out = edge_attention(q, k, neg, graph, variant=variant)
+    rows = torch.repeat_interleave(torch.arange(n, device="cuda"), graph.rowptr.diff().long())
+    hit = torch.zeros(n, heads, hn, dtype=torch.int32, device="cuda").index_add_(0, rows, bad[graph.col.long()].int()) > 0
+    assert hit.any() and torch.equal(out == float("-inf"), hit) and not out.isnan().any()
+    args = [x.detach().requires_grad_() for x in (q, k, v)]
+    grads = torch.autograd.grad(edge_attention(*args, graph, variant=variant), args, dout.masked_fill(bad, float("inf")))
+    hit = torch.zeros(n, heads, hn, dtype=torch.int32, device="cuda").index_add_(0, graph.col.long(), bad[rows].int()) > 0
+    assert hit.any() and torch.equal(grads[2] == float("inf"), hit) and not grads[2].isnan().any()
+
