@@ -338,7 +338,7 @@ int bf_bn_bwd_reduce(const void* dy, long long lddy, const void* x, long long ld
 // the sums' coefficients: out [5, cols] = mean, biased variance, 1 / std, a, b of y = x*a + b, with the running statistics (both or
 // neither) and their int64 count (or NULL) moved along; out [3, cols] = a, b, c0 of dx = dy*a + x*b + c0.  Rows: *count_dev, or count if NULL
 int bf_bn_finish(const float* s1, const float* s2, const float* count_dev, float count, const float* shift, const float* weight,
-                 const float* bias, float eps, int cols, float* out, float* run_mean, float* run_var, float momentum,
+                 const float* bias, float eps, int cols, float* out, float* run_mean, float* run_var, double momentum,
                  long long* tracked, cudaStream_t st);
 // out [2, cols] = a, b of y = x*a + b from running statistics
 int bf_bn_running(const float* mean, const float* var, const float* weight, const float* bias, float eps, float* out, int cols,

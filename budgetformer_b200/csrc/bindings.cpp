@@ -895,7 +895,7 @@ Tensor bn_finish(Tensor s1, Tensor s2, OptTensor count_dev, double count, OptTen
   check_cuda(bf_bn_finish(column_values(s1, s1, "s1"), column_values(s2, s1, "s2"), count_dev.has_value() ? count_dev->data_ptr<float>() : nullptr,
                           (float)count, column_values(shift, s1, "shift"), column_values(weight, s1, "weight"), column_values(bias, s1, "bias"),
                           (float)eps, (int)s1.numel(), out.data_ptr<float>(), column_values(run_mean, s1, "running mean"),
-                          column_values(run_var, s1, "running variance"), (float)momentum,
+                          column_values(run_var, s1, "running variance"), momentum,
                           tracked.has_value() ? (long long*)tracked->data_ptr<int64_t>() : nullptr, at::cuda::getCurrentCUDAStream()), "bn_finish");
   return out;
 }

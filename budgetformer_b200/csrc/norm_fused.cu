@@ -562,10 +562,11 @@ __global__ void __launch_bounds__(256) colstats_kernel(const T* __restrict__ x, 
 // From the column sums to the coefficients of col_affine, a thread a column.  Forward: `out` holds five rows of `cols` floats, mean,
 // variance (biased), 1 / std, a and b; the running statistics and their count move along when given (run_mean may be `shift`: a thread
 // reads its column before it writes it).  Backward: three rows, a, b and c0.  The number of rows is `count`, or *count_dev where the
-// sums come from several ranks.  Bound by the launch: 14 and 8 elementwise launches of 1.5 us each before, and one of 2 us now.
+// sums come from several ranks.  Products are rounded before they are subtracted: a fused multiply-add would leave the rounding error of a
+// mean's square as the variance of a single row or a constant column.  Bound by the launch: 14 and 8 elementwise launches of 1.5 us each before, and one of 2 us now.
 struct BnFinish {
   const float *s1, *s2, *count_dev, *shift, *weight, *bias;
-  float count, eps, momentum;
+  float count, eps, momentum, keep;             // keep: 1 - momentum
   float *run_mean, *run_var, *out;
   long long* tracked;
   int cols;
@@ -576,7 +577,7 @@ __global__ void __launch_bounds__(128) bn_finish_kernel(BnFinish f) {
   if (c >= f.cols) return;
   const float n = f.count_dev ? *f.count_dev : f.count;
   const float m1 = f.s1[c] / n;
-  float var = f.s2[c] / n - m1 * m1;
+  float var = __fsub_rn(f.s2[c] / n, __fmul_rn(m1, m1));
   if (var < 0.f) var = 0.f;                     // and NaN stays NaN
   const float mean = m1 + (f.shift ? f.shift[c] : 0.f);
   const float rstd = rsqrtf(var + f.eps);
@@ -585,11 +586,11 @@ __global__ void __launch_bounds__(128) bn_finish_kernel(BnFinish f) {
   f.out[f.cols + c] = var;
   f.out[2 * f.cols + c] = rstd;
   f.out[3 * f.cols + c] = a;
-  f.out[4 * f.cols + c] = (f.bias ? f.bias[c] : 0.f) - mean * a;
+  f.out[4 * f.cols + c] = __fsub_rn(f.bias ? f.bias[c] : 0.f, __fmul_rn(mean, a));
   if (f.run_mean) {
     const float unbias = n / fmaxf(n - 1.f, 1.f);
-    f.run_mean[c] = f.run_mean[c] * (1.f - f.momentum) + f.momentum * mean;
-    f.run_var[c] = f.run_var[c] * (1.f - f.momentum) + f.momentum * (var * unbias);
+    f.run_mean[c] = __fmaf_rn(f.momentum, mean, __fmul_rn(f.run_mean[c], f.keep));
+    f.run_var[c] = __fmaf_rn(f.momentum, __fmul_rn(var, unbias), __fmul_rn(f.run_var[c], f.keep));
   }
 }
 // Evaluation: a and b of y = x * a + b from the running statistics (out: two rows), for five launches of 1.5 us and 4 us of the host each
@@ -600,7 +601,7 @@ __global__ void __launch_bounds__(128) bn_running_kernel(const float* __restrict
   if (c >= cols) return;
   const float a = (weight ? weight[c] : 1.f) * rsqrtf(var[c] + eps);
   out[c] = a;
-  out[cols + c] = (bias ? bias[c] : 0.f) - mean[c] * a;
+  out[cols + c] = __fsub_rn(bias ? bias[c] : 0.f, __fmul_rn(mean[c], a));
 }
 // dx = g * rstd * (dy - mean(dy) - xhat * mean(dy * xhat)),  xhat = (x - mean) * rstd
 __global__ void __launch_bounds__(128) bn_bwd_finish_kernel(const float* __restrict__ sb, const float* __restrict__ sg,
@@ -612,7 +613,7 @@ __global__ void __launch_bounds__(128) bn_bwd_finish_kernel(const float* __restr
   const float n = count_dev ? *count_dev : count, r = rstd[c], a = (weight ? weight[c] : 1.f) * r, g = sg[c] / n;
   out[c] = a;
   out[cols + c] = -a * r * g;
-  out[2 * cols + c] = a * (mean[c] * r * g - sb[c] / n);
+  out[2 * cols + c] = a * __fsub_rn(__fmul_rn(mean[c] * r, g), sb[c] / n);
 }
 
 // TWO = false: y = x*a + b;  TWO = true: y = in2*a + x*b + c0
@@ -842,10 +843,11 @@ extern "C" int bf_bn_bwd_reduce(const void* dy, long long lddy, const void* x, l
 }
 
 extern "C" int bf_bn_finish(const float* s1, const float* s2, const float* count_dev, float count, const float* shift, const float* weight,
-                            const float* bias, float eps, int cols, float* out, float* run_mean, float* run_var, float momentum,
+                            const float* bias, float eps, int cols, float* out, float* run_mean, float* run_var, double momentum,
                             long long* tracked, cudaStream_t st) {
   if (cols < 0 || (run_mean == nullptr) != (run_var == nullptr)) return (int)cudaErrorInvalidValue;
-  const BnFinish f{s1, s2, count_dev, shift, weight, bias, count, eps, momentum, run_mean, run_var, out, tracked, cols};
+  const BnFinish f{s1, s2, count_dev, shift, weight, bias, count, eps, (float)momentum, (float)(1.0 - momentum), run_mean, run_var, out,
+                   tracked, cols};
   bn_finish_kernel<<<cols / 128 + 1, 128, 0, st>>>(f);
   return (int)cudaGetLastError();
 }

@@ -437,7 +437,7 @@ def test_ffn_rows_that_overlap(h, act):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_gelu_carries_values_that_are_not_finite(dtype):
-    """A NaN or an infinity in the bias reaches the activation as in PyTorch's GELU (NaN stays NaN, inf stays inf), in the product's
+    """A NaN or an infinity in the bias reaches the activation as in PyTorch's GELU (NaN stays NaN, inf stays inf, -inf gives NaN), in the product's
     epilogue with and without its pre-activation and in the one-kernel block, and the block's output."""
     from budgetformer_b200.ops.ffn import ffn_onchip
     torch.manual_seed(3)
@@ -445,7 +445,7 @@ def test_gelu_carries_values_that_are_not_finite(dtype):
     x = torch.randn(m, h, device="cuda").to(dtype)
     l1, l2 = torch.nn.Linear(h, 2 * h).cuda(), torch.nn.Linear(2 * h, h).cuda()
     with torch.no_grad():
-        for col, bad in ((5, float("nan")), (70, float("inf")), (100, -1e4), (33, 1e4)):
+        for col, bad in ((5, float("nan")), (70, float("inf")), (90, float("-inf")), (100, -1e4), (33, 1e4)):
             l1.bias[col] = bad
     b1, w1 = l1.bias.detach(), l1.weight.detach().to(dtype)
     want = torch.nn.functional.gelu(x.double() @ w1.double().t() + b1.double()).to(dtype)
@@ -455,8 +455,8 @@ def test_gelu_carries_values_that_are_not_finite(dtype):
     plain = ffn_onchip(x, l1.weight, l1.bias, l2.weight, l2.bias, act="gelu", residual=True)
     assert z[:, 5].isnan().all() and z[:, 70].isinf().all()
     for t in got + [hid]:
-        assert t[:, 5].isnan().all() and (t[:, 70] == float("inf")).all() and (t[:, 100] == 0).all()
-        rest = [c for c in range(2 * h) if c not in (5, 70)]
+        assert t[:, [5, 90]].isnan().all() and (t[:, 70] == float("inf")).all() and (t[:, 100] == 0).all()
+        rest = [c for c in range(2 * h) if c not in (5, 70, 90)]
         # one rounding (8 or 11 bits) of a value within its fp32 sums, a second where the pre-activation is rounded first
         assert torch.allclose(t[:, rest].float(), want[:, rest].float(), rtol=2.0 ** -7, atol=2.0 ** -7)
     assert y.isnan().all() and plain.isnan().all()

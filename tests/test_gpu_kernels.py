@@ -395,6 +395,38 @@ def test_batch_norm_coefficients_by_one_launch(h, affine, momentum, track, stats
     assert ya.dtype == x.dtype and (ya - yb).abs().max() <= 3e-5 * yb.abs().max()       # the running statistics' 1e-5 as well
 
 
+@pytest.mark.parametrize("rows,momentum", [(1, 0.1), (2, 0.3), (3001, 0.1)])
+def test_batch_norm_coefficients_equal_the_operators(rows, momentum):
+    """The coefficient kernels give what PyTorch's operators give, bit for bit: a single row and a constant column have no variance,
+    however large their mean."""
+    from budgetformer_b200.ops import _ext
+    ext, h = _ext.load(), 64
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, h, generator=g, device="cuda") * 10 ** torch.linspace(-3, 4.5, h, device="cuda")
+    x[:, 5] = 29952.0
+    x[:, 6] = 12345.67
+    shift, w, b = (torch.randn(h, generator=g, device="cuda") for _ in range(3))
+    n, eps = torch.full((1,), float(rows), device="cuda"), 1e-5      # on the device: a division by a host number is a multiplication
+    s1, s2 = (x - shift).sum(0), ((x - shift) ** 2).sum(0)
+    run_mean, run_var = shift.clone(), torch.rand(h, generator=g, device="cuda")
+    m1 = s1 / n
+    var = (s2 / n - m1 * m1).clamp_min(0.0)
+    mean = m1 + shift
+    rstd = torch.rsqrt(var + eps)
+    a = w * rstd
+    want = [mean, var, rstd, a, b - mean * a, run_mean.mul(1 - momentum).add(mean, alpha=momentum),
+            run_var.mul(1 - momentum).add(var * (n / (n - 1.0).clamp(min=1.0)), alpha=momentum)]
+    got = list(ext.bn_finish(s1, s2, None, float(rows), shift, w, b, eps, run_mean, run_var, momentum, None).unbind(0)) + [run_mean, run_var]
+    for i, (p, q) in enumerate(zip(got, want)):
+        assert torch.equal(p, q), i
+    if rows == 1:
+        assert not got[1].any()
+    sb, sg = (torch.randn(h, generator=g, device="cuda") * rows for _ in range(2))
+    want = [a, -a * rstd * (sg / n), a * (-(sb / n) + mean * rstd * (sg / n))]
+    for p, q in zip(ext.bn_bwd_finish(sb, sg, None, float(rows), mean, rstd, w).unbind(0), want):
+        assert torch.equal(p, q)
+
+
 def test_batch_norm_coefficients_with_the_count_on_the_device():
     """What a statistics group gives: sums and a number of rows that only the device knows."""
     from budgetformer_b200.ops import _ext
