@@ -51,7 +51,9 @@ __device__ __forceinline__ void set_bit(uint32_t& bits, bool pred, uint32_t bit,
 // GELU x * Phi(x) with the exact normal distribution function, by its lower tail: Phi(-m) = 2^-T(m), m = |x|.  T is smooth (close to
 // quadratic) and was fitted by a polynomial of degree 10 on [0, 8], least squares reweighted towards the largest error (Lawson's
 // method); it goes on rising up to the clamp at 30, where the tail is 0 in fp32.  Largest error of GELU over [-12, 12] 2.4e-7 (0.5 x (1 + erff)
-// 4.5e-7), relative 1.7e-5 down to x = -8 (1, since 1 + erff cancels), of its derivative 2.7e-7.  Half the instructions of erff.
+// 4.5e-7), relative 1.7e-5 down to x = -8 (1, since 1 + erff cancels).  Half the instructions of erff.  Of its derivative 2.7e-7 (with an erff
+// of no error 1.0e-7; relative from -8 to -1 2e-6 and 3e-2): of gradients rounded to bf16 one in 8,000 falls the other way than with
+// erff, and their error against 64 bits is the same to six digits (1.66e-3).
 __device__ __forceinline__ float ex2_approx(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
